@@ -710,6 +710,33 @@ def test_sampler_with_drawn_settings(V, rows):
         assert tok in ok, (r, o, k, tok, ok)
 
 
+@pytest.mark.parametrize("V", [1, 5, 1023, 5003, 151936])
+def test_sampler_lists_of_every_length(V):
+    """Top-k up to 1,024 goes by a list of the row's largest elements: k at both ends of that range and just beyond
+    it, at the row's length, with ties across the cut, with a bin too full for the list, with every later filter."""
+    g = gen(60 + V % 7)
+    rows, opts, ks = [], [], []
+    for k in (2, 3, 50, 1023, 1024, 1025, V):
+        for kind in range(4):
+            x = torch.randn(V, generator=g) * 2.5
+            if kind == 1:
+                x = (x * 2).round() / 2                          # many ties
+            if kind == 2:
+                x = x * 1e-4 - 40                                # all within a bin or two
+            if kind == 3 and V > 1:
+                x[torch.rand(V, generator=g) < 0.6] = float("-inf")
+            rows.append(x)
+            opts.append([(0.7, 1.0, 1.6)[(k + kind) % 3], (1.0, 0.9, 0.5, 1.0)[kind], (0.0, 0.0, 0.1, 0.4)[(kind + k) % 4],
+                         (0.03, 0.5, 0.97)[(k + kind) % 3]])
+            ks.append(k)
+    lg = torch.stack(rows)
+    got = _sample_rows(lg, opts, ks)
+    for r, (tok, o, k) in enumerate(zip(got, opts, ks)):
+        assert tok in _acceptable(lg[r], o[0], k, o[1], o[2], o[3]), (r, o, k, tok)
+    for n in (1, 20, 27):                                        # 8, 4 and 4 blocks a row: same tokens
+        assert _sample_rows(lg[:n], opts[:n], ks[:n]) == got[:n]
+
+
 def test_products_of_drawn_shapes_through_the_router():
     """Shapes drawn from a fixed seed across every regime of the product's routing
     (weight-streaming tcgen05 orientation with k split, single-SM tiles with
