@@ -482,6 +482,24 @@ def test_gemm_f32_is_true_float32(wdtype, M, N, K_):
     assert torch.equal(one[0], out[M // 2])
 
 
+@pytest.mark.parametrize("wdtype", [F32, BF16])
+@pytest.mark.parametrize("M,N,K_", [(1, 33, 4), (16, 31, 60), (17, 32, 64), (32, 65, 68), (33, 63, 132), (65, 200, 2052),
+                                    (129, 64, 1021), (9, 40, 37)])
+def test_gemm_f32_tiles(wdtype, M, N, K_):
+    """Edges of the three tile sizes and of the 64-wide steps of k, and rows that are no multiple of 16 bytes. A
+    sum of K products rounded K times is off by at most 2 K 2^-24 of the sum of the products' sizes."""
+    from lumenllm_b200.ops import kernels as K
+    g = gen(9)
+    a = torch.randn(M, K_, generator=g)
+    w = torch.randn(N, K_, generator=g).to(wdtype)
+    out = K.gemm_f32(dev(a), dev(w)).cpu().double()
+    ref = a.double() @ w.double().T
+    assert bool(((out - ref).abs() <= 2 * K_ * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T)).all())
+    assert float((out - ref).norm() / ref.norm()) < 2e-6 * math.sqrt(K_)
+    one = K.gemm_f32(dev(a[M // 2:M // 2 + 1].contiguous()), dev(w)).cpu().double()
+    assert torch.equal(one[0], out[M // 2])
+
+
 @pytest.mark.parametrize("M,N,K_", [(128, 256, 64), (200, 300, 320), (2048, 1024, 4096), (1, 256, 64),
                                     (8, 4096, 4096), (19, 311, 80), (33, 1000, 1000), (64, 6144, 1024),
                                     (65, 130, 72), (130, 17, 1000), (16, 151936 // 4 + 8, 256)])
