@@ -11,7 +11,14 @@
 //   r = sum_i g_i S_ij k_i,  w = sum_i g_i S_ij q_i,  u_j = beta (v_j - r),  o_j = w + u_j (k . q),
 //   S_ij <- g_i S_ij + k_i u_j,
 // so the DR_ROWS rows a thread keeps in registers are read once a token; the NS threads of a
-// column (adjacent lanes) add r and w by shuffles. What does not depend on the state is made for
+// column (adjacent lanes) add r by shuffles at once, since u_j waits for it, and w a chunk at a time: the
+// shares of eight tokens change lanes so that a lane adds up a token of its own (7 shuffles for 8 tokens
+// where one token after the other takes 8 log2(NS)).Four
+// warps of a block share a staged row, and what they read of it (48 values a thread and token) is what bounds a
+// token: 220 of its 430 cycles go to shared-memory reads, the rest to the chain of dependent steps. 2,048
+// tokens of 16 heads of 128 x 128: 466 us with the kernel that prepares them (732 with 16 threads a column, 8 rows
+// each, and w summed token by token), four sequences of 2,048 tokens in all: 400 (668), one token of 64 sequences: 36 (44).
+// What does not depend on the state is made for
 // all tokens at once by a kernel of its own (a warp a (token, head): normed q and k, the decays,
 // k . q and beta, one row [q | k | g | k.q, beta] of a scratch matrix), so that the walk itself is
 // nothing but the recurrence: rows are staged DR_CHUNK tokens at a time by asynchronous copies, the
@@ -19,8 +26,8 @@
 // state is stored [H, dv, d] (a column's rows lie together).
 #include "common.cuh"
 
-#define DR_THREADS 256
-#define DR_ROWS 8           // rows of S a thread keeps (2 groups of 4 consecutive rows), 16 for heads wider than 256
+#define DR_THREADS 128
+#define DR_ROWS 16          // rows of S a thread keeps (4 groups of 4 consecutive rows)
 #define DR_CHUNK 8
 #define DR_PREP_WARPS 4
 
@@ -28,6 +35,33 @@ __device__ __forceinline__ float dr_parts(const float* p, int S, size_t stride) 
     float x = p[0];
     for (int s = 1; s < S; ++s) x += p[(size_t)s * stride];
     return x;
+}
+// Two float32 operations in one instruction, each rounded as by itself.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpair2(f32x2 a) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(a));
+    return v;
 }
 __device__ __forceinline__ float dr_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ void dr_cp4(float* dst, const float* src) {
@@ -89,17 +123,18 @@ delta_prepare_kernel(const float* __restrict__ x, int C, int q_col, int k_col,
     }
 }
 
-// NS: threads that share a column of S (a power of two), ROWS: rows of it a thread keeps, NS ROWS >= d;
-// every offset of the walk is a constant of the instance. Eight rows a thread (16 threads a column at
-// 128 key channels) halves a token's chain of sums and doubles the blocks of a head.
-template <int NS, int ROWS>
+// NS: threads that share a column of S (a power of two), NS DR_ROWS >= d; every offset of the walk is a constant
+// of the instance. AHEAD: a token's rows are read from shared memory while the one before is worked on, which
+// takes twice the registers: for steps of several tokens a sequence. Same sums either way.
+template <int NS, bool AHEAD>
 __global__ void __launch_bounds__(DR_THREADS)
 delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __restrict__ prep,
                   float* __restrict__ state, size_t slot_stride, const int* __restrict__ cu_q,
-                  const int* __restrict__ seq_slot, float* __restrict__ y, int H, int d, int dv) {
+                  const int* __restrict__ seq_slot, float* __restrict__ y, int H, int d, int dv, int vec) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
+    constexpr int ROWS = DR_ROWS;
     constexpr int dp = NS * ROWS;                   // d padded to what the threads of a column hold
     constexpr int GR = ROWS / 4;
     constexpr int PW = 3 * dp + 4;
@@ -112,14 +147,23 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
     const int s = tid % NS, cj = tid / NS, j = blockIdx.z * cols + cj;
     const bool live = j < dv;
     float* Sj = state + (size_t)seq_slot[b] * slot_stride + ((size_t)h * dv + (live ? j : 0)) * d;
-    float S[ROWS];
+    f32x2 S[2 * GR];                                // rows 4 (i NS + s) .. + 3 in S[2 i], S[2 i + 1]
 #pragma unroll
-    for (int i = 0; i < GR; ++i)
+    for (int i = 0; i < GR; ++i) {
+        const int row0 = (i * NS + s) * 4;
+        if (vec) {                                  // d a multiple of 4 and the state's columns on 16 bytes
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (live && row0 < d) v = *reinterpret_cast<const float4*>(Sj + row0);
+            S[2 * i] = pair2(v.x, v.y);
+            S[2 * i + 1] = pair2(v.z, v.w);
+        } else {
+            float v[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int row = (i * NS + s) * 4 + c;
-            S[i * 4 + c] = (live && row < d) ? Sj[row] : 0.0f;
+            for (int c = 0; c < 4; ++c) v[c] = (live && row0 + c < d) ? Sj[row0 + c] : 0.0f;
+            S[2 * i] = pair2(v[0], v[1]);
+            S[2 * i + 1] = pair2(v[2], v[3]);
         }
+    }
 
     auto issue = [&](int t0, int buf) {
         const int nt = min(DR_CHUNK, t_end - t0);
@@ -150,70 +194,126 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
         __syncthreads();
         const float* rb = rows + buf * DR_CHUNK * PW;
         const float* vb = vs + buf * DR_CHUNK * cols;
-#pragma unroll 2
-        for (int t = 0; t < nt; ++t) {
-            const float* qn = rb + t * PW;
-            const float* kn = qn + dp;
-            const float* gd = kn + dp;
-            const float vj = vb[t * cols + cj];
-            float rp[GR], wp[GR];                   // a sum a group of four rows: short chains, not one long one
-            float4 k4[GR];
+        float wt[DR_CHUNK];                         // this lane's share of w (lane 0 of a column: and of u_j k.q)
+        struct Row { ulonglong2 q[GR], k[GR], g[GR]; float v, kq, beta; };
+        auto load = [&](int t) {
+            Row x;
+            const float* p = rb + t * PW + 4 * s;
 #pragma unroll
             for (int i = 0; i < GR; ++i) {
-                const int off = (i * NS + s) * 4;
-                const float4 g4 = *reinterpret_cast<const float4*>(gd + off);
-                const float4 q4 = *reinterpret_cast<const float4*>(qn + off);
-                k4[i] = *reinterpret_cast<const float4*>(kn + off);
-                S[i * 4 + 0] *= g4.x; S[i * 4 + 1] *= g4.y; S[i * 4 + 2] *= g4.z; S[i * 4 + 3] *= g4.w;
-                rp[i] = S[i * 4 + 0] * k4[i].x; rp[i] = fmaf(S[i * 4 + 1], k4[i].y, rp[i]);
-                rp[i] = fmaf(S[i * 4 + 2], k4[i].z, rp[i]); rp[i] = fmaf(S[i * 4 + 3], k4[i].w, rp[i]);
-                wp[i] = S[i * 4 + 0] * q4.x; wp[i] = fmaf(S[i * 4 + 1], q4.y, wp[i]);
-                wp[i] = fmaf(S[i * 4 + 2], q4.z, wp[i]); wp[i] = fmaf(S[i * 4 + 3], q4.w, wp[i]);
+                x.g[i] = *reinterpret_cast<const ulonglong2*>(p + 2 * dp + 4 * i * NS);
+                x.k[i] = *reinterpret_cast<const ulonglong2*>(p + dp + 4 * i * NS);
+                x.q[i] = *reinterpret_cast<const ulonglong2*>(p + 4 * i * NS);
             }
-            float r = rp[0] + rp[1], w = wp[0] + wp[1];
-            if (GR == 4) {
-                r += rp[GR - 2] + rp[GR - 1];
-                w += wp[GR - 2] + wp[GR - 1];
-            }
-#pragma unroll
-            for (int o = NS >> 1; o > 0; o >>= 1) {
-                r += __shfl_xor_sync(0xffffffffu, r, o);
-                w += __shfl_xor_sync(0xffffffffu, w, o);
-            }
-            const float uj = gd[dp + 1] * (vj - r);
+            const float2 e = *reinterpret_cast<const float2*>(rb + t * PW + 3 * dp);
+            x.kq = e.x;
+            x.beta = e.y;
+            x.v = vb[t * cols + cj];
+            return x;
+        };
+        // The chain from one token's S to the next one's is: S g, the sums of r over four short chains, their
+        // lanes, u_j, S. All else (w, the next token's rows) is put where it waits for shuffles.
+        auto walk = [&](const Row& x, Row& next, int t_next) {
+            f32x2 rp[GR], wp[2];
 #pragma unroll
             for (int i = 0; i < GR; ++i) {
-                S[i * 4 + 0] = fmaf(k4[i].x, uj, S[i * 4 + 0]); S[i * 4 + 1] = fmaf(k4[i].y, uj, S[i * 4 + 1]);
-                S[i * 4 + 2] = fmaf(k4[i].z, uj, S[i * 4 + 2]); S[i * 4 + 3] = fmaf(k4[i].w, uj, S[i * 4 + 3]);
+                S[2 * i] = mul2(S[2 * i], x.g[i].x);
+                S[2 * i + 1] = mul2(S[2 * i + 1], x.g[i].y);
             }
-            if (live && s == 0) y[(size_t)(t0 + t) * H * dv + h * dv + j] = fmaf(uj, gd[dp], w);
+#pragma unroll
+            for (int i = 0; i < GR; ++i) rp[i] = fma2(S[2 * i + 1], x.k[i].y, mul2(S[2 * i], x.k[i].x));
+            const float2 r2 = unpair2(add2(add2(rp[0], rp[1]), add2(rp[2], rp[3])));
+            float r = r2.x + r2.y;
+            if (AHEAD && t_next >= 0) next = load(t_next);
+#pragma unroll
+            for (int o = NS >> 1; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+#pragma unroll
+            for (int i = 0; i < GR; ++i) {
+                wp[i & 1] = i < 2 ? mul2(S[2 * i], x.q[i].x) : fma2(S[2 * i], x.q[i].x, wp[i & 1]);
+                wp[i & 1] = fma2(S[2 * i + 1], x.q[i].y, wp[i & 1]);
+            }
+            const float2 w2 = unpair2(add2(wp[0], wp[1]));
+            const float w = w2.x + w2.y;
+            const float uj = x.beta * (x.v - r);
+            const f32x2 u2 = pair2(uj, uj);
+#pragma unroll
+            for (int i = 0; i < GR; ++i) {
+                S[2 * i] = fma2(x.k[i].x, u2, S[2 * i]);
+                S[2 * i + 1] = fma2(x.k[i].y, u2, S[2 * i + 1]);
+            }
+            if (!AHEAD && t_next >= 0) next = load(t_next);
+            return s == 0 ? fmaf(uj, x.kq, w) : w;
+        };
+        Row now = load(0), next = now;
+        if (AHEAD && nt == DR_CHUNK) {                       // no branch between the tokens
+#pragma unroll
+            for (int t = 0; t < DR_CHUNK; ++t) {
+                wt[t] = walk(now, next, t + 1 < DR_CHUNK ? t + 1 : -1);
+                now = next;
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < DR_CHUNK; ++t) {
+                wt[t] = 0.0f;
+                if (t >= nt) continue;
+                wt[t] = walk(now, next, t + 1 < nt ? t + 1 : -1);
+                now = next;
+            }
+        }
+        // Halve the tokens a lane has with every step over the column's lanes; what is left of the steps adds
+        // up the one token it has. The tree of lanes is the same for every place in the chunk.
+        int n = DR_CHUNK, first = 0;
+#pragma unroll
+        for (int o = NS >> 1; o > 0; o >>= 1) {
+            if (n > 1) {
+                n >>= 1;
+                const bool up = (s & o) != 0;
+#pragma unroll
+                for (int i = 0; i < DR_CHUNK / 2; ++i) {
+                    if (i >= n) break;
+                    const float give = up ? wt[i] : wt[i + n], keep = up ? wt[i + n] : wt[i];
+                    wt[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+                first += up ? n : 0;
+            } else {
+                wt[0] += __shfl_xor_sync(0xffffffffu, wt[0], o);
+            }
+        }
+        constexpr int OWN = NS >= DR_CHUNK ? 1 : DR_CHUNK / NS, TWINS = NS > DR_CHUNK ? NS / DR_CHUNK : 1;
+        if (live && (s & (TWINS - 1)) == 0) {
+#pragma unroll
+            for (int i = 0; i < OWN; ++i)
+                if (first + i < nt) y[(size_t)(t0 + first + i) * H * dv + h * dv + j] = wt[i];
         }
         __syncthreads();                            // this chunk has been read by everyone before its buffer is filled again
     }
     if (live) {
 #pragma unroll
-        for (int i = 0; i < GR; ++i)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int row = (i * NS + s) * 4 + c;
-                if (row < d) Sj[row] = S[i * 4 + c];
+        for (int i = 0; i < GR; ++i) {
+            const int row0 = (i * NS + s) * 4;
+            const float2 a = unpair2(S[2 * i]), c = unpair2(S[2 * i + 1]);
+            if (vec) {
+                if (row0 < d) *reinterpret_cast<float4*>(Sj + row0) = make_float4(a.x, a.y, c.x, c.y);
+            } else {
+                if (row0 < d) Sj[row0] = a.x;
+                if (row0 + 1 < d) Sj[row0 + 1] = a.y;
+                if (row0 + 2 < d) Sj[row0 + 2] = c.x;
+                if (row0 + 3 < d) Sj[row0 + 3] = c.y;
             }
+        }
     }
 }
 
-// Threads a column and rows a thread for d key channels: 8 rows up to d = 256, 16 beyond.
-static inline void delta_rule_shape(int d, int* ns, int* rows) {
-    *rows = d <= 32 * DR_ROWS ? DR_ROWS : 2 * DR_ROWS;
+// Threads a column for d key channels.
+static inline int delta_rule_threads(int d) {
     int NS = 1;
-    while (NS * *rows < d) NS <<= 1;
-    *ns = NS;
+    while (NS * DR_ROWS < d) NS <<= 1;
+    return NS;
 }
 
 // Floats of scratch lumen_delta_rule needs for every (token, head) with d key channels.
 LUMEN_API int lumen_delta_rule_scratch_row(int d) {
-    int NS, rows;
-    delta_rule_shape(d, &NS, &rows);
-    return 3 * NS * rows + 4;
+    return 3 * delta_rule_threads(d) * DR_ROWS + 4;
 }
 
 // x float32 [N, C]: the convolved and activated q (G heads of d, from column q_col), k (k_col)
@@ -227,14 +327,13 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
                                const int* cu_q, const int* seq_slot, int n_seqs, float* y, float* prep, int N, int H,
                                int G, int d, int dv, cudaStream_t stream) {
     if (n_seqs <= 0 || N <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || d > 64 * DR_ROWS || uS < 1 || aS < 1 || H > 65535)
+    if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || d > 32 * DR_ROWS || uS < 1 || aS < 1 || H > 65535)
         return LUMEN_ERR_UNSUPPORTED;
     if (q_col < 0 || k_col < 0 || v_col < 0 || q_col + G * d > C || k_col + G * d > C || v_col + H * dv > C ||
         b_col < 0 || b_col + H > uW || !prep)
         return LUMEN_ERR_BAD_ARGUMENT;
-    int NS, rows;
-    delta_rule_shape(d, &NS, &rows);
-    const int cols = DR_THREADS / NS, dp = NS * rows;
+    const int NS = delta_rule_threads(d), cols = DR_THREADS / NS, dp = NS * DR_ROWS;
+    const int vec = (d & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
     dim3 pgrid(N, (H + DR_PREP_WARPS - 1) / DR_PREP_WARPS);
     if (pgrid.y > 65535) return LUMEN_ERR_UNSUPPORTED;
     lumen_launch(delta_prepare_kernel, pgrid, dim3(32 * DR_PREP_WARPS), 0, stream, x, C, q_col, k_col, u, uS,
@@ -243,25 +342,27 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
     dim3 grid(n_seqs, H, (dv + cols - 1) / cols);
     if (grid.z > 65535) return LUMEN_ERR_UNSUPPORTED;
     const size_t smem = (size_t)2 * DR_CHUNK * (3 * dp + 4 + cols) * sizeof(float);
-#define DR_LAUNCH(S, R)                                                                                               \
+#define DR_LAUNCH(S, A)                                                                                               \
     do {                                                                                                              \
-        auto k = delta_rule_kernel<S, R>;                                                                              \
+        auto k = delta_rule_kernel<S, A>;                                                                              \
         if (smem > 48 * 1024) {                                                                                       \
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
             if (e != cudaSuccess) return (int)e;                                                                      \
         }                                                                                                             \
         lumen_launch(k, grid, dim3(DR_THREADS), smem, stream, x, C, v_col, (const float*)prep, state,                 \
-                     (size_t)slot_stride, cu_q, seq_slot, y, H, d, dv);                                               \
+                     (size_t)slot_stride, cu_q, seq_slot, y, H, d, dv, vec);                                          \
     } while (0)
-    if (rows != DR_ROWS) DR_LAUNCH(32, 2 * DR_ROWS);
-    else switch (NS) {
-        case 1: DR_LAUNCH(1, DR_ROWS); break;
-        case 2: DR_LAUNCH(2, DR_ROWS); break;
-        case 4: DR_LAUNCH(4, DR_ROWS); break;
-        case 8: DR_LAUNCH(8, DR_ROWS); break;
-        case 16: DR_LAUNCH(16, DR_ROWS); break;
-        default: DR_LAUNCH(32, DR_ROWS); break;
+    const bool ahead = N > n_seqs;
+#define DR_GO(S) case S: if (ahead) DR_LAUNCH(S, true); else DR_LAUNCH(S, false); break
+    switch (NS) {
+        DR_GO(1);
+        DR_GO(2);
+        DR_GO(4);
+        DR_GO(8);
+        DR_GO(16);
+        DR_GO(32);
     }
+#undef DR_GO
 #undef DR_LAUNCH
     LUMEN_LAUNCH_CHECK();
     return 0;

@@ -376,6 +376,20 @@ def test_delta_rule_part_in_any_portions(m, dtype):
         close(got, ref, dtype)
 
 
+@pytest.mark.parametrize("d,dv", [(4, 5), (12, 130), (31, 16), (64, 33), (120, 17), (136, 9), (256, 40), (500, 3)])
+def test_delta_rule_head_sizes(d, dv):
+    """One to 32 threads a column, rows of the state that are and are not whole 16-byte pieces, value columns that end
+    inside a block; portions that end inside and at a run of eight tokens, and one token at a time."""
+    m = delta(2, 1, d, dv, 2, 3, 2)
+    mixer, w = mixer_part(m, 24, F32, seed=21)
+    g = torch.Generator().manual_seed(22)
+    ys = [torch.randn(n, 24, generator=g) for n in (41, 17)]
+    refs = [P.channel_delta(y, w, "l0.mix.", m, 1e-6) for y in ys]
+    pieces = [cut(ys[0], [8, 1, 1, 16, 15]), cut(ys[1], [3, 1, 0, 12, 1])]
+    for got, ref in zip(run_mixer(mixer, runtime(F32), pieces, twice=True), refs):
+        close(got, ref, F32)
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_the_state_remembers_far_back_and_forgets_by_channel(dtype):
     """Decays close to one and one loud early token: what the state holds of that token decides the
