@@ -17,13 +17,15 @@
 // held 75 cycles by each 128 x 64 x 16 product of S (32 cycles of arithmetic; 6 KB of operands
 // from shared memory) and 92 by each 128 x 128 x 16 product of O (64 of arithmetic), with one
 // block on the SM as with two, so a page costs 970 cycles of the pipe and two blocks an SM fill
-// it (1,860 cycles a page and block). The softmax of a page takes a warp 875 cycles alone and
-// about 1,000 beside its neighbour's, so it is not far behind: without any exponentials the
-// kernel is 7 % faster, with half of the S products 7 %, with half of the O products 6 %.
+// it (1,860 cycles a page and block). The softmax is not far behind: with its plain instructions it took a warp
+// 875 cycles a page alone and about 1,000 beside its neighbour's.
 // What was gained here: P in tensor memory instead of a 16 KB buffer in shared memory (no
 // write and read of P through shared memory, and no wait for the product of the page before
-// unless O is rescaled) 5 % at 8,192 tokens and 4 % at 2,048; one exponential in four on the
-// FMA pipe 10 % at 2,048. Making the operand descriptors once instead of per product changed
+// unless O is rescaled) 5 % at 8,192 tokens and 4 % at 2,048. The softmax's scale, sums and maxima are
+// instructions of two and three operands' worth (f32x2, max of three): the plain float32 ones run at half the pipe's
+// rate here, and with them a part of the exponentials had paid on the FMA pipe, which it no longer does
+// (us at 2,048 / 8,192 tokens and 5,435 after 24,576, 32 heads of 128: 55.7 / 537 / 2,312 before; 50.4 / 496 / 2,197
+// now; 51.2 / 509 / 2,386 with one exponential in four on the FMA pipe, 53.4 / 538 / 2,623 with two). Making the operand descriptors once instead of per product changed
 // nothing. Products with more columns were tried as a kernel of its own: one block an SM
 // with two Q tiles that share their K and V tiles, keys 128 at a time, S and O of both tiles
 // in all 512 columns of tensor memory, the tiles taken in turn by the tensor pipe. Right
@@ -74,7 +76,6 @@
 #define PT_ROWS 128
 #define PT_STAGES 2
 #define PT_RESCALE 8.0f
-#define PT_FMA_EX2_OF_4 1         // of every four exponentials, this many go to the FMA pipe
 
 __device__ __forceinline__ void pt_mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -157,19 +158,31 @@ __device__ __forceinline__ float pt_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 2^x without the special-function unit: x = n + f with n the nearest integer (the magic-number
-// add leaves n in the low mantissa bits), 2^f on [-0.5, 0.5] by a cubic (relative error 1e-4,
-// a twentieth of the rounding to bfloat16 that follows), and n added into the exponent bits.
-// The softmax does a part of its exponentials this way: the special-function unit makes 16 a
-// cycle and SM, and at head size 128 that is as long a job as the page's two products.
-__device__ __forceinline__ float pt_ex2_fma(float x) {
-    x = fmaxf(x, -125.0f);                       // also what a masked (-inf) score becomes: 2^-125, nothing
-    const float t = x + 12582912.0f;             // 1.5 * 2^23
-    const float f = x - (t - 12582912.0f);
-    float p = fmaf(0.05583828315138817f, f, 0.2426394820213318f);
-    p = fmaf(p, f, 0.6931367516517639f);
-    p = fmaf(p, f, 0.9999245405197144f);
-    return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
+// Two float32 operations in one instruction, each rounded as by itself (the plain instructions run at half the
+// pipe's rate on this chip).
+typedef unsigned long long pt_f2;
+__device__ __forceinline__ pt_f2 pt_pair(float lo, float hi) {
+    pt_f2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void pt_unpair(pt_f2 a, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+}
+__device__ __forceinline__ pt_f2 pt_fma2(pt_f2 a, pt_f2 b, pt_f2 c) {
+    pt_f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ pt_f2 pt_add2(pt_f2 a, pt_f2 b) {
+    pt_f2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ float pt_max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
 }
 __device__ __forceinline__ void pt_st32(uint32_t taddr, const float (&v)[32]) {
     asm volatile(
@@ -450,11 +463,11 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
             // row maximum of the raw scores, four independent chains (the scale is positive)
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int j = 0; j < 64; j += 4) {
-                mx4[0] = fmaxf(mx4[0], s[j]);
-                mx4[1] = fmaxf(mx4[1], s[j + 1]);
-                mx4[2] = fmaxf(mx4[2], s[j + 2]);
-                mx4[3] = fmaxf(mx4[3], s[j + 3]);
+            for (int j = 0; j < 64; j += 8) {
+                mx4[0] = pt_max3(mx4[0], s[j], s[j + 1]);
+                mx4[1] = pt_max3(mx4[1], s[j + 2], s[j + 3]);
+                mx4[2] = pt_max3(mx4[2], s[j + 4], s[j + 5]);
+                mx4[3] = pt_max3(mx4[3], s[j + 6], s[j + 7]);
             }
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
             // reference for the exponentials: moved only when the maximum has grown a lot
@@ -467,21 +480,23 @@ attn_prefill_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
                 }
             }
             const float nbase = (m_ref == -INFINITY) ? 0.0f : -m_ref;
-            float rs4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            pt_f2 rs[4] = {0ull, 0ull, 0ull, 0ull};
+            const pt_f2 scale2 = pt_pair(scale_log2, scale_log2), nbase2 = pt_pair(nbase, nbase);
 #pragma unroll
-            for (int j = 0; j < 64; j += 4) {
-                s[j] = pt_ex2(fmaf(s[j], scale_log2, nbase));
-                s[j + 1] = (PT_FMA_EX2_OF_4 >= 2) ? pt_ex2_fma(fmaf(s[j + 1], scale_log2, nbase))
-                                                  : pt_ex2(fmaf(s[j + 1], scale_log2, nbase));
-                s[j + 2] = pt_ex2(fmaf(s[j + 2], scale_log2, nbase));
-                s[j + 3] = (PT_FMA_EX2_OF_4 >= 1) ? pt_ex2_fma(fmaf(s[j + 3], scale_log2, nbase))
-                                                  : pt_ex2(fmaf(s[j + 3], scale_log2, nbase));
-                rs4[0] += s[j];
-                rs4[1] += s[j + 1];
-                rs4[2] += s[j + 2];
-                rs4[3] += s[j + 3];
+            for (int j = 0; j < 64; j += 8) {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    float& a = s[j + 2 * h];
+                    float& b = s[j + 2 * h + 1];
+                    pt_unpair(pt_fma2(pt_pair(a, b), scale2, nbase2), a, b);
+                    a = pt_ex2(a);
+                    b = pt_ex2(b);
+                    rs[h] = pt_add2(rs[h], pt_pair(a, b));
+                }
             }
-            l = l * corr + ((rs4[0] + rs4[1]) + (rs4[2] + rs4[3]));
+            float l_even, l_odd;
+            pt_unpair(pt_add2(pt_add2(rs[0], rs[1]), pt_add2(rs[2], rs[3])), l_even, l_odd);
+            l = l * corr + (l_even + l_odd);
             // O is rescaled rarely; only then must the PV product of the page before be done (it
             // is accumulating into O). P needs no such wait: it goes where this page's scores
             // were, and the product that read the P of two pages ago finished before these
