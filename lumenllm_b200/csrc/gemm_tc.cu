@@ -845,9 +845,15 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                 *reinterpret_cast<float4*>(myrow + (((uint32_t)j ^ sw) << 4)) =
                                     make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
                         } else {        // columns 2i, 2i+1 of this thread are gate_i, up_i
+                            // Rows beyond the matrix are zeros, which the division takes by its slow path: a warp
+                            // without a row leaves them out (300 rows x 24,576 x 4,096: 119 -> 89 us).
                             float z[16];
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) z[j] = tc_gate(v[2 * j], p.gelu) * v[2 * j + 1];
+                            for (int j = 0; j < 16; ++j) z[j] = 0.0f;
+                            if (row0 + q * 32 < p.M) {
+#pragma unroll                 // nor does a lane without one hold up its warp
+                                for (int j = 0; j < 16; ++j) z[j] = tc_gate(row_ok ? v[2 * j] : 1.0f, p.gelu) * v[2 * j + 1];
+                            }
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
                                 uint4 w;
@@ -1208,12 +1214,16 @@ static int tc2_launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
     return 0;
 }
 
-// Whether the two-SM kernel takes a prompt-sized product: at least one full wave of 256 x 256
-// tiles for the 74 pairs (fewer tiles are spread better by the single-SM kernel's narrow tiles).
+// Whether the two-SM kernel takes a prompt-sized product: at least three quarters of a wave of 256 x 256
+// tiles for the 74 pairs. Fewer tiles are spread better by the single-SM kernel's narrow tiles or its split k.
+// us, single-SM -> two-SM: 64 tiles, 1,024 x 4,096 x 12,288: 83.3 -> 75.2, 2,048 x 2,048 x 8,192: 61.3 -> 55.5; 60
+// tiles, 700 x 5,120 x 5,120: 46.8 -> 40.8, 1,536 x 2,560 x 2,048: 27.5 -> 23.3; 48 tiles, 700 x 4,096 x 4,096: 34.1 ->
+// 34.7, 3,000 x 1,024 x 2,048: 22.8 -> 23.4; 32 tiles, 1,024 x 2,048 x 8,192 (k in two): 38.6 -> 51.7. One row of tiles is
+// a stream over the weight, which all SMs share better in narrow tiles: 256 x 16,384 x 2,048: 31.1 -> 36.5.
 static bool tc_two_sm(int M, int N) {
     if (!g_tc_two_sm) return false;
     const long items = (long)((M + 255) / 256) * ((N + 255) / 256);
-    return items >= 74;
+    return items >= 74 || (items >= 56 && M > 256);
 }
 
 // Whether a product of this shape can be added to its output in place (epi 2): the shapes of

@@ -581,6 +581,30 @@ def test_tiled_form_of_a_weight(N, K_):
     assert float((part.sum(0).double() - x.double() @ w[:n].double().T).abs().max()) < 1e-3
 
 
+@pytest.mark.parametrize("M,I,H", [(257, 7200, 72), (300, 8192, 64), (385, 7168, 136), (1025, 1536, 64)])
+def test_gemm_tc_rows_that_end_inside_a_pair_of_tiles(M, I, H):
+    """The two-SM product from 56 tiles on, with rows that end inside one block's half of a tile or leave the other
+    half empty: plain, gated, and added to its output. Sums of H products of bfloat16 are exact to H 2^-24 of the
+    sum of their sizes; the gated result is rounded to bfloat16 once (2^-9)."""
+    from lumenllm_b200.ops import kernels as K
+    g = gen(17)
+    x = torch.randn(M, H, generator=g).to(BF16)
+    w = (torch.randn(2 * I, H, generator=g) / math.sqrt(H)).to(BF16)
+    tw = K.tile_weight(dev(w))
+    assert K.gemm_tc_adds(M, 2 * I)
+    ref = x.double() @ w.double().T
+    bound = 4 * H * 2.0 ** -24 * (x.abs().double() @ w.abs().double().T)
+    assert bool(((K.gemm_tc(dev(x), tw).cpu().double().sum(0) - ref).abs() <= bound).all())
+    h = torch.randn(M, 2 * I, generator=g)
+    hd = dev(h)
+    K.gemm_tc(dev(x), tw, add_to=hd)
+    assert bool(((hd.cpu().double() - h.double() - ref).abs() <= bound + 2.0 ** -23 * (h.abs() + ref.abs())).all())
+    z = K.gemm_tc(dev(x), tw, silu_interleaved=True).cpu().double()
+    zr = torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]
+    assert float(((z - zr).abs() / (zr.abs() + 1e-3)).max()) < 2.0 ** -8
+    K.check_error_flags()
+
+
 @pytest.mark.parametrize("M,I,H", [(300, 176, 80), (2048, 1536, 256), (40, 176, 80), (3, 12288, 128),
                                    (2048, 1300, 80), (100, 176, 80), (200, 520, 96)])
 def test_gemm_tc_with_silu_epilogue_on_interleaved_rows(M, I, H):
