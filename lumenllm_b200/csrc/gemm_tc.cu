@@ -19,7 +19,7 @@
 // over several tiles so that all SMs pull from HBM. A split writes partial sums [S, M, N] that
 // the consumer adds in rising order; S depends on the weight's shape only.
 //
-// Epilogues: float32 out; or, for a weight whose rows alternate gate_i, up_i, SiLU(gate)*up (or
+// Epilogues: float32 out; GELU of it in bfloat16 (two-SM kernel); or, for a weight whose rows alternate gate_i, up_i, SiLU(gate)*up (or
 // GELU(gate)*up) written as bfloat16 (no split then).
 //
 // A block-diagonal product is the same product with one difference: the weight's rows come in blocks
@@ -69,6 +69,7 @@
 #define TC_EPI_F32 0
 #define TC_EPI_SILU 1
 #define TC_EPI_ADD 2          // float32, added to what the output holds (two-SM kernel only)
+#define TC_EPI_GELU 4         // gelu_tanh of the product, bfloat16 (two-SM kernel only)
 #define TC_EPI_QKV 3          // heads of 128: q/k RMSNorm, rotation, q out in bfloat16, k and v into the paged cache (two-SM kernel only)
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -159,6 +160,9 @@ struct TcParams {
 // The activation of a gated unit's gate: SiLU, or gelu_tanh(x) = x sigmoid(2 sqrt(2/pi) (x + 0.044715 x^3)).
 __device__ __forceinline__ float tc_gate(float x, int gelu) {
     return x / (1.0f + expf(gelu ? -1.5957691216057308f * (x + 0.044715f * x * x * x) : -x));
+}
+__device__ __forceinline__ float tc_gelu(float z) {
+    return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
 // First column of the activations that the tile of weight rows from `row` on reads.
 __device__ __forceinline__ int tc_k0(const TcParams& p, int row) {
@@ -817,7 +821,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 // keeps the stores free of bank conflicts); when a block is full one thread hands
                 // it to the copy engine, which writes whole lines and clips at the matrix's edge.
                 // Two blocks alternate, so the next is filled while the last is being read.
-                constexpr int SUBS = (EPI != TC_EPI_SILU) ? 1 : 4;       // 32-column loads per staged block
+                constexpr int SUBS = EPI == TC_EPI_SILU ? 4 : (EPI == TC_EPI_GELU ? 2 : 1);      // 32-column loads per staged block
                 unsigned char* myrow0 = sOut + row_in_tile * 128;
                 const uint32_t sw = (uint32_t)(row_in_tile & 7);
 #pragma unroll 1
@@ -839,7 +843,19 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                     v[4 * j] *= f.x; v[4 * j + 1] *= f.y; v[4 * j + 2] *= f.z; v[4 * j + 3] *= f.w;
                                 }
                         }
-                        if (EPI != TC_EPI_SILU) {
+                        if (EPI == TC_EPI_GELU) {
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) {
+                                uint4 w = make_uint4(0u, 0u, 0u, 0u);
+                                if (row0 + q * 32 < p.M) {
+#pragma unroll
+                                    for (int j = 8 * h; j < 8 * h + 8; ++j) v[j] = tc_gelu(v[j]);
+                                    w.x = pack_bf16(v[8 * h], v[8 * h + 1]); w.y = pack_bf16(v[8 * h + 2], v[8 * h + 3]);
+                                    w.z = pack_bf16(v[8 * h + 4], v[8 * h + 5]); w.w = pack_bf16(v[8 * h + 6], v[8 * h + 7]);
+                                }
+                                *reinterpret_cast<uint4*>(myrow + (((uint32_t)(4 * sub + h) ^ sw) << 4)) = w;
+                            }
+                        } else if (EPI != TC_EPI_SILU) {
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
                                 *reinterpret_cast<float4*>(myrow + (((uint32_t)j ^ sw) << 4)) =
@@ -871,7 +887,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     epi_bar();
                     if (issuer) {
-                        const int col0 = (EPI != TC_EPI_SILU) ? tb * 256 + cb * 32 : tb * 128 + cb * 64;
+                        const int col0 = EPI == TC_EPI_SILU ? tb * 128 + cb * 64 : tb * 256 + cb * 32 * SUBS;
                         const int ncols = (EPI != TC_EPI_SILU) ? p.N : (p.N >> 1);
                         if (row0 < p.M && col0 < ncols) {
                             if (EPI == TC_EPI_ADD) tma_reduce_add_2d(&tmC, col0, row0, blk);
@@ -1230,10 +1246,14 @@ static bool tc_two_sm(int M, int N) {
 // the two-SM kernel with output rows that are multiples of 16 bytes.
 LUMEN_API int lumen_gemm_tc_adds(int M, int N) { return (!tc_swapped(M, TC_EPI_F32) && tc_two_sm(M, N) && (N & 3) == 0) ? 1 : 0; }
 
+// Whether GELU can go into the product's epilogue (epi 4): the two-SM kernel with output rows of whole 16 bytes.
+LUMEN_API int lumen_gemm_tc_gelu_ok(int M, int N) { return (!tc_swapped(M, TC_EPI_F32) && tc_two_sm(M, N) && (N & 7) == 0) ? 1 : 0; }
+
 // x bfloat16 [M, K]; W the tiled form (lumen_tile_weight) of a bfloat16 weight of w_rows padded
 // rows, of which the first N are used; K a multiple of 8; x 16-byte, W 128-byte aligned.
 // epi 2: out float32 [M, N] += x W^T, its columns times col_scale [N] where given (only where
 // lumen_gemm_tc_adds says so).
+// epi 4: out bfloat16 [M, N] = gelu_tanh(x W^T) (only where lumen_gemm_tc_gelu_ok says so).
 // epi 0: out float32 [S, M, N], S = lumen_gemm_tc_splits(M, N, K, 0).
 // epi 1: W's rows alternate gate_i, up_i; out bfloat16 [M, N / 2] = SiLU(gate) * up (gelu: GELU(gate) * up).
 static int gemm_tc_run(const void* x, const void* W, void* out, int M, int N, int K, int w_rows, int epi, int gelu,
@@ -1256,7 +1276,9 @@ LUMEN_API int lumen_gemm_tc_blocks(const void* x, const void* W, float* out, int
 static int gemm_tc_run(const void* x, const void* W, void* out, int M, int N, int K, int w_rows, int epi, int gelu,
                        const float* col_scale, int block_rows, int* err, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || (K & 7) || (epi != TC_EPI_F32 && epi != TC_EPI_SILU && epi != TC_EPI_ADD)) return LUMEN_ERR_UNSUPPORTED;
+    if (K <= 0 || (K & 7) || (epi != TC_EPI_F32 && epi != TC_EPI_SILU && epi != TC_EPI_ADD && epi != TC_EPI_GELU))
+        return LUMEN_ERR_UNSUPPORTED;
+    if (epi == TC_EPI_GELU && !lumen_gemm_tc_gelu_ok(M, N)) return LUMEN_ERR_UNSUPPORTED;
     if (epi == TC_EPI_ADD && !lumen_gemm_tc_adds(M, N)) return LUMEN_ERR_UNSUPPORTED;
     if (epi == TC_EPI_SILU && (N & 1)) return LUMEN_ERR_UNSUPPORTED;
     if (((uintptr_t)x & 15) || ((uintptr_t)W & 127) || w_rows < N || w_rows % TC_W_ROW_PAD) return LUMEN_ERR_BAD_ARGUMENT;
@@ -1307,10 +1329,11 @@ static int gemm_tc_run(const void* x, const void* W, void* out, int M, int N, in
         if ((rc = make_map(&mb, W, N, K, TC_BM, w_rows))) return rc;
         // the staged store needs output rows that are multiples of 16 bytes
         const int out_cols = epi != TC_EPI_SILU ? N : N / 2;
-        const int out_esz = epi != TC_EPI_SILU ? 4 : 2;
+        const int out_esz = epi != TC_EPI_SILU && epi != TC_EPI_GELU ? 4 : 2;
         CUtensorMap mc = ma;
         p.tma_out = ((out_cols * out_esz) % 16 == 0 && ((uintptr_t)out & 15) == 0) ? 1 : 0;
-        if (p.tma_out && (rc = make_out_map(&mc, out, M, out_cols, epi != TC_EPI_SILU))) return rc;
+        if (p.tma_out && (rc = make_out_map(&mc, out, M, out_cols, out_esz == 4))) return rc;
+        if (epi == TC_EPI_GELU) return p.tma_out ? tc2_launch<TC_EPI_GELU>(ma, mb, mc, p, stream) : LUMEN_ERR_BAD_ARGUMENT;
         if (epi == TC_EPI_ADD) return p.tma_out ? tc2_launch<TC_EPI_ADD>(ma, mb, mc, p, stream) : LUMEN_ERR_BAD_ARGUMENT;
         if (epi == TC_EPI_F32) return tc2_launch<TC_EPI_F32>(ma, mb, mc, p, stream);
         return tc2_launch<TC_EPI_SILU>(ma, mb, mc, p, stream);

@@ -1537,11 +1537,17 @@ def gemm_tc_adds(M, N) -> bool:
     return bool(int_fn("gemm_tc", "lumen_gemm_tc_adds", [c_int, c_int])(int(M), int(N)))
 
 
-def gemm_tc(x, w, silu_interleaved=False, add_to=None, act="silu", col_scale=None):
+def gemm_tc_gelu_takes(M, N) -> bool:
+    """Whether gemm_tc applies GELU in its epilogue for a product of this shape."""
+    return bool(int_fn("gemm_tc", "lumen_gemm_tc_gelu_ok", [c_int, c_int])(int(M), int(N)))
+
+
+def gemm_tc(x, w, silu_interleaved=False, add_to=None, act="silu", col_scale=None, gelu=False):
     """x @ w.T on the tcgen05 tensor cores. x bfloat16 [M, K], w a TiledWeight [N, K], K a
     multiple of 8. Returns float32 partials [S, M, N] (S = 1 unless M <= 256); or, with
     silu_interleaved (rows of w alternate gate_i, up_i), bfloat16 [M, N/2] = act(gate)*up, `act`
-    "silu" or "gelu"; or, with add_to (float32 [M, N], only where gemm_tc_adds(M, N)), adds the
+    "silu" or "gelu"; or, with gelu (only where gemm_tc_gelu_takes(M, N)), bfloat16 [M, N] =
+    gelu_tanh(product); or, with add_to (float32 [M, N], only where gemm_tc_adds(M, N)), adds the
     product, its columns times col_scale (float32 [N]) where given, to it in place (one float32
     add an element, by the copy engine) and returns None."""
     require(x, BF16, "gemm_tc.x")
@@ -1561,6 +1567,10 @@ def gemm_tc(x, w, silu_interleaved=False, add_to=None, act="silu", col_scale=Non
             require(col_scale, F32, "gemm_tc.col_scale")
             if col_scale.numel() != N:
                 raise KernelError(f"gemm_tc: {col_scale.numel()} factors for {N} columns")
+    elif gelu:
+        if silu_interleaved or not gemm_tc_gelu_takes(M, N):
+            raise KernelError(f"gemm_tc: a product [{M}, {N}] cannot go through GELU in its epilogue")
+        out, epi = torch.empty((M, N), dtype=BF16, device=x.device), 4
     elif silu_interleaved:
         if N % 2:
             raise KernelError("gemm_tc: gate/up rows must come in pairs")

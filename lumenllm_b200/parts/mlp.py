@@ -151,7 +151,9 @@ class GeluMLP:
     adds_residual = True      # forward takes `residual` and may add its update to it in place
 
     def forward(self, y, ctx, residual=None):
-        z = K.gelu_tanh(self.up(y, split_ok=True), self.runtime.dtype)      # adds the partial sums, float32
+        z = None if self.up.f32 else G.gemm_gelu(y, self.up.weight)
+        if z is None:
+            z = K.gelu_tanh(self.up(y, split_ok=True), self.runtime.dtype)  # adds the partial sums, float32
         return self.down(z, split_ok=True, add_to=residual)
 
 

@@ -605,6 +605,23 @@ def test_gemm_tc_rows_that_end_inside_a_pair_of_tiles(M, I, H):
     K.check_error_flags()
 
 
+@pytest.mark.parametrize("M,N,H", [(2048, 2048, 128), (300, 7432, 72), (769, 4104, 64), (257, 7176, 64)])
+def test_gemm_tc_with_gelu_epilogue(M, N, H):
+    """GELU in the two-SM product's epilogue: rows and columns that end inside a tile and a staged block of columns.
+    The float32 sums are rounded to bfloat16 once, after GELU (2^-9)."""
+    from lumenllm_b200.ops import gemm as G
+    from lumenllm_b200.ops import kernels as K
+    g = gen(18)
+    x = torch.randn(M, H, generator=g).to(BF16)
+    w = (torch.randn(N, H, generator=g) * 2 / math.sqrt(H)).to(BF16)
+    z = G.gemm_gelu(dev(x), K.tile_weight(dev(w))).cpu().double()
+    ref = torch.nn.functional.gelu(x.double() @ w.double().T, approximate="tanh")
+    assert z.shape == (M, N)
+    assert float(((z - ref).abs() / (ref.abs() + 1e-3)).max()) < 2.0 ** -8
+    assert G.gemm_gelu(dev(x[:100]), K.tile_weight(dev(w))) is None          # few rows: the split product
+    K.check_error_flags()
+
+
 @pytest.mark.parametrize("M,I,H", [(300, 176, 80), (2048, 1536, 256), (40, 176, 80), (3, 12288, 128),
                                    (2048, 1300, 80), (100, 176, 80), (200, 520, 96)])
 def test_gemm_tc_with_silu_epilogue_on_interleaved_rows(M, I, H):
