@@ -31,6 +31,7 @@ MODULES = {
     "gemm_tc": (["gemm_tc.cu"], ["common.cuh", "mma_utils.cuh"]),
     "attn_generic": (["attn_generic.cu"], ["common.cuh"]),
     "attn_latent": (["attn_latent.cu"], ["common.cuh", "mma_utils.cuh"]),
+    "attn_latent_tc": (["attn_latent_tc.cu"], ["common.cuh", "mma_utils.cuh"]),
     "layer_ops": (["layer_ops.cu"], ["common.cuh"]),
     "attn_talk": (["attn_talk.cu"], ["common.cuh", "mma_utils.cuh"]),
     "ssm": (["ssm.cu"], ["common.cuh"]),

@@ -1008,14 +1008,18 @@ def attn_latent_takes(width, value_dim, dtype) -> bool:
 ATTN_LATENT_DECODE_SPLIT = 8   # blocks that share a row's keys in steps of one token a sequence
 
 
-def attn_latent(q, cache, block_table, cu_q, seq_start, q_lens, value_dim, window, scale, n_seqs=None, n_split=1):
-    """Causal attention over a latent cache on the tensor cores (mma.sync): q bfloat16 [N, H, W],
+def attn_latent(q, cache, block_table, cu_q, seq_start, q_lens, value_dim, window, scale, n_seqs=None, n_split=1,
+                tensor_memory=None):
+    """Causal attention over a latent cache on the tensor cores (prompts of rows in whole 64-value blocks by
+    tcgen05, else mma.sync): q bfloat16 [N, H, W],
     already in the cache's space; cache bfloat16 [pages, 1, PAGE, W] (plain tiles), a row the key of
     every head and its first value_dim numbers the value of every head; a query at position p sees
     key j if 0 <= p - j < window (window 0: every earlier key). Returns float32 [N, H, value_dim].
     Prompts and decoded tokens alike; q_lens (host list) or, with q_lens None, n_seqs = B as in
     attn_prefill. n_split > 1 shares a row's keys out among that many blocks (a second kernel merges
-    them): for steps with few rows."""
+    them): for steps with few rows. tensor_memory: by tcgen05 (True, where the widths allow it), by mma.sync (False),
+    or by the number of rows: from 1,024 rows a sequence, or a device full of blocks, on (33 tokens of 16 heads 22 us by
+    tcgen05 and 18 by mma.sync, 300 tokens 30 and 48, 2,048 tokens 201 and 445)."""
     N, H, W = q.shape
     B = len(q_lens) if q_lens is not None else int(n_seqs)
     require(q, BF16, "attn_latent.q")
@@ -1027,11 +1031,21 @@ def attn_latent(q, cache, block_table, cu_q, seq_start, q_lens, value_dim, windo
     if cu_q.numel() < B + 1 or seq_start.numel() < B or block_table.shape[0] < B or \
             (q_lens is not None and sum(q_lens) != N):
         raise KernelError("attn_latent: metadata does not match the batch")
-    rows = ATTN_LATENT_ROWS
+    n_split = int(n_split)
+    if tensor_memory is None:
+        tensor_memory = N * H >= min(1024 * B, 128 * 74)
+    tc = tensor_memory and n_split == 1 and scale > 0 and bool(int_fn("attn_latent_tc", "lumen_attn_latent_tc_takes", [c_int, c_int])(W, int(value_dim)))
+    rows = 128 if tc else ATTN_LATENT_ROWS
     # sum of ceil(q_b H / rows) over any division of N tokens into B sequences is at most N H // rows + B
     n_tiles = sum((n * H + rows - 1) // rows for n in q_lens) if q_lens is not None else N * H // rows + B
     out = torch.empty((N, H, int(value_dim)), dtype=F32, device=q.device)
-    n_split = int(n_split)
+    if tc:
+        f = fn("attn_latent_tc", "lumen_attn_latent_tc",
+               [P, P, c_int, P, c_int, P, P, c_int, c_int, P, c_int, c_int, c_int, c_int, c_int, c_float, P, P])
+        check(f(ptr(q), ptr(cache), cache.shape[0], ptr(block_table), block_table.stride(0), ptr(cu_q), ptr(seq_start), B,
+                n_tiles, ptr(out), N, H, W, int(value_dim), int(window), float(scale), ptr(error_flag(q.device)),
+                stream_ptr()), "attn_latent_tc")
+        return out
     part = torch.empty((n_split, N * H, int(value_dim) + 2), dtype=F32, device=q.device) if n_split > 1 else None
     f = fn("attn_latent", "lumen_attn_latent",
            [P, P, P, c_int, P, P, c_int, c_int, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_float, P, P])

@@ -786,6 +786,18 @@ def test_latent_attention_kernel_against_plain_sums(H, W, dv, window):
         assert float((got - ref).abs().max()) < 2e-2
 
 
+@pytest.mark.parametrize("H,W,dv,window", [(16, 576, 512, 45), (16, 576, 512, 0), (3, 192, 64, 33), (70, 128, 128, 1),
+                                           (5, 64, 64, 0), (7, 448, 384, 100), (1, 320, 320, 64)])
+def test_latent_attention_of_whole_blocks(H, W, dv, window, monkeypatch):
+    """The same cases for rows of whole 64-value blocks, whose prompts go by tcgen05: one and two slices of value
+    columns (the second narrower), no columns outside the slice, row tiles of one and of many tokens."""
+    from functools import partial
+    from lumenllm_b200.ops import kernels as K
+    monkeypatch.setattr(K, "attn_latent", partial(K.attn_latent, tensor_memory=True))
+    test_latent_attention_kernel_against_plain_sums(H, W, dv, window)
+    K.check_error_flags()
+
+
 @pytest.mark.parametrize("N", [1, 9, 150])
 def test_products_of_every_head_on_the_tensor_cores(N):
     """Both per-head products of latent attention against float32 sums: the query into the latent
