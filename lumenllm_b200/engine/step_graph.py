@@ -24,11 +24,11 @@ import weakref
 from collections import OrderedDict
 from typing import Dict, List, Sequence, Tuple
 
-import numpy as np
 import torch
 
 from ..cache.kv import pages_for
 from ..ops import kernels as K
+from ..sampling.sampler import pack_options
 from .context import StepEntry, StepLayout, context_on, pack_step, padding_twin, upload
 
 # A prompt step of more tokens than this is launched kernel by kernel: the device then takes
@@ -60,8 +60,8 @@ def _pow2(n: int) -> int:
 
 
 class _Captured:
-    def __init__(self, graph, meta, opts, top_k, logits, next_tok, ctx):
-        self.graph, self.meta, self.opts, self.top_k = graph, meta, opts, top_k
+    def __init__(self, graph, meta, sampling, logits, next_tok, ctx):
+        self.graph, self.meta, self.sampling = graph, meta, sampling
         self.logits, self.next_tok, self.ctx = logits, next_tok, ctx
 
 
@@ -105,8 +105,8 @@ class StepGraphs:
         _, Bb, _, greedy = key
         dev = eng.device
         meta = torch.zeros((lay.total,), dtype=torch.int32, device=dev)
-        opts = torch.zeros((Bb, 4), dtype=torch.float32, device=dev)
-        top_k = torch.zeros((Bb,), dtype=torch.int32, device=dev)
+        sampling = torch.zeros((5 * Bb,), dtype=torch.float32, device=dev)      # as pack_options lays it out
+        opts, top_k = sampling[:4 * Bb].view(Bb, 4), sampling[4 * Bb:].view(torch.int32)
         next_tok = torch.zeros((Bb,), dtype=torch.int32, device=dev)
         q_lens, starts, slots, n_real = lists
         ctx = context_on(meta, lay, q_lens, starts, slots, n_real, eng.cache, eng.runtime)
@@ -145,7 +145,7 @@ class StepGraphs:
         finally:
             if was_enabled:
                 gc.enable()
-        cap = _Captured(graph, meta, opts, top_k, logits, next_tok, ctx)
+        cap = _Captured(graph, meta, sampling, logits, next_tok, ctx)
         cap.kernels_per_replay = native.launches - before
         return cap
 
@@ -183,13 +183,7 @@ class StepGraphs:
                 raise ValueError("tokens on the device can only feed a step of one token each")
             cap.ctx.tokens[:n].copy_(tokens_on_device[:n])
         if not greedy:
-            o = np.zeros((Bb, 4), dtype=np.float32)
-            k = np.zeros((Bb,), dtype=np.int32)
-            for i, (c, u) in enumerate(zip(configs, uniforms)):
-                o[i] = (c.temperature, c.top_p, c.min_p, u)
-                k[i] = c.top_k
-            cap.opts.copy_(torch.from_numpy(o).pin_memory(), non_blocking=True)
-            cap.top_k.copy_(torch.from_numpy(k).pin_memory(), non_blocking=True)
+            cap.sampling.copy_(torch.from_numpy(pack_options(configs, uniforms, Bb)).pin_memory(), non_blocking=True)
         cap.graph.replay()
         for e in se:
             eng.cache.commit(e.slot, len(e.tokens))

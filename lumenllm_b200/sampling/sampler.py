@@ -16,6 +16,7 @@ import os
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 _M64 = (1 << 64) - 1
@@ -56,6 +57,16 @@ def uniform(seed: int, stream: int, step: int) -> float:
     return (x >> 40) / float(1 << 24)
 
 
+def pack_options(configs, us, rows: int) -> np.ndarray:
+    """float32 [5 rows]: a row's (temperature, top_p, min_p, u) one behind the other, then the top-k of every
+    row as int32 bits; zeros for rows beyond the configs."""
+    out = np.zeros((5 * rows,), dtype=np.float32)
+    n = len(configs)
+    out[:4 * n] = [x for c, u in zip(configs, us) for x in (c.temperature, c.top_p, c.min_p, u)]
+    out[4 * rows:4 * rows + n].view(np.int32)[:] = [c.top_k for c in configs]
+    return out
+
+
 def fresh_seed() -> int:
     return int.from_bytes(os.urandom(8), "little")
 
@@ -74,8 +85,7 @@ class DeviceSampler:
             raise ValueError("one sampling config and one uniform number per row")
         if all(c.greedy for c in configs):
             return K.argmax(logits)
-        opts = torch.tensor([[c.temperature, c.top_p, c.min_p, u] for c, u in zip(configs, us)],
-                            dtype=torch.float32).pin_memory().to(self.device, non_blocking=True)
-        top_k = torch.tensor([c.top_k for c in configs], dtype=torch.int32) \
-            .pin_memory().to(self.device, non_blocking=True)
-        return K.sample(logits, opts, top_k)
+        # options and top-k go to the device in one copy (two, with a tensor each, were most of a small call's time)
+        host = torch.from_numpy(pack_options(configs, us, B)).pin_memory()
+        both = host.to(self.device, non_blocking=True)
+        return K.sample(logits, both[:4 * B].view(B, 4), both[4 * B:].view(torch.int32))
