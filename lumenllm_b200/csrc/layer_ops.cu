@@ -1213,6 +1213,105 @@ add_shaped_rmsnorm_kernel(float* __restrict__ h, const ShapedGroups gr, const fl
     }
 }
 
+// The same for a row that fits the block's threads, four values each, and up to two groups that are not picked from
+// places: decode steps, where the time is one round trip after another. The weights are in registers before the
+// wait, the first eight (rows beyond 2,048: four) partial sums of both groups are under way at once, two normed groups share a reduction, and x
+// stays in registers. Every sum has the order of the kernel above. Four rows of 2,048: 5.5 -> 3.8 us alone.
+template <typename TOut, int MAXT>
+__global__ void __launch_bounds__(MAXT)
+add_shaped_rmsnorm_row_kernel(float* __restrict__ h, const ShapedGroups gr, const float* __restrict__ wn, float eps_n,
+                              TOut* __restrict__ y, const int* __restrict__ rows, int H, int write_h) {
+    constexpr int V = 4, AHEAD = MAXT > 512 ? 4 : 8;
+    __shared__ float red[2][32];
+    pdl_trigger();
+    const int i = threadIdx.x * V;
+    const bool act = i < H;
+    Vals<V> zero;
+#pragma unroll
+    for (int k = 0; k < V; ++k) zero.v[k] = 0.0f;
+    const Vals<V> w1 = act && wn ? ldv<V>(wn + i) : zero, w2 = act && gr.wn2 ? ldv<V>(gr.wn2 + i) : zero;
+    Vals<V> wg[2], cg[2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        wg[g] = act && g < gr.n && gr.w[g] ? ldv<V>(gr.w[g] + i) : zero;
+        cg[g] = act && g < gr.n && gr.cols[g] ? ldv<V>(gr.cols[g] + i) : zero;
+    }
+    pdl_wait();
+    const int b = blockIdx.x;
+    const int r = rows ? rows[b] : b;
+    float* hr = h + (size_t)r * H;
+    Vals<V> x = act ? ldv<V>(gr.base ? gr.base + i : hr + i) : zero;
+    Vals<V> q[2][AHEAD];
+#pragma unroll
+    for (int g = 0; g < 2; ++g)
+#pragma unroll
+        for (int s = 0; s < AHEAD; ++s)
+            q[g][s] = act && g < gr.n && s < gr.S[g] ? ldv<V>(gr.p[g] + (size_t)s * gr.stride[g] + (size_t)r * H + i) : zero;
+    float scale[2], ss[2] = {0.0f, 0.0f};
+    Vals<V> v[2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        scale[g] = g < gr.n ? (gr.rowf[g] ? gr.scale[g] * gr.rowf[g][r] : gr.scale[g]) : 0.0f;
+        v[g] = q[g][0];
+#pragma unroll
+        for (int s = 1; s < AHEAD; ++s)
+            if (g < gr.n && s < gr.S[g])
+#pragma unroll
+                for (int k = 0; k < V; ++k) v[g].v[k] += q[g][s].v[k];
+        if (act && g < gr.n)
+            for (int s = AHEAD; s < gr.S[g]; ++s) {
+                const Vals<V> t = ldv<V>(gr.p[g] + (size_t)s * gr.stride[g] + (size_t)r * H + i);
+#pragma unroll
+                for (int k = 0; k < V; ++k) v[g].v[k] += t.v[k];
+            }
+        if (g < gr.n && gr.w[g])
+#pragma unroll
+            for (int k = 0; k < V; ++k) ss[g] += v[g].v[k] * v[g].v[k];
+    }
+    if ((gr.n > 0 && gr.w[0]) || (gr.n > 1 && gr.w[1])) {        // the groups' norms, both reductions at once (block_sum's order)
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = (blockDim.x + 31) >> 5;
+        const float a0 = warp_sum(ss[0]), a1 = warp_sum(ss[1]);
+        if (lane == 0) { red[0][warp] = a0; red[1][warp] = a1; }
+        __syncthreads();
+        const float b0 = warp_sum(lane < nwarp ? red[0][lane] : 0.0f), b1 = warp_sum(lane < nwarp ? red[1][lane] : 0.0f);
+        const float inv[2] = {gr.w[0] ? 1.0f / sqrtf(b0 / (float)H + gr.eps[0]) : 1.0f,
+                              gr.n > 1 && gr.w[1] ? 1.0f / sqrtf(b1 / (float)H + gr.eps[1]) : 1.0f};
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+            if (g < gr.n && gr.w[g])
+#pragma unroll
+                for (int k = 0; k < V; ++k) v[g].v[k] = v[g].v[k] * inv[g] * wg[g].v[k];
+    }
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        if (g >= gr.n) break;
+        if (gr.cols[g])
+#pragma unroll
+            for (int k = 0; k < V; ++k) v[g].v[k] *= cg[g].v[k];
+#pragma unroll
+        for (int k = 0; k < V; ++k) x.v[k] = fmaf(scale[g], v[g].v[k], x.v[k]);
+    }
+    if (act && write_h && (gr.n > 0 || gr.base)) stv<V>(hr + i, x);
+    if (!wn) {
+        if (act && y) stv<V>(y + (size_t)b * gr.ldy + i, x);
+        return;
+    }
+    float sx = 0.0f;
+#pragma unroll
+    for (int k = 0; k < V; ++k) sx += x.v[k] * x.v[k];
+    const float sn = 1.0f / sqrtf(block_sum(sx, red[0]) / (float)H + eps_n);
+    if (!act) return;
+    Vals<V> o;
+#pragma unroll
+    for (int k = 0; k < V; ++k) o.v[k] = x.v[k] * sn * w1.v[k];
+    stv<V>(y + (size_t)b * H + i, o);
+    if (gr.wn2) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) o.v[k] = x.v[k] * sn * w2.v[k];
+        stv<V>((TOut*)gr.y2 + (size_t)b * H + i, o);
+    }
+}
+
 // ptrs / strides / counts / scales / cols / weights / epss / row_factors / places / place_weights: host arrays of n_groups entries. y is
 // [n_rows, H] (ldy H) with wn, rows ldy apart without.
 LUMEN_API int lumen_add_shaped_rmsnorm(float* h, const void* const* ptrs, const long long* strides, const int* counts,
@@ -1254,6 +1353,17 @@ LUMEN_API int lumen_add_shaped_rmsnorm(float* h, const void* const* ptrs, const 
     const size_t smem = (size_t)H * (1 + normed) * sizeof(float);
     if (smem > 200 * 1024) return LUMEN_ERR_UNSUPPORTED;
     const int threads = row_threads(vec ? H / 4 : H, n_rows);
+    // few rows of at most 4,096 and up to two groups: a row in the registers of one block
+    if (vec && 4 * threads >= H && n_groups <= 2 && !gr.place[0] && !gr.place[1]) {
+#define ROW_GO(T, M)                                                                                                     \
+    lumen_launch(add_shaped_rmsnorm_row_kernel<T, M>, dim3(n_rows), dim3(threads), 0, stream, h, gr, wn, eps_n, (T*)y, rows, \
+                 H, write_h)
+        if (y_is_bf16) { if (threads <= 512) ROW_GO(__nv_bfloat16, 512); else ROW_GO(__nv_bfloat16, 1024); }
+        else { if (threads <= 512) ROW_GO(float, 512); else ROW_GO(float, 1024); }
+#undef ROW_GO
+        LUMEN_LAUNCH_CHECK();
+        return 0;
+    }
 #define SHAPED_GO(T, V_)                                                                                                 \
     do {                                                                                                                 \
         auto k = add_shaped_rmsnorm_kernel<T, V_>;                                                                       \

@@ -159,6 +159,45 @@ def test_rms_norm_with_shaped_updates(dtype, width, N):
     close(hd, x + value(*groups[0]) + value(*groups[1]), F32, "adding only")
 
 
+@pytest.mark.parametrize("width", [4, 2048, 2052, 4096])
+@pytest.mark.parametrize("normed", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_few_rows_of_up_to_two_shaped_updates(normed, width):
+    """Rows that one block holds in its registers: one, eight and eleven partial sums, a norm of either, both or
+    neither group, factors a row and a column, a stream that starts from one row, two norms of the sum, the sum itself
+    as the output, one group and none."""
+    from lumenllm_b200.ops import kernels as K
+    g = torch.Generator().manual_seed(width + sum(normed))
+    rn = lambda *s: torch.randn(*s, generator=g)
+    N = 5
+    h, w, w2, base = rn(N, width), 1 + 0.1 * rn(width), 1 + 0.1 * rn(width), rn(width)
+    for S in ((8, 11), (1, 9)):
+        groups = [(rn(S[0], N, width), 0.5, rn(width), 1 + 0.1 * rn(width) if normed[0] else None, 1e-5, rn(N)),
+                  (rn(S[1], N, width), -1.25, None, 1 + 0.1 * rn(width) if normed[1] else None, 1e-3)]
+
+        def value(d, s, c, nw, eps, rowf=None):
+            d = d.sum(0)
+            d = P.rms_norm(d, nw, eps) if nw is not None else d
+            d = s * (d if c is None else c * d)
+            return d if rowf is None else rowf[:, None] * d
+
+        for n in (0, 1, 2):
+            dev = [tuple(v.cuda() if isinstance(v, torch.Tensor) else v for v in gr) for gr in groups[:n]]
+            x = h + sum(value(*gr) for gr in groups[:n])
+            hd = h.clone().cuda()
+            ya, yb = K.add_shaped_rmsnorm(hd, dev, w.cuda(), 1e-6, F32, weight2=w2.cuda())
+            close(ya, P.rms_norm(x, w, 1e-6), F32, "first norm")
+            close(yb, P.rms_norm(x, w2, 1e-6), F32, "second norm")
+            close(hd, x, F32, "stream")
+            if n:
+                y = K.add_shaped_rmsnorm(hd, dev, w.cuda(), 1e-6, BF16, write_h=False, base=base.cuda())
+                xb = base + sum(value(*gr) for gr in groups[:n])
+                close(y, P.rms_norm(xb, w, 1e-6), BF16, "from one row")
+                out = torch.zeros(N, width + 4, dtype=F32, device="cuda")
+                K.add_shaped_rmsnorm(hd, dev, None, 0.0, F32, write_h=False, base=base.cuda(), cast_to=out[:, :width])
+                close(out[:, :width], xb, F32, "the sum itself")
+                assert not out[:, width:].any()
+
+
 def test_dynamic_tanh_takes_a_shaped_update():
     """The other norm, behind a layer whose updates have factors a column."""
     from lumenllm_b200.config.spec import PartSpec
