@@ -71,7 +71,7 @@ def gemm_gate_up_silu(x: torch.Tensor, w_interleaved, act="silu"):
 
 def gemm_gelu(x: torch.Tensor, w):
     """gelu_tanh(x w^T) in bfloat16 [M, N] in ONE kernel where the two-SM product takes the shape (its epilogue has
-    the float32 sums at hand; for 2,048 x 8,192 the activation kernel alone takes 25 us); else None, and the
+    the float32 sums at hand; 2,048 x 8,192 x 2,048: 58 us, 81 with the activation kernel behind); else None, and the
     caller takes the float32 product with the activation kernel behind it."""
     if takes_tc(x, w) and K.gemm_tc_gelu_takes(x.shape[0], w.shape[0]):
         return K.gemm_tc(x if x.is_contiguous() else x.contiguous(), w, gelu=True)
