@@ -13,11 +13,12 @@
 // so the DR_ROWS rows a thread keeps in registers are read once a token; the NS threads of a
 // column (adjacent lanes) add r by shuffles at once, since u_j waits for it, and w a chunk at a time: the
 // shares of eight tokens change lanes so that a lane adds up a token of its own (7 shuffles for 8 tokens
-// where one token after the other takes 8 log2(NS)).Four
-// warps of a block share a staged row, and what they read of it (48 values a thread and token) is what bounds a
-// token: 220 of its 430 cycles go to shared-memory reads, the rest to the chain of dependent steps. 2,048
-// tokens of 16 heads of 128 x 128: 466 us with the kernel that prepares them (732 with 16 threads a column, 8 rows
-// each, and w summed token by token), four sequences of 2,048 tokens in all: 400 (668), one token of 64 sequences: 36 (44).
+// where one token after the other takes 8 log2(NS)). Four warps of a block share a staged row, and what they read of
+// it (48 values a thread and token) is what bounds a token, with the chain of dependent steps: 220 of its 400
+// cycles go to shared-memory reads. 2,048 tokens of 16 heads of 128 x 128: 466 us with the kernel that
+// prepares them (732 with 16 threads a column, 8 rows each, and w summed token by token), four sequences of 2,048 tokens
+// in all: 400 (668), one token of 64 sequences: 36 (44). Two columns a thread over 16 lanes halve the reads and
+// lengthen the chain by two shuffles: 497 and 412 us.
 // What does not depend on the state is made for
 // all tokens at once by a kernel of its own (a warp a (token, head): normed q and k, the decays,
 // k . q and beta, one row [q | k | g | k.q, beta] of a scratch matrix), so that the walk itself is
