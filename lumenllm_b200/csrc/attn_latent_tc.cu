@@ -181,6 +181,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     __syncthreads();
     lt_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    int a_issued[2] = {0, 0}, v_issued[2] = {0, 0};          // the producer's copies into each stage
 
     if (warp == 0) {
         if (lane == 0) {
@@ -194,11 +195,13 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 if (na > 0) {
                     if (!mbar_wait(&a_empty[st], ph)) { *abort_flag = 1; atomicExch(err, 1); break; }
                     mbar_expect_tx(&a_full[st], (uint32_t)(na * LT_KBLOCK));
+                    ++a_issued[st];
                     for (int c = 0; c < wb; ++c)
                         if (c < v0 || c >= v0 + nv) lt_tma_2d(dst + c * LT_KBLOCK, &tmK, c * 64, row, &a_full[st]);
                 }
                 if (!mbar_wait(&v_empty[st], ph)) { *abort_flag = 1; atomicExch(err, 1); break; }
                 mbar_expect_tx(&v_full[st], (uint32_t)(nv * LT_KBLOCK));
+                ++v_issued[st];
                 for (int c = v0; c < v0 + nv; ++c) lt_tma_2d(dst + c * LT_KBLOCK, &tmK, c * 64, row, &v_full[st]);
             }
         }
@@ -348,6 +351,14 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
     }
 
+    if (threadIdx.x == 0) {
+        // the block's own copies have landed before it leaves; they have by now, unless a wait ran out
+        mbar_wait(q_full, 0);
+        for (int st = 0; st < 2; ++st) {
+            if (a_issued[st] > 0) mbar_wait(&a_full[st], (uint32_t)(a_issued[st] - 1) & 1u);
+            if (v_issued[st] > 0) mbar_wait(&v_full[st], (uint32_t)(v_issued[st] - 1) & 1u);
+        }
+    }
     lt_fence_before();
     __syncthreads();
     if (warp == 1) {
