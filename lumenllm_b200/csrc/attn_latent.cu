@@ -2,7 +2,9 @@
 // of every query head, and whose first dv values are the value of every head as well. Queries come
 // already carried into that space ([N, H, W], bfloat16), so all H heads of a token share every
 // cached row and a block's rows are (token, head) pairs: 64 consecutive rows of the query matrix
-// [N H, W] that belong to one sequence. The same kernel serves prompts and single decoded tokens.
+// [N H, W] that belong to one sequence. It serves single decoded tokens (a row's keys shared out among
+// blocks) and, where rows are not whole 64-value blocks, prompts as well; prompts of rows that are go to
+// attn_latent_tc.cu, whatever their length.
 //
 // Keys are walked 32 at a time (half a page; tiles start at multiples of 32 in absolute position,
 // so what a row computes depends only on its own position, never on the batch or on how a prompt

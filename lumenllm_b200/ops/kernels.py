@@ -1009,17 +1009,20 @@ ATTN_LATENT_DECODE_SPLIT = 8   # blocks that share a row's keys in steps of one 
 
 
 def attn_latent(q, cache, block_table, cu_q, seq_start, q_lens, value_dim, window, scale, n_seqs=None, n_split=1,
-                tensor_memory=None):
-    """Causal attention over a latent cache on the tensor cores (prompts of rows in whole 64-value blocks by
-    tcgen05, else mma.sync): q bfloat16 [N, H, W],
+                tensor_memory=True):
+    """Causal attention over a latent cache on the tensor cores: q bfloat16 [N, H, W],
     already in the cache's space; cache bfloat16 [pages, 1, PAGE, W] (plain tiles), a row the key of
     every head and its first value_dim numbers the value of every head; a query at position p sees
     key j if 0 <= p - j < window (window 0: every earlier key). Returns float32 [N, H, value_dim].
     Prompts and decoded tokens alike; q_lens (host list) or, with q_lens None, n_seqs = B as in
     attn_prefill. n_split > 1 shares a row's keys out among that many blocks (a second kernel merges
-    them): for steps with few rows. tensor_memory: by tcgen05 (True, where the widths allow it), by mma.sync (False),
-    or by the number of rows: from 1,024 rows a sequence, or a device full of blocks, on (33 tokens of 16 heads 22 us by
-    tcgen05 and 18 by mma.sync, 300 tokens 30 and 48, 2,048 tokens 201 and 445)."""
+    them): for steps with few rows. Which kernel runs is a matter of the widths and of n_split alone, never of the
+    step's size: with n_split 1 a row's result is the same bits alone and among others, however its prompt was cut and
+    whether the step was captured. Rows in whole 64-value blocks go by tcgen05 (n_split 1; tensor_memory False: not),
+    all others by mma.sync. us by tcgen05 / mma.sync at 16 heads of 576, 512 of them the value, window 1,024: one prompt of
+    8 tokens 11.4 / 11.0, 33: 11.5 / 11.2, 64: 13.3 / 15.1, 300: 29 / 48, 2,048: 211 / 446; 8 tokens after 1,500 in each
+    of 8 sequences 77 / 142; 64 sequences of one token after 1,500 beside a prompt of 33: 77 / 127; 16 prompts of
+    33 tokens (160 blocks, a few more than the SMs) 21 / 13."""
     N, H, W = q.shape
     B = len(q_lens) if q_lens is not None else int(n_seqs)
     require(q, BF16, "attn_latent.q")
@@ -1032,8 +1035,6 @@ def attn_latent(q, cache, block_table, cu_q, seq_start, q_lens, value_dim, windo
             (q_lens is not None and sum(q_lens) != N):
         raise KernelError("attn_latent: metadata does not match the batch")
     n_split = int(n_split)
-    if tensor_memory is None:
-        tensor_memory = N * H >= min(1024 * B, 128 * 74)
     tc = tensor_memory and n_split == 1 and scale > 0 and bool(int_fn("attn_latent_tc", "lumen_attn_latent_tc_takes", [c_int, c_int])(W, int(value_dim)))
     rows = 128 if tc else ATTN_LATENT_ROWS
     # sum of ceil(q_b H / rows) over any division of N tokens into B sequences is at most N H // rows + B

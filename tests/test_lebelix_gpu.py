@@ -798,6 +798,57 @@ def test_latent_attention_of_whole_blocks(H, W, dv, window, monkeypatch):
     K.check_error_flags()
 
 
+@pytest.mark.parametrize("H,W,dv,window", [(16, 576, 512, 100), (16, 576, 512, 0), (3, 192, 128, 70), (2, 64, 48, 0)])
+def test_a_latent_row_is_the_same_bits_in_any_step(H, W, dv, window):
+    """A prompt of 80 tokens alone, padded as a captured step pads it, among a long prompt and single tokens, and cut
+    into portions: the kernel is picked by the widths alone, and what a row computes depends on its position alone."""
+    from lumenllm_b200.ops import kernels as K
+    lens, starts = [80, 700, 1, 1], [0, 0, 90, 400]
+    table, cache, _, q = _latent_case(lens, starts, H, W, seed=33)
+    cache, table = cache.to(BF16).cuda(), table.cuda()
+
+    def run(pieces, captured=False):          # pieces: (sequence, its first query, number of queries)
+        n = [p[2] for p in pieces]
+        cu = torch.tensor([0] + list(torch.tensor(n).cumsum(0)), dtype=torch.int32).cuda()
+        st = torch.tensor([starts[b] + at for b, at, _ in pieces], dtype=torch.int32).cuda()
+        qq = torch.cat([q[b][at:at + m] for b, at, m in pieces])
+        if captured:                          # the padding sequence lies on the spare page
+            cu = torch.cat([cu, cu[-1:] + 16]).contiguous()
+            st = torch.cat([st, torch.zeros_like(st[:1])])
+            qq = torch.cat([qq, torch.zeros(16, H, W)])
+        tab = torch.stack([table[b] for b, _, _ in pieces] + ([torch.zeros_like(table[0])] if captured else [])).contiguous()
+        out = K.attn_latent(qq.to(BF16).cuda(), cache, tab, cu, st, None if captured else n, dv, window, 0.2, n_seqs=len(st))
+        return out.cpu()[:sum(n)]
+
+    alone = run([(0, 0, 80)])
+    assert torch.equal(run([(0, 0, 80)], captured=True), alone)
+    assert torch.equal(run([(b, 0, n) for b, n in enumerate(lens)])[:80], alone)
+    assert torch.equal(run([(2, 0, 1), (0, 0, 80), (1, 0, 700)])[1:81], alone)
+    assert torch.equal(torch.cat([run([(0, at, n)]) for at, n in ((0, 1), (1, 33), (34, 2), (36, 44))]), alone)
+    K.check_error_flags()
+
+
+@pytest.mark.parametrize("n", [66, 96, 300])
+def test_a_captured_prompt_of_latent_layers_equals_the_eager_one(n, tmp_path):
+    """Latent layers whose rows are whole 64-value blocks (16 heads): a prompt replayed from a graph, where padding
+    tokens and a padding sequence fill the bucket, gives the bits of the step that is launched kernel by kernel."""
+    from lumenllm_b200 import Engine, StepEntry
+    from lumenllm_b200.sampling import SamplingConfig
+    cfg = config(97, 64, 1e-6, [layer(latent(16, 32, 64, 32, 128, 0.1, size=50, rot=32), dense(80)),
+                                layer(latent(16, 32, 64, 64, 128, 0.1, rot=32, kv_from=0), None)])
+    folder = write_model(cfg, tmp_path / "blocks", seed=72)
+    toks = tokens_of(cfg, (n,), seed=73)[0]
+    _, w = P.load_model(folder)
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1024)
+    twin = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1024, use_graphs=False)
+    eng.run_device([(eng.alloc_slot(), toks)], [SamplingConfig()], [0.0])
+    got = eng.graphs.last.logits[:1].float().cpu()
+    assert eng.graphs.last.ctx.N == (n + 31) // 32 * 32
+    assert torch.equal(got, twin.step([StepEntry(twin.alloc_slot(), toks, [n - 1])]).cpu())
+    close(got, P.forward(cfg, w, toks)[-1:], "bfloat16")
+    eng.check_kernels()
+
+
 @pytest.mark.parametrize("N", [1, 9, 150])
 def test_products_of_every_head_on_the_tensor_cores(N):
     """Both per-head products of latent attention against float32 sums: the query into the latent
