@@ -23,8 +23,8 @@
 // 128 x 32 x 16 product reads 5 KB of shared memory for 16 cycles of arithmetic.
 // 2,048 tokens, 16 heads, W = 576, dv = 512, window 1,024: 211 us (mma.sync 445; 201 with one bfloat16 number a weight);
 // without the window 260 (625). Against 64 bits 2.7e-6 where mma.sync's rounded weights are 1.4e-3 off.
-// Every wait is bounded; when one runs out the block raises the error flag, lets the other roles run out, frees its
-// tensor memory and returns.
+// Every wait is bounded; when one runs out the block raises the error flag, the other roles give up on theirs, and the
+// block leaves once its own copies have landed and the products it has issued are done (waits with a bound of their own).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -98,6 +98,20 @@ __device__ __forceinline__ float lt_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// As mbar_wait, but given up as soon as another role of the block has.
+__device__ __forceinline__ bool lt_wait(uint64_t* bar, uint32_t parity, const volatile int* abort_flag) {
+    for (uint32_t it = 0; it < LUMEN_SPIN_LIMIT; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if ((it & 63u) == 63u && *abort_flag) return false;
+    }
+    return false;
+}
 // A 128-byte-swizzled operand: rows of 128 bytes, groups of 8 rows 1024 bytes apart; lbo: distance between the
 // 64-value blocks of an N-major operand.
 __device__ __forceinline__ uint64_t lt_desc(uint32_t smem_addr, uint32_t lbo_bytes) {
@@ -119,7 +133,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
 attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const int* __restrict__ block_table, int bt_stride, const int* __restrict__ cu_q,
                       const int* __restrict__ seq_start, int B, float* __restrict__ out, int H, int W, int dv, int window,
-                      float scale_log2, int* __restrict__ err) {
+                      float scale_log2, int give_up_at, int* __restrict__ err) {
     pdl_wait();      // nothing of this kernel touches global memory before this
     pdl_trigger();
     // operand tiles must start on 1024-byte boundaries; there is no static shared memory ahead of the dynamic part
@@ -142,7 +156,8 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     uint64_t* s_full = bars + 9;        // [2] S is in tensor memory
     uint64_t* p_ready = bars + 11;      // [2] P is in tensor memory, O corrected
     uint64_t* pv_done = bars + 13;      // [2] that tile's product is in O
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+    uint64_t* mma_done = bars + 15;     // all products of the block are done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     // which sequence, which tile of its rows; the last tiles of a sequence see the most keys and come first
@@ -165,7 +180,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 15; ++i) mbar_init(&bars[i], (i == 11 || i == 12) ? 4 : 1);
+        for (int i = 0; i < 16; ++i) mbar_init(&bars[i], (i == 11 || i == 12) ? 4 : 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmQ)) : "memory");
@@ -193,13 +208,13 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 const int row = bt[kt / (LUMEN_PAGE / LT_KEYS)] * LUMEN_PAGE + (kt % (LUMEN_PAGE / LT_KEYS)) * LT_KEYS;
                 unsigned char* dst = sK + st * wb * LT_KBLOCK;
                 if (na > 0) {
-                    if (!mbar_wait(&a_empty[st], ph)) { *abort_flag = 1; atomicExch(err, 1); break; }
+                    if (!lt_wait(&a_empty[st], ph, abort_flag)) { *abort_flag = 1; atomicExch(err, 1); break; }
                     mbar_expect_tx(&a_full[st], (uint32_t)(na * LT_KBLOCK));
                     ++a_issued[st];
                     for (int c = 0; c < wb; ++c)
                         if (c < v0 || c >= v0 + nv) lt_tma_2d(dst + c * LT_KBLOCK, &tmK, c * 64, row, &a_full[st]);
                 }
-                if (!mbar_wait(&v_empty[st], ph)) { *abort_flag = 1; atomicExch(err, 1); break; }
+                if (!lt_wait(&v_empty[st], ph, abort_flag)) { *abort_flag = 1; atomicExch(err, 1); break; }
                 mbar_expect_tx(&v_full[st], (uint32_t)(nv * LT_KBLOCK));
                 ++v_issued[st];
                 for (int c = v0; c < v0 + nv; ++c) lt_tma_2d(dst + c * LT_KBLOCK, &tmK, c * 64, row, &v_full[st]);
@@ -210,6 +225,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             constexpr uint32_t idesc_s = lt_idesc(LT_KEYS, 0);
             const uint32_t idesc_pv = lt_idesc(nv * 64, 1);
             const uint32_t q0 = smem_u32(sQ);
+            bool issued = false;
             auto scores = [&](int i) -> bool {          // S[i & 1] = Q K(i)^T
                 const int st = i & 1, ph = (i >> 1) & 1;
                 const uint32_t k0 = smem_u32(sK + st * wb * LT_KBLOCK), d = tmem_base + st * LT_KEYS;
@@ -222,19 +238,21 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     }
                 };
                 if (na > 0) {
-                    if (!mbar_wait(&a_full[st], ph)) return false;
+                    if (!lt_wait(&a_full[st], ph, abort_flag)) return false;
                     lt_fence_after();
                     for (int c = 0; c < wb; ++c)
                         if (c < v0 || c >= v0 + nv) block(c);
+                    issued = true;
                     lt_commit(&a_empty[st]);
                 }
-                if (!mbar_wait(&v_full[st], ph)) return false;
+                if (!lt_wait(&v_full[st], ph, abort_flag)) return false;
                 lt_fence_after();
                 for (int c = v0; c < v0 + nv; ++c) block(c);
+                issued = true;
                 lt_commit(&s_full[st]);
                 return true;
             };
-            bool ok = mbar_wait(q_full, 0);
+            bool ok = lt_wait(q_full, 0, abort_flag);
             if (ok) {
                 lt_fence_after();
                 ok = scores(0);
@@ -242,7 +260,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             for (int it = 0; ok && it < nkt && !*abort_flag; ++it) {
                 if (it + 1 < nkt && !scores(it + 1)) { ok = false; break; }
                 const int st = it & 1;
-                if (!mbar_wait(&p_ready[st], (it >> 1) & 1)) { ok = false; break; }
+                if (!lt_wait(&p_ready[st], (it >> 1) & 1, abort_flag)) { ok = false; break; }
                 lt_fence_after();
                 const uint32_t vt = smem_u32(sK + (st * wb + v0) * LT_KBLOCK);
 #pragma unroll
@@ -253,6 +271,12 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 lt_commit(&pv_done[st]);
             }
             if (!ok) { *abort_flag = 1; atomicExch(err, 1); }
+            // The block keeps its shared and tensor memory until the products that use them are done: a commit covers all
+            // that this lane has issued, those of a step that was broken off too.
+            if (issued) {
+                lt_commit(mma_done);
+                if (!mbar_wait(mma_done, 0)) atomicExch(err, 1);
+            }
         }
     } else {
         const int qd = warp & 3;                           // lanes of tensor memory this warp may read
@@ -267,7 +291,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int it = 0; it < nkt; ++it) {
             const int st = it & 1;
             if (__any_sync(0xffffffffu, *abort_flag != 0)) { ok = false; break; }
-            bool w = mbar_wait(&s_full[st], (it >> 1) & 1);
+            bool w = it != give_up_at && lt_wait(&s_full[st], (it >> 1) & 1, abort_flag);
             if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
             lt_fence_after();
             float s[32];
@@ -303,7 +327,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             l = l * corr + ((rs4[0] + rs4[1]) + (rs4[2] + rs4[3]));
             // only a rescale needs the product of the tile before to be done (it adds into O)
             if (it > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
-                w = mbar_wait(&pv_done[(it - 1) & 1], ((it - 1) >> 1) & 1);
+                w = lt_wait(&pv_done[(it - 1) & 1], ((it - 1) >> 1) & 1, abort_flag);
                 if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
                 lt_fence_after();
 #pragma unroll 1
@@ -327,7 +351,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if (lane == 0) lt_arrive(&p_ready[st]);
         }
         if (ok) {
-            const bool w = mbar_wait(&pv_done[(nkt - 1) & 1], ((nkt - 1) >> 1) & 1);
+            const bool w = lt_wait(&pv_done[(nkt - 1) & 1], ((nkt - 1) >> 1) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, w);
         }
         if (!ok) {
@@ -401,9 +425,11 @@ LUMEN_API int lumen_attn_latent_tc_takes(int W, int dv) {
 
 // q bfloat16 [N, H, W]; cache bfloat16 [n_pages, 1, PAGE, W] (plain tiles), both 16-byte aligned; out float32 [N, H, dv];
 // cu_q, seq_start, window as in lumen_attn_latent; n_tiles >= the sum over sequences of ceil(q_len H / 128).
+// give_up_at: the key tile of a block at which its softmax takes the wait for its scores as run out (-1: none; for tests of
+// what a block does then).
 LUMEN_API int lumen_attn_latent_tc(const void* q, const void* cache, int n_pages, const int* block_table, int bt_stride,
                                    const int* cu_q, const int* seq_start, int B, int n_tiles, float* out, int N, int H,
-                                   int W, int dv, int window, float scale, int* err, cudaStream_t stream) {
+                                   int W, int dv, int window, float scale, int give_up_at, int* err, cudaStream_t stream) {
     if (B <= 0 || n_tiles <= 0 || N <= 0) return 0;
     if (H <= 0 || window < 0 || !(scale > 0.0f) || !lumen_attn_latent_tc_takes(W, dv)) return LUMEN_ERR_UNSUPPORTED;
     if ((long long)N * H > 2147483647LL || (long long)n_pages * LUMEN_PAGE > 2147483647LL) return LUMEN_ERR_UNSUPPORTED;
@@ -417,7 +443,7 @@ LUMEN_API int lumen_attn_latent_tc(const void* q, const void* cache, int n_pages
     cudaError_t e = cudaFuncSetAttribute(attn_latent_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     lumen_launch(attn_latent_tc_kernel, dim3(n_tiles, (dv + LT_SLICE - 1) / LT_SLICE), dim3(LT_THREADS), smem, stream, mq, mk,
-                 block_table, bt_stride, cu_q, seq_start, B, out, H, W, dv, window, scale * 1.4426950408889634f, err);
+                 block_table, bt_stride, cu_q, seq_start, B, out, H, W, dv, window, scale * 1.4426950408889634f, give_up_at, err);
     LUMEN_LAUNCH_CHECK();
     return 0;
 }

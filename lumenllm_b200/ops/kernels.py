@@ -1042,9 +1042,9 @@ def attn_latent(q, cache, block_table, cu_q, seq_start, q_lens, value_dim, windo
     out = torch.empty((N, H, int(value_dim)), dtype=F32, device=q.device)
     if tc:
         f = fn("attn_latent_tc", "lumen_attn_latent_tc",
-               [P, P, c_int, P, c_int, P, P, c_int, c_int, P, c_int, c_int, c_int, c_int, c_int, c_float, P, P])
+               [P, P, c_int, P, c_int, P, P, c_int, c_int, P, c_int, c_int, c_int, c_int, c_int, c_float, c_int, P, P])
         check(f(ptr(q), ptr(cache), cache.shape[0], ptr(block_table), block_table.stride(0), ptr(cu_q), ptr(seq_start), B,
-                n_tiles, ptr(out), N, H, W, int(value_dim), int(window), float(scale), ptr(error_flag(q.device)),
+                n_tiles, ptr(out), N, H, W, int(value_dim), int(window), float(scale), -1, ptr(error_flag(q.device)),
                 stream_ptr()), "attn_latent_tc")
         return out
     part = torch.empty((n_split, N * H, int(value_dim) + 2), dtype=F32, device=q.device) if n_split > 1 else None

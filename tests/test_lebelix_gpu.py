@@ -828,6 +828,36 @@ def test_a_latent_row_is_the_same_bits_in_any_step(H, W, dv, window):
     K.check_error_flags()
 
 
+@pytest.mark.parametrize("H,W,dv", [(16, 576, 512), (4, 64, 64), (3, 448, 384)])
+def test_a_latent_block_that_gives_up_leaves_cleanly(H, W, dv):
+    """The softmax of every block takes one of its waits as run out, at the first key tile or at a later one, while
+    products and copies of the block are under way: the launch ends, the flag is raised, and launches right behind it
+    on the same stream, whose blocks get the same shared and tensor memory, give the bits they gave before."""
+    from lumenllm_b200.ops import kernels as K
+    from lumenllm_b200.ops.native import check, fn, ptr, stream_ptr
+    from ctypes import c_float, c_int, c_void_p as P_
+    lens, starts = [150, 300, 3], [0, 100, 260]
+    table, cache, _, q = _latent_case(lens, starts, H, W, seed=34)
+    q, cache, table = torch.cat(q).to(BF16).cuda(), cache.to(BF16).cuda(), table.cuda()
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32).cuda()
+    st = torch.tensor(starts, dtype=torch.int32).cuda()
+    good = lambda: K.attn_latent(q, cache, table, cu, st, lens, dv, 0, 0.2)
+    before = good()
+    K.check_error_flags()
+    f = fn("attn_latent_tc", "lumen_attn_latent_tc",
+           [P_, P_, c_int, P_, c_int, P_, P_, c_int, c_int, P_, c_int, c_int, c_int, c_int, c_int, c_float, c_int, P_, P_])
+    out = torch.empty_like(before)
+    tiles = sum((n * H + 127) // 128 for n in lens)
+    for at in (0, 1, 2, 5):
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        check(f(ptr(q), ptr(cache), cache.shape[0], ptr(table), table.stride(0), ptr(cu), ptr(st), len(lens), tiles,
+                ptr(out), sum(lens), H, W, dv, 0, 0.2, at, ptr(err), stream_ptr()), "attn_latent_tc")
+        after = [good() for _ in range(3)]
+        assert int(err.item()) == 1
+        assert all(torch.equal(a, before) for a in after)
+    K.check_error_flags()
+
+
 @pytest.mark.parametrize("n", [66, 96, 300])
 def test_a_captured_prompt_of_latent_layers_equals_the_eager_one(n, tmp_path):
     """Latent layers whose rows are whole 64-value blocks (16 heads): a prompt replayed from a graph, where padding
