@@ -1213,7 +1213,7 @@ add_shaped_rmsnorm_kernel(float* __restrict__ h, const ShapedGroups gr, const fl
     }
 }
 
-// The same for a row that fits the block's threads, four values each, and up to two groups that are not picked from
+// The same for few rows that fit a block's threads, four values each, and up to two groups that are not picked from
 // places: decode steps, where the time is one round trip after another. The weights are in registers before the
 // wait, the first eight (rows beyond 2,048: four) partial sums of both groups are under way at once, two normed groups share a reduction, and x
 // stays in registers. Every sum has the order of the kernel above. Four rows of 2,048: 5.5 -> 3.8 us alone.
@@ -1353,8 +1353,15 @@ LUMEN_API int lumen_add_shaped_rmsnorm(float* h, const void* const* ptrs, const 
     const size_t smem = (size_t)H * (1 + normed) * sizeof(float);
     if (smem > 200 * 1024) return LUMEN_ERR_UNSUPPORTED;
     const int threads = row_threads(vec ? H / 4 : H, n_rows);
-    // few rows of at most 4,096 and up to two groups: a row in the registers of one block
-    if (vec && 4 * threads >= H && n_groups <= 2 && !gr.place[0] && !gr.place[1]) {
+    // Few rows of at most 4,096 and up to two groups: a row in the registers of one block. Few: the blocks run all at
+    // once, which is one an SM above 256 threads and two up to that; a second round costs what the first does, where the
+    // general kernel's lighter blocks fill up (us, general / row kernel, two normed groups of four partial sums: 148 rows of
+    // 2,048 5.3 / 4.1, 149 rows 5.5 / 6.2; 295 rows of 1,024 5.2 / 3.7, 400 rows 5.8 / 6.1; one group without a norm, 2,048 rows
+    // of 1,024: 9.0 / 15.0). Beyond 2,048 values a block needs two groups and a norm or several partial sums of them to gain
+    // (four rows of 4,096, one partial sum of one group 3.3 / 3.8, of two groups 3.7 / 3.9; two groups with a norm 5.7 / 4.9).
+    const int at_once = threads > 256 ? 148 : 2 * 148 - 1;        // row_threads gives 256 from 296 rows on
+    if (vec && 4 * threads >= H && n_groups <= 2 && !gr.place[0] && !gr.place[1] && n_rows <= at_once &&
+        (H <= 2048 || (n_groups == 2 && (normed || gr.S[0] + gr.S[1] > 2)))) {
 #define ROW_GO(T, M)                                                                                                     \
     lumen_launch(add_shaped_rmsnorm_row_kernel<T, M>, dim3(n_rows), dim3(threads), 0, stream, h, gr, wn, eps_n, (T*)y, rows, \
                  H, write_h)

@@ -198,6 +198,34 @@ def test_few_rows_of_up_to_two_shaped_updates(normed, width):
                 assert not out[:, width:].any()
 
 
+@pytest.mark.parametrize("width,few,many", [(2048, 148, 149), (2048, 5, 290), (1024, 295, 296), (1024, 64, 600), (4096, 148, 150),
+                                            (1536, 100, 200)])
+@pytest.mark.parametrize("groups", [0, 1, 2])
+def test_shaped_updates_of_few_and_of_many_rows_give_the_same_bits(groups, width, few, many):
+    """The kernel that holds a row in one block's registers takes as many rows as run at once, the general one any
+    number: on both sides of that line a row's result is the same, and right."""
+    from lumenllm_b200.ops import kernels as K
+    g = torch.Generator().manual_seed(width + many)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    h, w = rn(many, width), 1 + 0.1 * rn(width)
+    gs = [(rn(3, many, width), 0.5, rn(width), 1 + 0.1 * rn(width), 1e-5), (rn(9, many, width), -1.25, None, None, 0.0)][:groups]
+
+    def run(n):
+        dev = [(d[:, :n].contiguous().cuda(), s, c if c is None else c.cuda(), nw if nw is None else nw.cuda(), eps) for d, s, c, nw, eps in gs]
+        hd = h[:n].clone().cuda()
+        return K.add_shaped_rmsnorm(hd, dev, w.cuda(), 1e-6, F32).cpu(), hd.cpu()
+
+    (ya, ha), (yb, hb) = run(few), run(many)
+    assert torch.equal(ya, yb[:few]) and torch.equal(ha, hb[:few])
+    x = h
+    for d, s, c, nw, eps in gs:
+        d = d.sum(0)
+        d = P.rms_norm(d, nw, eps) if nw is not None else d
+        x = x + s * (d if c is None else c * d)
+    close(hb, x, F32, "stream")
+    close(yb, P.rms_norm(x, w, 1e-6), F32, "norm")
+
+
 def test_dynamic_tanh_takes_a_shaped_update():
     """The other norm, behind a layer whose updates have factors a column."""
     from lumenllm_b200.config.spec import PartSpec
