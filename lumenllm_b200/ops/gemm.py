@@ -54,16 +54,31 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, split_ok: bool = False, add_to=N
     return part if split_ok else part.sum(dim=0)
 
 
+def gate_up_in_one(rows: int, width: int, k: int) -> bool:
+    """Whether a gate/up product [rows, k] x [width, k]^T goes through its activation in the product's epilogue. Up to 128 rows
+    the product streams the weights with k split, which the epilogue cannot have (at 100 rows of the 8B shape 41 + 6 us against
+    56 us), and up to 255 its one row of tiles is part empty (160 rows: 57 us and the activation behind it against 73); 256 rows
+    fill it, and more than 512 have tiles enough. Between, two things count. Below 56
+    tiles of 256 x 256 the float32 product can split k over idle SMs, which pays for long k and few tiles; from
+    56 on the two-SM kernel's epilogue, with its divisions, is longer than that of the float32 sums, which shows where k is
+    short or the last round of tiles is not full. us, one kernel / two, width x k:
+    300 rows 1,024 x 1,024 7.7 / 9.3; 6,144 x 1,024 10.4 / 18.5; 4,096 x 2,048 14.0 / 15.5; 2,816 x 2,048 12.9 / 16.9;
+    1,024 x 4,096 21.1 / 13.9; 4,096 x 4,096 23.4 / 19.4; 4,096 x 8,192 42.6 / 28.5; 6,144 x 8,192 45.2 / 41.8;
+    8,192 x 1,024 18.4 / 15.8; 16,384 x 1,024 29.1 / 24.0; 10,240 x 2,048 33.4 / 31.3; 16,384 x 2,048 35.0 / 35.1;
+    24,576 x 4,096 78.2 / 82.8; 448 rows 12,288 x 4,096 53.8 / 56.3, 8,192 x 4,096 33.9 / 32.3."""
+    if rows <= 256 or rows > 512:
+        return rows >= 256
+    tiles = (rows + 255) // 256 * ((width + 255) // 256)
+    if tiles >= 56:
+        return k >= 2048 and (tiles >= 128 or (tiles >= 80 and rows > 352))
+    return k <= 2048 or (tiles >= 36 and k <= 6144) or K.gemm_tc_splits(rows, width, k) == 1
+
+
 def gemm_gate_up_silu(x: torch.Tensor, w_interleaved, act="silu"):
     """silu(gate) * up (or, `act` "gelu", gelu_tanh(gate) * up) in bfloat16 [M, I] from x [M, K] and a weight [2I, K] whose rows
-    alternate gate_i, up_i, in ONE kernel where that is the faster way; else None, and the
-    caller takes the float32 product with the activation kernel behind it. One kernel: from 256
-    rows on. Below: up to 128 rows the product streams the weights with k split, which the epilogue
-    cannot have (at 100 rows of the 8B shape 41 + 6 us against 56 us); from 129 to 255 rows the two-SM
-    kernel's one row of tiles is part empty, and the split product is no slower (160 rows: 57 us and the
-    activation behind it against 73; 300 rows: 89 us in one kernel, where the product alone takes that)."""
-    rows = x.shape[0]
-    if rows >= 256 and takes_tc(x, w_interleaved):
+    alternate gate_i, up_i, in ONE kernel where that is the faster way (gate_up_in_one); else None, and the
+    caller takes the float32 product with the activation kernel behind it."""
+    if takes_tc(x, w_interleaved) and gate_up_in_one(x.shape[0], w_interleaved.shape[0], x.shape[1]):
         return K.gemm_tc(x if x.is_contiguous() else x.contiguous(), w_interleaved,
                          silu_interleaved=True, act=act)
     return None

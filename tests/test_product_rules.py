@@ -1,0 +1,25 @@
+"""Which products of a layer go through their activation in the product's own kernel: a rule on sizes."""
+import pytest
+
+
+@pytest.mark.parametrize("rows,width,k,one", [
+    # measured on both sides (one kernel against the product with the activation kernel behind it)
+    (257, 1024, 1024, True), (448, 2048, 1024, True), (384, 6144, 1024, True), (300, 2816, 2048, True), (320, 4096, 2048, True),
+    (320, 1024, 4096, False), (257, 4096, 4096, False), (320, 4096, 8192, False), (448, 2048, 8192, False), (257, 6144, 8192, False),
+    (320, 6912, 8192, True), (448, 5120, 8192, True), (384, 6144, 4096, True),
+    (257, 8192, 1024, False), (448, 8192, 4096, False), (384, 10240, 1024, False), (257, 10240, 2048, False), (448, 12288, 4096, True),
+    (448, 24576, 1024, False), (320, 16384, 2048, True), (300, 24576, 4096, True),
+    # whole tiles, and few rows
+    (256, 24576, 4096, True), (512, 4096, 8192, False), (511, 1024, 4096, False), (2048, 4096, 1024, True), (513, 4096, 8192, True), (128, 24576, 4096, False), (255, 24576, 4096, False),
+    (1, 24576, 4096, False)])
+def test_gate_up_products_with_their_activation_in_one_kernel(rows, width, k, one):
+    from lumenllm_b200.ops.gemm import gate_up_in_one
+    assert gate_up_in_one(rows, width, k) == one
+
+
+@pytest.mark.parametrize("width,k", [(512, 4096), (4096, 8192), (5120, 8192), (10240, 2048), (24576, 4096), (16384, 1024)])
+def test_a_captured_prompts_rows_take_the_way_of_the_eager_ones(width, k):
+    """A captured step rounds its rows up to a multiple of 32 and must give the bits of the eager one."""
+    from lumenllm_b200.ops.gemm import gate_up_in_one
+    for rows in range(257, 700):
+        assert gate_up_in_one(rows, width, k) == gate_up_in_one((rows + 31) // 32 * 32, width, k), rows
