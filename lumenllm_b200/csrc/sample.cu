@@ -11,17 +11,21 @@
 // order in which threads add: the same logits, options and u give the same
 // token in any batch.
 //
-// Three routes give the same answer. All start from the row's largest value. With top-k up to QCAP the list
-// route counts the row's elements in bins linear in (max - logit) / temperature (2,048 bins over 32 units,
+// Three routes give the same answer. All start from the row's largest value. With top-k up to QCAP (without a
+// later filter: QLIST_PLAIN) the list route counts the row's elements in bins linear in (max - logit) / temperature (2,048 bins over 32 units,
 // monotone in the logit, so a bin is a run of the rank order), gathers the elements of every bin up to the one
 // in which the k-th falls (k and a few as a rule) into one list, orders it by (logit down, index up) and does
 // top-p, min-p and the draw on the list's running weights: two passes over the row besides the maximum, and no
 // weight but the list's.
-// 8 rows of 151,936 with k = 50 and top-p: 64 us by the quick route, 23 by the list; 64 rows: 115 and 37.
-// The quick route, without top-k, bins the row once in the same way, with the exact weight of every bin (and the count, for a top-k beyond
-// the list); each selection then scans the bins, gathers the few hundred elements of the bin in which the target falls,
+// The list's ordering compares every two of its elements and takes a second round of the block's threads beyond 1,024, so a
+// k near that pays only where a later filter would cost the quick route a selection more. us a launch, rows of 151,936,
+// top-k alone / with top-p 0.9 / with min-p too: 8 rows by the quick route, whatever k, 45 / 57 / 69; by the list k = 50
+// 20 / 21 / 21, 500 28 / 28 / 28, 992 47 / 47 / 47, 1,024 56 / 57 / 57. 64 rows: quick 67 / 80 / 100, list k = 50 33 / 34 / 34,
+// 992 63 / 63 / 63, 1,024 73 / 73 / 74.
+// The quick route, for all else, bins the row once in the same way, with the exact weight of every bin (and the count, where there is a
+// top-k); each selection then scans the bins, gathers the few hundred elements of the bin in which the target falls,
 // orders them by (logit down, index up) and walks them. The radix descent over the keys is
-// the route for everything the others decline: min-p, a bin too full to gather (long runs
+// the route for everything the others decline: a bin too full to gather (long runs
 // of equal or nearly equal logits), a target in the last, open-ended bin.
 #include <cooperative_groups.h>
 #include <cstdint>
@@ -356,6 +360,7 @@ __global__ void argmax_final_kernel(const float* __restrict__ part_v, const int*
 #define QCMD_GATHER 1
 #define QCMD_MINKEY 2
 #define QLIST 2048         // elements the list route can hold: QCAP of top-k and a bin of QCAP
+#define QLIST_PLAIN 992    // largest top-k that goes by the list where no top-p and no min-p follows
 
 struct Quick {
     union {
@@ -821,7 +826,8 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
     // Every block: bin table of its share.
     for (int b = threadIdx.x; b < QB; b += blockDim.x) { quick.mass[b] = 0ull; quick.cnt[b] = 0u; }
     __syncthreads();
-    const bool by_list = top_k > 0 && top_k <= QCAP;
+    const bool filtered = (top_p > 0.0f && top_p < 1.0f) || min_p > 0.0f;
+    const bool by_list = top_k > 0 && top_k <= (filtered ? QCAP : QLIST_PLAIN);
     if (by_list) {
         int beg, end;
         row_share(V, rank, qc, &beg, &end);

@@ -796,6 +796,24 @@ def test_sampler_lists_of_every_length(V):
         assert _sample_rows(lg[:n], opts[:n], ks[:n]) == got[:n]
 
 
+@pytest.mark.parametrize("V", [1500, 151936])
+def test_top_k_alone_at_the_end_of_the_lists(V):
+    """Where top-k stands alone it goes by the list up to 992 and by the quick route beyond; a min-p that drops only
+    elements without weight keeps it on the list. Both give the same token."""
+    g = gen(71)
+    rows, opts, ks = [], [], []
+    for k in (991, 992, 993, 1008, 1024, 1025):
+        for temp, u in ((0.7, 0.03), (1.3, 0.5), (3.0, 0.999)):
+            rows.append(torch.randn(V, generator=g) * 2.5)
+            opts.append([temp, 1.0, 0.0, u])
+            ks.append(k)
+    lg = torch.stack(rows)
+    got = _sample_rows(lg, opts, ks)
+    assert got == _sample_rows(lg, [[t, 1.0, 1e-30, u] for t, _, _, u in opts], ks)
+    for r, (tok, o, k) in enumerate(zip(got, opts, ks)):
+        assert tok in _acceptable(lg[r], o[0], k, o[1], o[2], o[3]), (r, o, k, tok)
+
+
 def test_products_of_drawn_shapes_through_the_router():
     """Shapes drawn from a fixed seed across every regime of the product's routing
     (weight-streaming tcgen05 orientation with k split, single-SM tiles with
