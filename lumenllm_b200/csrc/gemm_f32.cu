@@ -1,8 +1,8 @@
 // True 32-bit matrix product C[M,N] = A[M,K] * W[N,K]^T with plain FFMA: no
 // tensor core, no TF32, no library. Each output element is summed over k in four
-// interleaved chains, each in ascending order (where rows are not a multiple of 16 bytes: in
-// one), whatever the tile, so the value of C[m,n] depends on row m of A
-// and row n of W only, never on M or on the other rows of the batch.
+// interleaved chains (of every 64 columns chain g takes the 16 from 16 g on), each in ascending order, that
+// are added as (c0 + c1) + (c2 + c3), in every kernel and tile here, so the value of C[m,n] depends on row m of A
+// and row n of W only, never on M, on the other rows of the batch, or on where the operands lie in memory.
 // W may be stored in float32 or in bfloat16 (widened exactly on load).
 //
 // What bounds it: the FMA pipe for many rows (128 products a cycle and SM, which take the two-product instruction:
@@ -21,8 +21,10 @@
 #define BM 64
 #define BN 64
 #define BK 16
+#define GK 4             // chains an output is summed in
 
-template <typename TW>
+// NG: chains that are not empty (four, or as many as a K of up to 32 has).
+template <typename TW, int NG>
 __global__ void __launch_bounds__(256)
 gemm_f32_kernel(const float* __restrict__ A, const TW* __restrict__ W, float* __restrict__ C, int M,
                 int N, int K) {
@@ -32,36 +34,43 @@ gemm_f32_kernel(const float* __restrict__ A, const TW* __restrict__ W, float* __
     __shared__ float Ws[BK][BN + 4];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[4][4];
+    float acc[NG][4][4];                       // chain g: the columns 16 g to 16 g + 15 of every 64
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int g = 0; g < NG; ++g)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[g][i][j] = 0.0f;
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // 64x16 tile of each operand, 4 elements a thread, k fastest in memory.
+    for (int kb = 0; kb < K; kb += GK * BK) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int idx = threadIdx.x + i * 256;  // 0..1023
-            const int r = idx >> 4, kk = idx & 15;
-            const int gm = m0 + r, gn = n0 + r, gk = k0 + kk;
-            As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * K + gk] : 0.0f;
-            Ws[kk][r] = (gn < N && gk < K) ? to_f32(W[(size_t)gn * K + gk]) : 0.0f;
+        for (int g = 0; g < NG; ++g) {
+            const int k0 = kb + g * BK;
+            if (k0 >= K) break;
+            // 64x16 tile of each operand, 4 elements a thread, k fastest in memory.
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int idx = threadIdx.x + i * 256;  // 0..1023
+                const int r = idx >> 4, kk = idx & 15;
+                const int gm = m0 + r, gn = n0 + r, gk = k0 + kk;
+                As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * K + gk] : 0.0f;
+                Ws[kk][r] = (gn < N && gk < K) ? to_f32(W[(size_t)gn * K + gk]) : 0.0f;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int kk = 0; kk < BK; ++kk) {
+                float a[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) b[j] = Ws[kk][tx * 4 + j];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[g][i][j] = fmaf(a[i], b[j], acc[g][i][j]);
+            }
+            __syncthreads();
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Ws[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -70,7 +79,8 @@ gemm_f32_kernel(const float* __restrict__ A, const TW* __restrict__ W, float* __
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int gn = n0 + tx * 4 + j;
-            if (gn < N) C[(size_t)gm * N + gn] = acc[i][j];
+            const float c01 = NG > 1 ? acc[0][i][j] + acc[NG > 1][i][j] : acc[0][i][j];
+            if (gn < N) C[(size_t)gm * N + gn] = NG > 2 ? c01 + (acc[NG > 2 ? 2 : 0][i][j] + acc[NG > 2 ? 3 : 0][i][j]) : c01;
         }
     }
 }
@@ -100,7 +110,6 @@ __device__ __forceinline__ unsigned long long twice(float x) {
 // piece c of row r lies at c ^ (r & 7), piece c of pair q at c ^ (q & 7): what eight lanes read at one k, and what
 // eight lanes write, touches every bank once.
 #define TK 64
-#define GK 4
 template <typename TW, int WM, int WN, int TM, int TN, int MINB>
 __global__ void __launch_bounds__(GK * WM * WN * 32, MINB)
 gemm_f32_tiled_kernel(const float* __restrict__ A, const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K) {
@@ -241,7 +250,10 @@ static int gemm_f32_go(const float* A, const TW* W, float* C, int M, int N, int 
     if ((M + BM - 1) / BM > 65535) return LUMEN_ERR_UNSUPPORTED;
     const bool vec = (K & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
     if (!vec) {
-        lumen_launch(gemm_f32_kernel<TW>, dim3((N + BN - 1) / BN, (M + BM - 1) / BM), dim3(256), 0, stream, A, W, C, M, N, K);
+        const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+        if (K <= BK) lumen_launch(gemm_f32_kernel<TW, 1>, grid, dim3(256), 0, stream, A, W, C, M, N, K);
+        else if (K <= 2 * BK) lumen_launch(gemm_f32_kernel<TW, 2>, grid, dim3(256), 0, stream, A, W, C, M, N, K);
+        else lumen_launch(gemm_f32_kernel<TW, GK>, grid, dim3(256), 0, stream, A, W, C, M, N, K);
         LUMEN_LAUNCH_CHECK();
         return 0;
     }

@@ -500,6 +500,31 @@ def test_gemm_f32_tiles(wdtype, M, N, K_):
     assert torch.equal(one[0], out[M // 2])
 
 
+@pytest.mark.parametrize("wdtype", [F32, BF16])
+@pytest.mark.parametrize("M,N,K_", [(5, 40, 4), (20, 33, 60), (70, 65, 132), (33, 64, 2052), (300, 100, 36), (9, 70, 1000)])
+def test_gemm_f32_adds_in_one_order_wherever_the_operands_lie(wdtype, M, N, K_):
+    """Operands that start on no 16-byte boundary, and rows of odd lengths, go to a kernel of their own: the same
+    bits as from aligned copies, and as with zeros added behind every row."""
+    from lumenllm_b200.ops import kernels as K
+    g = gen(19)
+    a, w = dev(torch.randn(M, K_, generator=g)), dev(torch.randn(N, K_, generator=g).to(wdtype))
+    ref = K.gemm_f32(a, w)
+
+    def moved(t):                                          # the same numbers one element further on
+        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+        buf[1:] = t.reshape(-1)
+        return buf[1:].view(t.shape)
+    for aa, ww in ((moved(a), w), (a, moved(w)), (moved(a), moved(w))):
+        assert torch.equal(K.gemm_f32(aa, ww), ref)
+    assert torch.equal(K.gemm_f32(a[:3].contiguous(), w), ref[:3])
+    wide = torch.cat([a, torch.zeros(M, 132, device=a.device)], 1), torch.cat([w, torch.zeros(N, 132, device=w.device, dtype=w.dtype)], 1)
+    assert torch.equal(K.gemm_f32(*wide), ref)
+    odd = K.gemm_f32(a[:, :K_ - 1].contiguous(), w[:, :K_ - 1].contiguous())          # K no multiple of 4
+    a[:, -1] = 0
+    w[:, -1] = 0
+    assert torch.equal(odd, K.gemm_f32(a, w))
+
+
 @pytest.mark.parametrize("M,N,K_", [(128, 256, 64), (200, 300, 320), (2048, 1024, 4096), (1, 256, 64),
                                     (8, 4096, 4096), (19, 311, 80), (33, 1000, 1000), (64, 6144, 1024),
                                     (65, 130, 72), (130, 17, 1000), (16, 151936 // 4 + 8, 256)])
