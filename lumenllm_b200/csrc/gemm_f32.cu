@@ -249,7 +249,12 @@ template <typename TW>
 static int gemm_f32_go(const float* A, const TW* W, float* C, int M, int N, int K, cudaStream_t stream) {
     if ((M + BM - 1) / BM > 65535) return LUMEN_ERR_UNSUPPORTED;
     const bool vec = (K & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
-    if (!vec) {
+    // More than 32 short rows go to the small-tile kernel: the large tiles' ring, four groups and their sums pay from some steps
+    // of 64 columns on (us, small / large tiles: 300 x 4,096 x 16 6.4 / 13.9, 4,000 x 4,096 x 16 32 / 120, 33 x 64 x 32 3.1 / 5.1,
+    // 1,000 x 1,000 x 48 8.9 / 10.0, 4,000 x 4,096 x 64 91 / 121, but 300 x 4,096 x 64 16.4 / 14.0). The same sums either way.
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    const bool is_short = M > 32 && (K <= 48 || (K <= 64 && tiles >= 512));
+    if (!vec || is_short) {
         const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
         if (K <= BK) lumen_launch(gemm_f32_kernel<TW, 1>, grid, dim3(256), 0, stream, A, W, C, M, N, K);
         else if (K <= 2 * BK) lumen_launch(gemm_f32_kernel<TW, 2>, grid, dim3(256), 0, stream, A, W, C, M, N, K);

@@ -501,10 +501,11 @@ def test_gemm_f32_tiles(wdtype, M, N, K_):
 
 
 @pytest.mark.parametrize("wdtype", [F32, BF16])
-@pytest.mark.parametrize("M,N,K_", [(5, 40, 4), (20, 33, 60), (70, 65, 132), (33, 64, 2052), (300, 100, 36), (9, 70, 1000)])
+@pytest.mark.parametrize("M,N,K_", [(5, 40, 4), (20, 33, 60), (70, 65, 132), (33, 64, 2052), (300, 100, 36), (9, 70, 1000), (16, 31, 16),
+                                    (31, 32, 32), (40, 65, 64), (1000, 2100, 64)])
 def test_gemm_f32_adds_in_one_order_wherever_the_operands_lie(wdtype, M, N, K_):
-    """Operands that start on no 16-byte boundary, and rows of odd lengths, go to a kernel of their own: the same
-    bits as from aligned copies, and as with zeros added behind every row."""
+    """Operands that start on no 16-byte boundary, rows of odd lengths, and more than 32 short rows go to a kernel of
+    their own: the same bits as from aligned copies, as with zeros added behind every row, and as from few rows."""
     from lumenllm_b200.ops import kernels as K
     g = gen(19)
     a, w = dev(torch.randn(M, K_, generator=g)), dev(torch.randn(N, K_, generator=g).to(wdtype))
