@@ -126,9 +126,9 @@ delta_prepare_kernel(const float* __restrict__ x, int C, int q_col, int k_col,
 
 // NS: threads that share a column of S (a power of two), NS DR_ROWS >= d; every offset of the walk is a constant
 // of the instance. AHEAD: a token's rows are read from shared memory while the one before is worked on, which
-// takes twice the registers: for steps of several tokens a sequence. Same sums either way.
-template <int NS, bool AHEAD>
-__global__ void __launch_bounds__(DR_THREADS)
+// takes twice the registers: for steps of several tokens a sequence. THREADS: of a block. Same sums either way.
+template <int NS, bool AHEAD, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __restrict__ prep,
                   float* __restrict__ state, size_t slot_stride, const int* __restrict__ cu_q,
                   const int* __restrict__ seq_slot, float* __restrict__ y, int H, int d, int dv, int vec) {
@@ -139,7 +139,7 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
     constexpr int dp = NS * ROWS;                   // d padded to what the threads of a column hold
     constexpr int GR = ROWS / 4;
     constexpr int PW = 3 * dp + 4;
-    constexpr int cols = DR_THREADS / NS;
+    constexpr int cols = THREADS / NS;
     float* rows = sm;                               // [2][DR_CHUNK][PW]
     float* vs = sm + 2 * DR_CHUNK * PW;             // [2][DR_CHUNK][cols]
     const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
@@ -170,12 +170,12 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
         const int nt = min(DR_CHUNK, t_end - t0);
         constexpr int pieces = PW / 4;
         float* rb = rows + buf * DR_CHUNK * PW;
-        for (int i = tid; i < nt * pieces; i += DR_THREADS) {
+        for (int i = tid; i < nt * pieces; i += THREADS) {
             const int tt = i / pieces, p = i - tt * pieces;
             dr_cp16(rb + tt * PW + 4 * p, prep + ((size_t)(t0 + tt) * H + h) * PW + 4 * p);
         }
         float* vb = vs + buf * DR_CHUNK * cols;
-        for (int i = tid; i < nt * cols; i += DR_THREADS) {
+        for (int i = tid; i < nt * cols; i += THREADS) {
             const int tt = i / cols, c = i - tt * cols, jj = blockIdx.z * cols + c;
             if (jj < dv) dr_cp4(vb + i, x + (size_t)(t0 + tt) * C + v_col + h * dv + jj);
             else vb[i] = 0.0f;
@@ -333,7 +333,12 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
     if (q_col < 0 || k_col < 0 || v_col < 0 || q_col + G * d > C || k_col + G * d > C || v_col + H * dv > C ||
         b_col < 0 || b_col + H > uW || !prep)
         return LUMEN_ERR_BAD_ARGUMENT;
-    const int NS = delta_rule_threads(d), cols = DR_THREADS / NS, dp = NS * DR_ROWS;
+    const int NS = delta_rule_threads(d), dp = NS * DR_ROWS;
+    // Heads wider than 256 leave a block of 128 threads four columns to share a staged row: right while every block has an SM,
+    // else twice as many (us, 128 / 256 threads, heads of 500 x 64: one sequence of 2,048 tokens, 64 blocks of 128, 629 / 821;
+    // four of 512 255 / 235; one token of 64 sequences 42 / 32, of 200 131 / 90).
+    const bool wide = NS == 32 && (long long)n_seqs * H * ((dv + DR_THREADS / NS - 1) / (DR_THREADS / NS)) > 148;
+    const int threads = wide ? 2 * DR_THREADS : DR_THREADS, cols = threads / NS;
     const int vec = (d & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
     dim3 pgrid(N, (H + DR_PREP_WARPS - 1) / DR_PREP_WARPS);
     if (pgrid.y > 65535) return LUMEN_ERR_UNSUPPORTED;
@@ -343,25 +348,27 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
     dim3 grid(n_seqs, H, (dv + cols - 1) / cols);
     if (grid.z > 65535) return LUMEN_ERR_UNSUPPORTED;
     const size_t smem = (size_t)2 * DR_CHUNK * (3 * dp + 4 + cols) * sizeof(float);
-#define DR_LAUNCH(S, A)                                                                                               \
+#define DR_LAUNCH(S, A, T)                                                                                            \
     do {                                                                                                              \
-        auto k = delta_rule_kernel<S, A>;                                                                              \
+        auto k = delta_rule_kernel<S, A, T>;                                                                           \
         if (smem > 48 * 1024) {                                                                                       \
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
             if (e != cudaSuccess) return (int)e;                                                                      \
         }                                                                                                             \
-        lumen_launch(k, grid, dim3(DR_THREADS), smem, stream, x, C, v_col, (const float*)prep, state,                 \
+        lumen_launch(k, grid, dim3(T), smem, stream, x, C, v_col, (const float*)prep, state,                 \
                      (size_t)slot_stride, cu_q, seq_slot, y, H, d, dv, vec);                                          \
     } while (0)
-    const bool ahead = N > n_seqs;
-#define DR_GO(S) case S: if (ahead) DR_LAUNCH(S, true); else DR_LAUNCH(S, false); break
+    // reading ahead takes twice the registers, and a second such block an SM is worth more (heads of 512 x 128, 8 a sequence, four
+    // sequences of 512 tokens: 845 us ahead, 750 not)
+    const bool ahead = N > n_seqs && !(wide && (long long)grid.x * grid.y * grid.z > 148);
+#define DR_GO(S, T) { if (ahead) DR_LAUNCH(S, true, T); else DR_LAUNCH(S, false, T); }
     switch (NS) {
-        DR_GO(1);
-        DR_GO(2);
-        DR_GO(4);
-        DR_GO(8);
-        DR_GO(16);
-        DR_GO(32);
+        case 1: DR_GO(1, DR_THREADS) break;
+        case 2: DR_GO(2, DR_THREADS) break;
+        case 4: DR_GO(4, DR_THREADS) break;
+        case 8: DR_GO(8, DR_THREADS) break;
+        case 16: DR_GO(16, DR_THREADS) break;
+        default: if (wide) DR_GO(32, 2 * DR_THREADS) else DR_GO(32, DR_THREADS)
     }
 #undef DR_GO
 #undef DR_LAUNCH

@@ -390,6 +390,32 @@ def test_delta_rule_head_sizes(d, dv):
         close(got, ref, F32)
 
 
+@pytest.mark.parametrize("tokens", [1, 19])
+@pytest.mark.parametrize("d,dv", [(257, 33), (512, 9), (300, 64)])
+def test_delta_rule_of_wide_heads_alone_and_among_many(d, dv, tokens):
+    """Heads wider than 256 go in blocks of four columns while every block has an SM, and of eight beyond: the same
+    bits for a sequence alone and among forty, with and without tokens to read ahead."""
+    from lumenllm_b200.ops import kernels as K
+    B, H = 40, 2
+    g = torch.Generator().manual_seed(d)
+    rn = lambda *s: torch.randn(*s, generator=g).cuda()
+    N, C = B * tokens, 2 * H * d + H * dv
+    x, u, a, dt, al, st = rn(N, C), rn(1, N, H), rn(1, N, H * d), rn(H * d), rn(H), rn(B, H, dv, d)
+
+    def run(b0, n):
+        s, rows_ = st[b0:b0 + n].clone(), slice(b0 * tokens, (b0 + n) * tokens)
+        y = K.delta_rule(x[rows_].contiguous(), 0, H * d, 2 * H * d, u[:, rows_].contiguous(), 0, a[:, rows_].contiguous(), dt, al, s,
+                         (torch.arange(n + 1, dtype=torch.int32) * tokens).cuda(), torch.arange(n, dtype=torch.int32).cuda(),
+                         n, H, H, d, dv)
+        return y, s
+
+    y, s = run(0, B)
+    assert torch.isfinite(y).all()
+    for b in (0, 17, B - 1):
+        yb, sb = run(b, 1)
+        assert torch.equal(yb, y[b * tokens:(b + 1) * tokens]) and torch.equal(sb, s[b:b + 1])
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_the_state_remembers_far_back_and_forgets_by_channel(dtype):
     """Decays close to one and one loud early token: what the state holds of that token decides the
