@@ -65,7 +65,12 @@ __device__ __forceinline__ void ag_block_reduce(float (&v)[NV], float (*red)[32]
 
 // VEC: rows of keys are read 16 bytes at a time (float32 plain tiles with d a multiple of 4, or swizzled tiles).
 // The products of a dot are added in the order of the key's numbers either way.
-template <typename T, typename TQ, int HB, bool VEC>
+// WIDE: four of a value row's numbers are read at a time instead of one and then the next for the whole page, so that more
+// of it is under way: float32 values beyond 384, where few blocks wait for memory (us, as the others / this: one token after
+// 1,000 keys, 16 sequences of 4 heads over one key head of 576 with values of 512: 981 / 651, of 4 heads of 512 1,126 / 774;
+// 300 tokens of 16 heads 440 / 284; 100 tokens of 8 heads of 384 after 1,000 562 / 672). The same sums. bfloat16 values gain
+// nothing by it.
+template <typename T, typename TQ, int HB, bool VEC, bool WIDE>
 __global__ void __launch_bounds__(AG_THREADS)
 attn_generic_kernel(const TQ* __restrict__ q, const T* __restrict__ kcache, const T* __restrict__ vcache,
                     const int* __restrict__ block_table, int bt_stride,
@@ -175,6 +180,21 @@ attn_generic_kernel(const TQ* __restrict__ q, const T* __restrict__ kcache, cons
                 const int r0 = j0 % LUMEN_PAGE, nr = min(LUMEN_PAGE - r0, last - j0 + 1);      // a run within a page
                 const T* vtile = vcache + ((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE * v_row;
                 const float* w = &ps[0][j0 - jbeg];
+                if (WIDE) {
+#pragma unroll 4
+                    for (int k = 0; k < nr; ++k) {
+                        float v[AG_ACC];
+#pragma unroll
+                        for (int i = 0; i < AG_ACC; ++i) {
+                            const int e = tid + i * AG_THREADS;
+                            v[i] = e < dv ? to_f32(vtile[tile_offset(v_layout, r0 + k, e, v_row)]) : 0.0f;
+                        }
+#pragma unroll
+                        for (int i = 0; i < AG_ACC; ++i)
+#pragma unroll
+                            for (int h = 0; h < HB; ++h) acc[h][i] = fmaf(w[h * AG_THREADS + k], v[i], acc[h][i]);
+                    }
+                } else
 #pragma unroll
                 for (int i = 0; i < AG_ACC; ++i) {
                     const int e = tid + i * AG_THREADS;
@@ -232,20 +252,21 @@ static int attn_generic_launch(const void* q, int q_is_f32, const void* kcache, 
     const int G = nq / nkv;
     int hb = 1;
     while (vec && hb < 4 && G % (2 * hb) == 0 && (long long)N * nq / (2 * hb) >= 2 * 148) hb *= 2;
-#define AG_GO(T, TQ, HB, VEC)                                                                                          \
-    lumen_launch(attn_generic_kernel<T, TQ, HB, VEC>, dim3(N, nq / HB), dim3(AG_THREADS), 0, stream, (const TQ*)q,     \
+#define AG_GO(T, TQ, HB, VEC, WIDE)                                                                                    \
+    lumen_launch(attn_generic_kernel<T, TQ, HB, VEC, WIDE>, dim3(N, nq / HB), dim3(AG_THREADS), 0, stream, (const TQ*)q, \
                  (const T*)kcache, (const T*)vcache, block_table, bt_stride, tok_seq, tok_pos, (TQ*)out, nq, nkv, d, dv, \
                  window, scale, layout, v_layout, opt)
-#define AG_PICK(T, TQ)                                                                                                 \
+#define AG_PICK(T, TQ, WIDE)                                                                                           \
     do {                                                                                                               \
-        if (!vec) AG_GO(T, TQ, 1, false);                                                                              \
-        else if (hb == 1) AG_GO(T, TQ, 1, true);                                                                       \
-        else if (hb == 2) AG_GO(T, TQ, 2, true);                                                                       \
-        else AG_GO(T, TQ, 4, true);                                                                                    \
+        if (!vec) AG_GO(T, TQ, 1, false, false);                                                                       \
+        else if (hb == 1) AG_GO(T, TQ, 1, true, WIDE);                                                                 \
+        else if (hb == 2) AG_GO(T, TQ, 2, true, WIDE);                                                                 \
+        else AG_GO(T, TQ, 4, true, WIDE);                                                                              \
     } while (0)
-    if (is_bf16 && !q_is_f32) AG_PICK(__nv_bfloat16, __nv_bfloat16);
-    else if (is_bf16) AG_PICK(__nv_bfloat16, float);
-    else AG_PICK(float, float);
+    if (is_bf16 && !q_is_f32) AG_PICK(__nv_bfloat16, __nv_bfloat16, false);
+    else if (is_bf16) AG_PICK(__nv_bfloat16, float, false);
+    else if (dv > 3 * AG_THREADS) AG_PICK(float, float, true);
+    else AG_PICK(float, float, false);
 #undef AG_PICK
 #undef AG_GO
     LUMEN_LAUNCH_CHECK();

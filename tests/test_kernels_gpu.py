@@ -197,6 +197,14 @@ def test_attention_generic(dtype, nq, nkv, d, window):
     assert float((out - ref).abs().max()) < tol
 
 
+@pytest.mark.parametrize("nq,nkv", [(8, 2), (4, 2), (3, 3)])
+@pytest.mark.parametrize("d,window", [(384, 0), (388, 50), (512, 0), (512, 33)])
+def test_attention_generic_with_wide_values(nq, nkv, d, window):
+    """float32 values beyond 384 numbers are read four at a time: on both sides of that line, one, two and four heads a
+    block, rows that end inside the last four."""
+    test_attention_generic(F32, nq, nkv, d, window)
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_attention_one_far_key_and_the_windows_edge(dtype):
     """One key among 700 is made to dominate: the output must be its value. With a window,
