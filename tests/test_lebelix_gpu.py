@@ -272,7 +272,10 @@ LATENTS = [latent(2, 8, 16, 24, 40, 0.2, size=11, rot=8),
            # divide a block's rows; a latent wider than 256; more heads than a block has rows
            latent(5, 16, 16, 32, 160, 0.2, size=45, rot=16),
            latent(3, 32, 32, 64, 320, 0.1, size=130, rot=32),
-           latent(70, 8, 16, 8, 48, 0.2, size=33, rot=8)]
+           latent(70, 8, 16, 8, 48, 0.2, size=33, rot=8),
+           # rows and values in whole 64-value blocks, whose prompts go by tcgen05: one and two slices of the value
+           latent(16, 16, 64, 8, 128, 0.2, size=70, rot=32),
+           latent(3, 32, 64, 24, 320, 0.1, rot=64)]
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
@@ -287,14 +290,15 @@ def test_latent_attention_part(m, dtype):
     close(got, ref, dtype)
 
 
+@pytest.mark.parametrize("d,r,D", [(48, 16, 64), (64, 64, 128)])          # the second: rows that go by tcgen05
 @pytest.mark.parametrize("decode", [False, True])
 @pytest.mark.parametrize("dtype", [F32, BF16])
-def test_one_loud_latent_at_every_edge_of_the_window(dtype, decode):
+def test_one_loud_latent_at_every_edge_of_the_window(dtype, decode, d, r, D):
     """Latent attention whose up-projections are identities, so that a head's plain key is the
     normed latent itself: one earlier token's latent is made to point where the last query points.
     It takes the query's weight just inside the window and none just outside, and at page
     borders; the window that differs by one gives a far result."""
-    H, d, r, R, D = 1, 48, 16, 48, 64
+    H, R = 1, d
     size = 130
     T = 300
     m = latent(H, d, r, R, R, 1.0, size=size, rot=16)
@@ -812,15 +816,57 @@ def test_latent_attention_kernel_against_plain_sums(H, W, dv, window):
         assert float((got - ref).abs().max()) < 2e-2
 
 
+def _latent_reference(q, rows, lens, starts, dv, window, scale, rounded=False):
+    """float64 [sum lens, H, dv]; `rounded`: with every weight, in units of its row's largest, rounded to bfloat16 for the
+    value sum, as a kernel with one bfloat16 number a weight would have it."""
+    out = []
+    for b, (n, s) in enumerate(zip(lens, starts)):
+        pos, j = torch.arange(s, s + n)[:, None], torch.arange(s + n)[None, :]
+        seen = (j <= pos) & ((pos - j < window) if window else torch.ones_like(j, dtype=torch.bool))
+        sc = torch.einsum("nhw,tw->nht", q[b].double(), rows[b].double()) * scale
+        sc = sc.masked_fill(~seen[:, None, :], float("-inf"))
+        w = torch.exp(sc - sc.amax(-1, keepdim=True))
+        out.append(torch.einsum("nht,tv->nhv", w.to(BF16).double() if rounded else w, rows[b][:, :dv].double()) / w.sum(-1)[..., None])
+    return torch.cat(out)
+
+
+def _latent_run(q, cache, table, lens, starts, dv, window, scale, **kw):
+    from lumenllm_b200.ops import kernels as K
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    return K.attn_latent(torch.cat(q).to(BF16).cuda(), cache.to(BF16).cuda(), table.cuda(), cu.cuda(),
+                         torch.tensor(starts, dtype=torch.int32).cuda(), lens, dv, window, scale, **kw).cpu().double()
+
+
 @pytest.mark.parametrize("H,W,dv,window", [(16, 576, 512, 45), (16, 576, 512, 0), (3, 192, 64, 33), (70, 128, 128, 1),
                                            (5, 64, 64, 0), (7, 448, 384, 100), (1, 320, 320, 64)])
-def test_latent_attention_of_whole_blocks(H, W, dv, window, monkeypatch):
-    """The same cases for rows of whole 64-value blocks, whose prompts go by tcgen05: one and two slices of value
-    columns (the second narrower), no columns outside the slice, row tiles of one and of many tokens."""
-    from functools import partial
+@pytest.mark.parametrize("rising", [0.0, 9.0, 25.0])
+def test_latent_attention_of_whole_blocks(H, W, dv, window, rising):
+    """Rows of whole 64-value blocks, which go by tcgen05 in every step that is not a decode step: one and two slices of
+    value columns (the second narrower), no columns outside the slice, row tiles of one and of many tokens. `rising`: the
+    scores grow by that many powers of two a tile of 32 keys, faster for some heads than for others, so that rows
+    move their reference (it lags by up to 2^8) at nearly every tile, on top of what they have summed.
+    A row's error is at most 2^-17 a weight for its two bfloat16 numbers, 2^-22 for its exponential, and W 2^-24 of the
+    score's size for the score: 1e-4 of the largest output stands for all; one bfloat16 number a weight is 5e-4 and more
+    off, which the plain sums with such weights show in every case of more than one key."""
     from lumenllm_b200.ops import kernels as K
-    monkeypatch.setattr(K, "attn_latent", partial(K.attn_latent, tensor_memory=True))
-    test_latent_attention_kernel_against_plain_sums(H, W, dv, window)
+    lens, starts, scale = [70, 1, 2, 60], [0, 299, 63, 250], 0.2
+    table, cache, rows, q = _latent_case(lens, starts, H, W, seed=31)
+    if rising:
+        # the last value of a row counts the keys, that of a query says how fast its scores grow (a row's numbers stay bfloat16)
+        for b, t in enumerate([s + n for s, n in zip(starts, lens)]):
+            rows[b][:, W - 1] = (torch.arange(t).float() // 8) * 0.25
+            for p_ in range((t + 63) // 64):
+                n = min(64, t - 64 * p_)
+                cache[table[b, p_], 0, :n] = rows[b][64 * p_:64 * p_ + n]
+            grow = rising * 0.6931 / scale * torch.tensor([1.0, 0.5, 1.0, 0.25])[torch.arange(H) % 4]
+            q[b][:, :, W - 1] = grow.to(BF16).float()
+    ref = _latent_reference(q, rows, lens, starts, dv, window, scale)
+    got = _latent_run(q, cache, table, lens, starts, dv, window, scale)
+    assert got.shape == ref.shape and torch.isfinite(got).all()
+    top = float(ref.abs().max())
+    assert float((got - ref).abs().max()) < 1e-4 * top
+    if window != 1:
+        assert float((_latent_reference(q, rows, lens, starts, dv, window, scale, rounded=True) - ref).abs().max()) > 5e-4 * top
     K.check_error_flags()
 
 
