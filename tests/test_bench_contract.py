@@ -53,3 +53,16 @@ def test_a_short_run_prints_the_whole_contract():
     assert rec["e2e"]["h2d_bytes_per_step"] > 0 and rec["e2e"]["d2h_bytes_per_step"] > 0
     assert rec["gpu_launches"] > 0
     assert {"sm_mhz", "sm_max_mhz", "reasons"} <= set(rec["clocks"])
+
+
+def test_every_kernel_of_a_step_has_a_class_in_the_comparison():
+    """The comparison's shares are by class of kernels: an entry point it does not know would be a class of its own."""
+    import re
+    from lumenllm_b200 import compare
+    from lumenllm_b200.ops import kernels
+    with open(kernels.__file__) as f:
+        names = set(re.findall(r'[^_]fn\(\s*"[a-z0-9_]+",\s*"(lumen_\w+)"', f.read()))
+    by_shape = {"lumen_gemm_tc", "lumen_gemm_tc_grouped", "lumen_moe_product"}       # classes by their arguments
+    elsewhere = {"lumen_gemm_f32", "lumen_tile_weight"}           # float32 models, and made when a model is built
+    assert len(names) > 40
+    assert names - set(compare.CLASSES) == by_shape | elsewhere
