@@ -21,8 +21,8 @@
 // part has barriers of its own, and the scores of the tile after next start on the first part. Everything arrives by
 // TMA (the cache's plain rows get the swizzle on the way). What bounds it is the tensor pipe's operand traffic: every
 // 128 x 32 x 16 product reads 5 KB of shared memory for 16 cycles of arithmetic.
-// 2,048 tokens, 16 heads, W = 576, dv = 512, window 1,024: 211 us (mma.sync 445; 201 with one bfloat16 number a weight);
-// without the window 260 (625). Against 64 bits 2.7e-6 where mma.sync's rounded weights are 1.4e-3 off.
+// 2,048 tokens, 16 heads, W = 576, dv = 512, window 1,024: 209 us (mma.sync 446; 201 with one bfloat16 number a weight);
+// without the window 259 (625). Against 64 bits 2.7e-6 where mma.sync's rounded weights are 1.4e-3 off.
 // Every wait is bounded; when one runs out the block raises the error flag, the other roles give up on theirs, and the
 // block leaves once its own copies have landed and the products it has issued are done (waits with a bound of their own).
 #include <cuda.h>

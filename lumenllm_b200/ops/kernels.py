@@ -1020,7 +1020,7 @@ def attn_latent(q, cache, block_table, cu_q, seq_start, q_lens, value_dim, windo
     step's size: with n_split 1 a row's result is the same bits alone and among others, however its prompt was cut and
     whether the step was captured. Rows in whole 64-value blocks go by tcgen05 (n_split 1; tensor_memory False: not),
     all others by mma.sync. us by tcgen05 / mma.sync at 16 heads of 576, 512 of them the value, window 1,024: one prompt of
-    8 tokens 11.4 / 11.0, 33: 11.5 / 11.2, 64: 13.3 / 15.1, 300: 29 / 48, 2,048: 211 / 446; 8 tokens after 1,500 in each
+    8 tokens 11.4 / 11.0, 33: 11.5 / 11.2, 64: 13.3 / 15.1, 300: 29 / 48, 2,048: 209 / 446; 8 tokens after 1,500 in each
     of 8 sequences 77 / 142; 64 sequences of one token after 1,500 beside a prompt of 33: 77 / 127; 16 prompts of
     33 tokens (160 blocks, a few more than the SMs) 21 / 13."""
     N, H, W = q.shape
