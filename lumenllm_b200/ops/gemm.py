@@ -61,7 +61,7 @@ def gate_up_in_one(rows: int, width: int, k: int) -> bool:
     fill it, and more than 512 have tiles enough. Between, two things count. Below 56
     tiles of 256 x 256 the float32 product can split k over idle SMs, which pays for long k and few tiles; from
     56 on the two-SM kernel's epilogue, with its divisions, is longer than that of the float32 sums, which shows where k is
-    short or the last round of tiles is not full. us, one kernel / two, width x k:
+    short or the last wave of tiles is not full. us, one kernel / two, width x k:
     300 rows 1,024 x 1,024 7.7 / 9.3; 6,144 x 1,024 10.4 / 18.5; 4,096 x 2,048 14.0 / 15.5; 2,816 x 2,048 12.9 / 16.9;
     1,024 x 4,096 21.1 / 13.9; 4,096 x 4,096 23.4 / 19.4; 4,096 x 8,192 42.6 / 28.5; 6,144 x 8,192 45.2 / 41.8;
     8,192 x 1,024 18.4 / 15.8; 16,384 x 1,024 29.1 / 24.0; 10,240 x 2,048 33.4 / 31.3; 16,384 x 2,048 35.0 / 35.1;
