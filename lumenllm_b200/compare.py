@@ -238,7 +238,7 @@ CLASSES = {
     "lumen_linear_attn": "linear attention: recurrence", "lumen_low_rank_decay": "linear attention: decays (+ bonus)",
     "lumen_add_shaped_rmsnorm": "norm", "lumen_rglru": "recurrent unit: recurrence",
     "lumen_gemm_tc_blocks": "block-diagonal product", "lumen_block_product": "block-diagonal product",
-    "lumen_shift_mix": "time mixing: token shift",
+    "lumen_shift_mix": "time mixing: token shift", "lumen_gemm_f32_tc": "float32 product",
 }
 
 

@@ -28,6 +28,7 @@ CSRC = Path(__file__).resolve().parent
 MODULES = {
     "core": (["core.cu"], ["common.cuh", "qk_head.cuh"]),
     "gemm_f32": (["gemm_f32.cu"], ["common.cuh"]),
+    "gemm_f32_tc": (["gemm_f32_tc.cu"], ["common.cuh", "mma_utils.cuh"]),
     "gemm_tc": (["gemm_tc.cu"], ["common.cuh", "mma_utils.cuh"]),
     "attn_generic": (["attn_generic.cu"], ["common.cuh"]),
     "attn_latent": (["attn_latent.cu"], ["common.cuh", "mma_utils.cuh"]),

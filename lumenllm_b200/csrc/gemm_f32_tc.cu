@@ -1,0 +1,466 @@
+// Float32 matrix product C[M,N] = A[M,K] * W[N,K]^T on the 5th-generation tensor cores, with the error of a 32-bit
+// product: every float32 operand is cut into three bfloat16 numbers that add up to it exactly (the number rounded to
+// eight significant bits, what is left rounded likewise, and what is left then), and of the nine products of parts the
+// six that reach 2^-25 of the whole are made, x1 y1 + (x1 y2 + x2 y1) + (x1 y3 + x2 y2 + x3 y1), each exactly, as a
+// product of two eight-bit numbers is. W may be bfloat16 (one part, three products, nothing left out).
+//
+// The tensor core's own sums are short: 64 values of k and their parts, small ones first, into a fresh accumulator, which
+// is then added to a running sum in registers, rounded to nearest. So an output is a chain of K / 64 float32 adds (in
+// up to eight shares of k, added in rising order) where the FFMA kernel's is K / 4. Against a 64-bit product, 2-norm,
+// this / FFMA: K = 1,000 9.7e-8 / 2.8e-7, 2,048 1.0e-7 / 4.1e-7, 8,192 1.2e-7 / 8.1e-7; of numbers that are all positive
+// 9.3e-8 / 1.3e-7, 8.8e-8 / 1.6e-7, 9.2e-8 / 3.1e-7.
+//
+// A block takes 128 rows of W (the 128-row side of the MMA) times up to 160 rows of A, for a share of k; the blocks of
+// one tile, one for each share, are a cluster and add up their sums through distributed shared memory. The number of
+// shares depends on N and K alone, so C[m,n] depends on row m of A and row n of W only, never on M or where they lie.
+//   warps 0..7   fetch the next 64 columns of both operands into registers while they cut the present ones and store the
+//                parts as 128-byte-swizzled tiles, two buffers;
+//   last warp    issues the products, allocates tensor memory;
+//   the others   add the finished accumulator (two of them, in tensor memory) to the sums in their registers.
+// Infinities and NaN have no parts: the rows that hold one are marked, and their outputs are made again with plain FMAs.
+//
+// What bounds it: for many rows cutting the operands, beside the tensor pipe (six bfloat16 products for one of 32 bits) and
+// shared memory (operands read by the products, parts written); for few rows the stream over W.
+// us, FFMA -> this: 300 rows x 16,384 outputs x 2,048 511 -> 187; 300 x 2,048 x 8,192 440 -> 151; 300 x 3,072 x 2,048
+// 115 -> 61; 100 x 2,048 x 8,192 222 -> 83; 16 x 32,768 x 2,048 95 -> 75; 8 x 2,048 x 8,192 60 -> 37.
+// Every wait is bounded; when one runs out the block raises the error flag, its other roles give up on theirs, and the
+// block leaves, through the same cluster barriers as ever, once the products it has issued are done.
+#include "common.cuh"
+#include "mma_utils.cuh"
+
+#define FT_ROWS 128                      // rows of W a block
+#define FT_BK 64
+#define FT_MAX_BN 160                    // rows of A a block
+#define FT_CONV 8                        // warps that fetch and cut
+#define FT_W_TILE (FT_ROWS * 128)        // bytes of one part of a tile of W
+#define FT_MAX_SHARES 8
+#define FT_MIN_N 1024                    // see lumen_gemm_f32_tc_takes
+#define FT_MIN_K 1024
+
+__device__ __forceinline__ void ft_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void ft_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void ft_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void ft_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void ft_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void ft_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// As mbar_wait, but given up as soon as another role of the block has.
+__device__ __forceinline__ bool ft_wait(uint64_t* bar, uint32_t parity, const volatile int* abort_flag) {
+    for (uint32_t it = 0; it < LUMEN_SPIN_LIMIT; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if ((it & 63u) == 63u && *abort_flag) return false;
+    }
+    return false;
+}
+// A K-major operand tile of 128-byte rows in the 128-byte swizzle, groups of 8 rows 1024 bytes apart.
+__device__ __forceinline__ uint64_t ft_desc(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+// D float32, A and B bfloat16, both K-major, M = 128.
+__device__ __forceinline__ uint32_t ft_idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(FT_ROWS >> 4) << 24);
+}
+__device__ __forceinline__ void ft_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ft_peer(uint32_t addr, uint32_t rank) {          // a float of another block's shared memory
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// Four values of a row as they lie in memory (zeros where there are none).
+template <typename T> struct FtRaw;
+template <> struct FtRaw<float> { float4 v; };
+template <> struct FtRaw<__nv_bfloat16> { uint2 v; };
+__device__ __forceinline__ void ft_fetch(FtRaw<float>& x, const float* p, int left, bool vec) {
+    x.v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (vec) {
+        if (left > 0) x.v = __ldg(reinterpret_cast<const float4*>(p));
+    } else {
+        if (left > 0) x.v.x = __ldg(p);
+        if (left > 1) x.v.y = __ldg(p + 1);
+        if (left > 2) x.v.z = __ldg(p + 2);
+        if (left > 3) x.v.w = __ldg(p + 3);
+    }
+}
+__device__ __forceinline__ void ft_fetch(FtRaw<__nv_bfloat16>& x, const __nv_bfloat16* p, int left, bool vec) {
+    x.v = make_uint2(0u, 0u);
+    if (vec) {
+        if (left > 0) x.v = __ldg(reinterpret_cast<const uint2*>(p));
+    } else {
+        const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+        if (left > 0) x.v.x = __ldg(q);
+        if (left > 1) x.v.x |= (uint32_t)__ldg(q + 1) << 16;
+        if (left > 2) x.v.y = __ldg(q + 2);
+        if (left > 3) x.v.y |= (uint32_t)__ldg(q + 3) << 16;
+    }
+}
+// Two numbers rounded to bfloat16, side by side; x becomes what is left of each (exactly).
+__device__ __forceinline__ uint32_t ft_cut(unsigned long long& x) {
+    uint32_t a, b;
+    unsigned long long r;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(x));
+    const uint32_t h = pack_bf16(__uint_as_float(a), __uint_as_float(b));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(h << 16), "r"(h & 0xffff0000u));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(x) : "l"(r), "l"(0xbf800000bf800000ull));       // x - r
+    return h;
+}
+// Cuts four values and stores their parts `part` bytes apart; 1 if one of them is not finite (or rounds to infinity).
+__device__ __forceinline__ int ft_store(const FtRaw<float>& x, unsigned char* dst, int part) {
+    unsigned long long a, b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(x.v.x), "f"(x.v.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(x.v.z), "f"(x.v.w));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        uint2 h;
+        h.x = ft_cut(a);
+        h.y = ft_cut(b);
+        *reinterpret_cast<uint2*>(dst + i * part) = h;
+    }
+    // nothing is left (or less than bfloat16 has numbers for, of values below 2^-110), or NaN: an infinity less itself
+    float u, v;
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(u), "=f"(v) : "l"(a));
+    return !(u + v == u + v);
+}
+__device__ __forceinline__ int ft_store(const FtRaw<__nv_bfloat16>& x, unsigned char* dst, int) {
+    *reinterpret_cast<uint2*>(dst) = x.v;
+    const uint32_t e = 0x7f80u;
+    return (x.v.x & e) == e || ((x.v.x >> 16) & e) == e || (x.v.y & e) == e || ((x.v.y >> 16) & e) == e;
+}
+
+template <typename TW, int BN>
+struct FtShape {
+    static constexpr int NW = sizeof(TW) == 4 ? 3 : 1;                   // parts of a weight
+    static constexpr int HALVES = BN > 64 ? 2 : 1;                       // groups of four adding warps, by columns
+    static constexpr int EPI = 4 * HALVES, WARPS = FT_CONV + EPI + 1;
+    static constexpr int A_TILE = BN * 128;
+    static constexpr int BUF = NW * FT_W_TILE + 3 * A_TILE;
+    static constexpr int TMEM = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
+    static constexpr int CTL = 1024;                                     // barriers, flags, marks
+    static constexpr int SMEM = 2 * BUF + CTL;
+    static constexpr int MINB = (BN <= 16 && 2 * SMEM <= 220 * 1024) ? 2 : 1;
+    static constexpr int SETS = MINB == 1 && BN <= 64 ? 2 : 1;           // blocks of W under way in registers
+    static_assert(BN * FT_ROWS * 4 <= 2 * BUF, "the sums are staged where the tiles were");
+};
+
+template <typename TW, int BN>
+__global__ void __launch_bounds__(32 * FtShape<TW, BN>::WARPS, FtShape<TW, BN>::MINB)
+gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn,
+                   int vec, int give_up_at, int* __restrict__ err) {
+    using F = FtShape<TW, BN>;
+    constexpr int NW = F::NW, EPI = F::EPI, ACOL = F::TMEM / 2;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char* tiles = smem;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * F::BUF);
+    uint64_t* full = bars;              // [2] the parts of a block of k are in shared memory
+    uint64_t* done = bars + 2;          // [2] its products are in the accumulator: the buffer is free, the sums can be taken
+    uint64_t* taken = bars + 4;         // [2] the accumulator has been read
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* any_odd = reinterpret_cast<volatile int*>(tmem_slot + 2);
+    unsigned char* odd_w = reinterpret_cast<unsigned char*>(bars + 16);      // [128] rows of W, [BN] rows of A with an infinity or NaN
+    unsigned char* odd_a = odd_w + FT_ROWS;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int S = gridDim.x, share = blockIdx.x;                             // the cluster is one tile's shares of k
+    const int m0 = blockIdx.y * bn, n0 = blockIdx.z * FT_ROWS;
+    const int num_kb = (K + FT_BK - 1) / FT_BK, per = (num_kb + S - 1) / S;
+    const int kb0 = min(share * per, num_kb), nk = min(kb0 + per, num_kb) - kb0;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&full[i], FT_CONV);
+            mbar_init(&done[i], 1);
+            mbar_init(&taken[i], EPI);
+        }
+        *abort_flag = 0;
+        *any_odd = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = threadIdx.x; i < FT_ROWS + BN; i += blockDim.x) odd_w[i] = 0;
+    if (warp == FT_CONV + EPI) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(F::TMEM)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    ft_fence_before();
+    __syncthreads();
+    ft_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();      // nothing of this kernel touches global memory before this
+    pdl_trigger();
+    const int rows = min(bn, M - m0), cols = min(FT_ROWS, N - n0);
+    float* sums = reinterpret_cast<float*>(tiles);             // [BN][128], over the tiles once they have been read
+
+    if (warp < FT_CONV) {
+        constexpr int LW = FT_ROWS / 16, LA = BN / 16;                       // fetches a thread: 16 threads a row
+        const int c = threadIdx.x & 15, r = threadIdx.x >> 4;
+        FtRaw<TW> rw[F::SETS][LW];
+        FtRaw<float> ra[LA];
+        auto fetch_w = [&](int kb, FtRaw<TW> (&x)[LW]) {
+            const int k = (kb0 + kb) * FT_BK + 4 * c;
+            const TW* p = W + (size_t)(n0 + r) * K + k;
+#pragma unroll
+            for (int i = 0; i < LW; ++i) ft_fetch(x[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < cols ? K - k : 0, vec);
+        };
+        auto fetch_a = [&](int kb) {
+            const int k = (kb0 + kb) * FT_BK + 4 * c;
+            const float* p = A + (size_t)(m0 + r) * K + k;
+#pragma unroll
+            for (int i = 0; i < LA; ++i) ft_fetch(ra[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < rows ? K - k : 0, vec);
+        };
+        // this thread's four values of row r: 8 bytes in the 16-byte piece c / 2, which lies at (c / 2) ^ (row & 7)
+        const uint32_t at = r * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8;
+        auto step = [&](int kb, FtRaw<TW> (&x)[LW]) -> bool {
+            const int b = kb & 1;
+            if (kb >= 2 && !__all_sync(0xffffffffu, ft_wait(&done[b], ((kb >> 1) & 1) ^ 1, abort_flag))) {
+                *abort_flag = 1;
+                if (lane == 0) atomicExch(err, 1);
+                return false;
+            }
+            unsigned char* tw = tiles + b * F::BUF + at;
+            unsigned char* ta = tw + NW * FT_W_TILE;
+            int odd = 0;                         // looked at once a block, so that the rows' cutting can be interleaved
+#pragma unroll
+            for (int i = 0; i < LW; ++i) odd |= ft_store(x[i], tw + i * 16 * 128, FT_W_TILE) << i;
+            fetch_w(kb + F::SETS, x);            // under way while the rows of A are cut, and while the products are waited for
+#pragma unroll
+            for (int i = 0; i < LA; ++i) odd |= ft_store(ra[i], ta + i * 16 * 128, F::A_TILE) << (LW + i);
+            fetch_a(kb + 1);
+            if (odd) {
+                *any_odd = 1;
+                for (int i = 0; i < LW; ++i)
+                    if (odd >> i & 1) odd_w[r + 16 * i] = 1;
+                for (int i = 0; i < LA; ++i)
+                    if (odd >> (LW + i) & 1) odd_a[r + 16 * i] = 1;
+            }
+            // The fence between these stores and the products' reads is the issuing thread's: here it would wait for the loads.
+            __syncwarp();
+            if (lane == 0) ft_arrive(&full[b]);
+            return true;
+        };
+#pragma unroll
+        for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
+        fetch_a(0);
+        for (int kb = 0; kb < nk; kb += F::SETS) {
+            if (!step(kb, rw[0])) break;
+            if (F::SETS == 2 && kb + 1 < nk && !step(kb + 1, rw[F::SETS - 1])) break;
+        }
+    } else if (warp == FT_CONV + EPI) {
+        if (lane == 0) {
+            const uint32_t idesc = ft_idesc(bn);
+            int issued = 0;
+            bool ok = true;
+            for (int kb = 0; kb < nk; ++kb) {
+                const int b = kb & 1;
+                ok = ft_wait(&full[b], (kb >> 1) & 1, abort_flag) &&
+                     (kb < 2 || ft_wait(&taken[b], ((kb >> 1) & 1) ^ 1, abort_flag));
+                if (!ok) break;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                ft_fence_after();
+                const uint32_t tw = smem_u32(tiles + b * F::BUF), ta = tw + NW * FT_W_TILE, d = tmem_base + b * ACOL;
+                uint32_t accumulate = 0;
+                auto product = [&](int pw, int pa) {
+                    const uint64_t wd = ft_desc(tw + pw * FT_W_TILE), ad = ft_desc(ta + pa * F::A_TILE);
+#pragma unroll
+                    for (int k = 0; k < FT_BK / 16; ++k) {
+                        ft_mma(d, wd + 2 * k, ad + 2 * k, idesc, accumulate);
+                        accumulate = 1;
+                    }
+                };
+                if (NW == 3) {
+                    product(2, 0);
+                    product(0, 2);
+                    product(1, 1);
+                    product(1, 0);
+                    product(0, 1);
+                } else {
+                    product(0, 2);
+                    product(0, 1);
+                }
+                product(0, 0);
+                ft_commit(&done[b]);
+                issued = kb + 1;
+            }
+            if (!ok) { *abort_flag = 1; atomicExch(err, 1); }
+            // the block keeps its shared and tensor memory until the products that use them are done
+            if (issued > 0 && !mbar_wait(&done[(issued - 1) & 1], ((issued - 1) >> 1) & 1)) atomicExch(err, 1);
+        }
+        __syncwarp();
+    } else {
+        constexpr int COLS = BN / F::HALVES;                    // rows of A an adding warp keeps
+        const int qd = warp & 3, first = ((warp - FT_CONV) >> 2) * COLS, n = qd * 32 + lane;
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16) + first;
+        float acc[COLS];
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
+        for (int kb = 0; kb < nk; ++kb) {
+            const int b = kb & 1;
+            const bool w = kb != give_up_at && ft_wait(&done[b], (kb >> 1) & 1, abort_flag);
+            if (!__all_sync(0xffffffffu, w)) {
+                *abort_flag = 1;
+                if (lane == 0) atomicExch(err, 1);
+                break;
+            }
+            ft_fence_after();
+#pragma unroll
+            for (int c0 = 0; c0 < COLS; c0 += 16) {
+                float v[16];
+                ft_ld16(lane_addr + b * ACOL + c0, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[c0 + j] += v[j];
+            }
+            ft_fence_before();
+            __syncwarp();
+            if (lane == 0) ft_arrive(&taken[b]);
+        }
+        // the last block's products are done, so no tile is read or written any more (unless a wait ran out)
+        if (S == 1 && !*any_odd) {
+            if (n < cols) {
+                float* dst = C + (size_t)(m0 + first) * N + n0 + n;
+#pragma unroll
+                for (int j = 0; j < COLS; ++j)
+                    if (first + j < rows) dst[(size_t)j * N] = acc[j];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) sums[(first + j) * FT_ROWS + n] = acc[j];
+        }
+    }
+
+    ft_fence_before();
+    __syncthreads();
+    ft_fence_after();
+    if (warp == FT_CONV + EPI)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(F::TMEM) : "memory");
+    const bool odd = *any_odd != 0;
+    if (S == 1 && !odd) return;
+    if (odd) {
+        for (int e = threadIdx.x; e < rows * FT_ROWS; e += blockDim.x) {
+            const int m = e / FT_ROWS, n = e % FT_ROWS;
+            if (n >= cols || !(odd_a[m] || odd_w[n])) continue;
+            float s = 0.0f;
+            const int k1 = min(K, (kb0 + nk) * FT_BK);
+            for (int k = kb0 * FT_BK; k < k1; ++k) s = fmaf(A[(size_t)(m0 + m) * K + k], to_f32(W[(size_t)(n0 + n) * K + k]), s);
+            sums[e] = s;
+        }
+    }
+    if (S > 1) ft_cluster_sync();
+    else __syncthreads();
+    for (int e = share * blockDim.x + threadIdx.x; e < rows * FT_ROWS; e += S * blockDim.x) {
+        const int m = e / FT_ROWS, n = e % FT_ROWS;
+        if (n >= cols) continue;
+        float s;
+        if (S > 1) {
+            const uint32_t a = smem_u32(sums + e);
+            s = ft_peer(a, 0);
+            for (int p = 1; p < S; ++p) s += ft_peer(a, p);
+        } else {
+            s = sums[e];
+        }
+        C[(size_t)(m0 + m) * N + n0 + n] = s;
+    }
+    if (S > 1) ft_cluster_sync();          // a block's sums stay until the others have read them
+}
+
+template <typename TW, int BN>
+static int gemm_f32_tc_go(const float* A, const TW* W, float* C, int M, int N, int K, int bn, int S, int give_up_at, int* err,
+                          cudaStream_t stream) {
+    using F = FtShape<TW, BN>;
+    auto k = gemm_f32_tc_kernel<TW, BN>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    const int vec = (K & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S, (M + bn - 1) / bn, (N + FT_ROWS - 1) / FT_ROWS);
+    cfg.blockDim = dim3(32 * F::WARPS);
+    cfg.dynamicSmemBytes = F::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = lumen_pdl_enabled() ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, k, A, W, C, M, N, K, bn, vec, give_up_at, err);
+    if (e != cudaSuccess) return (int)e;
+    LUMEN_LAUNCH_CHECK();
+    return 0;
+}
+
+// Shares of k: as many as keep the blocks of one row of tiles within the SMs, each with four blocks of k or more.
+static int gemm_f32_tc_shares(int N, int K) {
+    const int tiles = (N + FT_ROWS - 1) / FT_ROWS, num_kb = (K + FT_BK - 1) / FT_BK;
+    int S = 1;
+    while (S < FT_MAX_SHARES && 2 * S * tiles <= 148 && num_kb >= 8 * S) S *= 2;
+    return S;
+}
+
+template <typename TW>
+static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, int M, int N, int K, int give_up_at, int* err,
+                            cudaStream_t stream) {
+    const int S = gemm_f32_tc_shares(N, K);
+    const int tiles = (M + FT_MAX_BN - 1) / FT_MAX_BN;
+    const int bn = ((M + tiles - 1) / tiles + 15) / 16 * 16;
+    if (bn <= 16) return gemm_f32_tc_go<TW, 16>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
+    if (bn <= 32) return gemm_f32_tc_go<TW, 32>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
+    if (bn <= 64) return gemm_f32_tc_go<TW, 64>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
+    if (bn <= 96) return gemm_f32_tc_go<TW, 96>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
+    if (bn <= 128) return gemm_f32_tc_go<TW, 128>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
+    return gemm_f32_tc_go<TW, 160>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
+}
+
+// 1 if weights [N, K] go through this kernel, whatever M: by N and K alone, so that a row's value is the same in any batch.
+// Smaller weights leave most SMs idle and are FFMA's: 300 rows x 512 x 512 17.7 us there, 21.7 here; 300 x 1,024 x 300 13 / 21;
+// 2,048 x 256 x 256 11 / 18.
+LUMEN_API int lumen_gemm_f32_tc_takes(int N, int K) { return N >= FT_MIN_N && K >= FT_MIN_K ? 1 : 0; }
+
+// A float32 [M, K], W float32 or bfloat16 [N, K], C float32 [M, N], rows dense; any alignment their types have. give_up_at:
+// the block of k at which the adding warps take their wait as run out (-1: none; for tests of what a block does then).
+LUMEN_API int lumen_gemm_f32_tc(const float* A, const void* W, int w_is_bf16, float* C, int M, int N, int K, int give_up_at,
+                                int* err, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0) return LUMEN_ERR_BAD_ARGUMENT;
+    if ((M + 63) / 64 > 65535 || (N + FT_ROWS - 1) / FT_ROWS > 65535) return LUMEN_ERR_UNSUPPORTED;
+    return w_is_bf16 ? gemm_f32_tc_rows(A, (const __nv_bfloat16*)W, C, M, N, K, give_up_at, err, stream)
+                     : gemm_f32_tc_rows(A, (const float*)W, C, M, N, K, give_up_at, err, stream);
+}

@@ -1469,7 +1469,8 @@ def delta_rule(x, q_col, k_col, v_col, u, beta_col, a, dt_bias, a_log, state, cu
 
 
 def gemm_f32(a, w, out=None):
-    """C = a @ w.T in true float32 (FFMA). a float32 [M, K]; w [N, K] float32|bfloat16."""
+    """C = a @ w.T with 32-bit error. a float32 [M, K]; w [N, K] float32|bfloat16. The weight's size decides between the tensor
+    cores on three bfloat16 parts a number (csrc/gemm_f32_tc.cu) and FFMA, so a row's result is the same in any batch."""
     require(a, F32, "gemm_f32.a")
     M, K = a.shape
     N, K2 = w.shape
@@ -1479,6 +1480,10 @@ def gemm_f32(a, w, out=None):
         raise KernelError("gemm_f32.w must be a contiguous CUDA tensor")
     if out is None:
         out = torch.empty((M, N), dtype=F32, device=a.device)
+    if int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_takes", [c_int, c_int])(N, K):
+        f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, c_int, c_int, c_int, c_int, P, P])
+        check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), M, N, K, -1, ptr(error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
+        return out
     f = fn("gemm_f32", "lumen_gemm_f32", [P, P, c_int, P, c_int, c_int, c_int, P])
     check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), M, N, K, stream_ptr()), "gemm_f32")
     return out

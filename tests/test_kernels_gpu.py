@@ -534,6 +534,62 @@ def test_gemm_f32_adds_in_one_order_wherever_the_operands_lie(wdtype, M, N, K_):
     assert torch.equal(odd, K.gemm_f32(a, w))
 
 
+@pytest.mark.parametrize("wdtype", [F32, BF16])
+@pytest.mark.parametrize("M,N,K_", [(1, 1024, 1024), (16, 1025, 1028), (17, 1100, 1030), (33, 4096, 1088), (65, 1151, 2047), (97, 1024, 4096),
+                                    (129, 1300, 1024), (161, 1024, 1027), (300, 20000, 1024)])
+def test_gemm_f32_in_bfloat16_parts(wdtype, M, N, K_):
+    """Every tile width, one and several shares of k, ends inside tiles and rows of odd lengths. An exact product summed in
+    chains of K / 64 + 8 float32 adds, each after 24 adds that lose up to an ulp of a 64-value sum, with parts of
+    2^-25 left out: within (K / 64 + 40) 2^-24 of the sum of the products' sizes. Rows do not depend on the
+    batch or on where they lie, and what is not finite stays in its own outputs, with FFMA's values there."""
+    from lumenllm_b200.ops import kernels as K
+    from lumenllm_b200.ops.native import int_fn
+    from ctypes import c_int
+    assert int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_takes", [c_int, c_int])(N, K_)
+    g = gen(23)
+    a = torch.randn(M, K_, generator=g) * torch.logspace(-3, 3, K_)
+    w = (torch.randn(N, K_, generator=g) / torch.logspace(-3, 3, K_)).to(wdtype)
+    w[1] *= 2.0 ** -60
+    out = K.gemm_f32(dev(a), dev(w))
+    K.check_error_flags()
+    ref = a.double() @ w.double().T
+    assert bool(((out.cpu().double() - ref).abs() <= (K_ / 64 + 40) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T)).all())
+    buf = torch.empty(a.numel() + 1, device="cuda")
+    buf[1:] = dev(a).reshape(-1)
+    assert torch.equal(K.gemm_f32(buf[1:].view(M, K_), dev(w)), out)
+    assert torch.equal(K.gemm_f32(dev(a[M // 2:M // 2 + 1].contiguous()), dev(w))[0], out[M // 2])
+    odd_a, odd_w = a.clone(), w.clone()
+    odd_a[M - 1, 3], odd_w[N - 1, K_ - 1], odd_w[2, 5] = float("inf"), float("nan"), float("-inf")
+    got = K.gemm_f32(dev(odd_a), dev(odd_w)).cpu()
+    K.check_error_flags()
+    ok = torch.ones(M, N, dtype=torch.bool)
+    ok[M - 1], ok[:, N - 1], ok[:, 2] = False, False, False
+    assert torch.equal(got[ok], out.cpu()[ok])
+    assert bool(got[:, N - 1].isnan().all()) and torch.equal(got[:M - 1, 2], -float("inf") * odd_a[:M - 1, 5].sign())
+    mid = [n for n in range(N - 1) if n != 2]
+    assert torch.equal(got[M - 1, mid], float("inf") * odd_w[mid, 3].float().sign())
+
+
+def test_a_float32_product_that_gives_up_says_so():
+    """A wait that runs out raises the error flag, in clusters too, and the context stays usable."""
+    from ctypes import c_int, c_void_p
+    from lumenllm_b200.ops import kernels as K
+    from lumenllm_b200.ops.native import check, fn, ptr, stream_ptr
+    P = c_void_p
+    f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, c_int, c_int, c_int, c_int, P, P])
+    for M, N, K_ in ((20, 1024, 4096), (150, 20000, 1024)):
+        a, w = torch.ones(M, K_, device="cuda"), torch.ones(N, K_, device="cuda")
+        for at, raises in ((1, True), (-1, False)):
+            out = torch.empty(M, N, device="cuda")
+            check(f(ptr(a), ptr(w), 0, ptr(out), M, N, K_, at, ptr(K.error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
+            if raises:
+                with pytest.raises(K.KernelError):
+                    K.check_error_flags()
+            else:
+                K.check_error_flags()
+                assert bool((out == K_).all())
+
+
 @pytest.mark.parametrize("M,N,K_", [(128, 256, 64), (200, 300, 320), (2048, 1024, 4096), (1, 256, 64),
                                     (8, 4096, 4096), (19, 311, 80), (33, 1000, 1000), (64, 6144, 1024),
                                     (65, 130, 72), (130, 17, 1000), (16, 151936 // 4 + 8, 256)])
