@@ -13,9 +13,12 @@
 // A block takes 128 rows of W (the 128-row side of the MMA) times up to 160 rows of A, for a share of k; the blocks of
 // one tile, one for each share, are a cluster and add up their sums through distributed shared memory. The number of
 // shares depends on N and K alone, so C[m,n] depends on row m of A and row n of W only, never on M or where they lie.
-//   warps 0..7   fetch the next 64 columns of both operands into registers while they cut the present ones and store the
-//                parts as 128-byte-swizzled tiles, two buffers;
-//   last warp    issues the products, allocates tensor memory;
+//   warps 0..7   fetch the next 64 columns of W into registers while they cut the present ones and store the parts as
+//                128-byte-swizzled tiles, two buffers. Up to 32 rows of A go the same way; more are cut once, by a kernel
+//                ahead of this one, into the image their tiles have in shared memory (a block that cut 160 rows of A for its
+//                128 of W spent half of its time on them), and are copied by
+//   a warp       that does nothing else;
+//   a warp       issues the products, allocates tensor memory;
 //   the others   add the finished accumulator (two of them, in tensor memory) to the sums in their registers.
 // Infinities and NaN have no parts: the rows that hold one are marked, and their outputs are made again with plain FMAs.
 //
@@ -95,11 +98,11 @@ __device__ __forceinline__ uint32_t ft_idesc(int n) {
 __device__ __forceinline__ void ft_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float ft_peer(uint32_t addr, uint32_t rank) {          // a float of another block's shared memory
+__device__ __forceinline__ float4 ft_peer(uint32_t addr, uint32_t rank) {         // 16 bytes of another block's shared memory
     uint32_t a;
-    float v;
+    float4 v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
     return v;
 }
 
@@ -168,21 +171,23 @@ template <typename TW, int BN>
 struct FtShape {
     static constexpr int NW = sizeof(TW) == 4 ? 3 : 1;                   // parts of a weight
     static constexpr int HALVES = BN > 64 ? 2 : 1;                       // groups of four adding warps, by columns
-    static constexpr int EPI = 4 * HALVES, WARPS = FT_CONV + EPI + 1;
+    static constexpr bool IMAGE = BN > 32;                               // A arrives cut
+    static constexpr int EPI = 4 * HALVES, WARPS = FT_CONV + EPI + 1 + (IMAGE ? 1 : 0);
     static constexpr int A_TILE = BN * 128;
     static constexpr int BUF = NW * FT_W_TILE + 3 * A_TILE;
     static constexpr int TMEM = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
     static constexpr int CTL = 1024;                                     // barriers, flags, marks
     static constexpr int SMEM = 2 * BUF + CTL;
     static constexpr int MINB = (BN <= 16 && 2 * SMEM <= 220 * 1024) ? 2 : 1;
-    static constexpr int SETS = MINB == 1 && BN <= 64 ? 2 : 1;           // blocks of W under way in registers
+    static constexpr int SETS = MINB == 1 ? 2 : 1;                       // blocks of W under way in registers
     static_assert(BN * FT_ROWS * 4 <= 2 * BUF, "the sums are staged where the tiles were");
 };
 
 template <typename TW, int BN>
 __global__ void __launch_bounds__(32 * FtShape<TW, BN>::WARPS, FtShape<TW, BN>::MINB)
-gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn,
-                   int vec, int give_up_at, int* __restrict__ err) {
+gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict__ image, const unsigned char* __restrict__ image_odd,
+                   const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int vec, int give_up_at,
+                   int* __restrict__ err) {
     using F = FtShape<TW, BN>;
     constexpr int NW = F::NW, EPI = F::EPI, ACOL = F::TMEM / 2;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -191,7 +196,8 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
     uint64_t* full = bars;              // [2] the parts of a block of k are in shared memory
     uint64_t* done = bars + 2;          // [2] its products are in the accumulator: the buffer is free, the sums can be taken
     uint64_t* taken = bars + 4;         // [2] the accumulator has been read
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+    uint64_t* landed = bars + 6;        // [2] the parts of A have been copied
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* any_odd = reinterpret_cast<volatile int*>(tmem_slot + 2);
     unsigned char* odd_w = reinterpret_cast<unsigned char*>(bars + 16);      // [128] rows of W, [BN] rows of A with an infinity or NaN
@@ -208,32 +214,38 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
             mbar_init(&full[i], FT_CONV);
             mbar_init(&done[i], 1);
             mbar_init(&taken[i], EPI);
+            mbar_init(&landed[i], 1);
         }
         *abort_flag = 0;
         *any_odd = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < FT_ROWS + BN; i += blockDim.x) odd_w[i] = 0;
     if (warp == FT_CONV + EPI) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(F::TMEM)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    ft_fence_before();
-    __syncthreads();
-    ft_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
     pdl_wait();      // nothing of this kernel touches global memory before this
     pdl_trigger();
     const int rows = min(bn, M - m0), cols = min(FT_ROWS, N - n0);
+    int marked = 0;
+    for (int i = threadIdx.x; i < FT_ROWS + BN; i += blockDim.x) {
+        const int m = i - FT_ROWS;
+        odd_w[i] = F::IMAGE && m >= 0 && m < rows && image_odd[m0 + m];
+        marked |= odd_w[i];
+    }
+    ft_fence_before();
+    marked = __syncthreads_or(marked);
+    ft_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
     float* sums = reinterpret_cast<float*>(tiles);             // [BN][128], over the tiles once they have been read
 
     if (warp < FT_CONV) {
         constexpr int LW = FT_ROWS / 16, LA = BN / 16;                       // fetches a thread: 16 threads a row
         const int c = threadIdx.x & 15, r = threadIdx.x >> 4;
         FtRaw<TW> rw[F::SETS][LW];
-        FtRaw<float> ra[LA];
+        FtRaw<float> ra[F::IMAGE ? 1 : LA];
         auto fetch_w = [&](int kb, FtRaw<TW> (&x)[LW]) {
             const int k = (kb0 + kb) * FT_BK + 4 * c;
             const TW* p = W + (size_t)(n0 + r) * K + k;
@@ -243,8 +255,10 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
         auto fetch_a = [&](int kb) {
             const int k = (kb0 + kb) * FT_BK + 4 * c;
             const float* p = A + (size_t)(m0 + r) * K + k;
+            if constexpr (!F::IMAGE) {
 #pragma unroll
-            for (int i = 0; i < LA; ++i) ft_fetch(ra[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < rows ? K - k : 0, vec);
+                for (int i = 0; i < LA; ++i) ft_fetch(ra[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < rows ? K - k : 0, vec);
+            }
         };
         // this thread's four values of row r: 8 bytes in the 16-byte piece c / 2, which lies at (c / 2) ^ (row & 7)
         const uint32_t at = r * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8;
@@ -260,16 +274,19 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
             int odd = 0;                         // looked at once a block, so that the rows' cutting can be interleaved
 #pragma unroll
             for (int i = 0; i < LW; ++i) odd |= ft_store(x[i], tw + i * 16 * 128, FT_W_TILE) << i;
-            fetch_w(kb + F::SETS, x);            // under way while the rows of A are cut, and while the products are waited for
+            fetch_w(kb + F::SETS, x);            // under way while the products are waited for
+            if constexpr (!F::IMAGE) {
 #pragma unroll
-            for (int i = 0; i < LA; ++i) odd |= ft_store(ra[i], ta + i * 16 * 128, F::A_TILE) << (LW + i);
+                for (int i = 0; i < LA; ++i) odd |= ft_store(ra[i], ta + i * 16 * 128, F::A_TILE) << (LW + i);
+            }
             fetch_a(kb + 1);
             if (odd) {
                 *any_odd = 1;
                 for (int i = 0; i < LW; ++i)
                     if (odd >> i & 1) odd_w[r + 16 * i] = 1;
-                for (int i = 0; i < LA; ++i)
-                    if (odd >> (LW + i) & 1) odd_a[r + 16 * i] = 1;
+                if constexpr (!F::IMAGE)
+                    for (int i = 0; i < LA; ++i)
+                        if (odd >> (LW + i) & 1) odd_a[r + 16 * i] = 1;
             }
             // The fence between these stores and the products' reads is the issuing thread's: here it would wait for the loads.
             __syncwarp();
@@ -290,7 +307,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
             bool ok = true;
             for (int kb = 0; kb < nk; ++kb) {
                 const int b = kb & 1;
-                ok = ft_wait(&full[b], (kb >> 1) & 1, abort_flag) &&
+                ok = ft_wait(&full[b], (kb >> 1) & 1, abort_flag) && (!F::IMAGE || ft_wait(&landed[b], (kb >> 1) & 1, abort_flag)) &&
                      (kb < 2 || ft_wait(&taken[b], ((kb >> 1) & 1) ^ 1, abort_flag));
                 if (!ok) break;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -324,6 +341,27 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
             if (issued > 0 && !mbar_wait(&done[(issued - 1) & 1], ((issued - 1) >> 1) & 1)) atomicExch(err, 1);
         }
         __syncwarp();
+    } else if (F::IMAGE && warp == FT_CONV + EPI + 1) {
+        if (lane == 0) {
+            const unsigned char* from = image + ((size_t)blockIdx.y * num_kb + kb0) * 3 * bn * 128;
+            int asked = 0;
+            for (int kb = 0; kb < nk; ++kb) {
+                const int b = kb & 1;
+                if (kb >= 2 && !ft_wait(&done[b], ((kb >> 1) & 1) ^ 1, abort_flag)) {
+                    *abort_flag = 1;
+                    atomicExch(err, 1);
+                    break;
+                }
+                mbar_expect_tx(&landed[b], 3 * bn * 128);
+                for (int i = 0; i < 3; ++i)
+                    bulk_load(tiles + b * F::BUF + NW * FT_W_TILE + i * F::A_TILE, from + ((size_t)kb * 3 + i) * bn * 128, bn * 128, &landed[b]);
+                asked = kb + 1;
+            }
+            // the block stays until its copies have landed
+            for (int kb = max(0, asked - 2); kb < asked; ++kb)
+                if (!mbar_wait(&landed[kb & 1], (kb >> 1) & 1)) atomicExch(err, 1);
+        }
+        __syncwarp();
     } else {
         constexpr int COLS = BN / F::HALVES;                    // rows of A an adding warp keeps
         const int qd = warp & 3, first = ((warp - FT_CONV) >> 2) * COLS, n = qd * 32 + lane;
@@ -352,7 +390,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
             if (lane == 0) ft_arrive(&taken[b]);
         }
         // the last block's products are done, so no tile is read or written any more (unless a wait ran out)
-        if (S == 1 && !*any_odd) {
+        if (S == 1 && !*any_odd && !marked) {
             if (n < cols) {
                 float* dst = C + (size_t)(m0 + first) * N + n0 + n;
 #pragma unroll
@@ -370,7 +408,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
     ft_fence_after();
     if (warp == FT_CONV + EPI)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(F::TMEM) : "memory");
-    const bool odd = *any_odd != 0;
+    const bool odd = *any_odd != 0 || marked;
     if (S == 1 && !odd) return;
     if (odd) {
         for (int e = threadIdx.x; e < rows * FT_ROWS; e += blockDim.x) {
@@ -384,32 +422,85 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const TW* __restrict__ W, float*
     }
     if (S > 1) ft_cluster_sync();
     else __syncthreads();
-    for (int e = share * blockDim.x + threadIdx.x; e < rows * FT_ROWS; e += S * blockDim.x) {
+    for (int e = 4 * (share * blockDim.x + threadIdx.x); e < rows * FT_ROWS; e += 4 * S * blockDim.x) {
         const int m = e / FT_ROWS, n = e % FT_ROWS;
         if (n >= cols) continue;
-        float s;
+        float4 s = *reinterpret_cast<const float4*>(sums + e);
         if (S > 1) {
+            float4 part[FT_MAX_SHARES];                        // all on their way before the first is added
             const uint32_t a = smem_u32(sums + e);
-            s = ft_peer(a, 0);
-            for (int p = 1; p < S; ++p) s += ft_peer(a, p);
-        } else {
-            s = sums[e];
+#pragma unroll
+            for (int p = 0; p < FT_MAX_SHARES; ++p)
+                if (p < S) part[p] = ft_peer(a, p);
+            s = part[0];
+#pragma unroll
+            for (int p = 1; p < FT_MAX_SHARES; ++p)
+                if (p < S) {
+                    s.x += part[p].x;
+                    s.y += part[p].y;
+                    s.z += part[p].z;
+                    s.w += part[p].w;
+                }
         }
-        C[(size_t)(m0 + m) * N + n0 + n] = s;
+        float* dst = C + (size_t)(m0 + m) * N + n0 + n;
+        if ((N & 3) == 0 && ((uintptr_t)C & 15) == 0) {
+            *reinterpret_cast<float4*>(dst) = s;
+        } else {
+            dst[0] = s.x;
+            if (n + 1 < cols) dst[1] = s.y;
+            if (n + 2 < cols) dst[2] = s.z;
+            if (n + 3 < cols) dst[3] = s.w;
+        }
     }
     if (S > 1) ft_cluster_sync();          // a block's sums stay until the others have read them
 }
 
+// A cut into parts, in the image the blocks copy: tile of bn rows after tile, block of 64 columns after block, part after part, a
+// part bn rows of 128 bytes in the 128-byte swizzle. A block of threads a row (of the last tile's absent rows too, zeros).
+__global__ void __launch_bounds__(256)
+gemm_f32_image_kernel(const float* __restrict__ A, unsigned char* __restrict__ image, unsigned char* __restrict__ image_odd, int M, int K,
+                      int bn, int vec) {
+    pdl_wait();
+    pdl_trigger();
+    const int row = blockIdx.x, r = row % bn, num_kb = (K + FT_BK - 1) / FT_BK;
+    unsigned char* tile = image + (size_t)(row / bn) * num_kb * 3 * bn * 128 + r * 128;
+    int odd = 0;
+    for (int i = threadIdx.x; i < num_kb * 16; i += 256) {
+        const int c = i & 15;
+        FtRaw<float> x;
+        ft_fetch(x, A + (size_t)row * K + 4 * i, row < M ? K - 4 * i : 0, vec);
+        odd |= ft_store(x, tile + (size_t)(i >> 4) * 3 * bn * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8, bn * 128);
+    }
+    odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) image_odd[row] = odd != 0;
+}
+
+// Rows of A a block: as few tiles as there can be, of even height.
+static int gemm_f32_tc_tile(int M) {
+    const int tiles = (M + FT_MAX_BN - 1) / FT_MAX_BN;
+    return ((M + tiles - 1) / tiles + 15) / 16 * 16;
+}
+static size_t gemm_f32_tc_image(int M, int K) {               // bytes of the image, without the marks behind it
+    const int bn = gemm_f32_tc_tile(M);
+    return bn <= 32 ? 0 : (size_t)((M + bn - 1) / bn) * bn * ((K + FT_BK - 1) / FT_BK) * 3 * 128;
+}
+
 template <typename TW, int BN>
-static int gemm_f32_tc_go(const float* A, const TW* W, float* C, int M, int N, int K, int bn, int S, int give_up_at, int* err,
-                          cudaStream_t stream) {
+static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* work, int M, int N, int K, int bn, int S,
+                          int give_up_at, int* err, cudaStream_t stream) {
     using F = FtShape<TW, BN>;
     auto k = gemm_f32_tc_kernel<TW, BN>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
     if (e != cudaSuccess) return (int)e;
-    const int vec = (K & 3) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
+    const int vec_a = (K & 3) == 0 && ((uintptr_t)A & 15) == 0, vec_w = (K & 3) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
+    const int tiles = (M + bn - 1) / bn;
+    unsigned char* odd = F::IMAGE ? work + gemm_f32_tc_image(M, K) : nullptr;
+    if (F::IMAGE) {
+        lumen_launch(gemm_f32_image_kernel, dim3(tiles * bn), dim3(256), 0, stream, A, work, odd, M, K, bn, vec_a);
+        LUMEN_LAUNCH_CHECK();
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(S, (M + bn - 1) / bn, (N + FT_ROWS - 1) / FT_ROWS);
+    cfg.gridDim = dim3(S, tiles, (N + FT_ROWS - 1) / FT_ROWS);
     cfg.blockDim = dim3(32 * F::WARPS);
     cfg.dynamicSmemBytes = F::SMEM;
     cfg.stream = stream;
@@ -421,7 +512,8 @@ static int gemm_f32_tc_go(const float* A, const TW* W, float* C, int M, int N, i
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = lumen_pdl_enabled() ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, k, A, W, C, M, N, K, bn, vec, give_up_at, err);
+    e = cudaLaunchKernelEx(&cfg, k, A, (const unsigned char*)work, (const unsigned char*)odd, W, C, M, N, K, bn,
+                           F::IMAGE ? vec_w : vec_a && vec_w, give_up_at, err);
     if (e != cudaSuccess) return (int)e;
     LUMEN_LAUNCH_CHECK();
     return 0;
@@ -436,17 +528,19 @@ static int gemm_f32_tc_shares(int N, int K) {
 }
 
 template <typename TW>
-static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, int M, int N, int K, int give_up_at, int* err,
+static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, unsigned char* work, int M, int N, int K, int give_up_at, int* err,
                             cudaStream_t stream) {
-    const int S = gemm_f32_tc_shares(N, K);
-    const int tiles = (M + FT_MAX_BN - 1) / FT_MAX_BN;
-    const int bn = ((M + tiles - 1) / tiles + 15) / 16 * 16;
-    if (bn <= 16) return gemm_f32_tc_go<TW, 16>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
-    if (bn <= 32) return gemm_f32_tc_go<TW, 32>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
-    if (bn <= 64) return gemm_f32_tc_go<TW, 64>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
-    if (bn <= 96) return gemm_f32_tc_go<TW, 96>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
-    if (bn <= 128) return gemm_f32_tc_go<TW, 128>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
-    return gemm_f32_tc_go<TW, 160>(A, W, C, M, N, K, bn, S, give_up_at, err, stream);
+    const int S = gemm_f32_tc_shares(N, K), bn = gemm_f32_tc_tile(M);
+#define FT_GO(BN) \
+    if (bn <= BN) return gemm_f32_tc_go<TW, BN>(A, W, C, work, M, N, K, bn, S, give_up_at, err, stream)
+    FT_GO(16);
+    FT_GO(32);
+    FT_GO(64);
+    FT_GO(96);
+    FT_GO(128);
+    FT_GO(160);
+#undef FT_GO
+    return LUMEN_ERR_UNSUPPORTED;
 }
 
 // 1 if weights [N, K] go through this kernel, whatever M: by N and K alone, so that a row's value is the same in any batch.
@@ -454,13 +548,21 @@ static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, int M, int N,
 // 2,048 x 256 x 256 11 / 18.
 LUMEN_API int lumen_gemm_f32_tc_takes(int N, int K) { return N >= FT_MIN_N && K >= FT_MIN_K ? 1 : 0; }
 
-// A float32 [M, K], W float32 or bfloat16 [N, K], C float32 [M, N], rows dense; any alignment their types have. give_up_at:
-// the block of k at which the adding warps take their wait as run out (-1: none; for tests of what a block does then).
-LUMEN_API int lumen_gemm_f32_tc(const float* A, const void* W, int w_is_bf16, float* C, int M, int N, int K, int give_up_at,
-                                int* err, cudaStream_t stream) {
+// Bytes of scratch lumen_gemm_f32_tc needs.
+LUMEN_API long long lumen_gemm_f32_tc_scratch(int M, int K) {
+    const size_t image = M > 0 && K > 0 ? gemm_f32_tc_image(M, K) : 0;
+    return image ? (long long)(image + M + FT_MAX_BN) : 0;
+}
+
+// A float32 [M, K], W float32 or bfloat16 [N, K], C float32 [M, N], rows dense, of any alignment their types
+// have. work: lumen_gemm_f32_tc_scratch(M, K) bytes, 16-byte aligned. give_up_at: the block of k at which the adding warps
+// take their wait as run out (-1: none; for tests of what a block does then).
+LUMEN_API int lumen_gemm_f32_tc(const float* A, const void* W, int w_is_bf16, float* C, void* work, int M, int N, int K,
+                                int give_up_at, int* err, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0) return LUMEN_ERR_BAD_ARGUMENT;
+    if (K <= 0 || ((uintptr_t)work & 15) || (!work && gemm_f32_tc_image(M, K))) return LUMEN_ERR_BAD_ARGUMENT;
     if ((M + 63) / 64 > 65535 || (N + FT_ROWS - 1) / FT_ROWS > 65535) return LUMEN_ERR_UNSUPPORTED;
-    return w_is_bf16 ? gemm_f32_tc_rows(A, (const __nv_bfloat16*)W, C, M, N, K, give_up_at, err, stream)
-                     : gemm_f32_tc_rows(A, (const float*)W, C, M, N, K, give_up_at, err, stream);
+    unsigned char* w = (unsigned char*)work;
+    return w_is_bf16 ? gemm_f32_tc_rows(A, (const __nv_bfloat16*)W, C, w, M, N, K, give_up_at, err, stream)
+                     : gemm_f32_tc_rows(A, (const float*)W, C, w, M, N, K, give_up_at, err, stream);
 }

@@ -1481,8 +1481,12 @@ def gemm_f32(a, w, out=None):
     if out is None:
         out = torch.empty((M, N), dtype=F32, device=a.device)
     if int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_takes", [c_int, c_int])(N, K):
-        f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, c_int, c_int, c_int, c_int, P, P])
-        check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), M, N, K, -1, ptr(error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
+        size = int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_scratch", [c_int, c_int])
+        size.restype = c_longlong
+        n = size(M, K)
+        work = torch.empty((n,), dtype=torch.uint8, device=a.device) if n else None      # a cut into its parts
+        f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, P, c_int, c_int, c_int, c_int, P, P])
+        check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), ptr(work), M, N, K, -1, ptr(error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
         return out
     f = fn("gemm_f32", "lumen_gemm_f32", [P, P, c_int, P, c_int, c_int, c_int, P])
     check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), M, N, K, stream_ptr()), "gemm_f32")
