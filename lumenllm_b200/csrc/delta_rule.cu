@@ -76,25 +76,26 @@ template <int N> __device__ __forceinline__ void dr_wait() { asm volatile("cp.as
 
 // prep [N, H, 3 dp + 4]: row (n, h) = [q normed and scaled (dp) | k normed (dp) | decays (dp) | k . q, beta, 0, 0];
 // the dp - d values past a head's own are 0, 0 and 1.
-__global__ void __launch_bounds__(32 * DR_PREP_WARPS)
-delta_prepare_kernel(const float* __restrict__ x, int C, int q_col, int k_col,
-                     const float* __restrict__ u, int uS, size_t u_stride, int uW, int b_col,
-                     const float* __restrict__ a, int aS, size_t a_stride, const float* __restrict__ dt_bias,
-                     const float* __restrict__ a_log, float* __restrict__ prep, int N, int H, int G, int d, int dp) {
-    // No early trigger here: the walk that follows has about one block an SM and must find the SMs
-    // empty, so that its blocks are spread one an SM; started under this kernel's blocks they were
-    // packed several an SM wherever room was, and the walk took twice as long.
-    pdl_wait();
-    const int n = blockIdx.x, h = blockIdx.y * DR_PREP_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (h >= H) return;
-    const int g = h / (H / G);
-    const float a_neg = -expf(a_log[h]);
+// What a (token, head) needs, in one place.
+struct DrIn {
+    const float* x;           // [N, C]
+    const float* u;           // projection partial sums with the beta logits
+    const float* a;           // partial sums of the decay logits
+    const float* dt_bias;
+    const float* a_log;
+    size_t u_stride, a_stride;
+    int C, q_col, k_col, uS, uW, b_col, aS, H, G, d;
+};
+// One row, by a warp. out: dp floats each of q, k and decays, then k . q and beta.
+__device__ __forceinline__ void dr_prepare_row(const DrIn& in, int n, int h, int dp, float* out) {
+    const int lane = threadIdx.x & 31, d = in.d;
+    const int g = h / (in.H / in.G);
+    const float a_neg = -expf(in.a_log[h]);
     const float q_scale = rsqrtf((float)d);
-    const float* row = x + (size_t)n * C;
-    float* out = prep + ((size_t)n * H + h) * (3 * dp + 4);
+    const float* row = in.x + (size_t)n * in.C;
     float sq = 0.0f, sk = 0.0f;
     for (int e = lane; e < d; e += 32) {
-        const float qv = row[q_col + g * d + e], kv = row[k_col + g * d + e];
+        const float qv = row[in.q_col + g * d + e], kv = row[in.k_col + g * d + e];
         sq += qv * qv;
         sk += kv * kv;
     }
@@ -105,9 +106,9 @@ delta_prepare_kernel(const float* __restrict__ x, int C, int q_col, int k_col,
     for (int e = lane; e < dp; e += 32) {
         float qv = 0.0f, kv = 0.0f, gv = 1.0f;
         if (e < d) {
-            qv = row[q_col + g * d + e] * rq;
-            kv = row[k_col + g * d + e] * rk;
-            const float av = dr_parts(a + (size_t)n * H * d + h * d + e, aS, a_stride) + dt_bias[h * d + e];
+            qv = row[in.q_col + g * d + e] * rq;
+            kv = row[in.k_col + g * d + e] * rk;
+            const float av = dr_parts(in.a + (size_t)n * in.H * d + h * d + e, in.aS, in.a_stride) + in.dt_bias[h * d + e];
             gv = expf(a_neg * dr_softplus(av));
         }
         out[e] = qv;
@@ -119,22 +120,30 @@ delta_prepare_kernel(const float* __restrict__ x, int C, int q_col, int k_col,
     if (lane < 4) {
         float v = 0.0f;
         if (lane == 0) v = dot;
-        if (lane == 1) v = 1.0f / (1.0f + expf(-dr_parts(u + (size_t)n * uW + b_col + h, uS, u_stride)));
+        if (lane == 1) v = 1.0f / (1.0f + expf(-dr_parts(in.u + (size_t)n * in.uW + in.b_col + h, in.uS, in.u_stride)));
         out[3 * dp + lane] = v;
     }
+}
+
+__global__ void __launch_bounds__(32 * DR_PREP_WARPS)
+delta_prepare_kernel(const DrIn in, float* __restrict__ prep, int dp) {
+    // No early trigger here: the walk that follows has about one block an SM and must find the SMs
+    // empty, so that its blocks are spread one an SM; started under this kernel's blocks they were
+    // packed several an SM wherever room was, and the walk took twice as long.
+    pdl_wait();
+    const int n = blockIdx.x, h = blockIdx.y * DR_PREP_WARPS + (threadIdx.x >> 5);
+    if (h >= in.H) return;
+    dr_prepare_row(in, n, h, dp, prep + ((size_t)n * in.H + h) * (3 * dp + 4));
 }
 
 // NS: threads that share a column of S (a power of two), NS DR_ROWS >= d; every offset of the walk is a constant
 // of the instance. AHEAD: a token's rows are read from shared memory while the one before is worked on, which
 // takes twice the registers: for steps of several tokens a sequence. THREADS: of a block. Same sums either way.
+// row0: the row of the sequence's first token, the next ones row_stride floats on; zblock: which columns.
 template <int NS, bool AHEAD, int THREADS>
-__global__ void __launch_bounds__(THREADS)
-delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __restrict__ prep,
-                  float* __restrict__ state, size_t slot_stride, const int* __restrict__ cu_q,
-                  const int* __restrict__ seq_slot, float* __restrict__ y, int H, int d, int dv, int vec) {
-    pdl_trigger();
-    pdl_wait();
-    extern __shared__ __align__(16) float sm[];
+__device__ __forceinline__ void dr_walk(float* sm, const float* __restrict__ x, int C, int v_col, const float* __restrict__ row0,
+                                        size_t row_stride, int t_begin, int t_end, int zblock, float* __restrict__ S_head,
+                                        float* __restrict__ y, int H, int d, int dv, int vec) {
     constexpr int ROWS = DR_ROWS;
     constexpr int dp = NS * ROWS;                   // d padded to what the threads of a column hold
     constexpr int GR = ROWS / 4;
@@ -142,12 +151,10 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
     constexpr int cols = THREADS / NS;
     float* rows = sm;                               // [2][DR_CHUNK][PW]
     float* vs = sm + 2 * DR_CHUNK * PW;             // [2][DR_CHUNK][cols]
-    const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-    const int t_begin = cu_q[b], t_end = cu_q[b + 1];
-    if (t_end <= t_begin) return;
-    const int s = tid % NS, cj = tid / NS, j = blockIdx.z * cols + cj;
+    const int h = blockIdx.y, tid = threadIdx.x;
+    const int s = tid % NS, cj = tid / NS, j = zblock * cols + cj;
     const bool live = j < dv;
-    float* Sj = state + (size_t)seq_slot[b] * slot_stride + ((size_t)h * dv + (live ? j : 0)) * d;
+    float* Sj = S_head + (size_t)(live ? j : 0) * d;
     f32x2 S[2 * GR];                                // rows 4 (i NS + s) .. + 3 in S[2 i], S[2 i + 1]
 #pragma unroll
     for (int i = 0; i < GR; ++i) {
@@ -172,11 +179,11 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
         float* rb = rows + buf * DR_CHUNK * PW;
         for (int i = tid; i < nt * pieces; i += THREADS) {
             const int tt = i / pieces, p = i - tt * pieces;
-            dr_cp16(rb + tt * PW + 4 * p, prep + ((size_t)(t0 + tt) * H + h) * PW + 4 * p);
+            dr_cp16(rb + tt * PW + 4 * p, row0 + (size_t)(t0 + tt - t_begin) * row_stride + 4 * p);
         }
         float* vb = vs + buf * DR_CHUNK * cols;
         for (int i = tid; i < nt * cols; i += THREADS) {
-            const int tt = i / cols, c = i - tt * cols, jj = blockIdx.z * cols + c;
+            const int tt = i / cols, c = i - tt * cols, jj = zblock * cols + c;
             if (jj < dv) dr_cp4(vb + i, x + (size_t)(t0 + tt) * C + v_col + h * dv + jj);
             else vb[i] = 0.0f;
         }
@@ -305,6 +312,338 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
     }
 }
 
+template <int NS, bool AHEAD, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __restrict__ prep,
+                  float* __restrict__ state, size_t slot_stride, const int* __restrict__ cu_q,
+                  const int* __restrict__ seq_slot, float* __restrict__ y, int H, int d, int dv, int vec) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    constexpr int PW = 3 * NS * DR_ROWS + 4;
+    const int b = blockIdx.x, h = blockIdx.y, t_begin = cu_q[b], t_end = cu_q[b + 1];
+    if (t_end <= t_begin) return;
+    dr_walk<NS, AHEAD, THREADS>(sm, x, C, v_col, prep + ((size_t)t_begin * H + h) * PW, (size_t)H * PW, t_begin, t_end, blockIdx.z,
+                                state + (size_t)seq_slot[b] * slot_stride + (size_t)h * dv * d, y, H, d, dv, vec);
+}
+
+// ------------------------------------------------------------------- sixteen tokens at a time
+// For heads of 65 to 128 key channels a sequence's tokens go in chunks of sixteen (from its first of the step on). With
+// P_t = g_1 .. g_t the decays since the chunk's start, channel by channel, and S the state there,
+//   u_t = beta_t (v_t - S^T (P_t k_t) - sum_{i<t} A_ti u_i),   A_ti = k_t . (g_{i+1} .. g_t k_i)
+//   o_t = S^T (P_t q_t) + sum_{i<=t} B_ti u_i,                 B_ti = q_t . (g_{i+1} .. g_t k_i)
+//   S  <- P_16 S + sum_i (g_{i+1} .. g_16 k_i) u_i^T,
+// the same numbers as token by token, in another order of sums. A, B, the three sets of scaled vectors and
+// T = (1 + beta A)^-1 beta (so that u = T (v - S^T P k)) need no state: a kernel makes them for all chunks at once. Every
+// factor is a product of decays, at most 1, never a quotient; T's entries are at most 1 in size, as unit vectors and beta
+// below 1 make every step a contraction. What is left to the walk is three products with S a chunk, which have no chain
+// from token to token. A thread keeps 4 key channels of 4 columns of S, a warp all channels of four columns; sums over
+// channels change lanes a chunk at a time, 32 sums by 31 exchanges. Two warps keep the same four columns: one makes the sums
+// of P k and u, the other meanwhile those of P q and then o, and both move their S on. Zeros above the
+// diagonal are not multiplied, so that what is not finite in a token reaches no earlier one.
+// Sequences of fewer than sixteen tokens walk them one by one, with the sums of a decode step.
+// MEASURED
+#define DC_T 16
+#define DC_D 128
+#define DC_PITCH 20                                              // floats a row of T and of B
+#define DC_KT 0
+#define DC_QT (DC_T * DC_D)
+#define DC_KB (2 * DC_T * DC_D)
+#define DC_P (3 * DC_T * DC_D)
+#define DC_TM (DC_P + DC_D)
+#define DC_BM (DC_TM + DC_T * DC_PITCH)
+#define DC_REC (DC_BM + DC_T * DC_PITCH)                         // floats of a (chunk, head)
+#define DC_ROW (3 * DC_D + 4)                                    // a token's row, as above
+#define DC_WARPS 16                                              // of the kernel that prepares: one a token
+static_assert(DC_T * DC_ROW <= DC_REC, "a short sequence's rows lie in the record of its first chunk");
+
+// Where the chunks of sequence b start among all records: room for every cut of N tokens.
+__device__ __forceinline__ int dc_first(const int* cu_q, int b) { return cu_q[b] / DC_T + b; }
+
+__global__ void __launch_bounds__(32 * DC_WARPS)
+delta_chunk_prepare_kernel(const DrIn in, float* __restrict__ prep, const int* __restrict__ cu_q, int n_seqs) {
+    pdl_wait();              // no early trigger, as above
+    __shared__ __align__(16) float rows[DC_T * DC_ROW];
+    __shared__ float A[DC_T][DC_T + 1];
+    const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int lo = 0, hi = n_seqs - 1;                   // the last sequence whose records start at or before this one
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (dc_first(cu_q, mid) <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const int t_begin = cu_q[lo], t_end = cu_q[lo + 1], t0 = t_begin + ((int)blockIdx.x - dc_first(cu_q, lo)) * DC_T;
+    if (t0 < t_begin || t0 >= t_end) return;
+    const int nt = min(DC_T, t_end - t0);
+    float* rec = prep + ((size_t)blockIdx.x * in.H + h) * DC_REC;
+    const bool is_short = t_end - t_begin < DC_T;
+    {
+        float* row = is_short ? rec + warp * DC_ROW : rows + warp * DC_ROW;
+        if (warp < nt) {
+            dr_prepare_row(in, t0 + warp, h, DC_D, row);
+        } else if (!is_short) {                    // no token: nothing decays, nothing is written
+            for (int e = lane; e < DC_ROW; e += 32) row[e] = (e >= 2 * DC_D && e < 3 * DC_D) ? 1.0f : 0.0f;
+        }
+    }
+    if (is_short) return;
+    __syncthreads();
+    {                                              // columns i = warp of A and B, a lane four channels
+        const int i = warp;
+        float4 p = *reinterpret_cast<const float4*>(rows + i * DC_ROW + DC_D + 4 * lane);
+        f32x2 v[DC_T];                             // this lane's shares of A_ti and B_ti
+#pragma unroll
+        for (int t = 0; t < DC_T; ++t) {
+            v[t] = 0ull;
+            if (t < i) continue;
+            const float* r = rows + t * DC_ROW + 4 * lane;
+            const float4 q = *reinterpret_cast<const float4*>(r), k = *reinterpret_cast<const float4*>(r + DC_D);
+            if (t > i) {
+                const float4 g = *reinterpret_cast<const float4*>(r + 2 * DC_D);
+                p.x *= g.x;
+                p.y *= g.y;
+                p.z *= g.z;
+                p.w *= g.w;
+            }
+            v[t] = pair2(fmaf(p.y, k.y, p.x * k.x) + fmaf(p.w, k.w, p.z * k.z), fmaf(p.y, q.y, p.x * q.x) + fmaf(p.w, q.w, p.z * q.z));
+        }
+#pragma unroll
+        for (int o = 16; o > 1; o >>= 1) {         // lanes 2 t and 2 t + 1 get the sums of t, but for their own two shares
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int t = 0; t < o / 2; ++t) {
+                const f32x2 give = up ? v[t] : v[t + o / 2], keep = up ? v[t + o / 2] : v[t];
+                v[t] = add2(keep, __shfl_xor_sync(0xffffffffu, give, o));
+            }
+        }
+        const float2 ab = unpair2(add2(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1)));
+        const int t = lane >> 1;
+        if (t >= i) {
+            if (lane & 1) rec[DC_BM + t * DC_PITCH + i] = ab.y;
+            else A[t][i] = ab.x;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        if (lane < DC_T) {                         // column `lane` of T, from its diagonal down
+            float T[DC_T];
+#pragma unroll
+            for (int t = 0; t < DC_T; ++t) {
+                const float beta = rows[t * DC_ROW + 3 * DC_D + 1];
+                float s = 0.0f;
+#pragma unroll
+                for (int i = 0; i < t; ++i)
+                    if (i >= lane) s = fmaf(A[t][i], T[i], s);
+                T[t] = t < lane ? 0.0f : t == lane ? beta : -beta * s;
+                rec[DC_TM + t * DC_PITCH + lane] = T[t];
+            }
+        }
+    } else if (warp >= 4 && warp < 8) {            // a thread a channel
+        const int c = threadIdx.x - 4 * 32;
+        float P = 1.0f;
+#pragma unroll
+        for (int t = 0; t < DC_T; ++t) {
+            const float* r = rows + t * DC_ROW + c;
+            P *= r[2 * DC_D];
+            rec[DC_KT + t * DC_D + c] = P * r[DC_D];
+            rec[DC_QT + t * DC_D + c] = P * r[0];
+        }
+        rec[DC_P + c] = P;
+        float R = 1.0f;
+#pragma unroll
+        for (int t = DC_T - 1; t >= 0; --t) {
+            const float* r = rows + t * DC_ROW + c;
+            rec[DC_KB + t * DC_D + c] = R * r[DC_D];
+            R *= r[2 * DC_D];
+        }
+    }
+}
+
+#define DC_COLS 16                                              // columns of S a block: four a pair of warps
+#define DC_BUF (DC_REC + DC_T * DC_COLS)                        // floats of a staged chunk: the record, the values
+#define DC_THREADS 256
+#define DC_SMEM ((2 * DC_BUF + 2 * 4 * DC_T * 4) * (int)sizeof(float))
+
+// 32 pairs of sums over the lanes: lane l gets pair l.
+__device__ __forceinline__ f32x2 dc_reduce(f32x2 (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const f32x2 give = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+            v[i] = add2(keep, __shfl_xor_sync(0xffffffffu, give, o));
+        }
+    }
+    return v[0];
+}
+
+__global__ void __launch_bounds__(DC_THREADS)
+delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* __restrict__ prep, float* __restrict__ state,
+                   size_t slot_stride, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, float* __restrict__ y, int H,
+                   int d, int dv, int vec) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5 & 3, lane = tid & 31;
+    const bool reads = tid >= DC_THREADS / 2;                   // of the two warps of four columns: makes o
+    const int t_begin = cu_q[b], t_end = cu_q[b + 1];
+    if (t_end <= t_begin) return;
+    const float* rec0 = prep + ((size_t)dc_first(cu_q, b) * H + h) * DC_REC;
+    float* S_head = state + (size_t)seq_slot[b] * slot_stride + (size_t)h * dv * d;
+    if (t_end - t_begin < DC_T) {                              // 32 columns a block
+        if (blockIdx.z & 1) return;
+        dr_walk<8, false, DC_THREADS>(sm, x, C, v_col, rec0, DC_ROW, t_begin, t_end, blockIdx.z >> 1, S_head, y, H, d, dv, vec);
+        return;
+    }
+    const int j0 = blockIdx.z * DC_COLS + 4 * warp, c0 = 4 * lane;
+    float* xs = sm + 2 * DC_BUF + warp * DC_T * 4;              // these four columns' [16][4] numbers, twice
+    float* us = xs + 4 * DC_T * 4;
+    f32x2 S[4][2];                                              // channel c0 + c, columns j0 + 2 p and + 1
+    {
+        float v[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float* p = S_head + (size_t)(j0 + j) * d + c0;
+            const bool live = j0 + j < dv;
+            if (vec) {
+                float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (live && c0 < d) q = *reinterpret_cast<const float4*>(p);
+                v[j][0] = q.x; v[j][1] = q.y; v[j][2] = q.z; v[j][3] = q.w;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[j][c] = (live && c0 + c < d) ? p[c] : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            S[c][0] = pair2(v[0][c], v[1][c]);
+            S[c][1] = pair2(v[2][c], v[3][c]);
+        }
+    }
+    auto issue = [&](int t0, int chunk, int buf) {
+        float* to = sm + buf * DC_BUF;
+        const float* from = rec0 + (size_t)chunk * H * DC_REC;
+        for (int i = tid; i < DC_REC / 4; i += DC_THREADS) dr_cp16(to + 4 * i, from + 4 * i);
+        static_assert(DC_T * DC_COLS == DC_THREADS, "a thread a value");
+        const int t = t0 + tid / DC_COLS, j = blockIdx.z * DC_COLS + tid % DC_COLS;
+        if (t < t_end && j < dv) dr_cp4(to + DC_REC + tid, x + (size_t)t * C + v_col + h * dv + j);
+        else to[DC_REC + tid] = 0.0f;
+        dr_commit();
+    };
+    // rows of scaled vectors against S: lane l gets the sums of token l / 2, columns j0 + 2 (l % 2) and + 1
+    auto times_S = [&](const float* vecs) {
+        f32x2 v[32];
+#pragma unroll
+        for (int t = 0; t < DC_T; ++t) {
+            const float4 k = *reinterpret_cast<const float4*>(vecs + t * DC_D + c0);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                f32x2 r = mul2(pair2(k.x, k.x), S[0][p]);
+                r = fma2(pair2(k.y, k.y), S[1][p], r);
+                r = fma2(pair2(k.z, k.z), S[2][p], r);
+                v[2 * t + p] = fma2(pair2(k.w, k.w), S[3][p], r);
+            }
+        }
+        return dc_reduce(v);
+    };
+    issue(t_begin, 0, 0);
+    const int tt = lane >> 1, jp = 2 * (lane & 1);
+    for (int t0 = t_begin, it = 0; t0 < t_end; t0 += DC_T, ++it) {
+        const int nt = min(DC_T, t_end - t0);
+        if (t0 + DC_T < t_end) {
+            issue(t0 + DC_T, it + 1, (it + 1) & 1);             // under way while this chunk is worked on
+            dr_wait<1>();
+        } else {
+            dr_wait<0>();
+        }
+        __syncthreads();
+        const float* rec = sm + (it & 1) * DC_BUF;
+        // sum_{i <= tt} M[tt][i] z[i], from a start, in two chains
+        auto lower = [&](const float* M, const float* z, f32x2 s) {
+            float m[DC_T];
+#pragma unroll
+            for (int i = 0; i < DC_T; i += 4)
+                *reinterpret_cast<float4*>(m + i) = *reinterpret_cast<const float4*>(M + tt * DC_PITCH + i);
+            f32x2 s2 = 0ull;
+#pragma unroll
+            for (int i = 0; i < DC_T; i += 2) {
+                const f32x2 z0 = *reinterpret_cast<const f32x2*>(z + i * 4 + jp), z1 = *reinterpret_cast<const f32x2*>(z + i * 4 + 4 + jp);
+                if (i <= tt) s = fma2(pair2(m[i], m[i]), z0, s);
+                if (i + 1 <= tt) s2 = fma2(pair2(m[i + 1], m[i + 1]), z1, s2);
+            }
+            return add2(s, s2);
+        };
+        const f32x2 sums = times_S(rec + (reads ? DC_QT : DC_KT));
+        if (!reads) {
+            const float2 R = unpair2(sums);
+            const float2 v = *reinterpret_cast<const float2*>(rec + DC_REC + tt * DC_COLS + 4 * warp + jp);
+            *reinterpret_cast<float2*>(xs + tt * 4 + jp) = make_float2(v.x - R.x, v.y - R.y);
+            __syncwarp();
+            *reinterpret_cast<f32x2*>(us + tt * 4 + jp) = lower(rec + DC_TM, xs, 0ull);
+        }
+        __syncthreads();
+        if (reads) {
+            const float2 o = unpair2(lower(rec + DC_BM, us, sums));
+            if (tt < nt) {
+                float* dst = y + (size_t)(t0 + tt) * H * dv + (size_t)h * dv + j0 + jp;
+                if ((dv & 1) == 0) {
+                    if (j0 + jp < dv) *reinterpret_cast<float2*>(dst) = o;
+                } else {
+                    if (j0 + jp < dv) dst[0] = o.x;
+                    if (j0 + jp + 1 < dv) dst[1] = o.y;
+                }
+            }
+        }
+        const float4 P = *reinterpret_cast<const float4*>(rec + DC_P + c0);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            S[0][p] = mul2(pair2(P.x, P.x), S[0][p]);
+            S[1][p] = mul2(pair2(P.y, P.y), S[1][p]);
+            S[2][p] = mul2(pair2(P.z, P.z), S[2][p]);
+            S[3][p] = mul2(pair2(P.w, P.w), S[3][p]);
+        }
+        auto add = [&](int t) {
+            const float4 k = *reinterpret_cast<const float4*>(rec + DC_KB + t * DC_D + c0);
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(us + t * 4);
+            S[0][0] = fma2(pair2(k.x, k.x), u.x, S[0][0]);
+            S[0][1] = fma2(pair2(k.x, k.x), u.y, S[0][1]);
+            S[1][0] = fma2(pair2(k.y, k.y), u.x, S[1][0]);
+            S[1][1] = fma2(pair2(k.y, k.y), u.y, S[1][1]);
+            S[2][0] = fma2(pair2(k.z, k.z), u.x, S[2][0]);
+            S[2][1] = fma2(pair2(k.z, k.z), u.y, S[2][1]);
+            S[3][0] = fma2(pair2(k.w, k.w), u.x, S[3][0]);
+            S[3][1] = fma2(pair2(k.w, k.w), u.y, S[3][1]);
+        };
+        if (nt == DC_T) {
+#pragma unroll
+            for (int t = 0; t < DC_T; ++t) add(t);
+        } else {
+            for (int t = 0; t < nt; ++t) add(t);
+        }
+        __syncthreads();                            // this chunk has been read by everyone before its buffer is filled again
+    }
+    if (reads) return;                              // its S is the other warp's
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j0 + j >= dv) continue;
+        float* p = S_head + (size_t)(j0 + j) * d + c0;
+        float v[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float2 w = unpair2(S[c][j >> 1]);
+            v[c] = (j & 1) ? w.y : w.x;
+        }
+        if (vec) {
+            if (c0 < d) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (c0 + c < d) p[c] = v[c];
+        }
+    }
+}
+
 // Threads a column for d key channels.
 static inline int delta_rule_threads(int d) {
     int NS = 1;
@@ -312,16 +651,20 @@ static inline int delta_rule_threads(int d) {
     return NS;
 }
 
-// Floats of scratch lumen_delta_rule needs for every (token, head) with d key channels.
-LUMEN_API int lumen_delta_rule_scratch_row(int d) {
-    return 3 * delta_rule_threads(d) * DR_ROWS + 4;
+// Steps whose sequences go in chunks: heads of 65 to 128, and not one token a sequence.
+static inline bool delta_rule_chunks(int d, int N, int n_seqs) { return d > DC_D / 2 && d <= DC_D && N > n_seqs; }
+
+// Floats of scratch lumen_delta_rule needs for a step of N tokens in n_seqs sequences, H heads of d key channels.
+LUMEN_API long long lumen_delta_rule_scratch(int N, int n_seqs, int H, int d) {
+    if (delta_rule_chunks(d, N, n_seqs)) return ((long long)N / DC_T + n_seqs) * H * DC_REC;
+    return (long long)N * H * (3 * delta_rule_threads(d) * DR_ROWS + 4);
 }
 
 // x float32 [N, C]: the convolved and activated q (G heads of d, from column q_col), k (k_col)
 // and v (H heads of dv, v_col). u: the projection's partial sums [uS, N, uW] with the H beta
 // logits from column b_col. a: partial sums [aS, N, H d] of the decay logits (before dt_bias).
 // state float32, row seq_slot[b] of stride slot_stride holds [H, dv, d]. y float32 [N, H dv]. prep:
-// N H lumen_delta_rule_scratch_row(d) floats of scratch.
+// lumen_delta_rule_scratch(N, n_seqs, H, d) floats of scratch. cu_q covers at most N tokens.
 LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int v_col, const float* u, int uS,
                                long long u_stride, int uW, int b_col, const float* a, int aS, long long a_stride,
                                const float* dt_bias, const float* a_log, float* state, long long slot_stride,
@@ -340,10 +683,21 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
     const bool wide = NS == 32 && (long long)n_seqs * H * ((dv + DR_THREADS / NS - 1) / (DR_THREADS / NS)) > 148;
     const int threads = wide ? 2 * DR_THREADS : DR_THREADS, cols = threads / NS;
     const int vec = (d & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
+    const DrIn in = {x, u, a, dt_bias, a_log, (size_t)u_stride, (size_t)a_stride, C, q_col, k_col, uS, uW, b_col, aS, H, G, d};
+    if (delta_rule_chunks(d, N, n_seqs)) {
+        if ((dv + DC_COLS - 1) / DC_COLS > 65535) return LUMEN_ERR_UNSUPPORTED;
+        cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        lumen_launch(delta_chunk_prepare_kernel, dim3(N / DC_T + n_seqs, H), dim3(32 * DC_WARPS), 0, stream, in, prep, cu_q, n_seqs);
+        LUMEN_LAUNCH_CHECK();
+        lumen_launch(delta_chunk_kernel, dim3(n_seqs, H, (dv + DC_COLS - 1) / DC_COLS), dim3(DC_THREADS), DC_SMEM, stream, x, C, v_col,
+                     (const float*)prep, state, (size_t)slot_stride, cu_q, seq_slot, y, H, d, dv, vec);
+        LUMEN_LAUNCH_CHECK();
+        return 0;
+    }
     dim3 pgrid(N, (H + DR_PREP_WARPS - 1) / DR_PREP_WARPS);
     if (pgrid.y > 65535) return LUMEN_ERR_UNSUPPORTED;
-    lumen_launch(delta_prepare_kernel, pgrid, dim3(32 * DR_PREP_WARPS), 0, stream, x, C, q_col, k_col, u, uS,
-                 (size_t)u_stride, uW, b_col, a, aS, (size_t)a_stride, dt_bias, a_log, prep, N, H, G, d, dp);
+    lumen_launch(delta_prepare_kernel, pgrid, dim3(32 * DR_PREP_WARPS), 0, stream, in, prep, dp);
     LUMEN_LAUNCH_CHECK();
     dim3 grid(n_seqs, H, (dv + cols - 1) / cols);
     if (grid.z > 65535) return LUMEN_ERR_UNSUPPORTED;

@@ -1456,9 +1456,10 @@ def delta_rule(x, q_col, k_col, v_col, u, beta_col, a, dt_bias, a_log, state, cu
     require(cu_q, I32, "delta_rule.cu_q")
     require(seq_slot, I32, "delta_rule.seq_slot")
     y = torch.empty((N, heads * dv), dtype=F32, device=x.device)
-    # what does not depend on the state, a row a (token, head), made by the kernel's first launch
-    row = int_fn("delta_rule", "lumen_delta_rule_scratch_row", [c_int])(int(d))
-    prep = torch.empty((N, int(heads), row), dtype=F32, device=x.device)
+    # what does not depend on the state, made by the kernel's first launch
+    size = int_fn("delta_rule", "lumen_delta_rule_scratch", [c_int, c_int, c_int, c_int])
+    size.restype = c_longlong
+    prep = torch.empty((size(N, int(n_seqs), int(heads), int(d)),), dtype=F32, device=x.device)
     f = fn("delta_rule", "lumen_delta_rule",
            [P, c_int, c_int, c_int, c_int, P, c_int, c_longlong, c_int, c_int, P, c_int, c_longlong, P, P, P, c_longlong,
             P, P, c_int, P, P, c_int, c_int, c_int, c_int, c_int, P])

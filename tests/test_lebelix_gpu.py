@@ -420,6 +420,59 @@ def test_delta_rule_of_wide_heads_alone_and_among_many(d, dv, tokens):
         assert torch.equal(yb, y[b * tokens:(b + 1) * tokens]) and torch.equal(sb, s[b:b + 1])
 
 
+@pytest.mark.parametrize("d,dv,lens", [(128, 128, [16, 15, 33, 0, 1]), (65, 33, [40, 2]), (100, 17, [48, 16, 31]), (128, 5, [300]),
+                                       (96, 16, [7, 1])])
+def test_delta_rule_sixteen_tokens_at_a_time(d, dv, lens):
+    """Heads of 65 to 128 go in chunks of sixteen tokens where a sequence has that many: against 64-bit sums token by token (a
+    chain of float32 steps that are contractions: rounding of some 20 operations a token, remembered for at most the 300
+    tokens here), chunks that end part full, and next to shorter sequences, whose bits are a decode step's. What is not finite in a token
+    stays out of the earlier ones and of other sequences."""
+    from lumenllm_b200.ops import kernels as K
+    H, G, B, N = 4, 2, len(lens), sum(lens)
+    g = torch.Generator().manual_seed(d + dv)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    C = 2 * G * d + H * dv
+    x, u, a, dt, al, st = rn(N, C), rn(2, N, H), rn(1, N, H * d), rn(H * d), rn(H) - 2.0, rn(B, H, dv, d)
+    cu = torch.tensor([0] + [sum(lens[:i + 1]) for i in range(B)], dtype=torch.int32)
+
+    def run(x, cu, st, rows_=slice(None)):
+        s = st.cuda()
+        y = K.delta_rule(x[rows_].contiguous().cuda(), 0, G * d, 2 * G * d, u[:, rows_].contiguous().cuda(), 0, a[:, rows_].contiguous().cuda(),
+                         dt.cuda(), al.cuda(), s, cu.cuda(), torch.arange(len(cu) - 1, dtype=torch.int32).cuda(), len(cu) - 1, H, G, d, dv)
+        return y.cpu(), s.cpu()
+
+    def unit(t):
+        return t / (t.pow(2).sum(-1, True) + 1e-6).sqrt()
+    xd = x.double()
+    q = unit(xd[:, :G * d].view(N, G, d)).repeat_interleave(H // G, 1) * d ** -0.5
+    k = unit(xd[:, G * d:2 * G * d].view(N, G, d)).repeat_interleave(H // G, 1)
+    v, beta = xd[:, 2 * G * d:].view(N, H, dv), torch.sigmoid(u.double().sum(0))
+    decay = torch.exp(-al.double().exp()[:, None] * torch.nn.functional.softplus((a[0].double() + dt.double()).view(N, H, d)))
+    y, s = run(x, cu, st)
+    S, ref = st.double(), torch.empty(N, H, dv, dtype=torch.float64)
+    for b in range(B):
+        for n in range(int(cu[b]), int(cu[b + 1])):
+            S[b] = S[b] * decay[n][:, None]
+            S[b] += (beta[n][:, None] * (v[n] - (S[b] @ k[n][..., None])[..., 0]))[..., None] * k[n][:, None]
+            ref[n] = (S[b] @ q[n][..., None])[..., 0]
+    assert float((y.double().view(N, H, dv) - ref).norm() / ref.norm()) < 2e-6
+    assert float((s.double() - S).norm() / S.norm()) < 2e-6
+    one = torch.tensor([0, 1], dtype=torch.int32)
+    for b in range(B):
+        if 0 < lens[b] < 16:                        # token by token, as decode steps
+            sb = st[b:b + 1]
+            for n in range(int(cu[b]), int(cu[b + 1])):
+                yn, sb = run(x, one, sb, slice(n, n + 1))
+                assert torch.equal(yn[0], y[n])
+            assert torch.equal(sb[0], s[b])
+    bad = x.clone()
+    last = int(cu[1]) - 1
+    bad[last, 2 * G * d + 3] = float("inf")
+    yb, sb = run(bad, cu, st)
+    assert torch.equal(yb[:last], y[:last]) and torch.equal(yb[last + 1:], y[last + 1:]) and torch.equal(sb[1:], s[1:])
+    assert not bool(torch.isfinite(yb[last]).all())
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_the_state_remembers_far_back_and_forgets_by_channel(dtype):
     """Decays close to one and one loud early token: what the state holds of that token decides the
