@@ -232,6 +232,183 @@ attn_generic_kernel(const TQ* __restrict__ q, const T* __restrict__ kcache, cons
     }
 }
 
+// Float32 prompts without options, heads of up to 128: the kernel above with AP_Q neighbouring tokens a block, so that the keys and
+// values are fetched once for all of them (a token each read them again). A chunk's keys are staged in shared memory; products of two
+// rows share an instruction, each rounded as by itself, and every sum runs in the order of the kernel above: the same bits. Tokens of
+// different sequences in a block are walked one sequence after the other. A key past a row's own token is not multiplied into it.
+// MEASURED
+#define AP_Q 4
+typedef unsigned long long ap_f2;
+__device__ __forceinline__ ap_f2 ap_pair(float lo, float hi) {
+    ap_f2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 ap_unpair(ap_f2 a) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ void ap_fma(ap_f2& c, ap_f2 a, ap_f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void ap_mul(ap_f2& c, ap_f2 a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
+__host__ __device__ constexpr int ap_smem(int HB, int d) {           // floats: keys, queries, weights
+    return AG_THREADS * (d + 4) + (d + AG_THREADS) * (HB * AP_Q + 4);
+}
+
+template <int HB>
+__global__ void __launch_bounds__(AG_THREADS)
+attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kcache, const float* __restrict__ vcache,
+                       const int* __restrict__ block_table, int bt_stride, const int* __restrict__ tok_seq,
+                       const int* __restrict__ tok_pos, float* __restrict__ out, int N, int nq, int nkv, int d, int dv, float scale) {
+    pdl_wait();      // nothing of this kernel touches global memory before this
+    pdl_trigger();
+    constexpr int R = HB * AP_Q, RP = R + 4;         // rows (token t, head h: t HB + h); floats a key's weights lie apart
+    extern __shared__ __align__(16) float sm[];
+    float* ks = sm;                                  // [128][d + 4]
+    float* qs = ks + AG_THREADS * (d + 4);           // [d][RP]
+    float* ps = qs + d * RP;                         // [128][RP]
+    __shared__ float red[R][32];
+    const int tid = threadIdx.x, head0 = blockIdx.y * HB, kvh = head0 / (nq / nkv);
+    const int n0 = blockIdx.x * AP_Q, nt = min(AP_Q, N - n0);
+    for (int i = tid; i < R * d; i += AG_THREADS) {
+        const int r = i / d, e = i - r * d, t = r / HB;
+        qs[e * RP + r] = t < nt ? q[((size_t)(n0 + t) * nq + head0 + r % HB) * d + e] : 0.0f;
+    }
+    for (int g0 = 0, g1; g0 < nt; g0 = g1) {
+        const int seq = tok_seq[n0 + g0];
+        for (g1 = g0 + 1; g1 < nt && tok_seq[n0 + g1] == seq; ++g1) {}
+        const int* bt = block_table + (size_t)seq * bt_stride;
+        int pos[AP_Q], p_max = -1, p_min = 0x7fffffff;
+#pragma unroll
+        for (int t = 0; t < AP_Q; ++t) {
+            pos[t] = (t >= g0 && t < g1) ? tok_pos[n0 + t] : -1;       // -1: no row of this walk
+            if (pos[t] >= 0) {
+                p_max = max(p_max, pos[t]);
+                p_min = min(p_min, pos[t]);
+            }
+        }
+        float m[R], l[R];
+        ap_f2 acc[R / 2];                            // value number tid
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            m[r] = -INFINITY;
+            l[r] = 0.0f;
+            acc[r / 2] = 0ull;
+        }
+        for (int c = 0; c <= p_max / AG_THREADS; ++c) {
+            const int j = c * AG_THREADS + tid, jend = min(c * AG_THREADS + AG_THREADS - 1, p_max);
+            __syncthreads();                         // the keys and weights of the chunk before have been read
+            const int w4 = d / 4;
+            for (int i = tid; i < (jend - c * AG_THREADS + 1) * w4; i += AG_THREADS) {
+                const int r = i / w4, e = 4 * (i - r * w4), jj = c * AG_THREADS + r;
+                const float* src = kcache + (((size_t)bt[jj / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + jj % LUMEN_PAGE) * d + e;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(ks + r * (d + 4) + e)),
+                             "l"(src)
+                             : "memory");
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            float s[R], cm[R];
+            {
+                ap_f2 dot[R / 2];
+#pragma unroll
+                for (int r = 0; r < R / 2; ++r) dot[r] = 0ull;
+#pragma unroll 2
+                for (int e = 0; e < d; e += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(ks + tid * (d + 4) + e);
+                    const float k[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const ap_f2 kk = ap_pair(k[x], k[x]);
+#pragma unroll
+                        for (int r = 0; r < R / 4; ++r) {
+                            const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qs + (e + x) * RP + 4 * r);
+                            ap_fma(dot[2 * r], qq.x, kk);
+                            ap_fma(dot[2 * r + 1], qq.y, kk);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float2 v = ap_unpair(dot[r / 2]);
+                    const float x = __fmul_rn((r & 1) ? v.y : v.x, scale);
+                    s[r] = j <= pos[r / HB] ? x : -INFINITY;
+                    cm[r] = s[r];
+                }
+            }
+            ag_block_reduce<R, true>(cm, red);
+            __syncthreads();
+            float corr[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float m_new = fmaxf(m[r], cm[r]);
+                s[r] = j <= pos[r / HB] ? expf(s[r] - m_new) : 0.0f;
+                corr[r] = (m[r] == -INFINITY) ? 0.0f : expf(m[r] - m_new);
+                m[r] = m_new;
+            }
+#pragma unroll
+            for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(ps + tid * RP + r) = make_float4(s[r], s[r + 1], s[r + 2], s[r + 3]);
+#pragma unroll
+            for (int r = 0; r < R; r += 2) ap_mul(acc[r / 2], ap_pair(corr[r], corr[r + 1]));
+            ag_block_reduce<R, false>(s, red);       // has a __syncthreads before ps is read below
+#pragma unroll
+            for (int r = 0; r < R; ++r) l[r] = l[r] * corr[r] + s[r];
+            if (tid < dv) {
+                int j0 = c * AG_THREADS;
+                const int all = min(jend, p_min);    // in sight of every row
+                while (j0 <= all) {
+                    const int r0 = j0 % LUMEN_PAGE, nr = min(LUMEN_PAGE - r0, all - j0 + 1);      // a run within a page
+                    const float* v = vcache + (((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + r0) * dv + tid;
+                    const float* w = ps + (j0 - c * AG_THREADS) * RP;
+#pragma unroll 8
+                    for (int k = 0; k < nr; ++k) {
+                        const float x = v[(size_t)k * dv];
+                        const ap_f2 xx = ap_pair(x, x);
+#pragma unroll
+                        for (int r = 0; r < R / 4; ++r) {
+                            const ulonglong2 ww = *reinterpret_cast<const ulonglong2*>(w + k * RP + 4 * r);
+                            ap_fma(acc[2 * r], ww.x, xx);
+                            ap_fma(acc[2 * r + 1], ww.y, xx);
+                        }
+                    }
+                    j0 += nr;
+                }
+                for (; j0 <= jend; ++j0) {           // the last few, of some rows only
+                    const float x = vcache[(((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + j0 % LUMEN_PAGE) * dv + tid];
+#pragma unroll
+                    for (int r = 0; r < R; r += 2) {
+                        float2 a = ap_unpair(acc[r / 2]);
+                        if (j0 <= pos[r / HB]) a.x = fmaf(ps[(j0 - c * AG_THREADS) * RP + r], x, a.x);
+                        if (j0 <= pos[(r + 1) / HB]) a.y = fmaf(ps[(j0 - c * AG_THREADS) * RP + r + 1], x, a.y);
+                        acc[r / 2] = ap_pair(a.x, a.y);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int t = r / HB;
+            if (t < g0 || t >= g1 || tid >= dv) continue;
+            const float2 a = ap_unpair(acc[r / 2]);
+            const float inv = 1.0f / l[r];
+            out[((size_t)(n0 + t) * nq + head0 + r % HB) * dv + tid] = ((r & 1) ? a.y : a.x) * inv;
+        }
+    }
+}
+
+template <int HB>
+static int attn_prompt_f32_go(const float* q, const float* kcache, const float* vcache, const int* block_table, int bt_stride,
+                              const int* tok_seq, const int* tok_pos, float* out, int N, int nq, int nkv, int d, int dv, float scale,
+                              cudaStream_t stream) {
+    const int smem = ap_smem(HB, d) * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(attn_prompt_f32_kernel<HB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    lumen_launch(attn_prompt_f32_kernel<HB>, dim3((N + AP_Q - 1) / AP_Q, nq / HB), dim3(AG_THREADS), smem, stream, q, kcache, vcache,
+                 block_table, bt_stride, tok_seq, tok_pos, out, N, nq, nkv, d, dv, scale);
+    LUMEN_LAUNCH_CHECK();
+    return 0;
+}
+
 static int attn_generic_launch(const void* q, int q_is_f32, const void* kcache, const void* vcache,
                                const int* block_table, int bt_stride, const int* tok_seq, const int* tok_pos,
                                void* out, int is_bf16, int N, int nq, int nkv, int d, int dv, int window,
@@ -273,12 +450,27 @@ static int attn_generic_launch(const void* q, int q_is_f32, const void* kcache, 
     return 0;
 }
 
+// n_seqs: how many sequences the tokens come from (a sequence's lie together); it decides between kernels of the same bits.
 LUMEN_API int lumen_attn_generic(const void* q, const void* kcache, const void* vcache,
                                  const int* block_table, int bt_stride, const int* tok_seq,
-                                 const int* tok_pos, void* out, int is_bf16, int N, int nq, int nkv,
+                                 const int* tok_pos, void* out, int is_bf16, int N, int n_seqs, int nq, int nkv,
                                  int d, int dv, int window, float scale, int layout, int v_layout,
                                  cudaStream_t stream) {
     AttnOptions opt = {};
+    // several tokens a block where most blocks' tokens are of one sequence
+    const bool rows = !is_bf16 && window == 0 && layout == LUMEN_LAYOUT_LINEAR && v_layout == LUMEN_LAYOUT_LINEAR && d % 4 == 0 &&
+                      d > 0 && d <= AG_THREADS && dv > 0 && dv <= AG_THREADS && ((uintptr_t)kcache & 15) == 0 && nkv > 0 && nq > 0 &&
+                      nq % nkv == 0 && nq <= 65535 && n_seqs > 0 && N / n_seqs >= 2 * AP_Q;
+    if (rows) {
+#define AP_GO(HB)                                                                                                              \
+    return attn_prompt_f32_go<HB>((const float*)q, (const float*)kcache, (const float*)vcache, block_table, bt_stride, tok_seq, \
+                                  tok_pos, (float*)out, N, nq, nkv, d, dv, scale, stream)
+        const int G = nq / nkv;
+        if (G % 4 == 0) AP_GO(4);
+        if (G % 2 == 0) AP_GO(2);
+        AP_GO(1);
+#undef AP_GO
+    }
     return attn_generic_launch(q, 0, kcache, vcache, block_table, bt_stride, tok_seq, tok_pos, out, is_bf16, N, nq,
                                nkv, d, dv, window, scale, layout, v_layout, opt, stream);
 }

@@ -799,9 +799,9 @@ def attn_generic(q, kcache, vcache, block_table, tok_seq, tok_pos, window, scale
                           f"{d} / {dv} with {tuple(kcache.shape)} / {tuple(vcache.shape)}")
     out = torch.empty((N, nq, dv), dtype=q.dtype, device=q.device)
     f = fn("attn_generic", "lumen_attn_generic",
-           [P, P, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, P])
+           [P, P, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, P])
     check(f(ptr(q), ptr(kcache), ptr(vcache), ptr(block_table), block_table.stride(0), ptr(tok_seq),
-            ptr(tok_pos), ptr(out), _is_bf16(q), N, nq, nkv, d, dv, int(window), float(scale), int(layout),
+            ptr(tok_pos), ptr(out), _is_bf16(q), N, block_table.shape[0], nq, nkv, d, dv, int(window), float(scale), int(layout),
             int(v_layout), stream_ptr()), "attn_generic")
     return out
 

@@ -197,6 +197,25 @@ def test_attention_generic(dtype, nq, nkv, d, window):
     assert float((out - ref).abs().max()) < tol
 
 
+@pytest.mark.parametrize("nq,nkv,d,lens,starts", [(8, 2, 128, [70, 2, 130], [0, 299, 5]), (4, 2, 64, [1, 33], [128, 0]),
+                                                  (3, 3, 20, [41], [87]), (6, 1, 112, [127, 1, 3], [2, 63, 250])])
+def test_attention_of_float32_prompts_has_the_bits_of_single_tokens(nq, nkv, d, lens, starts):
+    """Prompts go four tokens a block, decode steps one: the same bits, also where a block's tokens are of two sequences and
+    where chunks of 128 keys end among a block's tokens; a later token's NaN value reaches no earlier one."""
+    from lumenllm_b200.ops import kernels as K
+    table, kc, vc, ks, vs, qs = _attn_case(lens, starts, nq, nkv, d, F32, 0, 6)
+    vc[table[0, (starts[0] + lens[0] - 1) // 64], :, (starts[0] + lens[0] - 1) % 64] = float("nan")
+    pos = torch.cat([torch.arange(s, s + n) for s, n in zip(starts, lens)]).to(I32)
+    seq = torch.cat([torch.full((n,), b) for b, n in enumerate(lens)]).to(I32)
+    q, kc, vc, table = dev(torch.cat(qs)), dev(kc), dev(vc), dev(table)
+    assert len(pos) >= 8 * len(lens)
+    out = K.attn_generic(q, kc, vc, table, dev(seq), dev(pos), 0, d ** -0.5).cpu()
+    one = torch.cat([K.attn_generic(q[n:n + 1].contiguous(), kc, vc, table, dev(seq[n:n + 1]), dev(pos[n:n + 1]), 0, d ** -0.5)
+                     for n in range(len(pos))]).cpu()
+    assert bool(one[lens[0] - 1].isnan().all()) and int(one.isnan().any(-1).any(-1).sum()) == 1
+    assert torch.equal(out.nan_to_num(7.0), one.nan_to_num(7.0))
+
+
 @pytest.mark.parametrize("nq,nkv", [(8, 2), (4, 2), (3, 3)])
 @pytest.mark.parametrize("d,window", [(384, 0), (388, 50), (512, 0), (512, 33)])
 def test_attention_generic_with_wide_values(nq, nkv, d, window):
