@@ -338,9 +338,10 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
 // factor is a product of decays, at most 1, never a quotient; T's entries are at most 1 in size, as unit vectors and beta
 // below 1 make every step a contraction. What is left to the walk is three products with S a chunk, which have no chain
 // from token to token. A thread keeps 4 key channels of 4 columns of S, a warp all channels of four columns; sums over
-// channels change lanes a chunk at a time, 32 sums by 31 exchanges. Two warps keep the same four columns: one makes the sums
-// of P k and u, the other meanwhile those of P q and then o, and both move their S on. Zeros above the
-// diagonal are not multiplied, so that what is not finite in a token reaches no earlier one.
+// channels change lanes a chunk at a time, 64 sums by 62 exchanges. What bounds it is instructions: pairs are of
+// neighbouring channels, as they lie in the records, and u is also written twice over, so that no operand of a two-product
+// instruction has to be put together. Zeros above the diagonal are not multiplied, so that what is not finite in a token
+// reaches no earlier one.
 // Sequences of fewer than sixteen tokens walk them one by one, with the sums of a decode step.
 // MEASURED
 #define DC_T 16
@@ -458,10 +459,10 @@ delta_chunk_prepare_kernel(const DrIn in, float* __restrict__ prep, const int* _
     }
 }
 
-#define DC_COLS 16                                              // columns of S a block: four a pair of warps
+#define DC_COLS 16                                              // columns of S a block: four a warp
 #define DC_BUF (DC_REC + DC_T * DC_COLS)                        // floats of a staged chunk: the record, the values
-#define DC_THREADS 256
-#define DC_SMEM ((2 * DC_BUF + 2 * 4 * DC_T * 4) * (int)sizeof(float))
+#define DC_WORK (DC_T * 4 * 4)                                  // floats a warp: v - S^T P k, u, u twice over
+#define DC_SMEM ((2 * DC_BUF + 4 * DC_WORK) * (int)sizeof(float))
 
 // 32 pairs of sums over the lanes: lane l gets pair l.
 __device__ __forceinline__ f32x2 dc_reduce(f32x2 (&v)[32]) {
@@ -478,57 +479,52 @@ __device__ __forceinline__ f32x2 dc_reduce(f32x2 (&v)[32]) {
     return v[0];
 }
 
-__global__ void __launch_bounds__(DC_THREADS)
+__global__ void __launch_bounds__(DR_THREADS)
 delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* __restrict__ prep, float* __restrict__ state,
                    size_t slot_stride, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, float* __restrict__ y, int H,
                    int d, int dv, int vec) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
-    const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5 & 3, lane = tid & 31;
-    const bool reads = tid >= DC_THREADS / 2;                   // of the two warps of four columns: makes o
+    const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
     if (t_end <= t_begin) return;
     const float* rec0 = prep + ((size_t)dc_first(cu_q, b) * H + h) * DC_REC;
     float* S_head = state + (size_t)seq_slot[b] * slot_stride + (size_t)h * dv * d;
-    if (t_end - t_begin < DC_T) {                              // 32 columns a block
-        if (blockIdx.z & 1) return;
-        dr_walk<8, false, DC_THREADS>(sm, x, C, v_col, rec0, DC_ROW, t_begin, t_end, blockIdx.z >> 1, S_head, y, H, d, dv, vec);
+    if (t_end - t_begin < DC_T) {
+        dr_walk<8, false, DR_THREADS>(sm, x, C, v_col, rec0, DC_ROW, t_begin, t_end, blockIdx.z, S_head, y, H, d, dv, vec);
         return;
     }
     const int j0 = blockIdx.z * DC_COLS + 4 * warp, c0 = 4 * lane;
-    float* xs = sm + 2 * DC_BUF + warp * DC_T * 4;              // these four columns' [16][4] numbers, twice
-    float* us = xs + 4 * DC_T * 4;
-    f32x2 S[4][2];                                              // channel c0 + c, columns j0 + 2 p and + 1
-    {
-        float v[4][4];
+    float* xs = sm + 2 * DC_BUF + warp * DC_WORK;               // [16][4]
+    float* us = xs + 4 * DC_T;                                  // [16][4]
+    float* uu = us + 4 * DC_T;                                  // [16][4][2]
+    f32x2 S[4][2];                                              // column j0 + j, channels c0 + 2 p and + 1
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float* p = S_head + (size_t)(j0 + j) * d + c0;
-            const bool live = j0 + j < dv;
-            if (vec) {
-                float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (live && c0 < d) q = *reinterpret_cast<const float4*>(p);
-                v[j][0] = q.x; v[j][1] = q.y; v[j][2] = q.z; v[j][3] = q.w;
-            } else {
+    for (int j = 0; j < 4; ++j) {
+        const float* p = S_head + (size_t)(j0 + j) * d + c0;
+        const bool live = j0 + j < dv;
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (vec) {
+            if (live && c0 < d) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+        } else {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) v[j][c] = (live && c0 + c < d) ? p[c] : 0.0f;
-            }
+            for (int c = 0; c < 4; ++c)
+                if (live && c0 + c < d) v[c] = p[c];
         }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            S[c][0] = pair2(v[0][c], v[1][c]);
-            S[c][1] = pair2(v[2][c], v[3][c]);
-        }
+        S[j][0] = pair2(v[0], v[1]);
+        S[j][1] = pair2(v[2], v[3]);
     }
     auto issue = [&](int t0, int chunk, int buf) {
         float* to = sm + buf * DC_BUF;
         const float* from = rec0 + (size_t)chunk * H * DC_REC;
-        for (int i = tid; i < DC_REC / 4; i += DC_THREADS) dr_cp16(to + 4 * i, from + 4 * i);
-        static_assert(DC_T * DC_COLS == DC_THREADS, "a thread a value");
-        const int t = t0 + tid / DC_COLS, j = blockIdx.z * DC_COLS + tid % DC_COLS;
-        if (t < t_end && j < dv) dr_cp4(to + DC_REC + tid, x + (size_t)t * C + v_col + h * dv + j);
-        else to[DC_REC + tid] = 0.0f;
+        for (int i = tid; i < DC_REC / 4; i += DR_THREADS) dr_cp16(to + 4 * i, from + 4 * i);
+#pragma unroll
+        for (int i = tid; i < DC_T * DC_COLS; i += DR_THREADS) {
+            const int t = t0 + i / DC_COLS, j = blockIdx.z * DC_COLS + i % DC_COLS;
+            if (t < t_end && j < dv) dr_cp4(to + DC_REC + i, x + (size_t)t * C + v_col + h * dv + j);
+            else to[DC_REC + i] = 0.0f;
+        }
         dr_commit();
     };
     // rows of scaled vectors against S: lane l gets the sums of token l / 2, columns j0 + 2 (l % 2) and + 1
@@ -536,14 +532,15 @@ delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* _
         f32x2 v[32];
 #pragma unroll
         for (int t = 0; t < DC_T; ++t) {
-            const float4 k = *reinterpret_cast<const float4*>(vecs + t * DC_D + c0);
+            const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(vecs + t * DC_D + c0);
+            float w[4];
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                f32x2 r = mul2(pair2(k.x, k.x), S[0][p]);
-                r = fma2(pair2(k.y, k.y), S[1][p], r);
-                r = fma2(pair2(k.z, k.z), S[2][p], r);
-                v[2 * t + p] = fma2(pair2(k.w, k.w), S[3][p], r);
+            for (int j = 0; j < 4; ++j) {
+                const float2 r = unpair2(fma2(k.y, S[j][1], mul2(k.x, S[j][0])));
+                w[j] = r.x + r.y;
             }
+            v[2 * t] = pair2(w[0], w[1]);
+            v[2 * t + 1] = pair2(w[2], w[3]);
         }
         return dc_reduce(v);
     };
@@ -574,46 +571,42 @@ delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* _
             }
             return add2(s, s2);
         };
-        const f32x2 sums = times_S(rec + (reads ? DC_QT : DC_KT));
-        if (!reads) {
-            const float2 R = unpair2(sums);
-            const float2 v = *reinterpret_cast<const float2*>(rec + DC_REC + tt * DC_COLS + 4 * warp + jp);
-            *reinterpret_cast<float2*>(xs + tt * 4 + jp) = make_float2(v.x - R.x, v.y - R.y);
-            __syncwarp();
-            *reinterpret_cast<f32x2*>(us + tt * 4 + jp) = lower(rec + DC_TM, xs, 0ull);
-        }
-        __syncthreads();
-        if (reads) {
-            const float2 o = unpair2(lower(rec + DC_BM, us, sums));
-            if (tt < nt) {
-                float* dst = y + (size_t)(t0 + tt) * H * dv + (size_t)h * dv + j0 + jp;
-                if ((dv & 1) == 0) {
-                    if (j0 + jp < dv) *reinterpret_cast<float2*>(dst) = o;
-                } else {
-                    if (j0 + jp < dv) dst[0] = o.x;
-                    if (j0 + jp + 1 < dv) dst[1] = o.y;
-                }
+        const float2 R = unpair2(times_S(rec + DC_KT));
+        const float2 v = *reinterpret_cast<const float2*>(rec + DC_REC + tt * DC_COLS + 4 * warp + jp);
+        *reinterpret_cast<float2*>(xs + tt * 4 + jp) = make_float2(v.x - R.x, v.y - R.y);
+        const f32x2 Q = times_S(rec + DC_QT);
+        __syncwarp();
+        const float2 u = unpair2(lower(rec + DC_TM, xs, 0ull));
+        *reinterpret_cast<float2*>(us + tt * 4 + jp) = u;
+        *reinterpret_cast<float4*>(uu + tt * 8 + 2 * jp) = make_float4(u.x, u.x, u.y, u.y);
+        __syncwarp();
+        const float2 o = unpair2(lower(rec + DC_BM, us, Q));
+        if (tt < nt) {
+            float* dst = y + (size_t)(t0 + tt) * H * dv + (size_t)h * dv + j0 + jp;
+            if ((dv & 1) == 0) {
+                if (j0 + jp < dv) *reinterpret_cast<float2*>(dst) = o;
+            } else {
+                if (j0 + jp < dv) dst[0] = o.x;
+                if (j0 + jp + 1 < dv) dst[1] = o.y;
             }
         }
-        const float4 P = *reinterpret_cast<const float4*>(rec + DC_P + c0);
+        const ulonglong2 P = *reinterpret_cast<const ulonglong2*>(rec + DC_P + c0);
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            S[0][p] = mul2(pair2(P.x, P.x), S[0][p]);
-            S[1][p] = mul2(pair2(P.y, P.y), S[1][p]);
-            S[2][p] = mul2(pair2(P.z, P.z), S[2][p]);
-            S[3][p] = mul2(pair2(P.w, P.w), S[3][p]);
+        for (int j = 0; j < 4; ++j) {
+            S[j][0] = mul2(P.x, S[j][0]);
+            S[j][1] = mul2(P.y, S[j][1]);
         }
         auto add = [&](int t) {
-            const float4 k = *reinterpret_cast<const float4*>(rec + DC_KB + t * DC_D + c0);
-            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(us + t * 4);
-            S[0][0] = fma2(pair2(k.x, k.x), u.x, S[0][0]);
-            S[0][1] = fma2(pair2(k.x, k.x), u.y, S[0][1]);
-            S[1][0] = fma2(pair2(k.y, k.y), u.x, S[1][0]);
-            S[1][1] = fma2(pair2(k.y, k.y), u.y, S[1][1]);
-            S[2][0] = fma2(pair2(k.z, k.z), u.x, S[2][0]);
-            S[2][1] = fma2(pair2(k.z, k.z), u.y, S[2][1]);
-            S[3][0] = fma2(pair2(k.w, k.w), u.x, S[3][0]);
-            S[3][1] = fma2(pair2(k.w, k.w), u.y, S[3][1]);
+            const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(rec + DC_KB + t * DC_D + c0);
+            const ulonglong2 u01 = *reinterpret_cast<const ulonglong2*>(uu + t * 8), u23 = *reinterpret_cast<const ulonglong2*>(uu + t * 8 + 4);
+            S[0][0] = fma2(k.x, u01.x, S[0][0]);
+            S[0][1] = fma2(k.y, u01.x, S[0][1]);
+            S[1][0] = fma2(k.x, u01.y, S[1][0]);
+            S[1][1] = fma2(k.y, u01.y, S[1][1]);
+            S[2][0] = fma2(k.x, u23.x, S[2][0]);
+            S[2][1] = fma2(k.y, u23.x, S[2][1]);
+            S[3][0] = fma2(k.x, u23.y, S[3][0]);
+            S[3][1] = fma2(k.y, u23.y, S[3][1]);
         };
         if (nt == DC_T) {
 #pragma unroll
@@ -623,17 +616,12 @@ delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* _
         }
         __syncthreads();                            // this chunk has been read by everyone before its buffer is filled again
     }
-    if (reads) return;                              // its S is the other warp's
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         if (j0 + j >= dv) continue;
         float* p = S_head + (size_t)(j0 + j) * d + c0;
-        float v[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const float2 w = unpair2(S[c][j >> 1]);
-            v[c] = (j & 1) ? w.y : w.x;
-        }
+        const float2 lo = unpair2(S[j][0]), hi = unpair2(S[j][1]);
+        const float v[4] = {lo.x, lo.y, hi.x, hi.y};
         if (vec) {
             if (c0 < d) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
         } else {
@@ -690,7 +678,7 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
         if (e != cudaSuccess) return (int)e;
         lumen_launch(delta_chunk_prepare_kernel, dim3(N / DC_T + n_seqs, H), dim3(32 * DC_WARPS), 0, stream, in, prep, cu_q, n_seqs);
         LUMEN_LAUNCH_CHECK();
-        lumen_launch(delta_chunk_kernel, dim3(n_seqs, H, (dv + DC_COLS - 1) / DC_COLS), dim3(DC_THREADS), DC_SMEM, stream, x, C, v_col,
+        lumen_launch(delta_chunk_kernel, dim3(n_seqs, H, (dv + DC_COLS - 1) / DC_COLS), dim3(DR_THREADS), DC_SMEM, stream, x, C, v_col,
                      (const float*)prep, state, (size_t)slot_stride, cu_q, seq_slot, y, H, d, dv, vec);
         LUMEN_LAUNCH_CHECK();
         return 0;
