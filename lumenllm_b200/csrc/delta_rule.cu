@@ -139,10 +139,11 @@ delta_prepare_kernel(const DrIn in, float* __restrict__ prep, int dp) {
 // NS: threads that share a column of S (a power of two), NS DR_ROWS >= d; every offset of the walk is a constant
 // of the instance. AHEAD: a token's rows are read from shared memory while the one before is worked on, which
 // takes twice the registers: for steps of several tokens a sequence. THREADS: of a block. Same sums either way.
-// row0: the row of the sequence's first token, the next ones row_stride floats on; zblock: which columns.
+// row0: the row of the sequence's first token, the next ones row_stride floats on, every sixteenth group_stride after the
+// one sixteen before; zblock: which columns.
 template <int NS, bool AHEAD, int THREADS>
 __device__ __forceinline__ void dr_walk(float* sm, const float* __restrict__ x, int C, int v_col, const float* __restrict__ row0,
-                                        size_t row_stride, int t_begin, int t_end, int zblock, float* __restrict__ S_head,
+                                        size_t row_stride, size_t group_stride, int t_begin, int t_end, int zblock, float* __restrict__ S_head,
                                         float* __restrict__ y, int H, int d, int dv, int vec) {
     constexpr int ROWS = DR_ROWS;
     constexpr int dp = NS * ROWS;                   // d padded to what the threads of a column hold
@@ -179,7 +180,7 @@ __device__ __forceinline__ void dr_walk(float* sm, const float* __restrict__ x, 
         float* rb = rows + buf * DR_CHUNK * PW;
         for (int i = tid; i < nt * pieces; i += THREADS) {
             const int tt = i / pieces, p = i - tt * pieces;
-            dr_cp16(rb + tt * PW + 4 * p, row0 + (size_t)(t0 + tt - t_begin) * row_stride + 4 * p);
+            dr_cp16(rb + tt * PW + 4 * p, row0 + (size_t)((t0 + tt - t_begin) >> 4) * group_stride + ((t0 + tt - t_begin) & 15) * row_stride + 4 * p);
         }
         float* vb = vs + buf * DR_CHUNK * cols;
         for (int i = tid; i < nt * cols; i += THREADS) {
@@ -323,7 +324,7 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
     constexpr int PW = 3 * NS * DR_ROWS + 4;
     const int b = blockIdx.x, h = blockIdx.y, t_begin = cu_q[b], t_end = cu_q[b + 1];
     if (t_end <= t_begin) return;
-    dr_walk<NS, AHEAD, THREADS>(sm, x, C, v_col, prep + ((size_t)t_begin * H + h) * PW, (size_t)H * PW, t_begin, t_end, blockIdx.z,
+    dr_walk<NS, AHEAD, THREADS>(sm, x, C, v_col, prep + ((size_t)t_begin * H + h) * PW, (size_t)H * PW, (size_t)16 * H * PW, t_begin, t_end, blockIdx.z,
                                 state + (size_t)seq_slot[b] * slot_stride + (size_t)h * dv * d, y, H, d, dv, vec);
 }
 
@@ -342,9 +343,11 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
 // neighbouring channels, as they lie in the records, and u is also written twice over, so that no operand of a two-product
 // instruction has to be put together. Zeros above the diagonal are not multiplied, so that what is not finite in a token
 // reaches no earlier one.
-// Sequences of fewer than sixteen tokens walk them one by one, with the sums of a decode step.
+// Sequences of fewer than DC_MIN tokens walk them one by one, with the sums of a decode step: a few chunks are no faster
+// (us, 16 heads of 128 x 128, chunks / tokens: 33 tokens 14.5 / 13.6, 64 sequences of 24 218 / 215, 200 tokens 36 / 50).
 // MEASURED
 #define DC_T 16
+#define DC_MIN 48
 #define DC_D 128
 #define DC_PITCH 20                                              // floats a row of T and of B
 #define DC_KT 0
@@ -356,7 +359,7 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
 #define DC_REC (DC_BM + DC_T * DC_PITCH)                         // floats of a (chunk, head)
 #define DC_ROW (3 * DC_D + 4)                                    // a token's row, as above
 #define DC_WARPS 16                                              // of the kernel that prepares: one a token
-static_assert(DC_T * DC_ROW <= DC_REC, "a short sequence's rows lie in the record of its first chunk");
+static_assert(DC_T * DC_ROW <= DC_REC, "a short sequence's rows lie in the records of its chunks");
 
 // Where the chunks of sequence b start among all records: room for every cut of N tokens.
 __device__ __forceinline__ int dc_first(const int* cu_q, int b) { return cu_q[b] / DC_T + b; }
@@ -377,7 +380,7 @@ delta_chunk_prepare_kernel(const DrIn in, float* __restrict__ prep, const int* _
     if (t0 < t_begin || t0 >= t_end) return;
     const int nt = min(DC_T, t_end - t0);
     float* rec = prep + ((size_t)blockIdx.x * in.H + h) * DC_REC;
-    const bool is_short = t_end - t_begin < DC_T;
+    const bool is_short = t_end - t_begin < DC_MIN;
     {
         float* row = is_short ? rec + warp * DC_ROW : rows + warp * DC_ROW;
         if (warp < nt) {
@@ -491,8 +494,8 @@ delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* _
     if (t_end <= t_begin) return;
     const float* rec0 = prep + ((size_t)dc_first(cu_q, b) * H + h) * DC_REC;
     float* S_head = state + (size_t)seq_slot[b] * slot_stride + (size_t)h * dv * d;
-    if (t_end - t_begin < DC_T) {
-        dr_walk<8, false, DR_THREADS>(sm, x, C, v_col, rec0, DC_ROW, t_begin, t_end, blockIdx.z, S_head, y, H, d, dv, vec);
+    if (t_end - t_begin < DC_MIN) {
+        dr_walk<8, true, DR_THREADS>(sm, x, C, v_col, rec0, DC_ROW, (size_t)H * DC_REC, t_begin, t_end, blockIdx.z, S_head, y, H, d, dv, vec);
         return;
     }
     const int j0 = blockIdx.z * DC_COLS + 4 * warp, c0 = 4 * lane;
