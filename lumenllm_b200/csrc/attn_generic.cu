@@ -236,6 +236,8 @@ attn_generic_kernel(const TQ* __restrict__ q, const T* __restrict__ kcache, cons
 // values are fetched once for all of them (a token each read them again). A chunk's keys are staged in shared memory; products of two
 // rows share an instruction, each rounded as by itself, and every sum runs in the order of the kernel above: the same bits. Tokens of
 // different sequences in a block are walked one sequence after the other. A key past a row's own token is not multiplied into it.
+// What bounds it is shared memory (a 16-byte read of a warp takes four cycles however many lanes share it): a thread makes the dots
+// of two keys and adds up two value numbers, for half of the rows, so that a read of queries or of weights serves twice.
 // MEASURED
 #define AP_Q 4
 typedef unsigned long long ap_f2;
@@ -269,7 +271,21 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
     float* ps = qs + d * RP;                         // [128][RP]
     __shared__ float red[R][32];
     const int tid = threadIdx.x, head0 = blockIdx.y * HB, kvh = head0 / (nq / nkv);
+    const int kp = tid & 63, half = tid >> 6;        // of a warp the same
     const int n0 = blockIdx.x * AP_Q, nt = min(AP_Q, N - n0);
+    // pairs of rows of this half, side by side
+    auto rows2 = [&](const float* p, ap_f2 (&x)[R / 4]) {
+        if constexpr (R >= 8) {
+#pragma unroll
+            for (int r = 0; r < R / 8; ++r) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + half * (R / 2) + 4 * r);
+                x[2 * r] = v.x;
+                x[2 * r + 1] = v.y;
+            }
+        } else {
+            x[0] = *reinterpret_cast<const ap_f2*>(p + half * (R / 2));
+        }
+    };
     for (int i = tid; i < R * d; i += AG_THREADS) {
         const int r = i / d, e = i - r * d, t = r / HB;
         qs[e * RP + r] = t < nt ? q[((size_t)(n0 + t) * nq + head0 + r % HB) * d + e] : 0.0f;
@@ -288,12 +304,12 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
             }
         }
         float m[R], l[R];
-        ap_f2 acc[R / 2];                            // value number tid
+        ap_f2 acc[2][R / 4];                         // value numbers kp and kp + 64, this half's rows
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             m[r] = -INFINITY;
             l[r] = 0.0f;
-            acc[r / 2] = 0ull;
+            acc[r & 1][r / 4] = 0ull;
         }
         for (int c = 0; c <= p_max / AG_THREADS; ++c) {
             const int j = c * AG_THREADS + tid, jend = min(c * AG_THREADS + AG_THREADS - 1, p_max);
@@ -310,29 +326,38 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
             __syncthreads();
             float s[R], cm[R];
             {
-                ap_f2 dot[R / 2];
+                ap_f2 dot[2][R / 4];
 #pragma unroll
-                for (int r = 0; r < R / 2; ++r) dot[r] = 0ull;
+                for (int r = 0; r < R / 4; ++r) dot[0][r] = dot[1][r] = 0ull;
 #pragma unroll 2
                 for (int e = 0; e < d; e += 4) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(ks + tid * (d + 4) + e);
-                    const float k[4] = {k4.x, k4.y, k4.z, k4.w};
+                    float k[2][4];
+                    *reinterpret_cast<float4*>(k[0]) = *reinterpret_cast<const float4*>(ks + kp * (d + 4) + e);
+                    *reinterpret_cast<float4*>(k[1]) = *reinterpret_cast<const float4*>(ks + (kp + 64) * (d + 4) + e);
 #pragma unroll
                     for (int x = 0; x < 4; ++x) {
-                        const ap_f2 kk = ap_pair(k[x], k[x]);
+                        ap_f2 qq[R / 4];
+                        rows2(qs + (e + x) * RP, qq);
+                        const ap_f2 k0 = ap_pair(k[0][x], k[0][x]), k1 = ap_pair(k[1][x], k[1][x]);
 #pragma unroll
                         for (int r = 0; r < R / 4; ++r) {
-                            const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qs + (e + x) * RP + 4 * r);
-                            ap_fma(dot[2 * r], qq.x, kk);
-                            ap_fma(dot[2 * r + 1], qq.y, kk);
+                            ap_fma(dot[0][r], qq[r], k0);
+                            ap_fma(dot[1][r], qq[r], k1);
                         }
                     }
                 }
+                // from here on a thread has the key tid, for all rows
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int r = 0; r < R / 4; ++r)
+                        *reinterpret_cast<ap_f2*>(ps + (kp + 64 * x) * RP + half * (R / 2) + 2 * r) = dot[x][r];
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(s + r) = *reinterpret_cast<const float4*>(ps + tid * RP + r);
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    const float2 v = ap_unpair(dot[r / 2]);
-                    const float x = __fmul_rn((r & 1) ? v.y : v.x, scale);
-                    s[r] = j <= pos[r / HB] ? x : -INFINITY;
+                    s[r] = j <= pos[r / HB] ? __fmul_rn(s[r], scale) : -INFINITY;
                     cm[r] = s[r];
                 }
             }
@@ -349,49 +374,63 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
 #pragma unroll
             for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(ps + tid * RP + r) = make_float4(s[r], s[r + 1], s[r + 2], s[r + 3]);
 #pragma unroll
-            for (int r = 0; r < R; r += 2) ap_mul(acc[r / 2], ap_pair(corr[r], corr[r + 1]));
+            for (int r = 0; r < R / 4; ++r) {
+                const ap_f2 c2 = half ? ap_pair(corr[R / 2 + 2 * r], corr[R / 2 + 2 * r + 1]) : ap_pair(corr[2 * r], corr[2 * r + 1]);
+                ap_mul(acc[0][r], c2);
+                ap_mul(acc[1][r], c2);
+            }
             ag_block_reduce<R, false>(s, red);       // has a __syncthreads before ps is read below
 #pragma unroll
             for (int r = 0; r < R; ++r) l[r] = l[r] * corr[r] + s[r];
-            if (tid < dv) {
+            const bool two = kp + 64 < dv;
+            if (kp < dv) {
                 int j0 = c * AG_THREADS;
                 const int all = min(jend, p_min);    // in sight of every row
                 while (j0 <= all) {
                     const int r0 = j0 % LUMEN_PAGE, nr = min(LUMEN_PAGE - r0, all - j0 + 1);      // a run within a page
-                    const float* v = vcache + (((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + r0) * dv + tid;
+                    const float* v = vcache + (((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + r0) * dv + kp;
                     const float* w = ps + (j0 - c * AG_THREADS) * RP;
 #pragma unroll 8
                     for (int k = 0; k < nr; ++k) {
-                        const float x = v[(size_t)k * dv];
-                        const ap_f2 xx = ap_pair(x, x);
+                        const float x0 = v[(size_t)k * dv], x1 = two ? v[(size_t)k * dv + 64] : 0.0f;
+                        const ap_f2 v0 = ap_pair(x0, x0), v1 = ap_pair(x1, x1);
+                        ap_f2 ww[R / 4];
+                        rows2(w + k * RP, ww);
 #pragma unroll
                         for (int r = 0; r < R / 4; ++r) {
-                            const ulonglong2 ww = *reinterpret_cast<const ulonglong2*>(w + k * RP + 4 * r);
-                            ap_fma(acc[2 * r], ww.x, xx);
-                            ap_fma(acc[2 * r + 1], ww.y, xx);
+                            ap_fma(acc[0][r], ww[r], v0);
+                            ap_fma(acc[1][r], ww[r], v1);
                         }
                     }
                     j0 += nr;
                 }
                 for (; j0 <= jend; ++j0) {           // the last few, of some rows only
-                    const float x = vcache[(((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + j0 % LUMEN_PAGE) * dv + tid];
+                    const float* v = vcache + (((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + j0 % LUMEN_PAGE) * dv + kp;
+                    const float x0 = v[0], x1 = two ? v[64] : 0.0f;
+                    const float* w = ps + (j0 - c * AG_THREADS) * RP + half * (R / 2);
 #pragma unroll
-                    for (int r = 0; r < R; r += 2) {
-                        float2 a = ap_unpair(acc[r / 2]);
-                        if (j0 <= pos[r / HB]) a.x = fmaf(ps[(j0 - c * AG_THREADS) * RP + r], x, a.x);
-                        if (j0 <= pos[(r + 1) / HB]) a.y = fmaf(ps[(j0 - c * AG_THREADS) * RP + r + 1], x, a.y);
-                        acc[r / 2] = ap_pair(a.x, a.y);
+                    for (int r = 0; r < R / 2; ++r) {
+                        if (j0 > (half ? pos[(R / 2 + r) / HB] : pos[r / HB])) continue;
+                        float2 a = ap_unpair(acc[0][r / 2]), b = ap_unpair(acc[1][r / 2]);
+                        float& a0 = (r & 1) ? a.y : a.x;
+                        float& b0 = (r & 1) ? b.y : b.x;
+                        a0 = fmaf(w[r], x0, a0);
+                        b0 = fmaf(w[r], x1, b0);
+                        acc[0][r / 2] = ap_pair(a.x, a.y);
+                        acc[1][r / 2] = ap_pair(b.x, b.y);
                     }
                 }
             }
         }
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int t = r / HB;
-            if (t < g0 || t >= g1 || tid >= dv) continue;
-            const float2 a = ap_unpair(acc[r / 2]);
-            const float inv = 1.0f / l[r];
-            out[((size_t)(n0 + t) * nq + head0 + r % HB) * dv + tid] = ((r & 1) ? a.y : a.x) * inv;
+        for (int r = 0; r < R / 2; ++r) {
+            const int row = half * (R / 2) + r, t = row / HB;
+            if (t < g0 || t >= g1) continue;
+            const float2 a = ap_unpair(acc[0][r / 2]), b = ap_unpair(acc[1][r / 2]);
+            const float inv = 1.0f / (half ? l[R / 2 + r] : l[r]);
+            float* dst = out + ((size_t)(n0 + t) * nq + head0 + row % HB) * dv + kp;
+            if (kp < dv) dst[0] = ((r & 1) ? a.y : a.x) * inv;
+            if (kp + 64 < dv) dst[64] = ((r & 1) ? b.y : b.x) * inv;
         }
     }
 }

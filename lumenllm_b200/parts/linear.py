@@ -1,8 +1,8 @@
 """y = x W^T for a weight stored [out, in] (crates/aegisllm-cuda/src/cuda/kernels/
 blackwell/sampling.cu:16-18). The result is float32.
 
-A weight kept in float32 (stored so, or a 32-bit run) is multiplied by the FFMA
-kernel in true 32-bit; a bfloat16 weight in a bfloat16 run goes to the tensor
+A weight kept in float32 (stored so, or a 32-bit run) is multiplied with the error
+of 32 bits (ops.kernels.gemm_f32); a bfloat16 weight in a bfloat16 run goes to the tensor
 cores with float32 accumulation. Several weights that read the same input are
 stacked row-wise at load so that they cost one product.
 """
