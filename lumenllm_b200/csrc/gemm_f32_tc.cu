@@ -13,12 +13,13 @@
 // A block takes 128 rows of W (the 128-row side of the MMA) times up to 160 rows of A, for a share of k; the blocks of
 // one tile, one for each share, are a cluster and add up their sums through distributed shared memory. The number of
 // shares depends on N and K alone, so C[m,n] depends on row m of A and row n of W only, never on M or where they lie.
-//   warps 0..7   two groups that take turns: a group cuts 64 columns of W, stores the parts as 128-byte-swizzled tiles (two
-//                buffers) and fetches its next 64 into registers, which are under way during the other group's turn. Up to 32 rows of A go the same way; more are cut once, by a kernel
+//   warps 0..7   fetch 64 columns of W into registers, cut them and store the parts as 128-byte-swizzled tiles, two buffers.
+//                With more than 64 rows of A, where the products take the time, they have the parts ready in registers
+//                when a buffer is free again. Up to 32 rows of A go the same way; more are cut once, by a kernel
 //                ahead of this one, into the image their tiles have in shared memory (a block that cut 160 rows of A for its
 //                128 of W spent half of its time on them), and are copied by
 //   a warp       that does nothing else;
-//   two warps    issue the products, in turns too (a lane that issues is held up until the tensor pipe takes its product, so a
+//   two warps    issue the products in turns (a lane that issues is held up until the tensor pipe takes its product, so a
 //                single one would leave the pipe idle while it goes through its barriers); one allocates tensor memory;
 //   the others   add the finished accumulator (two of them, in tensor memory) to the sums in their registers.
 // Infinities and NaN have no parts: the rows that hold one are marked, and their outputs are made again with plain FMAs.
@@ -35,9 +36,7 @@
 #define FT_ROWS 128                      // rows of W a block
 #define FT_BK 64
 #define FT_MAX_BN 160                    // rows of A a block
-#define FT_CONV 8                        // warps that fetch and cut, in two groups
-#define FT_GROUP (FT_CONV / 2 * 32)      // threads a group
-#define FT_PASS (FT_GROUP / 16)          // rows a group takes at once, sixteen threads a row
+#define FT_CONV 8                        // warps that fetch and cut
 #define FT_W_TILE (FT_ROWS * 128)        // bytes of one part of a tile of W
 #define FT_MAX_SHARES 8
 #define FT_MIN_N 1024                    // see lumen_gemm_f32_tc_takes
@@ -146,17 +145,17 @@ __device__ __forceinline__ uint32_t ft_cut(unsigned long long& x) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(x) : "l"(r), "l"(0xbf800000bf800000ull));       // x - r
     return h;
 }
-// Cuts four values and stores their parts `part` bytes apart; 1 if one of them is not finite (or rounds to infinity).
-__device__ __forceinline__ int ft_store(const FtRaw<float>& x, unsigned char* dst, int part) {
+// The parts of four values of a row.
+template <typename T> struct FtParts { uint2 h[sizeof(T) == 4 ? 3 : 1]; };
+// 1 if one of the values is not finite (or rounds to infinity).
+__device__ __forceinline__ int ft_parts(const FtRaw<float>& x, FtParts<float>& to) {
     unsigned long long a, b;
     asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(x.v.x), "f"(x.v.y));
     asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(x.v.z), "f"(x.v.w));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        uint2 h;
-        h.x = ft_cut(a);
-        h.y = ft_cut(b);
-        *reinterpret_cast<uint2*>(dst + i * part) = h;
+        to.h[i].x = ft_cut(a);
+        to.h[i].y = ft_cut(b);
     }
     // nothing is left (or less than bfloat16 has numbers for, of values below 2^-110), or NaN: an infinity less itself
     float u, v;
@@ -164,10 +163,23 @@ __device__ __forceinline__ int ft_store(const FtRaw<float>& x, unsigned char* ds
     asm("mov.b64 {%0, %1}, %2;" : "=f"(u), "=f"(v) : "l"(a));
     return !(u + v == u + v);
 }
-__device__ __forceinline__ int ft_store(const FtRaw<__nv_bfloat16>& x, unsigned char* dst, int) {
-    *reinterpret_cast<uint2*>(dst) = x.v;
+__device__ __forceinline__ int ft_parts(const FtRaw<__nv_bfloat16>& x, FtParts<__nv_bfloat16>& to) {
+    to.h[0] = x.v;
     const uint32_t e = 0x7f80u;
     return (x.v.x & e) == e || ((x.v.x >> 16) & e) == e || (x.v.y & e) == e || ((x.v.y >> 16) & e) == e;
+}
+// Parts go `part` bytes apart.
+template <typename T>
+__device__ __forceinline__ void ft_put(const FtParts<T>& x, unsigned char* dst, int part) {
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(x.h) / sizeof(x.h[0])); ++i) *reinterpret_cast<uint2*>(dst + i * part) = x.h[i];
+}
+template <typename T>
+__device__ __forceinline__ int ft_store(const FtRaw<T>& x, unsigned char* dst, int part) {
+    FtParts<T> p;
+    const int odd = ft_parts(x, p);
+    ft_put(p, dst, part);
+    return odd;
 }
 
 template <typename TW, int BN>
@@ -181,11 +193,14 @@ struct FtShape {
     static constexpr int TMEM = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
     static constexpr int CTL = 1024;                                     // barriers, flags, marks
     static constexpr int SMEM = 2 * BUF + CTL;
+    static constexpr int MINB = (BN <= 16 && 2 * SMEM <= 220 * 1024) ? 2 : 1;
+    static constexpr bool EARLY = BN > 64;                               // W is cut before there is room for it
+    static constexpr int SETS = MINB == 1 && !EARLY ? 2 : 1;             // blocks of W under way in registers
     static_assert(BN * FT_ROWS * 4 <= 2 * BUF, "the sums are staged where the tiles were");
 };
 
 template <typename TW, int BN>
-__global__ void __launch_bounds__(32 * FtShape<TW, BN>::WARPS, 1)
+__global__ void __launch_bounds__(32 * FtShape<TW, BN>::WARPS, FtShape<TW, BN>::MINB)
 gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict__ image, const unsigned char* __restrict__ image_odd,
                    const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int vec, int give_up_at,
                    int* __restrict__ err) {
@@ -212,7 +227,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&full[i], FT_CONV / 2);
+            mbar_init(&full[i], FT_CONV);
             mbar_init(&done[i], 1);
             mbar_init(&taken[i], EPI);
             mbar_init(&landed[i], 1);
@@ -243,48 +258,85 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
     float* sums = reinterpret_cast<float*>(tiles);             // [BN][128], over the tiles once they have been read
 
     if (warp < FT_CONV) {
-        constexpr int LW = FT_ROWS / FT_PASS, LA = F::IMAGE ? 0 : BN / FT_PASS;      // fetches a thread
-        const int c = threadIdx.x & 15, r = threadIdx.x % FT_GROUP >> 4, group = threadIdx.x / FT_GROUP;
-        FtRaw<TW> rw[LW];
-        FtRaw<float> ra[LA ? LA : 1];
-        auto fetch = [&](int kb) {
+        constexpr int LW = FT_ROWS / 16, LA = BN / 16;                       // fetches a thread: 16 threads a row
+        const int c = threadIdx.x & 15, r = threadIdx.x >> 4;
+        FtRaw<TW> rw[F::SETS][LW];
+        FtRaw<float> ra[F::IMAGE ? 1 : LA];
+        auto fetch_w = [&](int kb, FtRaw<TW> (&x)[LW]) {
             const int k = (kb0 + kb) * FT_BK + 4 * c;
-            const TW* pw = W + (size_t)(n0 + r) * K + k;
-            const float* pa = A + (size_t)(m0 + r) * K + k;
+            const TW* p = W + (size_t)(n0 + r) * K + k;
 #pragma unroll
-            for (int i = 0; i < LW; ++i)
-                ft_fetch(rw[i], pw + (size_t)(FT_PASS * i) * K, kb < nk && r + FT_PASS * i < cols ? K - k : 0, vec);
+            for (int i = 0; i < LW; ++i) ft_fetch(x[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < cols ? K - k : 0, vec);
+        };
+        auto fetch_a = [&](int kb) {
+            const int k = (kb0 + kb) * FT_BK + 4 * c;
+            const float* p = A + (size_t)(m0 + r) * K + k;
+            if constexpr (!F::IMAGE) {
 #pragma unroll
-            for (int i = 0; i < LA; ++i)
-                ft_fetch(ra[i], pa + (size_t)(FT_PASS * i) * K, kb < nk && r + FT_PASS * i < rows ? K - k : 0, vec);
+                for (int i = 0; i < LA; ++i) ft_fetch(ra[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < rows ? K - k : 0, vec);
+            }
         };
         // this thread's four values of row r: 8 bytes in the 16-byte piece c / 2, which lies at (c / 2) ^ (row & 7)
-        static_assert(FT_PASS == 8, "rows eight apart have one place for a piece");
-        unsigned char* tw = tiles + group * F::BUF + r * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8;
-        unsigned char* ta = tw + NW * FT_W_TILE;
-        fetch(group);
-        for (int kb = group; kb < nk; kb += 2) {
-            if (kb >= 2 && !__all_sync(0xffffffffu, ft_wait(&done[group], ((kb >> 1) & 1) ^ 1, abort_flag))) {
-                *abort_flag = 1;
-                if (lane == 0) atomicExch(err, 1);
-                break;
-            }
-            uint32_t odd = 0;                    // looked at once a block, so that the rows' cutting can be interleaved
-#pragma unroll
-            for (int i = 0; i < LW; ++i) odd |= (uint32_t)ft_store(rw[i], tw + i * FT_PASS * 128, FT_W_TILE) << i;
-#pragma unroll
-            for (int i = 0; i < LA; ++i) odd |= (uint32_t)ft_store(ra[i], ta + i * FT_PASS * 128, F::A_TILE) << (LW + i);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the next loads, which it would wait for
-            if (odd) {
-                *any_odd = 1;
-                for (int i = 0; i < LW; ++i)
-                    if (odd >> i & 1) odd_w[r + FT_PASS * i] = 1;
+        const uint32_t at = r * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8;
+        auto room = [&](int kb) -> bool {        // the buffer of block kb is free
+            if (kb < 2 || __all_sync(0xffffffffu, ft_wait(&done[kb & 1], ((kb >> 1) & 1) ^ 1, abort_flag))) return true;
+            *abort_flag = 1;
+            if (lane == 0) atomicExch(err, 1);
+            return false;
+        };
+        auto mark = [&](int odd) {               // looked at once a block, so that the rows' cutting can be interleaved
+            if (!odd) return;
+            *any_odd = 1;
+            for (int i = 0; i < LW; ++i)
+                if (odd >> i & 1) odd_w[r + 16 * i] = 1;
+            if constexpr (!F::IMAGE)
                 for (int i = 0; i < LA; ++i)
-                    if (odd >> (LW + i) & 1) odd_a[r + FT_PASS * i] = 1;
+                    if (odd >> (LW + i) & 1) odd_a[r + 16 * i] = 1;
+        };
+        if constexpr (F::EARLY) {
+            FtParts<TW> p[LW];
+            fetch_w(0, rw[0]);
+            for (int kb = 0; kb < nk; ++kb) {
+                int odd = 0;
+#pragma unroll
+                for (int i = 0; i < LW; ++i) odd |= ft_parts(rw[0][i], p[i]) << i;
+                fetch_w(kb + 1, rw[0]);
+                mark(odd);
+                if (!room(kb)) break;
+                unsigned char* tw = tiles + (kb & 1) * F::BUF + at;
+#pragma unroll
+                for (int i = 0; i < LW; ++i) ft_put(p[i], tw + i * 16 * 128, FT_W_TILE);
+                // the fence between these stores and the products' reads is the issuing lane's: here it would wait for the loads
+                __syncwarp();
+                if (lane == 0) ft_arrive(&full[kb & 1]);
             }
-            __syncwarp();
-            if (lane == 0) ft_arrive(&full[group]);
-            fetch(kb + 2);
+        } else {
+            auto step = [&](int kb, FtRaw<TW> (&x)[LW]) -> bool {
+                if (!room(kb)) return false;
+                unsigned char* tw = tiles + (kb & 1) * F::BUF + at;
+                unsigned char* ta = tw + NW * FT_W_TILE;
+                int odd = 0;
+#pragma unroll
+                for (int i = 0; i < LW; ++i) odd |= ft_store(x[i], tw + i * 16 * 128, FT_W_TILE) << i;
+                if constexpr (!F::IMAGE) {
+#pragma unroll
+                    for (int i = 0; i < LA; ++i) odd |= ft_store(ra[i], ta + i * 16 * 128, F::A_TILE) << (LW + i);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the next loads, which it would wait for
+                mark(odd);
+                __syncwarp();
+                if (lane == 0) ft_arrive(&full[kb & 1]);
+                fetch_w(kb + F::SETS, x);
+                fetch_a(kb + 1);
+                return true;
+            };
+#pragma unroll
+            for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
+            fetch_a(0);
+            for (int kb = 0; kb < nk; kb += F::SETS) {
+                if (!step(kb, rw[0])) break;
+                if (F::SETS == 2 && kb + 1 < nk && !step(kb + 1, rw[F::SETS - 1])) break;
+            }
         }
     } else if (warp == F::MMA || warp == F::MMA + 1) {
         if (lane == 0) {
@@ -296,6 +348,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
                 ok = (kb < 2 || ft_wait(&taken[b], ((kb >> 1) & 1) ^ 1, abort_flag)) &&
                      (!F::IMAGE || ft_wait(&landed[b], (kb >> 1) & 1, abort_flag)) && ft_wait(&full[b], (kb >> 1) & 1, abort_flag);
                 if (!ok) break;
+                if (F::EARLY) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 ft_fence_after();
                 const uint32_t tw = smem_u32(tiles + b * F::BUF), ta = tw + NW * FT_W_TILE, d = tmem_base + b * ACOL;
                 uint32_t accumulate = 0;
