@@ -237,7 +237,8 @@ attn_generic_kernel(const TQ* __restrict__ q, const T* __restrict__ kcache, cons
 // rows share an instruction, each rounded as by itself, and every sum runs in the order of the kernel above: the same bits. Tokens of
 // different sequences in a block are walked one sequence after the other. A key past a row's own token is not multiplied into it.
 // What bounds it is shared memory (a 16-byte read of a warp takes four cycles however many lanes share it): a thread makes the dots
-// of two keys and adds up two value numbers, for half of the rows, so that a read of queries or of weights serves twice.
+// of two keys and adds up two value numbers, for half of the rows, so that a read of queries or of weights serves twice. Then the
+// time of the longest block, a chunk after the other: so a page is looked up once a chunk, and values are fetched sixteen keys ahead.
 // MEASURED
 #define AP_Q 4
 typedef unsigned long long ap_f2;
@@ -261,7 +262,7 @@ template <int HB>
 __global__ void __launch_bounds__(AG_THREADS)
 attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kcache, const float* __restrict__ vcache,
                        const int* __restrict__ block_table, int bt_stride, const int* __restrict__ tok_seq,
-                       const int* __restrict__ tok_pos, float* __restrict__ out, int N, int nq, int nkv, int d, int dv, float scale) {
+                       const int* __restrict__ tok_pos, float* __restrict__ out, int N, int nq, int nkv, int d, int dv, float scale, int q_vec) {
     pdl_wait();      // nothing of this kernel touches global memory before this
     pdl_trigger();
     constexpr int R = HB * AP_Q, RP = R + 4;         // rows (token t, head h: t HB + h); floats a key's weights lie apart
@@ -286,9 +287,22 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
             x[0] = *reinterpret_cast<const ap_f2*>(p + half * (R / 2));
         }
     };
-    for (int i = tid; i < R * d; i += AG_THREADS) {
-        const int r = i / d, e = i - r * d, t = r / HB;
-        qs[e * RP + r] = t < nt ? q[((size_t)(n0 + t) * nq + head0 + r % HB) * d + e] : 0.0f;
+    const int warp = tid >> 5, e4 = 4 * (tid & 31);  // a warp a row, a lane 16 bytes of it
+#pragma unroll
+    for (int i = 0; i < R / 4; ++i) {
+        const int r = 4 * i + warp, t = r / HB;
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (e4 < d && t < nt) {
+            const float* p = q + ((size_t)(n0 + t) * nq + head0 + r % HB) * d + e4;
+            if (q_vec) x = *reinterpret_cast<const float4*>(p);
+            else x = make_float4(p[0], p[1], p[2], p[3]);
+        }
+        if (e4 < d) {
+            qs[e4 * RP + r] = x.x;
+            qs[(e4 + 1) * RP + r] = x.y;
+            qs[(e4 + 2) * RP + r] = x.z;
+            qs[(e4 + 3) * RP + r] = x.w;
+        }
     }
     for (int g0 = 0, g1; g0 < nt; g0 = g1) {
         const int seq = tok_seq[n0 + g0];
@@ -314,13 +328,16 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
         for (int c = 0; c <= p_max / AG_THREADS; ++c) {
             const int j = c * AG_THREADS + tid, jend = min(c * AG_THREADS + AG_THREADS - 1, p_max);
             __syncthreads();                         // the keys and weights of the chunk before have been read
-            const int w4 = d / 4;
-            for (int i = tid; i < (jend - c * AG_THREADS + 1) * w4; i += AG_THREADS) {
-                const int r = i / w4, e = 4 * (i - r * w4), jj = c * AG_THREADS + r;
-                const float* src = kcache + (((size_t)bt[jj / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + jj % LUMEN_PAGE) * d + e;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(ks + r * (d + 4) + e)),
-                             "l"(src)
-                             : "memory");
+            const int jc = c * AG_THREADS;           // a chunk is two pages, or less
+            const size_t page[2] = {((size_t)bt[jc / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE,
+                                    jc + LUMEN_PAGE <= jend ? ((size_t)bt[jc / LUMEN_PAGE + 1] * nkv + kvh) * LUMEN_PAGE : 0};
+            static_assert(AG_THREADS == 2 * LUMEN_PAGE, "");
+            if (e4 < d) {
+                for (int r = warp; r <= jend - jc; r += 4)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(ks + r * (d + 4) + e4)),
+                                 "l"(kcache + ((r < LUMEN_PAGE ? page[0] : page[1]) + r % LUMEN_PAGE) * d + e4)
+                                 : "memory");
             }
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
             __syncthreads();
@@ -384,28 +401,35 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
             for (int r = 0; r < R; ++r) l[r] = l[r] * corr[r] + s[r];
             const bool two = kp + 64 < dv;
             if (kp < dv) {
-                int j0 = c * AG_THREADS;
-                const int all = min(jend, p_min);    // in sight of every row
-                while (j0 <= all) {
-                    const int r0 = j0 % LUMEN_PAGE, nr = min(LUMEN_PAGE - r0, all - j0 + 1);      // a run within a page
-                    const float* v = vcache + (((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + r0) * dv + kp;
-                    const float* w = ps + (j0 - c * AG_THREADS) * RP;
-#pragma unroll 8
-                    for (int k = 0; k < nr; ++k) {
-                        const float x0 = v[(size_t)k * dv], x1 = two ? v[(size_t)k * dv + 64] : 0.0f;
-                        const ap_f2 v0 = ap_pair(x0, x0), v1 = ap_pair(x1, x1);
-                        ap_f2 ww[R / 4];
-                        rows2(w + k * RP, ww);
+                const int all = min(jend, p_min) - jc + 1;       // keys of the chunk in sight of every row
+                constexpr int AHEAD = 16;
+                float x0[AHEAD], x1[AHEAD];
+                auto value = [&](int k, int i) {
+                    const float* v = vcache + ((k < LUMEN_PAGE ? page[0] : page[1]) + k % LUMEN_PAGE) * dv + kp;
+                    x0[i] = k < all ? v[0] : 0.0f;
+                    x1[i] = k < all && two ? v[64] : 0.0f;
+                };
 #pragma unroll
-                        for (int r = 0; r < R / 4; ++r) {
-                            ap_fma(acc[0][r], ww[r], v0);
-                            ap_fma(acc[1][r], ww[r], v1);
+                for (int i = 0; i < AHEAD; ++i) value(i, i);
+                for (int k0 = 0; k0 < all; k0 += AHEAD) {
+#pragma unroll
+                    for (int i = 0; i < AHEAD; ++i) {
+                        const ap_f2 v0 = ap_pair(x0[i], x0[i]), v1 = ap_pair(x1[i], x1[i]);
+                        value(k0 + AHEAD + i, i);
+                        if (k0 + i < all) {
+                            ap_f2 ww[R / 4];
+                            rows2(ps + (k0 + i) * RP, ww);
+#pragma unroll
+                            for (int r = 0; r < R / 4; ++r) {
+                                ap_fma(acc[0][r], ww[r], v0);
+                                ap_fma(acc[1][r], ww[r], v1);
+                            }
                         }
                     }
-                    j0 += nr;
                 }
+                int j0 = jc + max(all, 0);
                 for (; j0 <= jend; ++j0) {           // the last few, of some rows only
-                    const float* v = vcache + (((size_t)bt[j0 / LUMEN_PAGE] * nkv + kvh) * LUMEN_PAGE + j0 % LUMEN_PAGE) * dv + kp;
+                    const float* v = vcache + ((j0 - jc < LUMEN_PAGE ? page[0] : page[1]) + j0 % LUMEN_PAGE) * dv + kp;
                     const float x0 = v[0], x1 = two ? v[64] : 0.0f;
                     const float* w = ps + (j0 - c * AG_THREADS) * RP + half * (R / 2);
 #pragma unroll
@@ -443,7 +467,7 @@ static int attn_prompt_f32_go(const float* q, const float* kcache, const float* 
     cudaError_t e = cudaFuncSetAttribute(attn_prompt_f32_kernel<HB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     lumen_launch(attn_prompt_f32_kernel<HB>, dim3((N + AP_Q - 1) / AP_Q, nq / HB), dim3(AG_THREADS), smem, stream, q, kcache, vcache,
-                 block_table, bt_stride, tok_seq, tok_pos, out, N, nq, nkv, d, dv, scale);
+                 block_table, bt_stride, tok_seq, tok_pos, out, N, nq, nkv, d, dv, scale, ((uintptr_t)q & 15) == 0);
     LUMEN_LAUNCH_CHECK();
     return 0;
 }
