@@ -14,8 +14,7 @@
 // one tile, one for each share, are a cluster and add up their sums through distributed shared memory. The number of
 // shares depends on N and K alone, so C[m,n] depends on row m of A and row n of W only, never on M or where they lie.
 //   warps 0..7   fetch 64 columns of W into registers, cut them and store the parts as 128-byte-swizzled tiles, two buffers.
-//                With more than 64 rows of A, where the products take the time, they have the parts ready in registers
-//                when a buffer is free again. Up to 32 rows of A go the same way; more are cut once, by a kernel
+//                Up to 32 rows of A go the same way; more are cut once, by a kernel
 //                ahead of this one, into the image their tiles have in shared memory (a block that cut 160 rows of A for its
 //                128 of W spent half of its time on them), and are copied by
 //   a warp       that does nothing else;
@@ -145,17 +144,17 @@ __device__ __forceinline__ uint32_t ft_cut(unsigned long long& x) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(x) : "l"(r), "l"(0xbf800000bf800000ull));       // x - r
     return h;
 }
-// The parts of four values of a row.
-template <typename T> struct FtParts { uint2 h[sizeof(T) == 4 ? 3 : 1]; };
-// 1 if one of the values is not finite (or rounds to infinity).
-__device__ __forceinline__ int ft_parts(const FtRaw<float>& x, FtParts<float>& to) {
+// Cuts four values and stores their parts `part` bytes apart; 1 if one of them is not finite (or rounds to infinity).
+__device__ __forceinline__ int ft_store(const FtRaw<float>& x, unsigned char* dst, int part) {
     unsigned long long a, b;
     asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(x.v.x), "f"(x.v.y));
     asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(x.v.z), "f"(x.v.w));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        to.h[i].x = ft_cut(a);
-        to.h[i].y = ft_cut(b);
+        uint2 h;
+        h.x = ft_cut(a);
+        h.y = ft_cut(b);
+        *reinterpret_cast<uint2*>(dst + i * part) = h;
     }
     // nothing is left (or less than bfloat16 has numbers for, of values below 2^-110), or NaN: an infinity less itself
     float u, v;
@@ -163,23 +162,10 @@ __device__ __forceinline__ int ft_parts(const FtRaw<float>& x, FtParts<float>& t
     asm("mov.b64 {%0, %1}, %2;" : "=f"(u), "=f"(v) : "l"(a));
     return !(u + v == u + v);
 }
-__device__ __forceinline__ int ft_parts(const FtRaw<__nv_bfloat16>& x, FtParts<__nv_bfloat16>& to) {
-    to.h[0] = x.v;
+__device__ __forceinline__ int ft_store(const FtRaw<__nv_bfloat16>& x, unsigned char* dst, int) {
+    *reinterpret_cast<uint2*>(dst) = x.v;
     const uint32_t e = 0x7f80u;
     return (x.v.x & e) == e || ((x.v.x >> 16) & e) == e || (x.v.y & e) == e || ((x.v.y >> 16) & e) == e;
-}
-// Parts go `part` bytes apart.
-template <typename T>
-__device__ __forceinline__ void ft_put(const FtParts<T>& x, unsigned char* dst, int part) {
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(x.h) / sizeof(x.h[0])); ++i) *reinterpret_cast<uint2*>(dst + i * part) = x.h[i];
-}
-template <typename T>
-__device__ __forceinline__ int ft_store(const FtRaw<T>& x, unsigned char* dst, int part) {
-    FtParts<T> p;
-    const int odd = ft_parts(x, p);
-    ft_put(p, dst, part);
-    return odd;
 }
 
 template <typename TW, int BN>
@@ -194,8 +180,7 @@ struct FtShape {
     static constexpr int CTL = 1024;                                     // barriers, flags, marks
     static constexpr int SMEM = 2 * BUF + CTL;
     static constexpr int MINB = (BN <= 16 && 2 * SMEM <= 220 * 1024) ? 2 : 1;
-    static constexpr bool EARLY = BN > 64;                               // W is cut before there is room for it
-    static constexpr int SETS = MINB == 1 && !EARLY ? 2 : 1;             // blocks of W under way in registers
+    static constexpr int SETS = MINB == 1 ? 2 : 1;                       // blocks of W under way in registers
     static_assert(BN * FT_ROWS * 4 <= 2 * BUF, "the sums are staged where the tiles were");
 };
 
@@ -293,50 +278,31 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
                 for (int i = 0; i < LA; ++i)
                     if (odd >> (LW + i) & 1) odd_a[r + 16 * i] = 1;
         };
-        if constexpr (F::EARLY) {
-            FtParts<TW> p[LW];
-            fetch_w(0, rw[0]);
-            for (int kb = 0; kb < nk; ++kb) {
-                int odd = 0;
+        auto step = [&](int kb, FtRaw<TW> (&x)[LW]) -> bool {
+            if (!room(kb)) return false;
+            unsigned char* tw = tiles + (kb & 1) * F::BUF + at;
+            unsigned char* ta = tw + NW * FT_W_TILE;
+            int odd = 0;
 #pragma unroll
-                for (int i = 0; i < LW; ++i) odd |= ft_parts(rw[0][i], p[i]) << i;
-                fetch_w(kb + 1, rw[0]);
-                mark(odd);
-                if (!room(kb)) break;
-                unsigned char* tw = tiles + (kb & 1) * F::BUF + at;
+            for (int i = 0; i < LW; ++i) odd |= ft_store(x[i], tw + i * 16 * 128, FT_W_TILE) << i;
+            if constexpr (!F::IMAGE) {
 #pragma unroll
-                for (int i = 0; i < LW; ++i) ft_put(p[i], tw + i * 16 * 128, FT_W_TILE);
-                // the fence between these stores and the products' reads is the issuing lane's: here it would wait for the loads
-                __syncwarp();
-                if (lane == 0) ft_arrive(&full[kb & 1]);
+                for (int i = 0; i < LA; ++i) odd |= ft_store(ra[i], ta + i * 16 * 128, F::A_TILE) << (LW + i);
             }
-        } else {
-            auto step = [&](int kb, FtRaw<TW> (&x)[LW]) -> bool {
-                if (!room(kb)) return false;
-                unsigned char* tw = tiles + (kb & 1) * F::BUF + at;
-                unsigned char* ta = tw + NW * FT_W_TILE;
-                int odd = 0;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the next loads, which it would wait for
+            mark(odd);
+            __syncwarp();
+            if (lane == 0) ft_arrive(&full[kb & 1]);
+            fetch_w(kb + F::SETS, x);
+            fetch_a(kb + 1);
+            return true;
+        };
 #pragma unroll
-                for (int i = 0; i < LW; ++i) odd |= ft_store(x[i], tw + i * 16 * 128, FT_W_TILE) << i;
-                if constexpr (!F::IMAGE) {
-#pragma unroll
-                    for (int i = 0; i < LA; ++i) odd |= ft_store(ra[i], ta + i * 16 * 128, F::A_TILE) << (LW + i);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the next loads, which it would wait for
-                mark(odd);
-                __syncwarp();
-                if (lane == 0) ft_arrive(&full[kb & 1]);
-                fetch_w(kb + F::SETS, x);
-                fetch_a(kb + 1);
-                return true;
-            };
-#pragma unroll
-            for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
-            fetch_a(0);
-            for (int kb = 0; kb < nk; kb += F::SETS) {
-                if (!step(kb, rw[0])) break;
-                if (F::SETS == 2 && kb + 1 < nk && !step(kb + 1, rw[F::SETS - 1])) break;
-            }
+        for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
+        fetch_a(0);
+        for (int kb = 0; kb < nk; kb += F::SETS) {
+            if (!step(kb, rw[0])) break;
+            if (F::SETS == 2 && kb + 1 < nk && !step(kb + 1, rw[F::SETS - 1])) break;
         }
     } else if (warp == F::MMA || warp == F::MMA + 1) {
         if (lane == 0) {
@@ -348,7 +314,6 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
                 ok = (kb < 2 || ft_wait(&taken[b], ((kb >> 1) & 1) ^ 1, abort_flag)) &&
                      (!F::IMAGE || ft_wait(&landed[b], (kb >> 1) & 1, abort_flag)) && ft_wait(&full[b], (kb >> 1) & 1, abort_flag);
                 if (!ok) break;
-                if (F::EARLY) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 ft_fence_after();
                 const uint32_t tw = smem_u32(tiles + b * F::BUF), ta = tw + NW * FT_W_TILE, d = tmem_base + b * ACOL;
                 uint32_t accumulate = 0;
