@@ -6,8 +6,8 @@
 // channel). Query/key head of value head h: h / (H / G). Everything is float32.
 //
 // A block takes one (sequence, head, slice of value channels) and walks the sequence's tokens of
-// the step strictly in order, so a token's sums do not depend on how the sequence was cut or
-// batched. A column j of S is independent of the others:
+// the step strictly in order (heads of 65 to 128 have another way for prompts, below), so a token's sums do not depend on how the
+// sequence was cut or batched. A column j of S is independent of the others:
 //   r = sum_i g_i S_ij k_i,  w = sum_i g_i S_ij q_i,  u_j = beta (v_j - r),  o_j = w + u_j (k . q),
 //   S_ij <- g_i S_ij + k_i u_j,
 // so the DR_ROWS rows a thread keeps in registers are read once a token; the NS threads of a
@@ -345,7 +345,9 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
 // reaches no earlier one.
 // Sequences of fewer than DC_MIN tokens walk them one by one, with the sums of a decode step: a few chunks are no faster
 // (us, 16 heads of 128 x 128, chunks / tokens: 33 tokens 14.5 / 13.6, 64 sequences of 24 218 / 215, 200 tokens 36 / 50).
-// MEASURED
+// 2,048 tokens of 16 heads of 128 x 128: 303 us with the kernel ahead (465 token by token), four sequences of 512 241 (339), nine
+// of 300 286 (396), one of 200 36 (50). The walk issues 1,480 instructions a chunk and warp, one in 2.6 cycles. Tried: two warps for the
+// same columns, one for P k and u, one for P q and o: 286 for one sequence, but 255 and 313 for four and nine.
 #define DC_T 16
 #define DC_MIN 48
 #define DC_D 128
@@ -380,16 +382,20 @@ delta_chunk_prepare_kernel(const DrIn in, float* __restrict__ prep, const int* _
     if (t0 < t_begin || t0 >= t_end) return;
     const int nt = min(DC_T, t_end - t0);
     float* rec = prep + ((size_t)blockIdx.x * in.H + h) * DC_REC;
-    const bool is_short = t_end - t_begin < DC_MIN;
+    if (t_end - t_begin < DC_MIN) {                // rows only; the warps of the first blocks share out all heads' tokens
+        const int i = h * DC_WARPS + warp;
+        if (i < nt * in.H)
+            dr_prepare_row(in, t0 + i / in.H, i % in.H, DC_D, prep + ((size_t)blockIdx.x * in.H + i % in.H) * DC_REC + i / in.H * DC_ROW);
+        return;
+    }
     {
-        float* row = is_short ? rec + warp * DC_ROW : rows + warp * DC_ROW;
+        float* row = rows + warp * DC_ROW;
         if (warp < nt) {
             dr_prepare_row(in, t0 + warp, h, DC_D, row);
-        } else if (!is_short) {                    // no token: nothing decays, nothing is written
+        } else {                                   // no token: nothing decays, nothing is written
             for (int e = lane; e < DC_ROW; e += 32) row[e] = (e >= 2 * DC_D && e < 3 * DC_D) ? 1.0f : 0.0f;
         }
     }
-    if (is_short) return;
     __syncthreads();
     {                                              // columns i = warp of A and B, a lane four channels
         const int i = warp;
