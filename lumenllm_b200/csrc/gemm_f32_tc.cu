@@ -23,10 +23,13 @@
 //   the others   add the finished accumulator (two of them, in tensor memory) to the sums in their registers.
 // Infinities and NaN have no parts: the rows that hold one are marked, and their outputs are made again with plain FMAs.
 //
-// What bounds it: for many rows cutting the operands, beside the tensor pipe (six bfloat16 products for one of 32 bits) and
-// shared memory (operands read by the products, parts written); for few rows the stream over W.
-// us, FFMA -> this: 300 rows x 16,384 outputs x 2,048 511 -> 187; 300 x 2,048 x 8,192 440 -> 151; 300 x 3,072 x 2,048
-// 115 -> 61; 100 x 2,048 x 8,192 222 -> 83; 16 x 32,768 x 2,048 95 -> 75; 8 x 2,048 x 8,192 60 -> 37.
+// What bounds it: for many rows the chain of a buffer, parts stored (1,270 cycles a block of 64 columns), products (1,900, the tensor
+// pipe's time for 24 of 128 x 160 x 16) and the barriers between, of which two are under way; for few rows the stream over W, of which
+// 64 KB an SM are under way; and some 9 us a block for its start, first fetch and sums.
+// us, FFMA -> this (with the kernel ahead): 300 rows x 16,384 outputs x 2,048 511 -> 122 (1.0 PFLOP/s of bfloat16 products); 300 x 2,048 x 8,192 440 -> 105;
+// 300 x 3,072 x 2,048 115 -> 42; 100 x 2,048 x 8,192 221 -> 61; 64 x 16,384 x 2,048 115 -> 50; 16 x 32,768 x 2,048 94 -> 72;
+// 8 x 2,048 x 8,192 59 -> 32; 8 x 1,024 x 1,024 9.0 -> 8.9. Tried, 300 x 16,384 x 2,048: A cut by every block 169; one warp issuing, loads
+// asked for before the fence 136; two groups of cutting warps in turns 147; parts waiting in registers for a buffer 172.
 // Every wait is bounded; when one runs out the block raises the error flag, its other roles give up on theirs, and the
 // block leaves, through the same cluster barriers as ever, once the products it has issued are done.
 #include "common.cuh"
