@@ -220,6 +220,7 @@ CLASSES = {
     "lumen_attn_decode": "attention", "lumen_attn_decode_qkv": "attention", "lumen_attn_prefill_tc": "attention",
     "lumen_attn_prefill": "attention", "lumen_attn_generic": "attention", "lumen_attn_talk": "attention",
     "lumen_attn_talk_prompt": "attention", "lumen_argmax": "sampling", "lumen_sample": "sampling",
+    "lumen_sample_held": "sampling",
     "lumen_gemm_tc_qkv": "qkv product + q/k norm + cache write",
     "lumen_conv_silu": "recurrence: convolution", "lumen_ssm_scan": "state-space: recurrence",
     "lumen_gated_part_norm": "state-space: gate + norm", "lumen_xielu": "activation",

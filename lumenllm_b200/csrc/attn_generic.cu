@@ -274,7 +274,8 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
     __shared__ float red[R][32];
     const int tid = threadIdx.x, head0 = blockIdx.y * HB, kvh = head0 / (nq / nkv);
     const int kp = tid & 63, half = tid >> 6;        // of a warp the same
-    const int n0 = blockIdx.x * AP_Q, nt = min(AP_Q, N - n0);
+    // the upper half of the heads from the last tokens on, so that blocks that see many keys and few share an SM
+    const int n0 = (int)(2 * blockIdx.y < gridDim.y ? blockIdx.x : gridDim.x - 1 - blockIdx.x) * AP_Q, nt = min(AP_Q, N - n0);
     // pairs of rows of this half, side by side
     auto rows2 = [&](const float* p, ap_f2 (&x)[R / 4]) {
         if constexpr (R >= 8) {
@@ -405,27 +406,41 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
                 const int all = min(jend, p_min) - jc + 1;       // keys of the chunk in sight of every row
                 constexpr int AHEAD = 16;
                 float x0[AHEAD], x1[AHEAD];
-                auto value = [&](int k, int i) {
-                    const float* v = vcache + ((k < LUMEN_PAGE ? page[0] : page[1]) + k % LUMEN_PAGE) * dv + kp;
-                    x0[i] = k < all ? v[0] : 0.0f;
-                    x1[i] = k < all && two ? v[64] : 0.0f;
-                };
-#pragma unroll
-                for (int i = 0; i < AHEAD; ++i) value(i, i);
-                for (int k0 = 0; k0 < all; k0 += AHEAD) {
+                static_assert(LUMEN_PAGE % AHEAD == 0, "");
+                auto fetch = [&](int k0) {               // keys k0 to k0 + 15 of the chunk, of one page
+                    const float* v = vcache + ((k0 < LUMEN_PAGE ? page[0] : page[1]) + k0 % LUMEN_PAGE) * dv + kp;
 #pragma unroll
                     for (int i = 0; i < AHEAD; ++i) {
-                        const ap_f2 v0 = ap_pair(x0[i], x0[i]), v1 = ap_pair(x1[i], x1[i]);
-                        value(k0 + AHEAD + i, i);
-                        if (k0 + i < all) {
-                            ap_f2 ww[R / 4];
-                            rows2(ps + (k0 + i) * RP, ww);
+                        x0[i] = k0 + i < all ? v[(size_t)i * dv] : 0.0f;
+                        x1[i] = k0 + i < all && two ? v[(size_t)i * dv + 64] : 0.0f;
+                    }
+                };
+                auto add = [&](int k, float a, float b) {
+                    const ap_f2 v0 = ap_pair(a, a), v1 = ap_pair(b, b);
+                    ap_f2 ww[R / 4];
+                    rows2(ps + k * RP, ww);
 #pragma unroll
-                            for (int r = 0; r < R / 4; ++r) {
-                                ap_fma(acc[0][r], ww[r], v0);
-                                ap_fma(acc[1][r], ww[r], v1);
-                            }
-                        }
+                    for (int r = 0; r < R / 4; ++r) {
+                        ap_fma(acc[0][r], ww[r], v0);
+                        ap_fma(acc[1][r], ww[r], v1);
+                    }
+                };
+                fetch(0);
+                for (int k0 = 0; k0 < all; k0 += AHEAD) {
+                    float y0[AHEAD], y1[AHEAD];
+#pragma unroll
+                    for (int i = 0; i < AHEAD; ++i) {
+                        y0[i] = x0[i];
+                        y1[i] = x1[i];
+                    }
+                    fetch(min(k0 + AHEAD, AG_THREADS - AHEAD));      // of the last batch again, if there is none
+                    if (k0 + AHEAD <= all) {
+#pragma unroll
+                        for (int i = 0; i < AHEAD; ++i) add(k0 + i, y0[i], y1[i]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < AHEAD; ++i)
+                            if (k0 + i < all) add(k0 + i, y0[i], y1[i]);
                     }
                 }
                 int j0 = jc + max(all, 0);

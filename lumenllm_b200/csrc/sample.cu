@@ -766,11 +766,22 @@ __device__ int sample_list(Cluster& cluster, const float* lg, int V, int rank, i
     return (int)~(unsigned)q.sorted[q.sel_pos];
 }
 
-// opts: per row (temperature, top_p, min_p, u); top_k: per row. A cluster of 1 to QC blocks a row
-// (the launch says how many); the token does not depend on how many.
+// A row's options: opts per row (temperature, top_p, min_p, u), top_k per row. On the device, or, for a caller who has them on the host
+// and few rows, in the launch itself: no copy ahead of the kernel, no memory for it (8 rows of 151,936 through DeviceSampler.pick: PICKED).
+struct SampleAt {
+    const float* opts;
+    const int* top_k;
+};
+#define SM_HELD_ROWS 64
+struct SampleHeld {
+    float opts[4 * SM_HELD_ROWS];
+    int top_k[SM_HELD_ROWS];
+};
+
+// A cluster of 1 to QC blocks a row (the launch says how many); the token does not depend on how many.
+template <typename Options>
 __global__ void __launch_bounds__(SM_THREADS)
-sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
-              const float* __restrict__ opts, const int* __restrict__ top_k_arr,
+sample_kernel(const float* __restrict__ logits, long long row_stride, int V, const __grid_constant__ Options o,
               int* __restrict__ out) {
     pdl_wait();      // nothing of this kernel touches global memory before this
     pdl_trigger();
@@ -781,11 +792,11 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
     __shared__ Shared sh;
     __shared__ Quick quick;
     const float* lg = logits + (size_t)row * row_stride;
-    const float temperature = opts[row * 4 + 0];
-    const float top_p = opts[row * 4 + 1];
-    const float min_p = opts[row * 4 + 2];
-    const float u = opts[row * 4 + 3];
-    const int top_k = top_k_arr[row];
+    const float temperature = o.opts[row * 4 + 0];
+    const float top_p = o.opts[row * 4 + 1];
+    const float min_p = o.opts[row * 4 + 2];
+    const float u = o.opts[row * 4 + 3];
+    const int top_k = o.top_k[row];
 
     // Every block: largest value (lowest index) and largest finite value of its share, told to all.
     {
@@ -993,10 +1004,8 @@ LUMEN_API int lumen_argmax(const float* logits, long long row_stride, int B, int
     return 0;
 }
 
-LUMEN_API int lumen_sample(const float* logits, long long row_stride, int B, int V,
-                           const float* opts, const int* top_k, int* out, cudaStream_t stream) {
-    if (B <= 0) return 0;
-    if (V <= 0) return LUMEN_ERR_BAD_ARGUMENT;
+template <typename Options>
+static int sample_go(const float* logits, long long row_stride, int B, int V, const Options& o, int* out, cudaStream_t stream) {
     // blocks a row: as many as keep about 148 SMs busy, so a few rows are spread wide and many
     // rows are not slowed down by blocks that mostly wait for their cluster's first
     const int qc = B <= 16 ? 8 : (B <= 32 ? 4 : (B <= 64 ? 2 : 1));
@@ -1014,8 +1023,28 @@ LUMEN_API int lumen_sample(const float* logits, long long row_stride, int B, int
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = lumen_pdl_enabled() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, sample_kernel, logits, row_stride, V, opts, top_k, out);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, sample_kernel<Options>, logits, row_stride, V, o, out);
     if (e != cudaSuccess) return (int)e;
     LUMEN_LAUNCH_CHECK();
     return 0;
+}
+
+LUMEN_API int lumen_sample(const float* logits, long long row_stride, int B, int V,
+                           const float* opts, const int* top_k, int* out, cudaStream_t stream) {
+    if (B <= 0) return 0;
+    if (V <= 0) return LUMEN_ERR_BAD_ARGUMENT;
+    return sample_go(logits, row_stride, B, V, SampleAt{opts, top_k}, out, stream);
+}
+
+LUMEN_API int lumen_sample_held_rows(void) { return SM_HELD_ROWS; }
+
+// The same with opts [B, 4] and top_k [B] on the host, read before the call returns; B up to lumen_sample_held_rows().
+LUMEN_API int lumen_sample_held(const float* logits, long long row_stride, int B, int V,
+                                const float* opts, const int* top_k, int* out, cudaStream_t stream) {
+    if (B <= 0) return 0;
+    if (V <= 0 || B > SM_HELD_ROWS || !opts || !top_k) return LUMEN_ERR_BAD_ARGUMENT;
+    SampleHeld o = {};
+    for (int i = 0; i < 4 * B; ++i) o.opts[i] = opts[i];
+    for (int i = 0; i < B; ++i) o.top_k[i] = top_k[i];
+    return sample_go(logits, row_stride, B, V, o, out, stream);
 }

@@ -1708,6 +1708,25 @@ def sample(logits, opts, top_k, out=None):
     return out
 
 
+def sample_held_rows() -> int:
+    """Rows that sample_held takes."""
+    return int_fn("sample", "lumen_sample_held_rows", [])()
+
+
+def sample_held(logits, opts, top_k):
+    """sample with the options on the host, which go to the device in the launch itself: opts an array('f') of 4 B numbers,
+    top_k an array('i') of B; B up to sample_held_rows()."""
+    require(logits, F32, "sample.logits", contiguous=False)
+    B, V = logits.shape
+    if logits.stride(1) != 1 or opts.typecode != "f" or len(opts) != 4 * B or top_k.typecode != "i" or len(top_k) != B:
+        raise KernelError("sample: bad shapes")
+    out = torch.empty((B,), dtype=I32, device=logits.device)
+    f = fn("sample", "lumen_sample_held", [P, c_longlong, c_int, c_int, P, P, P, P])
+    check(f(ptr(logits), logits.stride(0), B, V, opts.buffer_info()[0], top_k.buffer_info()[0], ptr(out), stream_ptr()),
+          "sample")
+    return out
+
+
 _err_flags = {}
 
 

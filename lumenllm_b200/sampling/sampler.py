@@ -13,6 +13,7 @@ request samples the same tokens alone and in any batch.
 from __future__ import annotations
 
 import os
+from array import array
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -85,7 +86,11 @@ class DeviceSampler:
             raise ValueError("one sampling config and one uniform number per row")
         if all(c.greedy for c in configs):
             return K.argmax(logits)
-        # options and top-k go to the device in one copy (two, with a tensor each, were most of a small call's time)
+        if B <= K.sample_held_rows():       # in the launch: a copy ahead of it was most of a small call's time
+            opts = array("f")
+            for c, u in zip(configs, us):
+                opts.extend((c.temperature, c.top_p, c.min_p, u))
+            return K.sample_held(logits, opts, array("i", [int(c.top_k) for c in configs]))
         host = torch.from_numpy(pack_options(configs, us, B)).pin_memory()
         both = host.to(self.device, non_blocking=True)
         return K.sample(logits, both[:4 * B].view(B, 4), both[4 * B:].view(torch.int32))

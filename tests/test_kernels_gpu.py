@@ -803,6 +803,22 @@ def test_sampler_against_the_plain_one(V):
     assert _sample_rows(lg[3:4], opts[3:4], ks[3:4]) == got[3:4]
 
 
+@pytest.mark.parametrize("rows", [1, 7, 64, 65])
+def test_options_in_the_launch_or_on_the_device(rows):
+    """Up to 64 rows' options go to the device in the launch itself: the tokens of options that lie on the device."""
+    from lumenllm_b200.ops import kernels as K
+    from lumenllm_b200.sampling import DeviceSampler, SamplingConfig, uniform
+    from lumenllm_b200.sampling.sampler import pack_options
+    g = gen(rows)
+    logits = dev(torch.randn(rows, 5003, generator=g) * 3)
+    configs = [SamplingConfig(temperature=(0.0, 0.7, 1.3)[i % 3], top_k=(0, 20, 1, 1500)[i % 4], top_p=(1.0, 0.8)[i % 2],
+                              min_p=(0.0, 0.05)[i // 2 % 2]) for i in range(1, rows + 1)]
+    us = [uniform(3, i, 1) for i in range(rows)]
+    both = torch.from_numpy(pack_options(configs, us, rows)).cuda()
+    want = K.sample(logits, both[:4 * rows].view(rows, 4), both[4 * rows:].view(torch.int32))
+    assert torch.equal(DeviceSampler(logits.device).pick(logits, configs, us), want)
+
+
 def test_sampler_edges():
     V = 777
     lg = torch.full((6, V), -5.0)
