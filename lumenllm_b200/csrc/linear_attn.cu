@@ -575,9 +575,7 @@ __global__ void __launch_bounds__(128)
 low_rank_decay_kernel(const float* __restrict__ u, int S, size_t split_stride, int W, int c_col, int R,
                       const float* __restrict__ w, const float* __restrict__ bias, float inv_tau,
                       float* __restrict__ alpha, int N, int C, int twice, const BonusOf bo) {
-    // no early trigger for prompts: see linear_attn_prep_kernel. Steps of a few tokens (decoding) have no such walk behind them, and
-    // what follows starts 2 us earlier.
-    if (N <= LD_TOK) pdl_trigger();
+    // no early trigger: see linear_attn_prep_kernel
     __shared__ __align__(16) float ts[LD_RANK][LD_TOK + 4];
     const int n0 = blockIdx.y * LD_TOK, channel_blocks = (C + 128 * CPT - 1) / (128 * CPT);
     if ((int)blockIdx.x >= channel_blocks) {
