@@ -239,8 +239,8 @@ attn_generic_kernel(const TQ* __restrict__ q, const T* __restrict__ kcache, cons
 // What bounds it is shared memory (a 16-byte read of a warp takes four cycles however many lanes share it): a thread makes the dots
 // of two keys and adds up two value numbers, for half of the rows, so that a read of queries or of weights serves twice. Then the
 // time of the longest block, a chunk after the other: so a page is looked up once a chunk, and values are fetched sixteen keys ahead.
-// 300 tokens of 16 heads of 128 over 4 key heads, inside the step: 122 us a layer with a token a block, 56 so (63 with one key and one
-// value number a thread).
+// 300 tokens of 16 heads of 128 over 4 key heads, inside the step: 122 us a layer with a token a block, 46 so (63 with one key and one
+// value number a thread, 56 with a predicate a key and long blocks beside long ones).
 #define AP_Q 4
 typedef unsigned long long ap_f2;
 __device__ __forceinline__ ap_f2 ap_pair(float lo, float hi) {

@@ -190,7 +190,7 @@ struct FtShape {
 template <typename TW, int BN>
 __global__ void __launch_bounds__(32 * FtShape<TW, BN>::WARPS, FtShape<TW, BN>::MINB)
 gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict__ image, const unsigned char* __restrict__ image_odd,
-                   const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int vec, int give_up_at,
+                   const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int vec, int early, int give_up_at,
                    int* __restrict__ err) {
     using F = FtShape<TW, BN>;
     constexpr int NW = F::NW, EPI = F::EPI, ACOL = F::TMEM / 2;
@@ -230,9 +230,29 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    pdl_wait();      // nothing of this kernel touches global memory before this
-    pdl_trigger();
     const int rows = min(bn, M - m0), cols = min(FT_ROWS, N - n0);
+    // fetches of a cutting warp's thread: 16 threads a row
+    constexpr int LW = FT_ROWS / 16, LA = BN / 16;
+    const int c = threadIdx.x & 15, r = threadIdx.x >> 4;
+    FtRaw<TW> rw[F::SETS][LW];
+    auto fetch_w = [&](int kb, FtRaw<TW> (&x)[LW]) {
+        const int k = (kb0 + kb) * FT_BK + 4 * c;
+        const TW* p = W + (size_t)(n0 + r) * K + k;
+#pragma unroll
+        for (int i = 0; i < LW; ++i) ft_fetch(x[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < cols ? K - k : 0, vec);
+    };
+    // A model's weights never change: its first ones are asked for before the kernel ahead has ended. Nothing else of this
+    // kernel touches global memory before the wait.
+    if (early && warp < FT_CONV) {
+#pragma unroll
+        for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (!early && warp < FT_CONV) {
+#pragma unroll
+        for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
+    }
     int marked = 0;
     for (int i = threadIdx.x; i < FT_ROWS + BN; i += blockDim.x) {
         const int m = i - FT_ROWS;
@@ -246,16 +266,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
     float* sums = reinterpret_cast<float*>(tiles);             // [BN][128], over the tiles once they have been read
 
     if (warp < FT_CONV) {
-        constexpr int LW = FT_ROWS / 16, LA = BN / 16;                       // fetches a thread: 16 threads a row
-        const int c = threadIdx.x & 15, r = threadIdx.x >> 4;
-        FtRaw<TW> rw[F::SETS][LW];
         FtRaw<float> ra[F::IMAGE ? 1 : LA];
-        auto fetch_w = [&](int kb, FtRaw<TW> (&x)[LW]) {
-            const int k = (kb0 + kb) * FT_BK + 4 * c;
-            const TW* p = W + (size_t)(n0 + r) * K + k;
-#pragma unroll
-            for (int i = 0; i < LW; ++i) ft_fetch(x[i], p + (size_t)(16 * i) * K, kb < nk && r + 16 * i < cols ? K - k : 0, vec);
-        };
         auto fetch_a = [&](int kb) {
             const int k = (kb0 + kb) * FT_BK + 4 * c;
             const float* p = A + (size_t)(m0 + r) * K + k;
@@ -300,8 +311,6 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
             fetch_a(kb + 1);
             return true;
         };
-#pragma unroll
-        for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
         fetch_a(0);
         for (int kb = 0; kb < nk; kb += F::SETS) {
             if (!step(kb, rw[0])) break;
@@ -493,7 +502,7 @@ static size_t gemm_f32_tc_image(int M, int K) {               // bytes of the im
 
 template <typename TW, int BN>
 static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* work, int M, int N, int K, int bn, int S,
-                          int give_up_at, int* err, cudaStream_t stream) {
+                          int early, int give_up_at, int* err, cudaStream_t stream) {
     using F = FtShape<TW, BN>;
     auto k = gemm_f32_tc_kernel<TW, BN>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
@@ -519,7 +528,7 @@ static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* 
     cfg.attrs = attr;
     cfg.numAttrs = lumen_pdl_enabled() ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, k, A, (const unsigned char*)work, (const unsigned char*)odd, W, C, M, N, K, bn,
-                           F::IMAGE ? vec_w : vec_a && vec_w, give_up_at, err);
+                           F::IMAGE ? vec_w : vec_a && vec_w, early, give_up_at, err);
     if (e != cudaSuccess) return (int)e;
     LUMEN_LAUNCH_CHECK();
     return 0;
@@ -534,11 +543,11 @@ static int gemm_f32_tc_shares(int N, int K) {
 }
 
 template <typename TW>
-static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, unsigned char* work, int M, int N, int K, int give_up_at, int* err,
-                            cudaStream_t stream) {
+static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, unsigned char* work, int M, int N, int K, int early, int give_up_at,
+                            int* err, cudaStream_t stream) {
     const int S = gemm_f32_tc_shares(N, K), bn = gemm_f32_tc_tile(M);
 #define FT_GO(BN) \
-    if (bn <= BN) return gemm_f32_tc_go<TW, BN>(A, W, C, work, M, N, K, bn, S, give_up_at, err, stream)
+    if (bn <= BN) return gemm_f32_tc_go<TW, BN>(A, W, C, work, M, N, K, bn, S, early, give_up_at, err, stream)
     FT_GO(16);
     FT_GO(32);
     FT_GO(64);
@@ -561,14 +570,15 @@ LUMEN_API long long lumen_gemm_f32_tc_scratch(int M, int K) {
 }
 
 // A float32 [M, K], W float32 or bfloat16 [N, K], C float32 [M, N], rows dense, of any alignment their types
-// have. work: lumen_gemm_f32_tc_scratch(M, K) bytes, 16-byte aligned. give_up_at: the block of k at which the adding warps
+// have. work: lumen_gemm_f32_tc_scratch(M, K) bytes, 16-byte aligned. early: W was written before the kernels that are still on
+// their way in the stream (a model's weights), and may be read before they end. give_up_at: the block of k at which the adding warps
 // take their wait as run out (-1: none; for tests of what a block does then).
 LUMEN_API int lumen_gemm_f32_tc(const float* A, const void* W, int w_is_bf16, float* C, void* work, int M, int N, int K,
-                                int give_up_at, int* err, cudaStream_t stream) {
+                                int early, int give_up_at, int* err, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || ((uintptr_t)work & 15) || (!work && gemm_f32_tc_image(M, K))) return LUMEN_ERR_BAD_ARGUMENT;
     if ((M + 63) / 64 > 65535 || (N + FT_ROWS - 1) / FT_ROWS > 65535) return LUMEN_ERR_UNSUPPORTED;
     unsigned char* w = (unsigned char*)work;
-    return w_is_bf16 ? gemm_f32_tc_rows(A, (const __nv_bfloat16*)W, C, w, M, N, K, give_up_at, err, stream)
-                     : gemm_f32_tc_rows(A, (const float*)W, C, w, M, N, K, give_up_at, err, stream);
+    return w_is_bf16 ? gemm_f32_tc_rows(A, (const __nv_bfloat16*)W, C, w, M, N, K, early, give_up_at, err, stream)
+                     : gemm_f32_tc_rows(A, (const float*)W, C, w, M, N, K, early, give_up_at, err, stream);
 }

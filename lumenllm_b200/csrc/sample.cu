@@ -767,7 +767,7 @@ __device__ int sample_list(Cluster& cluster, const float* lg, int V, int rank, i
 }
 
 // A row's options: opts per row (temperature, top_p, min_p, u), top_k per row. On the device, or, for a caller who has them on the host
-// and few rows, in the launch itself: no copy ahead of the kernel, no memory for it (8 rows of 151,936 through DeviceSampler.pick: PICKED).
+// and few rows, in the launch itself: no copy ahead of the kernel, no memory for it (8 rows of 151,936 through DeviceSampler.pick: 21 us, 37 with a copy).
 struct SampleAt {
     const float* opts;
     const int* top_k;

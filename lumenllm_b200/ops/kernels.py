@@ -1469,9 +1469,10 @@ def delta_rule(x, q_col, k_col, v_col, u, beta_col, a, dt_bias, a_log, state, cu
     return y
 
 
-def gemm_f32(a, w, out=None):
+def gemm_f32(a, w, out=None, weight_ready=False):
     """C = a @ w.T with 32-bit error. a float32 [M, K]; w [N, K] float32|bfloat16. The weight's size decides between the tensor
-    cores on three bfloat16 parts a number (csrc/gemm_f32_tc.cu) and FFMA, so a row's result is the same in any batch."""
+    cores on three bfloat16 parts a number (csrc/gemm_f32_tc.cu) and FFMA, so a row's result is the same in any batch.
+    weight_ready: no kernel that may still be running writes w (a model's weights), so it may be read ahead of its turn."""
     require(a, F32, "gemm_f32.a")
     M, K = a.shape
     N, K2 = w.shape
@@ -1486,8 +1487,8 @@ def gemm_f32(a, w, out=None):
         size.restype = c_longlong
         n = size(M, K)
         work = torch.empty((n,), dtype=torch.uint8, device=a.device) if n else None      # a cut into its parts
-        f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, P, c_int, c_int, c_int, c_int, P, P])
-        check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), ptr(work), M, N, K, -1, ptr(error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
+        f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, P, c_int, c_int, c_int, c_int, c_int, P, P])
+        check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), ptr(work), M, N, K, 1 if weight_ready else 0, -1, ptr(error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
         return out
     f = fn("gemm_f32", "lumen_gemm_f32", [P, P, c_int, P, c_int, c_int, c_int, P])
     check(f(ptr(a), ptr(w), _is_bf16(w), ptr(out), M, N, K, stream_ptr()), "gemm_f32")

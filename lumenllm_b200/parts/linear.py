@@ -71,5 +71,5 @@ class Linear:
         if self.f32:
             if x.dtype != torch.float32:
                 x = x.float()
-            return K.gemm_f32(x, self.weight)
+            return K.gemm_f32(x, self.weight, weight_ready=True)
         return G.gemm_bf16(x, self.weight, split_ok=split_ok, add_to=add_to, col_scale=factor)

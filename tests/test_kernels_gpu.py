@@ -595,13 +595,13 @@ def test_a_float32_product_that_gives_up_says_so():
     from lumenllm_b200.ops import kernels as K
     from lumenllm_b200.ops.native import check, fn, ptr, stream_ptr
     P = c_void_p
-    f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, P, c_int, c_int, c_int, c_int, P, P])
+    f = fn("gemm_f32_tc", "lumen_gemm_f32_tc", [P, P, c_int, P, P, c_int, c_int, c_int, c_int, c_int, P, P])
     work = torch.empty(3 << 20, dtype=torch.uint8, device="cuda")
     for M, N, K_ in ((20, 1024, 4096), (150, 20000, 1024)):
         a, w = torch.ones(M, K_, device="cuda"), torch.ones(N, K_, device="cuda")
         for at, raises in ((1, True), (-1, False)):
             out = torch.empty(M, N, device="cuda")
-            check(f(ptr(a), ptr(w), 0, ptr(out), ptr(work), M, N, K_, at, ptr(K.error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
+            check(f(ptr(a), ptr(w), 0, ptr(out), ptr(work), M, N, K_, 0, at, ptr(K.error_flag(a.device)), stream_ptr()), "gemm_f32_tc")
             if raises:
                 with pytest.raises(K.KernelError):
                     K.check_error_flags()
