@@ -171,7 +171,8 @@ __device__ __forceinline__ int ft_store(const FtRaw<__nv_bfloat16>& x, unsigned 
     return (x.v.x & e) == e || ((x.v.x >> 16) & e) == e || (x.v.y & e) == e || ((x.v.y >> 16) & e) == e;
 }
 
-template <typename TW, int BN>
+// DEEP: a block has an SM to itself and two blocks of W under way (up to 16 rows, where two blocks share an SM if there are that many).
+template <typename TW, int BN, bool DEEP>
 struct FtShape {
     static constexpr int NW = sizeof(TW) == 4 ? 3 : 1;                   // parts of a weight
     static constexpr int HALVES = BN > 64 ? 2 : 1;                       // groups of four adding warps, by columns
@@ -182,17 +183,18 @@ struct FtShape {
     static constexpr int TMEM = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
     static constexpr int CTL = 1024;                                     // barriers, flags, marks
     static constexpr int SMEM = 2 * BUF + CTL;
-    static constexpr int MINB = (BN <= 16 && 2 * SMEM <= 220 * 1024) ? 2 : 1;
+    static constexpr int MINB = DEEP ? 1 : 2;
+    static_assert(DEEP || 2 * SMEM <= 220 * 1024, "two blocks fit an SM");
     static constexpr int SETS = MINB == 1 ? 2 : 1;                       // blocks of W under way in registers
     static_assert(BN * FT_ROWS * 4 <= 2 * BUF, "the sums are staged where the tiles were");
 };
 
-template <typename TW, int BN>
-__global__ void __launch_bounds__(32 * FtShape<TW, BN>::WARPS, FtShape<TW, BN>::MINB)
+template <typename TW, int BN, bool DEEP>
+__global__ void __launch_bounds__(32 * FtShape<TW, BN, DEEP>::WARPS, FtShape<TW, BN, DEEP>::MINB)
 gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict__ image, const unsigned char* __restrict__ image_odd,
                    const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int vec, int early, int give_up_at,
                    int* __restrict__ err) {
-    using F = FtShape<TW, BN>;
+    using F = FtShape<TW, BN, DEEP>;
     constexpr int NW = F::NW, EPI = F::EPI, ACOL = F::TMEM / 2;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* tiles = smem;
@@ -500,11 +502,11 @@ static size_t gemm_f32_tc_image(int M, int K) {               // bytes of the im
     return bn <= 32 ? 0 : (size_t)((M + bn - 1) / bn) * bn * ((K + FT_BK - 1) / FT_BK) * 3 * 128;
 }
 
-template <typename TW, int BN>
+template <typename TW, int BN, bool DEEP>
 static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* work, int M, int N, int K, int bn, int S,
                           int early, int give_up_at, int* err, cudaStream_t stream) {
-    using F = FtShape<TW, BN>;
-    auto k = gemm_f32_tc_kernel<TW, BN>;
+    using F = FtShape<TW, BN, DEEP>;
+    auto k = gemm_f32_tc_kernel<TW, BN, DEEP>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
     if (e != cudaSuccess) return (int)e;
     const int vec_a = (K & 3) == 0 && ((uintptr_t)A & 15) == 0, vec_w = (K & 3) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
@@ -546,14 +548,16 @@ template <typename TW>
 static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, unsigned char* work, int M, int N, int K, int early, int give_up_at,
                             int* err, cudaStream_t stream) {
     const int S = gemm_f32_tc_shares(N, K), bn = gemm_f32_tc_tile(M);
-#define FT_GO(BN) \
-    if (bn <= BN) return gemm_f32_tc_go<TW, BN>(A, W, C, work, M, N, K, bn, S, early, give_up_at, err, stream)
-    FT_GO(16);
-    FT_GO(32);
-    FT_GO(64);
-    FT_GO(96);
-    FT_GO(128);
-    FT_GO(160);
+#define FT_GO(BN, DEEP) \
+    if (bn <= BN) return gemm_f32_tc_go<TW, BN, DEEP>(A, W, C, work, M, N, K, bn, S, early, give_up_at, err, stream)
+    // two blocks an SM where there are more blocks than SMs (DEEPTIMES)
+    if ((long long)S * ((N + FT_ROWS - 1) / FT_ROWS) > 148) FT_GO(16, false);
+    FT_GO(16, true);
+    FT_GO(32, true);
+    FT_GO(64, true);
+    FT_GO(96, true);
+    FT_GO(128, true);
+    FT_GO(160, true);
 #undef FT_GO
     return LUMEN_ERR_UNSUPPORTED;
 }
