@@ -6,7 +6,7 @@
 //
 // The tensor core's own sums are short: 64 values of k and their parts, small ones first, into a fresh accumulator, which
 // is then added to a running sum in registers, rounded to nearest. So an output is a chain of K / 64 float32 adds (in
-// up to eight shares of k, added in rising order) where the FFMA kernel's is K / 4. Against a 64-bit product, 2-norm,
+// up to four shares of k, added in rising order) where the FFMA kernel's is K / 4. Against a 64-bit product, 2-norm,
 // this / FFMA: K = 1,000 9.7e-8 / 2.8e-7, 2,048 1.0e-7 / 4.1e-7, 8,192 1.2e-7 / 8.1e-7; of numbers that are all positive
 // 9.3e-8 / 1.3e-7, 8.8e-8 / 1.6e-7, 9.2e-8 / 3.1e-7.
 //
@@ -40,7 +40,7 @@
 #define FT_MAX_BN 160                    // rows of A a block
 #define FT_CONV 8                        // warps that fetch and cut
 #define FT_W_TILE (FT_ROWS * 128)        // bytes of one part of a tile of W
-#define FT_MAX_SHARES 8
+#define FT_MAX_SHARES 4                  // a cluster of eight, one block an SM, finds place 15 times at the most, one of four 33 times
 #define FT_MIN_N 1024                    // see lumen_gemm_f32_tc_takes
 #define FT_MIN_K 1024
 
