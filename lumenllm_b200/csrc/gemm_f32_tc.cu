@@ -7,8 +7,8 @@
 // The tensor core's own sums are short: 64 values of k and their parts, small ones first, into a fresh accumulator, which
 // is then added to a running sum in registers, rounded to nearest. So an output is a chain of K / 64 float32 adds (in
 // up to four shares of k, added in rising order) where the FFMA kernel's is K / 4. Against a 64-bit product, 2-norm,
-// this / FFMA: K = 1,000 9.7e-8 / 2.8e-7, 2,048 1.0e-7 / 4.1e-7, 8,192 1.2e-7 / 8.1e-7; of numbers that are all positive
-// 9.3e-8 / 1.3e-7, 8.8e-8 / 1.6e-7, 9.2e-8 / 3.1e-7.
+// this / FFMA: K = 1,000 9.7e-8 / 2.8e-7, 2,048 1.0e-7 / 4.1e-7, 8,192 1.4e-7 / 8.1e-7; of numbers that are all positive
+// 9.4e-8 / 1.3e-7, 8.8e-8 / 1.6e-7, 9.4e-8 / 3.1e-7.
 //
 // A block takes 128 rows of W (the 128-row side of the MMA) times up to 160 rows of A, for a share of k; the blocks of
 // one tile, one for each share, are a cluster and add up their sums through distributed shared memory. The number of
@@ -26,10 +26,11 @@
 // What bounds it: for many rows the chain of a buffer, parts stored (1,270 cycles a block of 64 columns), products (1,900, the tensor
 // pipe's time for 24 of 128 x 160 x 16) and the barriers between, of which two are under way; for few rows the stream over W, of which
 // 64 KB an SM are under way; and some 9 us a block for its start, first fetch and sums.
-// us, FFMA -> this (with the kernel ahead): 300 rows x 16,384 outputs x 2,048 511 -> 122 (1.0 PFLOP/s of bfloat16 products); 300 x 2,048 x 8,192 440 -> 105;
-// 300 x 3,072 x 2,048 115 -> 42; 100 x 2,048 x 8,192 221 -> 61; 64 x 16,384 x 2,048 115 -> 50; 16 x 32,768 x 2,048 94 -> 72;
-// 8 x 2,048 x 8,192 59 -> 32; 8 x 1,024 x 1,024 9.0 -> 8.9. Tried, 300 x 16,384 x 2,048: A cut by every block 169; one warp issuing, loads
-// asked for before the fence 136; two groups of cutting warps in turns 147; parts waiting in registers for a buffer 172.
+// us, FFMA -> this (with the kernel ahead): 300 rows x 16,384 outputs x 2,048 511 -> 118 (1.0 PFLOP/s of bfloat16 products); 300 x 2,048 x 8,192 438 -> 67;
+// 300 x 2,048 x 2,048 114 -> 23; 300 x 3,072 x 2,048 114 -> 41; 100 x 2,048 x 8,192 221 -> 56; 64 x 16,384 x 2,048 114 -> 48; 16 x 32,768 x 2,048
+// 94 -> 73; 8 x 16,384 x 2,048 60 -> 48; 8 x 2,048 x 8,192 59 -> 39; 8 x 1,024 x 1,024 8.8 -> 8.3. Tried, 300 x 16,384 x 2,048: A cut by every block 169; one
+// warp issuing, loads asked for before the fence 136; two groups of cutting warps in turns 147; parts waiting in registers for a buffer
+// 172. Eight shares: 300 x 2,048 x 8,192 101, 300 x 2,048 x 2,048 43, 8 x 2,048 x 8,192 32.
 // Every wait is bounded; when one runs out the block raises the error flag, its other roles give up on theirs, and the
 // block leaves, through the same cluster barriers as ever, once the products it has issued are done.
 #include "common.cuh"
@@ -550,7 +551,8 @@ static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, unsigned char
     const int S = gemm_f32_tc_shares(N, K), bn = gemm_f32_tc_tile(M);
 #define FT_GO(BN, DEEP) \
     if (bn <= BN) return gemm_f32_tc_go<TW, BN, DEEP>(A, W, C, work, M, N, K, bn, S, early, give_up_at, err, stream)
-    // two blocks an SM where there are more blocks than SMs (DEEPTIMES)
+    // two blocks an SM where there are more blocks than SMs (8 x 16,384 x 2,048, 128 blocks: 48 us, 52 with one
+    // block of weights under way)
     if ((long long)S * ((N + FT_ROWS - 1) / FT_ROWS) > 148) FT_GO(16, false);
     FT_GO(16, true);
     FT_GO(32, true);
