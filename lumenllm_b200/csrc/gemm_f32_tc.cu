@@ -41,7 +41,7 @@
 #define FT_MAX_BN 160                    // rows of A a block
 #define FT_CONV 8                        // warps that fetch and cut
 #define FT_W_TILE (FT_ROWS * 128)        // bytes of one part of a tile of W
-#define FT_MAX_SHARES 4                  // a cluster of eight, one block an SM, finds place 15 times at the most, one of four 33 times
+#define FT_MAX_SHARES 4                  // 16 clusters of eight blocks that fill an SM each take two rounds, 32 of four one
 #define FT_MIN_N 1024                    // see lumen_gemm_f32_tc_takes
 #define FT_MIN_K 1024
 
