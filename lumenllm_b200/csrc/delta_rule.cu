@@ -648,12 +648,13 @@ static inline int delta_rule_threads(int d) {
     return NS;
 }
 
-// Steps whose sequences go in chunks: heads of 65 to 128, and not one token a sequence.
-static inline bool delta_rule_chunks(int d, int N, int n_seqs) { return d > DC_D / 2 && d <= DC_D && N > n_seqs; }
+// Steps in which a sequence may go in chunks: heads of 65 to 128, and tokens for one long enough. Whether it does is its own
+// number of tokens alone: not how many sequences there are beside it, empty ones among them.
+static inline bool delta_rule_chunks(int d, int N, int one_each) { return d > DC_D / 2 && d <= DC_D && !one_each && N >= DC_MIN; }
 
 // Floats of scratch lumen_delta_rule needs for a step of N tokens in n_seqs sequences, H heads of d key channels.
-LUMEN_API long long lumen_delta_rule_scratch(int N, int n_seqs, int H, int d) {
-    if (delta_rule_chunks(d, N, n_seqs)) return ((long long)N / DC_T + n_seqs) * H * DC_REC;
+LUMEN_API long long lumen_delta_rule_scratch(int N, int n_seqs, int one_each, int H, int d) {
+    if (delta_rule_chunks(d, N, one_each)) return ((long long)N / DC_T + n_seqs) * H * DC_REC;
     return (long long)N * H * (3 * delta_rule_threads(d) * DR_ROWS + 4);
 }
 
@@ -661,11 +662,12 @@ LUMEN_API long long lumen_delta_rule_scratch(int N, int n_seqs, int H, int d) {
 // and v (H heads of dv, v_col). u: the projection's partial sums [uS, N, uW] with the H beta
 // logits from column b_col. a: partial sums [aS, N, H d] of the decay logits (before dt_bias).
 // state float32, row seq_slot[b] of stride slot_stride holds [H, dv, d]. y float32 [N, H dv]. prep:
-// lumen_delta_rule_scratch(N, n_seqs, H, d) floats of scratch. cu_q covers at most N tokens.
+// lumen_delta_rule_scratch(N, n_seqs, one_each, H, d) floats of scratch. cu_q covers at most N tokens. one_each: no sequence has
+// more than one token (a decode step).
 LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int v_col, const float* u, int uS,
                                long long u_stride, int uW, int b_col, const float* a, int aS, long long a_stride,
                                const float* dt_bias, const float* a_log, float* state, long long slot_stride,
-                               const int* cu_q, const int* seq_slot, int n_seqs, float* y, float* prep, int N, int H,
+                               const int* cu_q, const int* seq_slot, int n_seqs, int one_each, float* y, float* prep, int N, int H,
                                int G, int d, int dv, cudaStream_t stream) {
     if (n_seqs <= 0 || N <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || d > 32 * DR_ROWS || uS < 1 || aS < 1 || H > 65535)
@@ -681,7 +683,7 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
     const int threads = wide ? 2 * DR_THREADS : DR_THREADS, cols = threads / NS;
     const int vec = (d & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
     const DrIn in = {x, u, a, dt_bias, a_log, (size_t)u_stride, (size_t)a_stride, C, q_col, k_col, uS, uW, b_col, aS, H, G, d};
-    if (delta_rule_chunks(d, N, n_seqs)) {
+    if (delta_rule_chunks(d, N, one_each)) {
         if ((dv + DC_COLS - 1) / DC_COLS > 65535) return LUMEN_ERR_UNSUPPORTED;
         cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM);
         if (e != cudaSuccess) return (int)e;

@@ -473,6 +473,34 @@ def test_delta_rule_sixteen_tokens_at_a_time(d, dv, lens):
     assert not bool(torch.isfinite(yb[last]).all())
 
 
+@pytest.mark.parametrize("lens", [[60] + [0] * 70, [1] * 63 + [60] + [0] * 64, [2, 50, 47, 1, 128, 16]])
+def test_a_sequence_goes_as_it_does_alone_whatever_is_beside_it(lens):
+    """Chunks or token by token, and where the chunks lie, is a sequence's own number of tokens alone, also where there are more
+    sequences than tokens: the bits of a call by itself."""
+    from lumenllm_b200.ops import kernels as K
+    H, G, d, dv, B, N = 2, 1, 128, 16, len(lens), sum(lens)
+    g = torch.Generator().manual_seed(N)
+    rn = lambda *s: torch.randn(*s, generator=g).cuda()
+    C = 2 * G * d + H * dv
+    x, u, a, dt, al, st = rn(N, C), rn(1, N, H), rn(1, N, H * d), rn(H * d), rn(H) - 2.0, rn(B, H, dv, d)
+
+    def run(lens, rows, s):
+        cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32).cuda()
+        slots = torch.arange(len(lens), dtype=torch.int32).cuda()
+        y = K.delta_rule(x[rows].contiguous(), 0, G * d, 2 * G * d, u[:, rows].contiguous(), 0, a[:, rows].contiguous(), dt, al, s, cu, slots,
+                         len(lens), H, G, d, dv)
+        return y, s
+
+    y, s = run(lens, slice(0, N), st.clone())
+    for b, n in enumerate(lens):
+        if n:
+            at = sum(lens[:b])
+            yb, sb = run([n], slice(at, at + n), st[b:b + 1].clone())
+            assert torch.equal(yb, y[at:at + n]) and torch.equal(sb[0], s[b])
+        else:
+            assert torch.equal(s[b], st[b])
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_the_state_remembers_far_back_and_forgets_by_channel(dtype):
     """Decays close to one and one loud early token: what the state holds of that token decides the
