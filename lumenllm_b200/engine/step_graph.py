@@ -97,8 +97,10 @@ class StepGraphs:
             Bb = _bucket(n)
             return Bb, Bb, [1] * (Bb - n)
         Bb = _bucket(n + 1)                              # the first padding sequence takes the
-        Nb = _token_bucket(n_tok)                        # tokens that fill the bucket (maybe none),
-        return Nb, Bb, [Nb - n_tok] + [0] * (Bb - n - 1)  # the others are empty
+        # tokens that fill the bucket (maybe none), the others are empty. More tokens than sequences, so that
+        # many prompts of a token or two are never taken for the decode step of as many sequences.
+        Nb = _token_bucket(max(n_tok, Bb + 1))
+        return Nb, Bb, [Nb - n_tok] + [0] * (Bb - n - 1)
 
     def _capture(self, key, lay: StepLayout, lists, host) -> _Captured:
         eng = self.engine

@@ -229,3 +229,15 @@ def test_the_shape_of_a_captured_step_depends_on_counts_alone():
     for lens in ([5], [1, 2], [600, 300], [31] * 7):
         n_tok, n_seq, pads = StepGraphs.plan(lens)
         assert n_tok == sum(lens) + sum(pads) and n_seq == len(lens) + len(pads) and n_tok > n_seq
+
+
+def test_a_captured_prompt_step_is_never_taken_for_a_decode_step():
+    """Captured steps are kept by their buckets; many prompts of a token or two fill as many tokens as sequences, and must
+    not replay (or be replayed as) the decode step of that many sequences."""
+    from lumenllm_b200.engine.step_graph import StepGraphs
+    for n in (1, 2, 15, 16, 17, 31, 32, 33, 63, 64, 65, 130):
+        for more in (1, 2, n, 3 * n + 5):
+            lens = [1 + more] + [1] * (n - 1)
+            n_tok, n_seq, pads = StepGraphs.plan(lens)
+            assert n_tok == sum(lens) + sum(pads) and n_seq == n + len(pads) and min(pads) >= 0
+            assert n_tok > n_seq and (n_tok, n_seq) != StepGraphs.plan([1] * n_seq)[:2]
