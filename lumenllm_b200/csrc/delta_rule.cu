@@ -139,11 +139,10 @@ delta_prepare_kernel(const DrIn in, float* __restrict__ prep, int dp) {
 // NS: threads that share a column of S (a power of two), NS DR_ROWS >= d; every offset of the walk is a constant
 // of the instance. AHEAD: a token's rows are read from shared memory while the one before is worked on, which
 // takes twice the registers: for steps of several tokens a sequence. THREADS: of a block. Same sums either way.
-// row0: the row of the sequence's first token, the next ones row_stride floats on, every sixteenth group_stride after the
-// one sixteen before; zblock: which columns.
+// row0: the row of the sequence's first token, the next ones row_stride floats on; zblock: which columns.
 template <int NS, bool AHEAD, int THREADS>
 __device__ __forceinline__ void dr_walk(float* sm, const float* __restrict__ x, int C, int v_col, const float* __restrict__ row0,
-                                        size_t row_stride, size_t group_stride, int t_begin, int t_end, int zblock, float* __restrict__ S_head,
+                                        size_t row_stride, int t_begin, int t_end, int zblock, float* __restrict__ S_head,
                                         float* __restrict__ y, int H, int d, int dv, int vec) {
     constexpr int ROWS = DR_ROWS;
     constexpr int dp = NS * ROWS;                   // d padded to what the threads of a column hold
@@ -180,7 +179,7 @@ __device__ __forceinline__ void dr_walk(float* sm, const float* __restrict__ x, 
         float* rb = rows + buf * DR_CHUNK * PW;
         for (int i = tid; i < nt * pieces; i += THREADS) {
             const int tt = i / pieces, p = i - tt * pieces;
-            dr_cp16(rb + tt * PW + 4 * p, row0 + (size_t)((t0 + tt - t_begin) >> 4) * group_stride + ((t0 + tt - t_begin) & 15) * row_stride + 4 * p);
+            dr_cp16(rb + tt * PW + 4 * p, row0 + (size_t)(t0 + tt - t_begin) * row_stride + 4 * p);
         }
         float* vb = vs + buf * DR_CHUNK * cols;
         for (int i = tid; i < nt * cols; i += THREADS) {
@@ -324,7 +323,7 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
     constexpr int PW = 3 * NS * DR_ROWS + 4;
     const int b = blockIdx.x, h = blockIdx.y, t_begin = cu_q[b], t_end = cu_q[b + 1];
     if (t_end <= t_begin) return;
-    dr_walk<NS, AHEAD, THREADS>(sm, x, C, v_col, prep + ((size_t)t_begin * H + h) * PW, (size_t)H * PW, (size_t)16 * H * PW, t_begin, t_end, blockIdx.z,
+    dr_walk<NS, AHEAD, THREADS>(sm, x, C, v_col, prep + ((size_t)t_begin * H + h) * PW, (size_t)H * PW, t_begin, t_end, blockIdx.z,
                                 state + (size_t)seq_slot[b] * slot_stride + (size_t)h * dv * d, y, H, d, dv, vec);
 }
 
@@ -345,6 +344,9 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
 // reaches no earlier one.
 // Sequences of fewer than DC_MIN tokens walk them one by one, with the sums of a decode step: a few chunks are no faster
 // (us, 16 heads of 128 x 128, chunks / tokens: 33 tokens 14.5 / 13.6, 64 sequences of 24 218 / 215, 200 tokens 36 / 50).
+// Their rows lie where their tokens' shares of records would (a record a sequence of any length took 66 MB for 128 sequences of two
+// tokens of 16 heads; 11 so), and a step that is known to have no longer sequences goes to the kernels above (us, 128 sequences of two tokens
+// 136 here, 128 there; 200 of eight 317 / 302).
 // 2,048 tokens of 16 heads of 128 x 128: 303 us with the kernel ahead (465 token by token), four sequences of 512 241 (339), nine
 // of 300 286 (396), one of 200 36 (50). The walk issues 1,480 instructions a chunk and warp, one in 2.6 cycles. Tried: two warps for the
 // same columns, one for P k and u, one for P q and o: 286 for one sequence, but 255 and 313 for four and nine.
@@ -361,10 +363,28 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
 #define DC_REC (DC_BM + DC_T * DC_PITCH)                         // floats of a (chunk, head)
 #define DC_ROW (3 * DC_D + 4)                                    // a token's row, as above
 #define DC_WARPS 16                                              // of the kernel that prepares: one a token
-static_assert(DC_T * DC_ROW <= DC_REC, "a short sequence's rows lie in the records of its chunks");
+#define DC_TOKEN (DC_REC / DC_T)                                 // floats of scratch a (token, head)
+static_assert(DC_REC % DC_T == 0 && DC_ROW <= DC_TOKEN && DC_TOKEN % 4 == 0 && DC_ROW % 4 == 0, "a short sequence's rows lie where its share of a record would");
 
-// Where the chunks of sequence b start among all records: room for every cut of N tokens.
+// The block of the preparing kernel that sequence b's chunks begin at: room for every cut of N tokens.
 __device__ __forceinline__ int dc_first(const int* cu_q, int b) { return cu_q[b] / DC_T + b; }
+// The last sequence whose blocks begin at or before block x: for a whole warp, 32 sequences a look.
+__device__ __forceinline__ int dc_of_block(const int* cu_q, int n_seqs, int x) {
+    int lo = 0, n = n_seqs;
+    while (n > 1) {
+        const int step = (n + 31) / 32, b = lo + (int)(threadIdx.x & 31) * step;
+        const unsigned before = __ballot_sync(0xffffffffu, b < lo + n && dc_first(cu_q, min(b, n_seqs)) <= x);
+        const int k = max(__popc(before) - 1, 0);           // they are ordered: the first k + 1 lanes
+        n = min(step, n - k * step);
+        lo += k * step;
+    }
+    return lo;
+}
+// Where sequence b's share of the scratch begins, in (token, head) floats: records chunk by chunk, or rows token by token, all heads
+// side by side. A sequence in chunks may need one record more than its tokens' shares, the others do not.
+__host__ __device__ __forceinline__ size_t dc_place(int tokens, int seqs) {
+    return (size_t)tokens * DC_TOKEN + (size_t)DC_REC * (seqs < tokens / DC_MIN ? seqs : tokens / DC_MIN);
+}
 
 __global__ void __launch_bounds__(32 * DC_WARPS)
 delta_chunk_prepare_kernel(const DrIn in, float* __restrict__ prep, const int* __restrict__ cu_q, int n_seqs) {
@@ -372,22 +392,18 @@ delta_chunk_prepare_kernel(const DrIn in, float* __restrict__ prep, const int* _
     __shared__ __align__(16) float rows[DC_T * DC_ROW];
     __shared__ float A[DC_T][DC_T + 1];
     const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int lo = 0, hi = n_seqs - 1;                   // the last sequence whose records start at or before this one
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (dc_first(cu_q, mid) <= (int)blockIdx.x) lo = mid;
-        else hi = mid - 1;
-    }
+    const int lo = dc_of_block(cu_q, n_seqs, (int)blockIdx.x);
     const int t_begin = cu_q[lo], t_end = cu_q[lo + 1], t0 = t_begin + ((int)blockIdx.x - dc_first(cu_q, lo)) * DC_T;
     if (t0 < t_begin || t0 >= t_end) return;
     const int nt = min(DC_T, t_end - t0);
-    float* rec = prep + ((size_t)blockIdx.x * in.H + h) * DC_REC;
+    float* place = prep + dc_place(t_begin, lo) * in.H;
     if (t_end - t_begin < DC_MIN) {                // rows only; the warps of the first blocks share out all heads' tokens
         const int i = h * DC_WARPS + warp;
         if (i < nt * in.H)
-            dr_prepare_row(in, t0 + i / in.H, i % in.H, DC_D, prep + ((size_t)blockIdx.x * in.H + i % in.H) * DC_REC + i / in.H * DC_ROW);
+            dr_prepare_row(in, t0 + i / in.H, i % in.H, DC_D, place + ((size_t)(t0 - t_begin) * in.H + i) * DC_ROW);
         return;
     }
+    float* rec = place + ((size_t)((t0 - t_begin) / DC_T) * in.H + h) * DC_REC;
     {
         float* row = rows + warp * DC_ROW;
         if (warp < nt) {
@@ -498,10 +514,10 @@ delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* _
     const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
     if (t_end <= t_begin) return;
-    const float* rec0 = prep + ((size_t)dc_first(cu_q, b) * H + h) * DC_REC;
+    const float* rec0 = prep + dc_place(t_begin, b) * H;
     float* S_head = state + (size_t)seq_slot[b] * slot_stride + (size_t)h * dv * d;
     if (t_end - t_begin < DC_MIN) {
-        dr_walk<8, true, DR_THREADS>(sm, x, C, v_col, rec0, DC_ROW, (size_t)H * DC_REC, t_begin, t_end, blockIdx.z, S_head, y, H, d, dv, vec);
+        dr_walk<8, true, DR_THREADS>(sm, x, C, v_col, rec0 + (size_t)h * DC_ROW, (size_t)H * DC_ROW, t_begin, t_end, blockIdx.z, S_head, y, H, d, dv, vec);
         return;
     }
     const int j0 = blockIdx.z * DC_COLS + 4 * warp, c0 = 4 * lane;
@@ -526,7 +542,7 @@ delta_chunk_kernel(const float* __restrict__ x, int C, int v_col, const float* _
     }
     auto issue = [&](int t0, int chunk, int buf) {
         float* to = sm + buf * DC_BUF;
-        const float* from = rec0 + (size_t)chunk * H * DC_REC;
+        const float* from = rec0 + ((size_t)chunk * H + h) * DC_REC;
         for (int i = tid; i < DC_REC / 4; i += DR_THREADS) dr_cp16(to + 4 * i, from + 4 * i);
 #pragma unroll
         for (int i = tid; i < DC_T * DC_COLS; i += DR_THREADS) {
@@ -650,11 +666,11 @@ static inline int delta_rule_threads(int d) {
 
 // Steps in which a sequence may go in chunks: heads of 65 to 128, and tokens for one long enough. Whether it does is its own
 // number of tokens alone: not how many sequences there are beside it, empty ones among them.
-static inline bool delta_rule_chunks(int d, int N, int one_each) { return d > DC_D / 2 && d <= DC_D && !one_each && N >= DC_MIN; }
+static inline bool delta_rule_chunks(int d, int longest) { return d > DC_D / 2 && d <= DC_D && longest >= DC_MIN; }
 
 // Floats of scratch lumen_delta_rule needs for a step of N tokens in n_seqs sequences, H heads of d key channels.
-LUMEN_API long long lumen_delta_rule_scratch(int N, int n_seqs, int one_each, int H, int d) {
-    if (delta_rule_chunks(d, N, one_each)) return ((long long)N / DC_T + n_seqs) * H * DC_REC;
+LUMEN_API long long lumen_delta_rule_scratch(int N, int n_seqs, int longest, int H, int d) {
+    if (delta_rule_chunks(d, longest)) return (long long)dc_place(N, n_seqs) * H;
     return (long long)N * H * (3 * delta_rule_threads(d) * DR_ROWS + 4);
 }
 
@@ -662,12 +678,12 @@ LUMEN_API long long lumen_delta_rule_scratch(int N, int n_seqs, int one_each, in
 // and v (H heads of dv, v_col). u: the projection's partial sums [uS, N, uW] with the H beta
 // logits from column b_col. a: partial sums [aS, N, H d] of the decay logits (before dt_bias).
 // state float32, row seq_slot[b] of stride slot_stride holds [H, dv, d]. y float32 [N, H dv]. prep:
-// lumen_delta_rule_scratch(N, n_seqs, one_each, H, d) floats of scratch. cu_q covers at most N tokens. one_each: no sequence has
-// more than one token (a decode step).
+// lumen_delta_rule_scratch(N, n_seqs, longest, H, d) floats of scratch. cu_q covers at most N tokens. longest: no sequence has
+// more tokens (N where that is not known); it decides what is launched, not how a sequence is summed.
 LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int v_col, const float* u, int uS,
                                long long u_stride, int uW, int b_col, const float* a, int aS, long long a_stride,
                                const float* dt_bias, const float* a_log, float* state, long long slot_stride,
-                               const int* cu_q, const int* seq_slot, int n_seqs, int one_each, float* y, float* prep, int N, int H,
+                               const int* cu_q, const int* seq_slot, int n_seqs, int longest, float* y, float* prep, int N, int H,
                                int G, int d, int dv, cudaStream_t stream) {
     if (n_seqs <= 0 || N <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || d > 32 * DR_ROWS || uS < 1 || aS < 1 || H > 65535)
@@ -683,7 +699,7 @@ LUMEN_API int lumen_delta_rule(const float* x, int C, int q_col, int k_col, int 
     const int threads = wide ? 2 * DR_THREADS : DR_THREADS, cols = threads / NS;
     const int vec = (d & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
     const DrIn in = {x, u, a, dt_bias, a_log, (size_t)u_stride, (size_t)a_stride, C, q_col, k_col, uS, uW, b_col, aS, H, G, d};
-    if (delta_rule_chunks(d, N, one_each)) {
+    if (delta_rule_chunks(d, longest)) {
         if ((dv + DC_COLS - 1) / DC_COLS > 65535) return LUMEN_ERR_UNSUPPORTED;
         cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM);
         if (e != cudaSuccess) return (int)e;

@@ -70,6 +70,12 @@ class StepContext:
         return max(self.q_lens)
 
     @property
+    def longest(self) -> Optional[int]:
+        """The most tokens a sequence brings, or None where that is not known: a captured prompt step is replayed for
+        other divisions of its tokens than the one whose lists are here."""
+        return None if self.extras.get("captured") and not self.is_decode else self.max_q
+
+    @property
     def max_len(self) -> int:
         return max(s + q for s, q in zip(self.starts, self.q_lens))
 

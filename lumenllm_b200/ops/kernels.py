@@ -1433,12 +1433,13 @@ def shift_mix(y, mu, state, tok_seq, cu_q, seq_slot):
 
 
 def delta_rule(x, q_col, k_col, v_col, u, beta_col, a, dt_bias, a_log, state, cu_q, seq_slot, n_seqs, heads, kv_heads,
-               d, dv, one_each=False):
+               d, dv, longest=None):
     """The gated delta rule with a decay a key channel (csrc/delta_rule.cu). x float32 [N, C]: q
     (kv_heads heads of d from q_col), k (k_col), v (heads of dv from v_col), convolved and activated;
     u: projection partial sums with the heads' beta logits from beta_col; a: partial sums [.., N,
     heads * d] of the decay logits; state float32 [slots, heads, dv, d] (row seq_slot[b] sequence
-    b's, updated in place). one_each: no sequence has more than one token (a decode step). Returns float32 [N, heads * dv]."""
+    b's, updated in place). longest: no sequence has more tokens, if the host knows (it decides
+    what is launched, not how a sequence is summed). Returns float32 [N, heads * dv]."""
     require(x, F32, "delta_rule.x")
     u, uS = _partials(u, "delta_rule.u")
     a, aS = _partials(a, "delta_rule.a")
@@ -1457,16 +1458,16 @@ def delta_rule(x, q_col, k_col, v_col, u, beta_col, a, dt_bias, a_log, state, cu
     require(seq_slot, I32, "delta_rule.seq_slot")
     y = torch.empty((N, heads * dv), dtype=F32, device=x.device)
     # what does not depend on the state, made by the kernel's first launch
-    one_each = 1 if one_each else 0
+    longest = N if longest is None else int(longest)
     size = int_fn("delta_rule", "lumen_delta_rule_scratch", [c_int, c_int, c_int, c_int, c_int])
     size.restype = c_longlong
-    prep = torch.empty((size(N, int(n_seqs), one_each, int(heads), int(d)),), dtype=F32, device=x.device)
+    prep = torch.empty((size(N, int(n_seqs), longest, int(heads), int(d)),), dtype=F32, device=x.device)
     f = fn("delta_rule", "lumen_delta_rule",
            [P, c_int, c_int, c_int, c_int, P, c_int, c_longlong, c_int, c_int, P, c_int, c_longlong, P, P, P, c_longlong,
             P, P, c_int, c_int, P, P, c_int, c_int, c_int, c_int, c_int, P])
     check(f(ptr(x), C, int(q_col), int(k_col), int(v_col), ptr(u), uS, N * u.shape[2], u.shape[2], int(beta_col), ptr(a),
             aS, N * heads * d, ptr(dt_bias), ptr(a_log), ptr(state), state.stride(0), ptr(cu_q), ptr(seq_slot),
-            int(n_seqs), one_each, ptr(y), ptr(prep), N, int(heads), int(kv_heads), int(d), int(dv), stream_ptr()), "delta_rule")
+            int(n_seqs), longest, ptr(y), ptr(prep), N, int(heads), int(kv_heads), int(d), int(dv), stream_ptr()), "delta_rule")
     return y
 
 

@@ -93,6 +93,6 @@ class ChannelDeltaMixer:
         a = self.a2(K.cols_cast(u, self.C + self.H, self.ra, dt), split_ok=True)
         g = self.g2(K.cols_cast(u, self.C + self.H + self.ra, self.rg, dt), split_ok=True)
         o = K.delta_rule(x, 0, self.G * self.d, 2 * self.G * self.d, u, self.C, a, self.dt_bias, self.a_log, S,
-                         ctx.cu_q, ctx.seq_slot, ctx.B, self.H, self.G, self.d, self.dv, ctx.is_decode)
+                         ctx.cu_q, ctx.seq_slot, ctx.B, self.H, self.G, self.d, self.dv, ctx.longest)
         v = K.head_norm_gate(o, self.norm_w, self.eps, g, 0, self.H, dt)
         return self.o(v, split_ok=True, add_to=residual)

@@ -178,3 +178,18 @@ def test_plain_latent_attention_equals_expanded_keys_and_values():
             out[i, hd] = p @ vh[lo:i + 1]
     ref = out.reshape(T, H * dv) @ w[pre + "o"].T
     assert float((got - ref).abs().max()) < 1e-10
+
+
+def test_scratch_of_the_delta_rule_follows_the_tokens():
+    """Sequences of a token or two beside prompts (or alone) ask for their own rows, not for sixteen tokens' worth each: a row is
+    388 floats a (token, head), a token in chunks 432, and a chunk more a sequence of 48 tokens or more."""
+    from ctypes import c_int, c_longlong
+    from lumenllm_b200.ops.native import int_fn
+    size = int_fn("delta_rule", "lumen_delta_rule_scratch", [c_int] * 5)
+    size.restype = c_longlong
+    H = 16
+    for lens in ([2] * 128, [1] * 64 + [300], [24] * 64, [1] * 200 + [64], [2048], [300] * 9, [47], [49] * 7):
+        need = sum(432 * n + 6912 if n >= 48 else 432 * n for n in lens) * H
+        got = size(sum(lens), len(lens), sum(lens), H, 128)
+        assert got <= 1.5 * 388 * sum(lens) * H
+        assert got >= need or sum(lens) < 48

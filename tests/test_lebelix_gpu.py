@@ -473,7 +473,8 @@ def test_delta_rule_sixteen_tokens_at_a_time(d, dv, lens):
     assert not bool(torch.isfinite(yb[last]).all())
 
 
-@pytest.mark.parametrize("lens", [[60] + [0] * 70, [1] * 63 + [60] + [0] * 64, [2, 50, 47, 1, 128, 16]])
+@pytest.mark.parametrize("lens", [[60] + [0] * 70, [1] * 63 + [60] + [0] * 64, [2, 50, 47, 1, 128, 16], [3, 200, 2],
+                                  [2] * 200 + [49] * 3])
 def test_a_sequence_goes_as_it_does_alone_whatever_is_beside_it(lens):
     """Chunks or token by token, and where the chunks lie, is a sequence's own number of tokens alone, also where there are more
     sequences than tokens: the bits of a call by itself."""
