@@ -204,7 +204,10 @@ class Engine:
 
     def _split(self, entries: List[StepEntry]):
         """Cuts a step into passes of at most max_step_tokens tokens. Returns the passes
-        and, for every output row in pass order, its index in the caller's order."""
+        and, for every output row in pass order, its index in the caller's order. In a model
+        whose sums depend on where a step's tokens begin, a sequence that does not fit what is
+        left of a pass begins the next one: its cut, and so its results, are the same alone and
+        behind any others."""
         budget = self.max_step_tokens
         row0, rows = 0, []
         for e in entries:
@@ -221,6 +224,10 @@ class Engine:
                     parts.append(cur)
                     cur, room = [], budget
                 n = min(room, len(toks) - off)
+                if self.model.cut_matters and n < len(toks) - off and room < budget:
+                    parts.append(cur)
+                    cur, room = [], budget
+                    continue
                 want_here = sorted(w for w in rows[ei] if off <= w < off + n)
                 wl = []
                 for w in want_here:

@@ -50,6 +50,8 @@ class DecoderModel:
         self.graph_safe = all(b.graph_safe if hasattr(b, "graph_safe") else
                               (getattr(b.mixer, "graph_safe", False) and getattr(b.ffn, "graph_safe", False))
                               for b in self.blocks)
+        # whether a token's sums depend on where its sequence's tokens of the step begin
+        self.cut_matters = any(getattr(b.mixer, "cut_matters", False) for b in self.blocks)
 
     # what the cache must hold, per schedule entry
     def cache_needs(self) -> Dict[int, CacheNeed]:

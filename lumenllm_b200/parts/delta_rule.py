@@ -72,6 +72,11 @@ class ChannelDeltaMixer:
         self.n_state = self.H * self.dv * self.d
         self.n_conv = (self.taps - 1) * self.C
 
+    @property
+    def cut_matters(self):
+        """Prompts of heads of 65 to 128 go in chunks of sixteen tokens from the step's first one on (csrc/delta_rule.cu)."""
+        return 64 < self.d <= 128
+
     def cache_need(self):
         return None
 

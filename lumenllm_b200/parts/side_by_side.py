@@ -97,6 +97,10 @@ class SideBySide:
     def graph_safe(self):
         return all(getattr(m, "graph_safe", False) for m in self.mixers)
 
+    @property
+    def cut_matters(self):
+        return any(getattr(m, "cut_matters", False) for m in self.mixers)
+
     def cache_need(self):
         return next((n for n in (m.cache_need() for m in self.mixers) if n is not None), None)
 

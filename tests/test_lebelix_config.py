@@ -180,6 +180,28 @@ def test_plain_latent_attention_equals_expanded_keys_and_values():
     assert float((got - ref).abs().max()) < 1e-10
 
 
+def test_pieces_of_a_long_step_follow_the_sequence_alone():
+    """Where a model's sums depend on the cut, a sequence's pieces are those it has alone; elsewhere passes are filled up."""
+    from types import SimpleNamespace
+    from lumenllm_b200.engine import Engine, StepEntry
+    g = torch.Generator().manual_seed(4)
+    for _ in range(200):
+        budget = int(torch.randint(1, 60, (1,), generator=g))
+        lens = torch.randint(1, 150, (int(torch.randint(1, 7, (1,), generator=g)),), generator=g).tolist()
+        entries = [StepEntry(i, [100 * i + t for t in range(n)], [0, n - 1]) for i, n in enumerate(lens)]
+        for matters in (True, False):
+            model = SimpleNamespace(cut_matters=matters)
+            parts, origin = Engine._split(SimpleNamespace(max_step_tokens=budget, model=model), entries)
+            assert all(0 < sum(len(e.tokens) for e in p) <= budget and len({e.slot for e in p}) == len(p) for p in parts)
+            assert sorted(origin) == list(range(2 * len(lens)))
+            for e in entries:
+                pieces = [x.tokens for p in parts for x in p if x.slot == e.slot]
+                assert sum(pieces, []) == list(e.tokens)
+                if matters:
+                    n = len(e.tokens)
+                    assert [len(x) for x in pieces] == [min(budget, n - at) for at in range(0, n, budget)]
+
+
 def test_scratch_of_the_delta_rule_follows_the_tokens():
     """Sequences of a token or two beside prompts (or alone) ask for their own rows, not for sixteen tokens' worth each: a row is
     388 floats a (token, head), a token in chunks 432, and a chunk more a sequence of 48 tokens or more."""

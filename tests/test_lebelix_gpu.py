@@ -758,6 +758,31 @@ def test_a_model_of_delta_rule_layers_only(dtype, tmp_path):
     eng.check_kernels()
 
 
+def test_a_long_sequence_is_cut_as_it_is_alone(tmp_path):
+    """Steps beyond max_step_tokens: heads of 128 go in chunks from a piece's first token on, so a sequence is cut where its own
+    tokens say, whatever lies ahead of it; a float32 run's logits are the same bits alone and behind others."""
+    from lumenllm_b200.engine import Engine, StepEntry
+    cfg = config(50, 64, 1e-5, [layer(delta(2, 1, 128, 16, 3, 2, 2), dense(40)), layer(delta(2, 2, 100, 36, 2, 3, 5), None)])
+    folder = write_model(cfg, tmp_path / "m", seed=82)
+    eng = Engine.from_folder(folder, dtype="float32", max_tokens=2048, max_slots=4, max_step_tokens=200)
+    toks = tokens_of(cfg, (7, 150, 61, 470), seed=83)
+
+    def step(which):
+        slots = [eng.alloc_slot() for _ in which]
+        out = eng.step([StepEntry(s, toks[i], list(range(len(toks[i])))) for s, i in zip(slots, which)])
+        for s in slots:
+            eng.free_slot(s)
+        return out.split([len(toks[i]) for i in which])
+
+    alone = [step([i])[0] for i in range(4)]
+    for which in ([0, 1], [0, 1, 2], [2, 0, 3, 1], [3, 1, 2, 0]):
+        for i, got in zip(which, step(which)):
+            assert torch.equal(got, alone[i])
+    _, w = P.load_model(folder)
+    close(alone[3], P.forward(cfg, w, toks[3]), "float32")
+    eng.check_kernels()
+
+
 def test_a_long_prompt_whose_products_add_into_the_stream(tmp_path):
     """A prompt long and wide enough for the output products to add their result to the residual
     stream in their epilogue (no update is handed on then), with every kind of mixer."""
