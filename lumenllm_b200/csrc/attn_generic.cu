@@ -475,6 +475,19 @@ attn_prompt_f32_kernel(const float* __restrict__ q, const float* __restrict__ kc
     }
 }
 
+// Heads a block of it: more of them share the staged keys, but a block's time grows with its rows, so a step of few tokens takes as few
+// as keep the SMs busy (us, 1 / 2 / 4 heads a block, 16 heads of 128 over 4: 8 tokens 6.5 / 7.7 / 10.1, after 3,000 others 156 / 195 / 260;
+// 48 tokens, 192 blocks of one head, 8.5 / 9.2 / 11.8; 64 tokens, 256, 11.2 / 9.7 / 12.6; 3 x 48, 576, 17.6 / 11.0 / 12.4; 3 x 64, 768, 19.6 /
+// 19.4 / 16.3; 300, 1,200, 59 / 52 / 43. With a token a block 8 tokens take 7.6 and 274, 300 106). The same bits.
+static int attn_prompt_heads(int N, int nq, int nkv) {
+    const long long blocks = (long long)((N + AP_Q - 1) / AP_Q) * nq;
+    const int G = nq / nkv;
+    int hb = 1;
+    while (hb < 4 && G % (2 * hb) == 0 && blocks / (2 * hb) >= (hb == 1 ? 128 : 148)) hb *= 2;
+    return hb;
+}
+LUMEN_API int lumen_attn_prompt_heads(int N, int nq, int nkv) { return attn_prompt_heads(N, nq, nkv); }
+
 template <int HB>
 static int attn_prompt_f32_go(const float* q, const float* kcache, const float* vcache, const int* block_table, int bt_stride,
                               const int* tok_seq, const int* tok_pos, float* out, int N, int nq, int nkv, int d, int dv, float scale,
@@ -544,9 +557,9 @@ LUMEN_API int lumen_attn_generic(const void* q, const void* kcache, const void* 
 #define AP_GO(HB)                                                                                                              \
     return attn_prompt_f32_go<HB>((const float*)q, (const float*)kcache, (const float*)vcache, block_table, bt_stride, tok_seq, \
                                   tok_pos, (float*)out, N, nq, nkv, d, dv, scale, stream)
-        const int G = nq / nkv;
-        if (G % 4 == 0) AP_GO(4);
-        if (G % 2 == 0) AP_GO(2);
+        const int hb = attn_prompt_heads(N, nq, nkv);
+        if (hb == 4) AP_GO(4);
+        if (hb == 2) AP_GO(2);
         AP_GO(1);
 #undef AP_GO
     }

@@ -198,7 +198,8 @@ def test_attention_generic(dtype, nq, nkv, d, window):
 
 
 @pytest.mark.parametrize("nq,nkv,d,lens,starts", [(8, 2, 128, [70, 2, 130], [0, 299, 5]), (4, 2, 64, [1, 33], [128, 0]),
-                                                  (3, 3, 20, [41], [87]), (6, 1, 112, [127, 1, 3], [2, 63, 250])])
+                                                  (3, 3, 20, [41], [87]), (6, 1, 112, [127, 1, 3], [2, 63, 250]),
+                                                  (16, 4, 64, [190, 20], [7, 300])])
 def test_attention_of_float32_prompts_has_the_bits_of_single_tokens(nq, nkv, d, lens, starts):
     """Prompts go four tokens a block, decode steps one: the same bits, also where a block's tokens are of two sequences and
     where chunks of 128 keys end among a block's tokens; a later token's NaN value reaches no earlier one."""

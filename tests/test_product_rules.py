@@ -1,4 +1,6 @@
-"""Which products of a layer go through their activation in the product's own kernel: a rule on sizes."""
+"""Which kernels take a product, and how attention is divided into blocks: rules on sizes."""
+from ctypes import c_int
+
 import pytest
 
 
@@ -23,3 +25,14 @@ def test_a_captured_prompts_rows_take_the_way_of_the_eager_ones(width, k):
     from lumenllm_b200.ops.gemm import gate_up_in_one
     for rows in range(257, 700):
         assert gate_up_in_one(rows, width, k) == gate_up_in_one((rows + 31) // 32 * 32, width, k), rows
+
+
+def test_heads_a_block_of_float32_prompt_attention():
+    """Steps of few tokens keep the SMs busy with a head a block; long prompts share the staged keys among four, of one group."""
+    from lumenllm_b200.ops.native import int_fn
+    heads = lambda *a: int_fn("attn_generic", "lumen_attn_prompt_heads", [c_int] * 3)(*a)
+    assert [heads(n, 16, 4) for n in (8, 16, 48, 64, 128, 192, 300, 2000)] == [1, 1, 1, 2, 2, 4, 4, 4]
+    assert [heads(n, 8, 2) for n in (8, 100, 128, 200, 300)] == [1, 1, 2, 2, 4]
+    for n in (8, 300, 5000):
+        for nq, nkv in ((16, 16), (12, 6), (6, 2), (64, 8)):
+            assert nq // nkv % heads(n, nq, nkv) == 0
