@@ -1,14 +1,18 @@
 // Float32 matrix product C[M,N] = A[M,K] * W[N,K]^T on the 5th-generation tensor cores, with the error of a 32-bit
-// product: every float32 operand is cut into three bfloat16 numbers that add up to it exactly (the number rounded to
-// eight significant bits, what is left rounded likewise, and what is left then), and of the nine products of parts the
-// six that reach 2^-25 of the whole are made, x1 y1 + (x1 y2 + x2 y1) + (x1 y3 + x2 y2 + x3 y1), each exactly, as a
-// product of two eight-bit numbers is. W may be bfloat16 (one part, three products, nothing left out).
+// product: every float32 operand is cut into three bfloat16 numbers, x = x1 + 2^-8 x2 + 2^-16 x3 exactly, from the smallest
+// number to where one rounds to infinity (x1 is the number rounded to eight significant bits, x2 2^8 times what is left,
+// rounded likewise, x3 2^8 times what is left then: scaled, so that the parts of a small number are still bfloat16 numbers).
+// Of the nine products of parts the six largest are made, x3 y1 + x1 y3 + x2 y2, 2^-8 of that + x2 y1 + x1 y2, 2^-8 of that
+// + x1 y1 (the accumulator is scaled by the instruction that goes on with it), each exactly, as a product of two eight-bit numbers is. The three
+// left out reach 2^-24 of a product (2^-27.4 rms). A subnormal operand has fewer bits in front, and counts as if it were off by up to
+// the spacing of the numbers there, 2^-149. W may be bfloat16 (one part, three products, nothing left out).
 //
-// The tensor core's own sums are short: 64 values of k and their parts, small ones first, into a fresh accumulator, which
-// is then added to a running sum in registers, rounded to nearest. So an output is a chain of K / 64 float32 adds (in
+// The tensor core's own sums are short: 64 values of k and their parts, small ones first, into a fresh accumulator, which loses up to
+// an ulp an instruction and is then added to a running sum in registers, rounded to nearest. So an output is a chain of K / 64 float32 adds (in
 // up to four shares of k, added in rising order) where the FFMA kernel's is K / 4. Against a 64-bit product, 2-norm,
 // this / FFMA: K = 1,000 9.7e-8 / 2.8e-7, 2,048 1.0e-7 / 4.1e-7, 8,192 1.4e-7 / 8.1e-7; of numbers that are all positive
-// 9.4e-8 / 1.3e-7, 8.8e-8 / 1.6e-7, 9.4e-8 / 3.1e-7.
+// 9.4e-8 / 1.3e-7, 8.8e-8 / 1.6e-7, 9.4e-8 / 3.1e-7. Rows of zeros but for a few numbers gain nothing by short chains: one number of 2,048
+// 4.5e-8 / 2.5e-8, 16 7.2e-8 / 5.8e-8, 64 8.1e-8 / 8.4e-8.
 //
 // A block takes 128 rows of W (the 128-row side of the MMA) times up to 160 rows of A, for a share of k; the blocks of
 // one tile, one for each share, are a cluster and add up their sums through distributed shared memory. The number of
@@ -21,16 +25,19 @@
 //   two warps    issue the products in turns (a lane that issues is held up until the tensor pipe takes its product, so a
 //                single one would leave the pipe idle while it goes through its barriers); one allocates tensor memory;
 //   the others   add the finished accumulator (two of them, in tensor memory) to the sums in their registers.
-// Infinities and NaN have no parts: the rows that hold one are marked, and their outputs are made again with plain FMAs.
+// An infinity or a NaN leaves NaN in its parts, and so in its outputs: a block's sums that are not finite, for this or any other
+// reason, are made again with plain FMAs.
 //
 // What bounds it: for many rows the chain of a buffer, parts stored (1,270 cycles a block of 64 columns), products (1,900, the tensor
 // pipe's time for 24 of 128 x 160 x 16) and the barriers between, of which two are under way; for few rows the stream over W, of which
 // 64 KB an SM are under way; and some 9 us a block for its start, first fetch and sums.
-// us, FFMA -> this (with the kernel ahead): 300 rows x 16,384 outputs x 2,048 511 -> 118 (1.0 PFLOP/s of bfloat16 products); 300 x 2,048 x 8,192 438 -> 67;
-// 300 x 2,048 x 2,048 114 -> 23; 300 x 3,072 x 2,048 114 -> 41; 100 x 2,048 x 8,192 221 -> 56; 64 x 16,384 x 2,048 114 -> 48; 16 x 32,768 x 2,048
-// 94 -> 73; 8 x 16,384 x 2,048 60 -> 48; 8 x 2,048 x 8,192 59 -> 39; 8 x 1,024 x 1,024 8.8 -> 8.3. Tried, 300 x 16,384 x 2,048: A cut by every block 169; one
-// warp issuing, loads asked for before the fence 136; two groups of cutting warps in turns 147; parts waiting in registers for a buffer
-// 172. Eight shares: 300 x 2,048 x 8,192 101, 300 x 2,048 x 2,048 43, 8 x 2,048 x 8,192 32.
+// us, L2 cold, FFMA -> this (with the kernel ahead): 300 rows x 16,384 outputs x 2,048 518 -> 120 (1.0 PFLOP/s of bfloat16 products); 300 x 2,048 x
+// 8,192 447 -> 69; 300 x 2,048 x 2,048 121 -> 30; 300 x 3,072 x 2,048 121 -> 48; 100 x 2,048 x 8,192 226 -> 60; 64 x 16,384 x 2,048 123 -> 54; 16 x
+// 32,768 x 2,048 107 -> 84; 8 x 16,384 x 2,048 72 -> 57; 8 x 2,048 x 8,192 117 -> 55; 8 x 1,024 x 1,024 21 -> 14. Parts that were not
+// scaled, with marks of the rows that hold something that is not finite: 126 for the first, 6 % over all sizes. Tried, 300 x 16,384 x 2,048, L2 warm (118
+// then): A cut by every block 169; one warp issuing, loads asked for before the fence 136; two groups of cutting warps in turns 147; parts
+// waiting in registers for a buffer 172. Eight shares: 300 x 2,048 x 8,192 101 (67), 300 x 2,048 x 2,048 43 (23), but 8 x 2,048 x 8,192 32 (39):
+// few rows over a long k pay for many.
 // Every wait is bounded; when one runs out the block raises the error flag, its other roles give up on theirs, and the
 // block leaves, through the same cluster barriers as ever, once the products it has issued are done.
 #include "common.cuh"
@@ -59,6 +66,14 @@ __device__ __forceinline__ void ft_mma(uint32_t d_tmem, uint64_t adesc, uint64_t
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The same onto 2^-8 times the accumulator.
+__device__ __forceinline__ void ft_mma_2m8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.eq.b32 p, 0, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 8;\n}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc)
         : "memory");
 }
 __device__ __forceinline__ void ft_ld16(uint32_t taddr, float (&v)[16]) {
@@ -138,7 +153,7 @@ __device__ __forceinline__ void ft_fetch(FtRaw<__nv_bfloat16>& x, const __nv_bfl
         if (left > 3) x.v.y |= (uint32_t)__ldg(q + 3) << 16;
     }
 }
-// Two numbers rounded to bfloat16, side by side; x becomes what is left of each (exactly).
+// Two numbers rounded to bfloat16, side by side; x becomes what is left of each, times 2^8 (exactly).
 __device__ __forceinline__ uint32_t ft_cut(unsigned long long& x) {
     uint32_t a, b;
     unsigned long long r;
@@ -146,10 +161,11 @@ __device__ __forceinline__ uint32_t ft_cut(unsigned long long& x) {
     const uint32_t h = pack_bf16(__uint_as_float(a), __uint_as_float(b));
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(h << 16), "r"(h & 0xffff0000u));
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(x) : "l"(r), "l"(0xbf800000bf800000ull));       // x - r
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(0x4380000043800000ull));
     return h;
 }
-// Cuts four values and stores their parts `part` bytes apart; 1 if one of them is not finite (or rounds to infinity).
-__device__ __forceinline__ int ft_store(const FtRaw<float>& x, unsigned char* dst, int part) {
+// Cuts four values and stores their parts `part` bytes apart. What is not finite (or rounds to infinity) leaves NaN in its second part.
+__device__ __forceinline__ void ft_store(const FtRaw<float>& x, unsigned char* dst, int part) {
     unsigned long long a, b;
     asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(x.v.x), "f"(x.v.y));
     asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(x.v.z), "f"(x.v.w));
@@ -160,17 +176,8 @@ __device__ __forceinline__ int ft_store(const FtRaw<float>& x, unsigned char* ds
         h.y = ft_cut(b);
         *reinterpret_cast<uint2*>(dst + i * part) = h;
     }
-    // nothing is left (or less than bfloat16 has numbers for, of values below 2^-110), or NaN: an infinity less itself
-    float u, v;
-    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(u), "=f"(v) : "l"(a));
-    return !(u + v == u + v);
 }
-__device__ __forceinline__ int ft_store(const FtRaw<__nv_bfloat16>& x, unsigned char* dst, int) {
-    *reinterpret_cast<uint2*>(dst) = x.v;
-    const uint32_t e = 0x7f80u;
-    return (x.v.x & e) == e || ((x.v.x >> 16) & e) == e || (x.v.y & e) == e || ((x.v.y >> 16) & e) == e;
-}
+__device__ __forceinline__ void ft_store(const FtRaw<__nv_bfloat16>& x, unsigned char* dst, int) { *reinterpret_cast<uint2*>(dst) = x.v; }
 
 // DEEP: a block has an SM to itself and two blocks of W under way (up to 16 rows, where two blocks share an SM if there are that many).
 template <typename TW, int BN, bool DEEP>
@@ -182,7 +189,7 @@ struct FtShape {
     static constexpr int A_TILE = BN * 128;
     static constexpr int BUF = NW * FT_W_TILE + 3 * A_TILE;
     static constexpr int TMEM = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
-    static constexpr int CTL = 1024;                                     // barriers, flags, marks
+    static constexpr int CTL = 1024;                                     // barriers, flags
     static constexpr int SMEM = 2 * BUF + CTL;
     static constexpr int MINB = DEEP ? 1 : 2;
     static_assert(DEEP || 2 * SMEM <= 220 * 1024, "two blocks fit an SM");
@@ -192,8 +199,7 @@ struct FtShape {
 
 template <typename TW, int BN, bool DEEP>
 __global__ void __launch_bounds__(32 * FtShape<TW, BN, DEEP>::WARPS, FtShape<TW, BN, DEEP>::MINB)
-gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict__ image, const unsigned char* __restrict__ image_odd,
-                   const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int vec, int early, int give_up_at,
+gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict__ image, const TW* __restrict__ W, float* __restrict__ C, int M, int N, int K, int bn, int vec, int early, int give_up_at,
                    int* __restrict__ err) {
     using F = FtShape<TW, BN, DEEP>;
     constexpr int NW = F::NW, EPI = F::EPI, ACOL = F::TMEM / 2;
@@ -207,8 +213,6 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* any_odd = reinterpret_cast<volatile int*>(tmem_slot + 2);
-    unsigned char* odd_w = reinterpret_cast<unsigned char*>(bars + 16);      // [128] rows of W, [BN] rows of A with an infinity or NaN
-    unsigned char* odd_a = odd_w + FT_ROWS;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = gridDim.x, share = blockIdx.x;                             // the cluster is one tile's shares of k
@@ -256,14 +260,8 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
 #pragma unroll
         for (int i = 0; i < F::SETS; ++i) fetch_w(i, rw[i]);
     }
-    int marked = 0;
-    for (int i = threadIdx.x; i < FT_ROWS + BN; i += blockDim.x) {
-        const int m = i - FT_ROWS;
-        odd_w[i] = F::IMAGE && m >= 0 && m < rows && image_odd[m0 + m];
-        marked |= odd_w[i];
-    }
     ft_fence_before();
-    marked = __syncthreads_or(marked);
+    __syncthreads();
     ft_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     float* sums = reinterpret_cast<float*>(tiles);             // [BN][128], over the tiles once they have been read
@@ -286,28 +284,17 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
             if (lane == 0) atomicExch(err, 1);
             return false;
         };
-        auto mark = [&](int odd) {               // looked at once a block, so that the rows' cutting can be interleaved
-            if (!odd) return;
-            *any_odd = 1;
-            for (int i = 0; i < LW; ++i)
-                if (odd >> i & 1) odd_w[r + 16 * i] = 1;
-            if constexpr (!F::IMAGE)
-                for (int i = 0; i < LA; ++i)
-                    if (odd >> (LW + i) & 1) odd_a[r + 16 * i] = 1;
-        };
         auto step = [&](int kb, FtRaw<TW> (&x)[LW]) -> bool {
             if (!room(kb)) return false;
             unsigned char* tw = tiles + (kb & 1) * F::BUF + at;
             unsigned char* ta = tw + NW * FT_W_TILE;
-            int odd = 0;
 #pragma unroll
-            for (int i = 0; i < LW; ++i) odd |= ft_store(x[i], tw + i * 16 * 128, FT_W_TILE) << i;
+            for (int i = 0; i < LW; ++i) ft_store(x[i], tw + i * 16 * 128, FT_W_TILE);
             if constexpr (!F::IMAGE) {
 #pragma unroll
-                for (int i = 0; i < LA; ++i) odd |= ft_store(ra[i], ta + i * 16 * 128, F::A_TILE) << (LW + i);
+                for (int i = 0; i < LA; ++i) ft_store(ra[i], ta + i * 16 * 128, F::A_TILE);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the next loads, which it would wait for
-            mark(odd);
             __syncwarp();
             if (lane == 0) ft_arrive(&full[kb & 1]);
             fetch_w(kb + F::SETS, x);
@@ -331,26 +318,25 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
                 if (!ok) break;
                 ft_fence_after();
                 const uint32_t tw = smem_u32(tiles + b * F::BUF), ta = tw + NW * FT_W_TILE, d = tmem_base + b * ACOL;
-                uint32_t accumulate = 0;
-                auto product = [&](int pw, int pa) {
+                // first: what the accumulator does at this product's start, 0 it begins anew, 1 goes on, 2 goes on 2^-8 times
+                auto product = [&](int pw, int pa, int first) {
                     const uint64_t wd = ft_desc(tw + pw * FT_W_TILE), ad = ft_desc(ta + pa * F::A_TILE);
+                    if (first == 2) ft_mma_2m8(d, wd, ad, idesc);
+                    else ft_mma(d, wd, ad, idesc, first);
 #pragma unroll
-                    for (int k = 0; k < FT_BK / 16; ++k) {
-                        ft_mma(d, wd + 2 * k, ad + 2 * k, idesc, accumulate);
-                        accumulate = 1;
-                    }
+                    for (int k = 1; k < FT_BK / 16; ++k) ft_mma(d, wd + 2 * k, ad + 2 * k, idesc, 1);
                 };
                 if (NW == 3) {
-                    product(2, 0);
-                    product(0, 2);
-                    product(1, 1);
-                    product(1, 0);
-                    product(0, 1);
+                    product(2, 0, 0);
+                    product(0, 2, 1);
+                    product(1, 1, 1);
+                    product(1, 0, 2);
+                    product(0, 1, 1);
                 } else {
-                    product(0, 2);
-                    product(0, 1);
+                    product(0, 2, 0);
+                    product(0, 1, 2);
                 }
-                product(0, 0);
+                product(0, 0, 2);
                 ft_commit(&done[b]);
                 issued = kb + 1;
             }
@@ -408,7 +394,12 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
             if (lane == 0) ft_arrive(&taken[b]);
         }
         // the last block's products are done, so no tile is read or written any more (unless a wait ran out)
-        if (S == 1 && !*any_odd && !marked) {
+        bool odd = false;
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) odd |= first + j < rows && !isfinite(acc[j]);
+        if (odd) *any_odd = 1;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI) : "memory");
+        if (S == 1 && !*any_odd) {
             if (n < cols) {
                 float* dst = C + (size_t)(m0 + first) * N + n0 + n;
 #pragma unroll
@@ -426,12 +417,12 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
     ft_fence_after();
     if (warp == F::MMA)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(F::TMEM) : "memory");
-    const bool odd = *any_odd != 0 || marked;
+    const bool odd = *any_odd != 0;
     if (S == 1 && !odd) return;
     if (odd) {
         for (int e = threadIdx.x; e < rows * FT_ROWS; e += blockDim.x) {
             const int m = e / FT_ROWS, n = e % FT_ROWS;
-            if (n >= cols || !(odd_a[m] || odd_w[n])) continue;
+            if (n >= cols || isfinite(sums[e])) continue;
             float s = 0.0f;
             const int k1 = min(K, (kb0 + nk) * FT_BK);
             for (int k = kb0 * FT_BK; k < k1; ++k) s = fmaf(A[(size_t)(m0 + m) * K + k], to_f32(W[(size_t)(n0 + n) * K + k]), s);
@@ -476,21 +467,17 @@ gemm_f32_tc_kernel(const float* __restrict__ A, const unsigned char* __restrict_
 // A cut into parts, in the image the blocks copy: tile of bn rows after tile, block of 64 columns after block, part after part, a
 // part bn rows of 128 bytes in the 128-byte swizzle. A block of threads a row (of the last tile's absent rows too, zeros).
 __global__ void __launch_bounds__(256)
-gemm_f32_image_kernel(const float* __restrict__ A, unsigned char* __restrict__ image, unsigned char* __restrict__ image_odd, int M, int K,
-                      int bn, int vec) {
+gemm_f32_image_kernel(const float* __restrict__ A, unsigned char* __restrict__ image, int M, int K, int bn, int vec) {
     pdl_wait();
     pdl_trigger();
     const int row = blockIdx.x, r = row % bn, num_kb = (K + FT_BK - 1) / FT_BK;
     unsigned char* tile = image + (size_t)(row / bn) * num_kb * 3 * bn * 128 + r * 128;
-    int odd = 0;
     for (int i = threadIdx.x; i < num_kb * 16; i += 256) {
         const int c = i & 15;
         FtRaw<float> x;
         ft_fetch(x, A + (size_t)row * K + 4 * i, row < M ? K - 4 * i : 0, vec);
-        odd |= ft_store(x, tile + (size_t)(i >> 4) * 3 * bn * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8, bn * 128);
+        ft_store(x, tile + (size_t)(i >> 4) * 3 * bn * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8, bn * 128);
     }
-    odd = __syncthreads_or(odd);
-    if (threadIdx.x == 0) image_odd[row] = odd != 0;
 }
 
 // Rows of A a block: as few tiles as there can be, of even height.
@@ -498,7 +485,7 @@ static int gemm_f32_tc_tile(int M) {
     const int tiles = (M + FT_MAX_BN - 1) / FT_MAX_BN;
     return ((M + tiles - 1) / tiles + 15) / 16 * 16;
 }
-static size_t gemm_f32_tc_image(int M, int K) {               // bytes of the image, without the marks behind it
+static size_t gemm_f32_tc_image(int M, int K) {               // bytes of the image
     const int bn = gemm_f32_tc_tile(M);
     return bn <= 32 ? 0 : (size_t)((M + bn - 1) / bn) * bn * ((K + FT_BK - 1) / FT_BK) * 3 * 128;
 }
@@ -512,9 +499,8 @@ static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* 
     if (e != cudaSuccess) return (int)e;
     const int vec_a = (K & 3) == 0 && ((uintptr_t)A & 15) == 0, vec_w = (K & 3) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
     const int tiles = (M + bn - 1) / bn;
-    unsigned char* odd = F::IMAGE ? work + gemm_f32_tc_image(M, K) : nullptr;
     if (F::IMAGE) {
-        lumen_launch(gemm_f32_image_kernel, dim3(tiles * bn), dim3(256), 0, stream, A, work, odd, M, K, bn, vec_a);
+        lumen_launch(gemm_f32_image_kernel, dim3(tiles * bn), dim3(256), 0, stream, A, work, M, K, bn, vec_a);
         LUMEN_LAUNCH_CHECK();
     }
     cudaLaunchConfig_t cfg = {};
@@ -530,14 +516,14 @@ static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = lumen_pdl_enabled() ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, k, A, (const unsigned char*)work, (const unsigned char*)odd, W, C, M, N, K, bn,
+    e = cudaLaunchKernelEx(&cfg, k, A, (const unsigned char*)work, W, C, M, N, K, bn,
                            F::IMAGE ? vec_w : vec_a && vec_w, early, give_up_at, err);
     if (e != cudaSuccess) return (int)e;
     LUMEN_LAUNCH_CHECK();
     return 0;
 }
 
-// Shares of k: as many as keep the blocks of one row of tiles within the SMs, each with four blocks of k or more.
+// Shares of k: as many as keep the blocks of one row of tiles within the SMs, with four blocks of k each, taken over all.
 static int gemm_f32_tc_shares(int N, int K) {
     const int tiles = (N + FT_ROWS - 1) / FT_ROWS, num_kb = (K + FT_BK - 1) / FT_BK;
     int S = 1;
@@ -571,8 +557,7 @@ LUMEN_API int lumen_gemm_f32_tc_takes(int N, int K) { return N >= FT_MIN_N && K 
 
 // Bytes of scratch lumen_gemm_f32_tc needs.
 LUMEN_API long long lumen_gemm_f32_tc_scratch(int M, int K) {
-    const size_t image = M > 0 && K > 0 ? gemm_f32_tc_image(M, K) : 0;
-    return image ? (long long)(image + M + FT_MAX_BN) : 0;
+    return M > 0 && K > 0 ? (long long)gemm_f32_tc_image(M, K) : 0;
 }
 
 // A float32 [M, K], W float32 or bfloat16 [N, K], C float32 [M, N], rows dense, of any alignment their types

@@ -590,6 +590,32 @@ def test_gemm_f32_in_bfloat16_parts(wdtype, M, N, K_):
     assert torch.equal(got[M - 1, mid], float("inf") * odd_w[mid, 3].float().sign())
 
 
+@pytest.mark.parametrize("wdtype", [F32, BF16])
+@pytest.mark.parametrize("M", [20, 150])
+def test_gemm_f32_over_the_whole_range(wdtype, M):
+    """One product an output, of numbers from the smallest float32 to the largest: every part of every operand counts. The parts that are
+    left out reach 2^-24 of a product and the accumulator loses up to an ulp (2^-23) of it, so within 2^-22, and three of the
+    smallest numbers where the product itself is that small. A subnormal operand's first part may be zero and the parts left out
+    then 2^-134 2^-16 of the other operand, and the tensor core keeps as much of a subnormal part's product: within its own spacing, 2^-149. No product of parts overflows where the number does not."""
+    from lumenllm_b200.ops import kernels as K
+    N, K_ = 1100, 1088
+    g = gen(M)
+    numbers = lambda n, top: ((1 + torch.rand(n, generator=g)).double() * 2.0 ** torch.linspace(-148, top, n).round().double()).float()
+    a, w = torch.zeros(M, K_), torch.zeros(N, K_)
+    a[:, 700], w[:, 700] = numbers(M, 127), numbers(N, 127) * torch.randn(N, generator=g).sign()
+    a[M - 1, 700], a[M - 2, 700] = torch.finfo(F32).max, float(1.99999 * 2.0 ** 63)
+    w[5, 700] = float(1.99999 * 2.0 ** 63)
+    w = w.to(wdtype)
+    out = K.gemm_f32(dev(a), dev(w)).cpu().double()
+    K.check_error_flags()
+    ref = a[:, 700].double()[:, None] * w[:, 700].double()
+    x, y = a[:, 700].double().abs()[:, None], w[:, 700].double().abs()
+    subnormal = y * (x < 2.0 ** -126) + x * (y < 2.0 ** -126)
+    near = (out - ref).abs() <= ref.abs() * 2.0 ** -22 + (3 + subnormal) * 2.0 ** -149
+    assert bool((near | (ref.abs() > torch.finfo(F32).max * (1 - 2.0 ** -22))).all())
+    assert bool((out[ref.abs() >= 2.0 ** 128].isinf()).all())
+
+
 def test_a_float32_product_that_gives_up_says_so():
     """A wait that runs out raises the error flag, in clusters too, and the context stays usable."""
     from ctypes import c_int, c_void_p
