@@ -51,6 +51,7 @@
 #define FT_MAX_SHARES 4                  // 16 clusters of eight blocks that fill an SM each take two rounds, 32 of four one
 #define FT_MIN_N 1024                    // see lumen_gemm_f32_tc_takes
 #define FT_MIN_K 1024
+#define FT_IMAGE_MAX (128ll << 20)       // bytes of cut activations at a time: about what stays in L2, and hundreds of tiles
 
 __device__ __forceinline__ void ft_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -485,9 +486,15 @@ static int gemm_f32_tc_tile(int M) {
     const int tiles = (M + FT_MAX_BN - 1) / FT_MAX_BN;
     return ((M + tiles - 1) / tiles + 15) / 16 * 16;
 }
+// Tiles of bn rows that are cut at a time; more go through the same scratch one lot after the other (six bytes a number of A
+// would be 1.26 GB for 8,192 rows of 25,600).
+static int gemm_f32_tc_lot(int M, int K, int bn) {
+    const long long tile = (long long)bn * ((K + FT_BK - 1) / FT_BK) * 3 * 128, tiles = (M + bn - 1) / bn;
+    return (int)(tiles * tile <= FT_IMAGE_MAX ? tiles : FT_IMAGE_MAX / tile > 0 ? FT_IMAGE_MAX / tile : 1);
+}
 static size_t gemm_f32_tc_image(int M, int K) {               // bytes of the image
     const int bn = gemm_f32_tc_tile(M);
-    return bn <= 32 ? 0 : (size_t)((M + bn - 1) / bn) * bn * ((K + FT_BK - 1) / FT_BK) * 3 * 128;
+    return bn <= 32 ? 0 : (size_t)gemm_f32_tc_lot(M, K, bn) * bn * ((K + FT_BK - 1) / FT_BK) * 3 * 128;
 }
 
 template <typename TW, int BN, bool DEEP>
@@ -498,13 +505,8 @@ static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* 
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
     if (e != cudaSuccess) return (int)e;
     const int vec_a = (K & 3) == 0 && ((uintptr_t)A & 15) == 0, vec_w = (K & 3) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
-    const int tiles = (M + bn - 1) / bn;
-    if (F::IMAGE) {
-        lumen_launch(gemm_f32_image_kernel, dim3(tiles * bn), dim3(256), 0, stream, A, work, M, K, bn, vec_a);
-        LUMEN_LAUNCH_CHECK();
-    }
+    const int lot = F::IMAGE ? gemm_f32_tc_lot(M, K, bn) * bn : M;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(S, tiles, (N + FT_ROWS - 1) / FT_ROWS);
     cfg.blockDim = dim3(32 * F::WARPS);
     cfg.dynamicSmemBytes = F::SMEM;
     cfg.stream = stream;
@@ -516,10 +518,18 @@ static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = lumen_pdl_enabled() ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, k, A, (const unsigned char*)work, W, C, M, N, K, bn,
-                           F::IMAGE ? vec_w : vec_a && vec_w, early, give_up_at, err);
-    if (e != cudaSuccess) return (int)e;
-    LUMEN_LAUNCH_CHECK();
+    for (int m = 0; m < M; m += lot) {           // the kernel that cuts the next lot waits for the product of the one before
+        const int rows = lot < M - m ? lot : M - m, tiles = (rows + bn - 1) / bn;
+        if (F::IMAGE) {
+            lumen_launch(gemm_f32_image_kernel, dim3(tiles * bn), dim3(256), 0, stream, A + (size_t)m * K, work, rows, K, bn, vec_a);
+            LUMEN_LAUNCH_CHECK();
+        }
+        cfg.gridDim = dim3(S, tiles, (N + FT_ROWS - 1) / FT_ROWS);
+        e = cudaLaunchKernelEx(&cfg, k, A + (size_t)m * K, (const unsigned char*)work, W, C + (size_t)m * N, rows, N, K, bn,
+                               F::IMAGE ? vec_w : vec_a && vec_w, early, give_up_at, err);
+        if (e != cudaSuccess) return (int)e;
+        LUMEN_LAUNCH_CHECK();
+    }
     return 0;
 }
 

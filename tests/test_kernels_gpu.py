@@ -590,6 +590,24 @@ def test_gemm_f32_in_bfloat16_parts(wdtype, M, N, K_):
     assert torch.equal(got[M - 1, mid], float("inf") * odd_w[mid, 3].float().sign())
 
 
+@pytest.mark.parametrize("M,K_", [(1400, 16384), (5000, 4700)])
+def test_gemm_f32_whose_activations_are_cut_in_lots(M, K_):
+    """More rows than are cut at a time: every row has the bits it has by itself, on both sides of where a lot ends."""
+    from ctypes import c_int, c_longlong
+    from lumenllm_b200.ops import kernels as K
+    from lumenllm_b200.ops.native import int_fn
+    size = int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_scratch", [c_int, c_int])
+    size.restype = c_longlong
+    assert size(M, K_) < 6 * M * K_
+    g = gen(M)
+    a, w = dev(torch.randn(M, K_, generator=g)), dev(torch.randn(1030, K_, generator=g))
+    out = K.gemm_f32(a, w)
+    K.check_error_flags()
+    for at in range(0, M, 100):
+        rows = slice(at, min(at + 100, M))
+        assert torch.equal(K.gemm_f32(a[rows].contiguous(), w), out[rows])
+
+
 @pytest.mark.parametrize("wdtype", [F32, BF16])
 @pytest.mark.parametrize("M", [20, 150])
 def test_gemm_f32_over_the_whole_range(wdtype, M):
