@@ -1471,10 +1471,11 @@ def delta_rule(x, q_col, k_col, v_col, u, beta_col, a, dt_bias, a_log, state, cu
     return y
 
 
-def gemm_f32(a, w, out=None, weight_ready=False):
+def gemm_f32(a, w, out=None, weight_ready=False, ffma=False):
     """C = a @ w.T with 32-bit error. a float32 [M, K]; w [N, K] float32|bfloat16. The weight's size decides between the tensor
     cores on three bfloat16 parts a number (csrc/gemm_f32_tc.cu) and FFMA, so a row's result is the same in any batch.
-    weight_ready: no kernel that may still be running writes w (a model's weights), so it may be read ahead of its turn."""
+    weight_ready: no kernel that may still be running writes w (a model's weights), so it may be read ahead of its turn.
+    ffma: plain FFMA whatever the size, for comparisons that are to share nothing with the tensor cores."""
     require(a, F32, "gemm_f32.a")
     M, K = a.shape
     N, K2 = w.shape
@@ -1484,7 +1485,7 @@ def gemm_f32(a, w, out=None, weight_ready=False):
         raise KernelError("gemm_f32.w must be a contiguous CUDA tensor")
     if out is None:
         out = torch.empty((M, N), dtype=F32, device=a.device)
-    if int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_takes", [c_int, c_int])(N, K):
+    if not ffma and int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_takes", [c_int, c_int])(N, K):
         size = int_fn("gemm_f32_tc", "lumen_gemm_f32_tc_scratch", [c_int, c_int])
         size.restype = c_longlong
         n = size(M, K)

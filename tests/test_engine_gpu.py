@@ -720,3 +720,33 @@ def test_a_long_prompt_at_real_layer_sizes():
         del eng
         torch.cuda.empty_cache()
         check(got, plain, dtype, "long prompt at the 14B layer sizes")
+
+
+def test_a_float32_model_whose_weights_have_three_parts(monkeypatch):
+    """Float32 weights large enough for the tensor cores' float32 product, through a model: a prompt and decoded tokens against
+    the plain implementation and against the same run with every product by plain FFMA (products off by 4e-7, some nine one after
+    the other that add up like unrelated errors, 1.2e-6, three times that allowed; parts left out would be 4e-6 a product)."""
+    from lumenllm_b200 import Engine, StepEntry
+    from lumenllm_b200.config import config_from_dict
+    from lumenllm_b200.engine.model import expected_tensors
+    from lumenllm_b200.ops import kernels as K
+    from lumenllm_b200.weights import random_weights
+    cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=2, hidden_size=1024, num_attention_heads=8,
+               num_key_value_heads=4, head_dim=128, intermediate_size=2048, vocab_size=2000, rope_theta=1000000.0, rms_norm_eps=1e-6,
+               max_position_embeddings=4096, tie_word_embeddings=False)
+    spec = config_from_dict(cfg).model_spec()
+    weights = random_weights(expected_tensors(spec), 9, 0.03, 0.1, torch.float32, device="cuda")
+    toks = seeded_tokens(2000, [93], 7)[0]
+    plain = plain_ref(cfg, {k: v.cpu() for k, v in weights.items()}, toks)[[0, 44, 89, 90, 91, 92]]
+    default, runs = K.gemm_f32, []
+    for ffma in (False, True):
+        if ffma:
+            monkeypatch.setattr(K, "gemm_f32", lambda *a, **kw: default(*a, ffma=True, **kw))
+        eng = Engine(spec, weights, dtype="float32", max_tokens=256)
+        s = eng.alloc_slot()
+        out = [eng.step([StepEntry(s, toks[:90], [0, 44, 89])])] + [eng.step([StepEntry(s, [toks[90 + k]], [0])]) for k in range(3)]
+        got = torch.cat(out).cpu()
+        eng.check_kernels()
+        check(got, plain, "float32", f"three parts a weight, ffma={ffma}")
+        runs.append(got)
+    assert 0 < float((runs[0] - runs[1]).norm() / runs[1].norm()) < 4e-6

@@ -590,6 +590,21 @@ def test_gemm_f32_in_bfloat16_parts(wdtype, M, N, K_):
     assert torch.equal(got[M - 1, mid], float("inf") * odd_w[mid, 3].float().sign())
 
 
+@pytest.mark.parametrize("wdtype", [F32, BF16])
+@pytest.mark.parametrize("M,N,K_", [(8, 1024, 2048), (150, 1100, 1030), (300, 2048, 4096)])
+def test_gemm_f32_by_ffma_for_large_weights(wdtype, M, N, K_):
+    """The plain 32-bit kernel can be asked for at any size: it is another kernel (other bits), and farther from the 64-bit product
+    than the tensor cores on three parts a number (chains of K / 4 adds against K / 64)."""
+    from lumenllm_b200.ops import kernels as K
+    g = gen(31)
+    a, w = torch.randn(M, K_, generator=g), torch.randn(N, K_, generator=g).to(wdtype)
+    ref = a.double() @ w.double().T
+    got, plain = K.gemm_f32(dev(a), dev(w)).cpu(), K.gemm_f32(dev(a), dev(w), ffma=True).cpu()
+    K.check_error_flags()
+    error = [float((x.double() - ref).norm() / ref.norm()) for x in (got, plain)]
+    assert not torch.equal(got, plain) and error[0] < error[1] < 1e-6
+
+
 @pytest.mark.parametrize("M,K_", [(1400, 16384), (5000, 4700)])
 def test_gemm_f32_whose_activations_are_cut_in_lots(M, K_):
     """More rows than are cut at a time: every row has the bits it has by itself, on both sides of where a lot ends."""
