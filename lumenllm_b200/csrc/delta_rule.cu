@@ -6,8 +6,9 @@
 // channel). Query/key head of value head h: h / (H / G). Everything is float32.
 //
 // A block takes one (sequence, head, slice of value channels) and walks the sequence's tokens of
-// the step strictly in order (heads of 65 to 128 have another way for prompts, below), so a token's sums do not depend on how the
-// sequence was cut or batched. A column j of S is independent of the others:
+// the step strictly in order, so a token's sums do not depend on how the
+// sequence was cut or batched (heads of 65 to 128 go in chunks where a sequence has 48 tokens or more in the step, below: their sums
+// depend on where it is cut, never on other sequences). A column j of S is independent of the others:
 //   r = sum_i g_i S_ij k_i,  w = sum_i g_i S_ij q_i,  u_j = beta (v_j - r),  o_j = w + u_j (k . q),
 //   S_ij <- g_i S_ij + k_i u_j,
 // so the DR_ROWS rows a thread keeps in registers are read once a token; the NS threads of a
@@ -15,10 +16,10 @@
 // shares of eight tokens change lanes so that a lane adds up a token of its own (7 shuffles for 8 tokens
 // where one token after the other takes 8 log2(NS)). Four warps of a block share a staged row, and what they read of
 // it (48 values a thread and token) is what bounds a token, with the chain of dependent steps: 220 of its 400
-// cycles go to shared-memory reads. 2,048 tokens of 16 heads of 128 x 128: 466 us with the kernel that
-// prepares them (732 with 16 threads a column, 8 rows each, and w summed token by token), four sequences of 2,048 tokens
-// in all: 400 (668), one token of 64 sequences: 36 (44). Two columns a thread over 16 lanes halve the reads and
-// lengthen the chain by two shuffles: 497 and 412 us.
+// cycles go to shared-memory reads. Of 16 heads of 128 x 128, one token of 64 sequences: 36 us with the kernel that
+// prepares them (44 with 16 threads a column, 8 rows each, and w summed token by token), 200 sequences of eight tokens 302. Prompts, before
+// they went in chunks: 2,048 tokens 466 (732), four sequences of 2,048 tokens in all 400 (668); two columns a thread over 16 lanes halve the
+// reads and lengthen the chain by two shuffles: 497 and 412.
 // What does not depend on the state is made for
 // all tokens at once by a kernel of its own (a warp a (token, head): normed q and k, the decays,
 // k . q and beta, one row [q | k | g | k.q, beta] of a scratch matrix), so that the walk itself is
@@ -343,7 +344,8 @@ delta_rule_kernel(const float* __restrict__ x, int C, int v_col, const float* __
 // instruction has to be put together. Zeros above the diagonal are not multiplied, so that what is not finite in a token
 // reaches no earlier one.
 // Sequences of fewer than DC_MIN tokens walk them one by one, with the sums of a decode step: a few chunks are no faster
-// (us, 16 heads of 128 x 128, chunks / tokens: 33 tokens 14.5 / 13.6, 64 sequences of 24 218 / 215, 200 tokens 36 / 50).
+// (us, 16 heads of 128 x 128, chunks / tokens: 33 tokens 14.5 / 13.6, 64 sequences of 24 218 / 215, 200 tokens 36 / 50). How a sequence
+// goes is its own number of tokens in the step alone.
 // Their rows lie where their tokens' shares of records would (a record a sequence of any length took 66 MB for 128 sequences of two
 // tokens of 16 heads; 11 so), and a step that is known to have no longer sequences goes to the kernels above (us, 128 sequences of two tokens
 // 136 here, 128 there; 200 of eight 317 / 302).

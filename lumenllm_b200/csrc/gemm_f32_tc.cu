@@ -562,7 +562,7 @@ static int gemm_f32_tc_rows(const float* A, const TW* W, float* C, unsigned char
 
 // 1 if weights [N, K] go through this kernel, whatever M: by N and K alone, so that a row's value is the same in any batch.
 // Smaller weights leave most SMs idle and are FFMA's: 300 rows x 512 x 512 17.7 us there, 21.7 here; 300 x 1,024 x 300 13 / 21;
-// 2,048 x 256 x 256 11 / 18.
+// 2,048 x 256 x 256 11 / 18. Weights that are long one way only (16,384 x 896) have not been measured and stay there too.
 LUMEN_API int lumen_gemm_f32_tc_takes(int N, int K) { return N >= FT_MIN_N && K >= FT_MIN_K ? 1 : 0; }
 
 // Bytes of scratch lumen_gemm_f32_tc needs.
