@@ -231,6 +231,18 @@ def test_the_shape_of_a_captured_step_depends_on_counts_alone():
         assert n_tok == sum(lens) + sum(pads) and n_seq == len(lens) + len(pads) and n_tok > n_seq
 
 
+def test_a_captured_prompt_step_knows_no_lengths():
+    """Its lists are those of the step it was captured with; a decode step's lengths, and an eager step's, are known."""
+    import torch
+    from lumenllm_b200.engine.context import StepLayout, context_on
+    for lens, captured, longest in (([5, 60], False, 60), ([1, 1, 1], False, 1), ([5, 60], True, None), ([1, 1, 1], True, 1), ([2], True, None)):
+        lay = StepLayout.of(len(lens), sum(lens), 0, 1, 0)
+        ctx = context_on(torch.zeros(lay.total, dtype=torch.int32), lay, lens, [0] * len(lens), list(range(len(lens))), len(lens), None, None)
+        if captured:
+            ctx.extras["captured"] = True
+        assert ctx.longest == longest
+
+
 def test_a_captured_prompt_step_is_never_taken_for_a_decode_step():
     """Captured steps are kept by their buckets; many prompts of a token or two fill as many tokens as sequences, and must
     not replay (or be replayed as) the decode step of that many sequences."""

@@ -783,6 +783,31 @@ def test_a_long_sequence_is_cut_as_it_is_alone(tmp_path):
     eng.check_kernels()
 
 
+def test_a_captured_prompt_step_serves_other_lengths(tmp_path):
+    """A captured step is replayed for any division of its tokens, also for sequences long enough to go in chunks where the one it was
+    captured with had none: the bits of the step launched kernel by kernel."""
+    from lumenllm_b200 import SamplingConfig
+    from lumenllm_b200.engine import Engine, StepEntry
+    cfg = config(50, 64, 1e-5, [layer(delta(2, 1, 128, 16, 3, 2, 2), dense(40)), layer(delta(2, 2, 100, 36, 2, 3, 5), None)])
+    eng = Engine.from_folder(write_model(cfg, tmp_path / "m", seed=84), dtype="float32", max_tokens=1024, max_slots=4)
+    shapes = set()
+    for k, lens in enumerate([(30, 31, 29), (60, 20, 10), (1, 2, 90), (47, 1, 48)]):
+        toks, out = tokens_of(cfg, lens, seed=85 + k), []
+        for captured in (True, False):
+            slots = [eng.alloc_slot() for _ in lens]
+            if captured:
+                eng.run_device(list(zip(slots, toks)), [SamplingConfig(temperature=0.0)] * 3, [0.0] * 3)
+                out.append(eng.graphs.last.logits[:3].clone())
+            else:
+                out.append(eng.step([StepEntry(s, t, [len(t) - 1]) for s, t in zip(slots, toks)]))
+            for s in slots:
+                eng.free_slot(s)
+        assert torch.equal(out[0], out[1])
+        shapes |= set(eng.graphs.captured)
+    assert len(shapes) == 1
+    eng.check_kernels()
+
+
 def test_a_long_prompt_whose_products_add_into_the_stream(tmp_path):
     """A prompt long and wide enough for the output products to add their result to the residual
     stream in their epilogue (no update is handed on then), with every kind of mixer."""
