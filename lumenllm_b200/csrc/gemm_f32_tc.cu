@@ -51,7 +51,7 @@
 #define FT_MAX_SHARES 4                  // 16 clusters of eight blocks that fill an SM each take two rounds, 32 of four one
 #define FT_MIN_N 1024                    // see lumen_gemm_f32_tc_takes
 #define FT_MIN_K 1024
-#define FT_IMAGE_MAX (128ll << 20)       // bytes of cut activations at a time: about what stays in L2, and hundreds of tiles
+#define FT_IMAGE_MAX (256ll << 20)       // bytes of cut activations at a time (or one tile): products of a millisecond and more
 
 __device__ __forceinline__ void ft_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -505,7 +505,22 @@ static int gemm_f32_tc_go(const float* A, const TW* W, float* C, unsigned char* 
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
     if (e != cudaSuccess) return (int)e;
     const int vec_a = (K & 3) == 0 && ((uintptr_t)A & 15) == 0, vec_w = (K & 3) == 0 && ((uintptr_t)W & (4 * sizeof(TW) - 1)) == 0;
-    const int lot = F::IMAGE ? gemm_f32_tc_lot(M, K, bn) * bn : M;
+    int lot = M;
+    if (F::IMAGE) {
+        // of the lots that fit, the one whose blocks take the fewest rounds on the SMs (ms, all at once / in lots: 8,192 x 2,048 x 25,600
+        // 5.33 / 5.46, 1.28 GB / 0.25; 6,000 x 3,000 x 16,384 4.38 / 4.44; 3,000 x 2,048 x 16,384 1.74 / 1.62)
+        const long long most = gemm_f32_tc_lot(M, K, bn), tiles = (M + bn - 1) / bn, tile_blocks = (long long)S * ((N + FT_ROWS - 1) / FT_ROWS);
+        const int at_once = S == 1 ? 148 : 144;
+        auto rounds = [&](long long t) { return (t * tile_blocks + at_once - 1) / at_once; };
+        long long fewest = 0;
+        for (long long t = most; most < tiles && t > most / 2; --t) {
+            const long long all = tiles / t * rounds(t) + rounds(tiles % t);
+            if (fewest == 0 || all < fewest) {
+                fewest = all;
+                lot = (int)t * bn;
+            }
+        }
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(32 * F::WARPS);
     cfg.dynamicSmemBytes = F::SMEM;

@@ -610,7 +610,7 @@ def test_gemm_f32_by_ffma_for_large_weights(wdtype, M, N, K_):
     assert not torch.equal(got, plain) and error[0] < error[1] < 1e-6
 
 
-@pytest.mark.parametrize("M,K_", [(1400, 16384), (5000, 4700)])
+@pytest.mark.parametrize("M,K_", [(2800, 16384), (10000, 4700)])
 def test_gemm_f32_whose_activations_are_cut_in_lots(M, K_):
     """More rows than are cut at a time: every row has the bits it has by itself, on both sides of where a lot ends."""
     from ctypes import c_int, c_longlong
@@ -623,8 +623,8 @@ def test_gemm_f32_whose_activations_are_cut_in_lots(M, K_):
     a, w = dev(torch.randn(M, K_, generator=g)), dev(torch.randn(1030, K_, generator=g))
     out = K.gemm_f32(a, w)
     K.check_error_flags()
-    for at in range(0, M, 100):
-        rows = slice(at, min(at + 100, M))
+    for at in range(0, M, 250):
+        rows = slice(at, min(at + 250, M))
         assert torch.equal(K.gemm_f32(a[rows].contiguous(), w), out[rows])
 
 
